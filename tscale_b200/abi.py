@@ -165,6 +165,24 @@ def lib():
     return _lib
 
 
+_binding = None
+
+
+def native():
+    """The compiled torch-tensor binding (_native.so), bound to the library that lib() loaded.  Raises if it has not been built."""
+    global _binding
+    if _binding is None:
+        import torch  # noqa: F401  (its libraries have to be in the process first)
+        try:
+            from . import _native
+        except ImportError as e:
+            raise ImportError("tscale_b200: _native.so cannot be loaded (%s); build it with `make -C tscale_b200/csrc` "
+                              "(or __graft_entry__.build())." % e) from e
+        _native.bind(lib()._handle)
+        _binding = _native
+    return _binding
+
+
 class TsaError(RuntimeError):
     def __init__(self, code, text):
         RuntimeError.__init__(self, "tsa status %d: %s" % (code, text))

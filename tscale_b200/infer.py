@@ -9,8 +9,8 @@ import torch
 
 from . import abi
 from .abi import check
-from .ops import _ptr, _stream
 
+_native = abi.native()
 _MATS = ("qk", "qv", "k", "v", "combiner", "expand", "contract")
 
 
@@ -89,8 +89,7 @@ class InferContext:
         assert labels.dtype == torch.int32 and labels.dim() == 2 and labels.shape[0] == self.n_seq and labels.is_contiguous()
         if want_prediction and prediction is None:
             prediction = torch.empty((self.n_seq, m.vocab), dtype=torch.float32, device=m.device)
-        check(abi.lib().tsa_infer_step(ctypes.byref(m.c), self.layer_seqs, _ptr(self.ctx_lens), self.capacity, _ptr(labels), labels.shape[1],
-                                       self.n_seq, self.max_ctx if max_ctx_bound is None else int(max_ctx_bound), _ptr(prediction), _ptr(logits), _ptr(self.workspace), self.workspace.numel(),
-                                       _ptr(self.status), _stream()))
+        check(_native.infer_step(m.c, self.layer_seqs, self.ctx_lens, self.capacity, labels, labels.shape[1], self.n_seq,
+                                 self.max_ctx if max_ctx_bound is None else int(max_ctx_bound), prediction, logits, self.workspace, self.status))
         self.max_ctx += 1
         return prediction

@@ -2,7 +2,8 @@
 
 Names follow the reference's attention operators (code/gpt/compute/gpt_cuda.cu:445-564, 618-894):
 qk = queries, qv = keys, v = values, per-head scale planes [H][len], grouped spans for the mask.
-Everything runs on the GPU through libtsa_b200.so; torch only owns the memory and the stream.
+Everything runs on the GPU through libtsa_b200.so; torch only owns the memory and the stream.  The calls a step runs through
+go by way of the compiled binding (_native.so, csrc/torch_binding.cpp); the rest uses ctypes.
 """
 import ctypes
 
@@ -11,6 +12,8 @@ import torch
 
 from . import abi
 from .abi import Ptr2D, check
+
+_native = abi.native()
 
 _DT = {"i8": abi.TSA_I8, "e4m3": abi.TSA_E4M3, torch.float16: abi.TSA_F16, torch.bfloat16: abi.TSA_BF16,
        torch.float32: abi.TSA_F32}
@@ -46,6 +49,7 @@ class Mask:
         self.groups, self.group_ptr = groups, group_ptr          # numpy int32 [n][130], [tiles+1]
         self.rev_groups, self.rev_group_ptr = rev_groups, rev_group_ptr
         self._dev = {}
+        self._last = (None, None)  # device of the last call and its arrays
 
     @staticmethod
     def _run_grouper(fn, cap):
@@ -154,34 +158,30 @@ class Mask:
         return m
 
     def dev(self, device):
+        last = self._last
+        if last[0] == device:
+            return last[1]
         key = str(device)
         if key not in self._dev:
             self._dev[key] = tuple(torch.from_numpy(np.ascontiguousarray(a)).to(device)
                                    for a in (self.groups, self.group_ptr, self.rev_groups, self.rev_group_ptr))
+        self._last = (device, self._dev[key])
         return self._dev[key]
 
 
 def quant_rows(src, kind, dst, tile, vec_scale=0.0, length=None):
     """Per-row, per-tile quantiser.  kind 'rms' | 'absmax'; dst 'i8' | 'e4m3'.
     Returns (bytes uint8 [rows][x], scale f32 [x/tile][rows])."""
-    rows, xs = src.shape
-    length = rows if length is None else length
-    out = torch.empty((rows, xs), dtype=torch.uint8, device=src.device)
-    scale = torch.empty((xs // tile, rows), dtype=torch.float32, device=src.device)
-    check(abi.lib().tsa_quant_rows(abi.TSA_QUANT_RMS if kind == "rms" else abi.TSA_QUANT_ABSMAX, _DT[src.dtype], _DT[dst],
-                                   vec_scale, p2d(src), p2d(out), p2d(scale), length, tile, _stream()))
+    rc, out, scale = _native.quant_rows(abi.TSA_QUANT_RMS if kind == "rms" else abi.TSA_QUANT_ABSMAX, src, _DT[dst], vec_scale,
+                                        src.shape[0] if length is None else length, tile)
+    check(rc)
     return out, scale
 
 
 def norm_rope_quant(src, rope, dst, heads, head_dim, vec_scale=1.0, direction=1.0, length=None):
     """Per-head RMS normalise, rope (None: no rotation), quantise.  Returns (bytes uint8 [rows][H*D], scale f32 [H][rows])."""
-    rows = src.shape[0]
-    length = rows if length is None else length
-    out = torch.empty((rows, heads * head_dim), dtype=torch.uint8, device=src.device)
-    scale = torch.empty((heads, rows), dtype=torch.float32, device=src.device)
-    check(abi.lib().tsa_norm_rope_quant(_DT[src.dtype], _DT[dst], vec_scale, p2d(src), p2d(rope),
-                                        _DT[rope.dtype] if rope is not None else abi.TSA_F32, direction, p2d(out), p2d(scale),
-                                        heads, head_dim, length, _stream()))
+    rc, out, scale = _native.norm_rope_quant(src, rope, _DT[dst], heads, head_dim, vec_scale, direction, src.shape[0] if length is None else length)
+    check(rc)
     return out, scale
 
 
@@ -189,41 +189,31 @@ def matmul_norm_rope_quant(x, w, rope, dst, heads, head_dim, vec_scale=1.0, src_
     """The projection x @ w^T fused with norm_rope_quant: x [rows][dim], w [H*D][dim] both int8 (exact int32 products) or both
     e4m3 bytes (src="e4m3", f32 accumulation), rope f32 [rows][D] or None; dst "i8" / "e4m3" (quantised bytes) or torch.float16 /
     torch.bfloat16 (the normalised, rotated values).  Returns (out [rows][H*D], scale f32 [H][rows])."""
-    rows = x.shape[0]
-    length = rows if length is None else length
-    out = torch.empty((rows, heads * head_dim), dtype=torch.uint8 if isinstance(dst, str) else dst, device=x.device)
-    scale = torch.empty((heads, rows), dtype=torch.float32, device=x.device)
-    check(abi.lib().tsa_matmul_norm_rope_quant(_DT[src], _DT[dst], vec_scale, src_scale, p2d(x), p2d(w), p2d(rope), direction, p2d(out), p2d(scale),
-                                               heads, head_dim, length, _ptr(status), _stream()))
+    rc, out, scale = _native.matmul_norm_rope_quant(_DT[src], x, w, rope, _DT[dst], heads, head_dim, vec_scale, src_scale, direction,
+                                                    x.shape[0] if length is None else length, status)
+    check(rc)
     return out, scale
 
 
 def rope_norm_bwd(src, grad, rope, heads, head_dim, direction=1.0):
     """Gradient with respect to the raw projections given the gradient with respect to the roped unit-RMS vectors."""
-    out = torch.empty_like(grad)
-    check(abi.lib().tsa_rope_norm_bwd(_DT[src.dtype], _DT[grad.dtype], p2d(src), p2d(grad), p2d(rope),
-                                      _DT[rope.dtype] if rope is not None else abi.TSA_F32, direction, p2d(out), heads, head_dim,
-                                      src.shape[0], _stream()))
+    rc, out = _native.rope_norm_bwd(src, grad, rope, heads, head_dim, direction)
+    check(rc)
     return out
 
 
 def kv_product(k, val, heads, head_dim, kv_mult=1.0, out_dtype=None, out=None):
     """Combiner input [rows][H*D*4] from k and the attention output."""
     out_dtype = (k.dtype if out is None else out.dtype) if out_dtype is None else out_dtype
-    if out is None:
-        out = torch.empty((k.shape[0], heads * head_dim * 4), dtype=out_dtype, device=k.device)
-    check(abi.lib().tsa_kv_product(_DT[k.dtype], _DT[out_dtype], p2d(k), p2d(val), kv_mult, p2d(out), heads, head_dim, k.shape[0], _stream()))
+    rc, out = _native.kv_product(k, val, heads, head_dim, kv_mult, _DT[out_dtype], out)
+    check(rc)
     return out
 
 
 def kv_product_bwd(k, val, dkv, heads, head_dim):
     """Returns (dK, dVal [rows][H*D] of dkv's dtype, dScale f32 [H][rows])."""
-    rows = k.shape[0]
-    dk = torch.empty((rows, heads * head_dim), dtype=dkv.dtype, device=k.device)
-    dv = torch.empty_like(dk)
-    ds = torch.empty((heads, rows), dtype=torch.float32, device=k.device)
-    check(abi.lib().tsa_kv_product_bwd(_DT[k.dtype], _DT[dkv.dtype], p2d(k), p2d(val), p2d(dkv), p2d(dk), p2d(dv), p2d(ds),
-                                       heads, head_dim, rows, _stream()))
+    rc, dk, dv, ds = _native.kv_product_bwd(k, val, dkv, heads, head_dim)
+    check(rc)
     return dk, dv, ds
 
 
@@ -239,6 +229,12 @@ def att_fwd(cfg, qk, qv, v, qv_scale, mask, slope, heads, qk_scale=None, v_scale
     either tensors or (data_ptr, stride_bytes) pairs for buffers of other GPUs mapped into this process (tsa_att_fwd_to).
     combiner_k (bf16 [len][H*D]): the kernel also forms the combiner input kv (bf16 [len][4*H*D], tsa_att_fwd_kv) and the
     call returns (out, sumWeightLog, kv)."""
+    groups, gptr, _, _ = mask.dev(qk.device)
+    if combiner_k is None and not out_copies:
+        rc, out, lse = _native.att_fwd(cfg, global_scale, qk, qv, v, qk_scale, qv_scale, v_scale, groups, gptr, slope, out, lse, heads,
+                                       mask.len_att_tiles, workspace, status)
+        check(rc)
+        return out, lse
     L = abi.lib()
     dev = qk.device
     rows = qk.shape[0]
@@ -249,7 +245,6 @@ def att_fwd(cfg, qk, qv, v, qv_scale, mask, slope, heads, qk_scale=None, v_scale
         lse = torch.empty((heads, rows), dtype=torch.float32, device=dev)
     if workspace is None:
         workspace = torch.empty(max(1, L.tsa_att_fwd_workspace_bytes(ctypes.byref(cfg), heads, rows)), dtype=torch.uint8, device=dev)
-    groups, gptr, _, _ = mask.dev(dev)
     if combiner_k is not None:
         if out_copies:
             raise ValueError("att_fwd: out_copies and combiner_k exclude each other")
@@ -260,18 +255,13 @@ def att_fwd(cfg, qk, qv, v, qv_scale, mask, slope, heads, qk_scale=None, v_scale
                                kv_mult, p2d(kv), heads, mask.len_att_tiles, _ptr(workspace), workspace.numel(), _ptr(status),
                                _stream()))
         return out, lse, kv
-    if out_copies:
-        outs = (Ptr2D * (1 + len(out_copies)))()
-        outs[0] = p2d(out)
-        for i, c in enumerate(out_copies):
-            outs[1 + i] = p2d(c) if isinstance(c, torch.Tensor) else Ptr2D(int(c[0]), int(c[1]), out.shape[1], out.shape[0])
-        check(L.tsa_att_fwd_to(ctypes.byref(cfg), _ptr(global_scale), p2d(qk), p2d(qv), p2d(qk_scale), p2d(qv_scale),
-                               p2d(v), p2d(v_scale), _ptr(groups), _ptr(gptr), slope, outs, len(outs), p2d(lse), heads,
-                               mask.len_att_tiles, _ptr(workspace), workspace.numel(), _ptr(status), _stream()))
-        return out, lse
-    check(L.tsa_att_fwd(ctypes.byref(cfg), _ptr(global_scale), p2d(qk), p2d(qv), p2d(qk_scale), p2d(qv_scale),
-                        p2d(v), p2d(v_scale), _ptr(groups), _ptr(gptr), slope, p2d(out), p2d(lse), heads,
-                        mask.len_att_tiles, _ptr(workspace), workspace.numel(), _ptr(status), _stream()))
+    outs = (Ptr2D * (1 + len(out_copies)))()
+    outs[0] = p2d(out)
+    for i, c in enumerate(out_copies):
+        outs[1 + i] = p2d(c) if isinstance(c, torch.Tensor) else Ptr2D(int(c[0]), int(c[1]), out.shape[1], out.shape[0])
+    check(L.tsa_att_fwd_to(ctypes.byref(cfg), _ptr(global_scale), p2d(qk), p2d(qv), p2d(qk_scale), p2d(qv_scale),
+                           p2d(v), p2d(v_scale), _ptr(groups), _ptr(gptr), slope, outs, len(outs), p2d(lse), heads,
+                           mask.len_att_tiles, _ptr(workspace), workspace.numel(), _ptr(status), _stream()))
     return out, lse
 
 
@@ -297,29 +287,16 @@ def att_fwd_host(cfg, qk, qv, v, qv_scale, mask, slope, heads, out, lse=None, qk
 def att_bwd(cfg, qk, qv, v, qv_scale, d_out, out, lse, mask, slope, heads, qk_scale=None, v_scale=None,
             global_scale=None, d_scale=None, grad_mult=1.0, workspace=None, status=None):
     """Backward.  Returns (dQK, dQV, dV) with respect to the true-scale vectors."""
-    L = abi.lib()
-    dev = qk.device
-    rows = qk.shape[0]
-    gt = {abi.TSA_F16: torch.float16, abi.TSA_BF16: torch.bfloat16, abi.TSA_F32: torch.float32}[cfg.grad_dtype]
-    dq = torch.empty((rows, heads * cfg.head_dim_qk), dtype=gt, device=dev)
-    dk = torch.empty((rows, heads * cfg.head_dim_qk), dtype=gt, device=dev)
-    dv = torch.empty((rows, heads * cfg.head_dim_v), dtype=gt, device=dev)
-    if workspace is None:
-        workspace = torch.empty(max(1, L.tsa_att_bwd_workspace_bytes(ctypes.byref(cfg), heads, rows)), dtype=torch.uint8, device=dev)
-    groups, gptr, rgroups, rgptr = mask.dev(dev)
-    check(L.tsa_att_bwd(ctypes.byref(cfg), _ptr(global_scale), p2d(qk), p2d(qv), p2d(qk_scale), p2d(qv_scale),
-                        p2d(v), p2d(v_scale), p2d(d_out), p2d(out), p2d(d_scale), p2d(lse),
-                        _ptr(groups), _ptr(gptr), _ptr(rgroups), _ptr(rgptr), slope, grad_mult,
-                        p2d(dq), p2d(dk), p2d(dv), heads, mask.len_att_tiles,
-                        _ptr(workspace), workspace.numel(), _ptr(status), _stream()))
+    groups, gptr, rgroups, rgptr = mask.dev(qk.device)
+    rc, dq, dk, dv = _native.att_bwd(cfg, global_scale, qk, qv, v, qk_scale, qv_scale, v_scale, d_out, out, d_scale, lse, groups, gptr,
+                                     rgroups, rgptr, slope, grad_mult, heads, mask.len_att_tiles, workspace, status)
+    check(rc)
     return dq, dk, dv
 
 
 def calc_dscale(out, d_out, heads, head_dim_v):
-    rows = out.shape[0]
-    res = torch.empty((heads, rows), dtype=torch.float32, device=out.device)
-    check(abi.lib().tsa_calc_dscale(_DT[out.dtype], _DT[d_out.dtype], p2d(out), p2d(d_out), p2d(res), heads, head_dim_v,
-                                    rows, _stream()))
+    rc, res = _native.calc_dscale(out, d_out, heads, head_dim_v)
+    check(rc)
     return res
 
 
@@ -354,28 +331,22 @@ class KVCache:
         self.max_ctx = 0
 
     def append(self, k_new, k_scale_new, v_new, v_scale_new, status=None):
-        check(abi.lib().tsa_kv_append(ctypes.byref(self.cfg), _ptr(self.seqs), _ptr(self.ctx_lens), self.n_seq, self.capacity,
-                                      p2d(k_new), p2d(k_scale_new), p2d(v_new), p2d(v_scale_new), self.heads,
-                                      _ptr(status), _stream()))
+        check(_native.kv_append(self.cfg, self.seqs, self.ctx_lens, self.n_seq, self.capacity, k_new, k_scale_new, v_new, v_scale_new,
+                                self.heads, status))
         self.max_ctx = min(self.capacity, self.max_ctx + 1)
 
     def decode(self, q, q_scale, window, slope, out=None, status=None):
-        L = abi.lib()
-        if out is None:
-            out = torch.empty((self.n_seq, self.heads * self.head_dim), dtype=self.out_dtype, device=q.device)
-        need = L.tsa_att_decode_workspace_bytes(ctypes.byref(self.cfg), self.n_seq, self.heads, self.capacity)
-        if self.workspace is None or self.workspace.numel() < need:
+        if self.workspace is None:
+            need = abi.lib().tsa_att_decode_workspace_bytes(ctypes.byref(self.cfg), self.n_seq, self.heads, self.capacity)
             self.workspace = torch.empty(max(1, need), dtype=torch.uint8, device=q.device)
-        check(L.tsa_att_decode(ctypes.byref(self.cfg), _ptr(self.seqs), _ptr(self.ctx_lens), self.n_seq, self.max_ctx,
-                               p2d(q), p2d(q_scale), window, slope, p2d(out), self.heads,
-                               _ptr(self.workspace), self.workspace.numel(), _ptr(status), _stream()))
+        rc, out = _native.att_decode(self.cfg, self.seqs, self.ctx_lens, self.n_seq, self.max_ctx, q, q_scale, window, slope, out, self.heads,
+                                     self.workspace, status)
+        check(rc)
         return out
 
     def decode_static(self, q, q_scale, window, slope, out=None, status=None):
         """The same step through tsa_att_decode_static: no workspace, the library's built-in scratch array."""
-        if out is None:
-            out = torch.empty((self.n_seq, self.heads * self.head_dim), dtype=self.out_dtype, device=q.device)
-        check(abi.lib().tsa_att_decode_static(ctypes.byref(self.cfg), _ptr(self.seqs), _ptr(self.ctx_lens), self.n_seq,
-                                              self.max_ctx, p2d(q), p2d(q_scale), window, slope, p2d(out), self.heads,
-                                              _ptr(status), _stream()))
+        rc, out = _native.att_decode(self.cfg, self.seqs, self.ctx_lens, self.n_seq, self.max_ctx, q, q_scale, window, slope, out, self.heads,
+                                     None, status)
+        check(rc)
         return out
