@@ -94,7 +94,7 @@ __device__ __forceinline__ void PlanSync()
 __device__ bool DecodePlan(const TDecodeParams &p, int slot, int *pSeq, int *pBeg, int *pEnd)
 {
     __shared__ int red[DEC_WARPS];
-    __shared__ int sliceBase[DEC_WARPS * 32 + 1];
+    __shared__ int scanRed[DEC_WARPS];
     __shared__ int found[3];
     const int tid = threadIdx.x, nThreads = DEC_WARPS * 32;
     // total number of keys
@@ -160,19 +160,27 @@ __device__ bool DecodePlan(const TDecodeParams &p, int slot, int *pSeq, int *pBe
     for (int s = s0; s < s1; ++s) {
         mine += (SeqKeys(p.CtxLens, p.CtxBias, s, p.Window) + chunk - 1) / chunk;
     }
-    sliceBase[tid + 1] = mine;
+    // exclusive scan over the threads' counts: shuffles inside a warp, the warps' sums through shared memory (one thread walking
+    // 128 sums in shared memory took 2 us of every call)
+    int base = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, base, o);
+        base += (tid & 31) >= o ? v : 0;
+    }
+    if ((tid & 31) == 31) {
+        scanRed[tid >> 5] = base;
+    }
     if (tid == 0) {
-        sliceBase[0] = 0;
         found[0] = -1;
     }
     PlanSync();
-    if (tid == 0) {
-        for (int i = 1; i <= nThreads; ++i) {
-            sliceBase[i] += sliceBase[i - 1];
-        }
+    base -= mine;
+    int slots = 0;
+    for (int w = 0; w < DEC_WARPS; ++w) {
+        base += w < (tid >> 5) ? scanRed[w] : 0;
+        slots += scanRed[w];
     }
-    PlanSync();
-    int base = sliceBase[tid];
     const bool writePlan = blockIdx.x == 0;
     if (writePlan && tid == 0) {
         p.Plan[0] = chunk;
@@ -194,7 +202,7 @@ __device__ bool DecodePlan(const TDecodeParams &p, int slot, int *pSeq, int *pBe
         base += n;
     }
     if (writePlan && tid == nThreads - 1) {
-        p.Plan[1 + p.NSeq] = sliceBase[nThreads];
+        p.Plan[1 + p.NSeq] = slots;
     }
     PlanSync();
     *pSeq = found[0];
@@ -247,6 +255,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 4) DecodePartialKernel(TDecode
     constexpr int HPW = 32 / LPH;     // heads per warp-wide load
     const int chunk = blockIdx.x;     // chunk slot (FINAL: the sequence)
     int seq, cBeg, cEnd;
+    PdlTrigger();
+    PdlWait();
     if (FINAL) {
         seq = blockIdx.x;
         const int len = CtxLenOf(p, seq);
@@ -445,28 +455,73 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 4) DecodePartialKernel(TDecode
     }
 }
 
-// merge chunk partials of one (sequence, head): block = D threads
+// Merge of the chunk partials of one (sequence, head) and the sink.  D / 4 lanes take a chunk's accumulator 16 bytes each and
+// the block's DEC_MERGE_THREADS / (D / 4) lane groups take every so-many-th chunk, all loads of a group independent of one
+// another; the groups' sums meet in shared memory.  A thread per column that walked the chunks one after another was bound by
+// the latency of that walk: 31 us for the 63 chunks of one 1000-token sequence (12 heads x 64), 11 us for the ten chunks per
+// sequence of a full batch.
+constexpr int DEC_MERGE_THREADS = 256;
 template <int D>
-__global__ void __launch_bounds__(D) DecodeCombineKernel(TDecodeParams p)
+__global__ void __launch_bounds__(DEC_MERGE_THREADS) DecodeCombineKernel(TDecodeParams p)
 {
-    int seq = blockIdx.y, head = blockIdx.x, x = threadIdx.x;
-    int ctxLen = CtxLenOf(p, seq);
-    float res = 0;
+    constexpr int LPC = D / 4, GROUPS = DEC_MERGE_THREADS / LPC;
+    __shared__ float redMax[DEC_MERGE_THREADS / 32];
+    __shared__ float sumL[GROUPS];
+    __shared__ float4 sumAcc[GROUPS][LPC];
+    const int seq = blockIdx.y, head = blockIdx.x, tid = threadIdx.x;
+    const int group = tid / LPC, sub = tid % LPC;
+    PdlTrigger();
+    PdlWait();
+    const int ctxLen = CtxLenOf(p, seq);
+    float m = 0; // the sink has logit 0 (softMax.Add(0), cpu_infer.cpp:444)
     if (ctxLen > 0) {
         const int first = p.Plan[1 + seq];
         const int chunks = p.Plan[2 + seq] - first;
         const float *base = p.Partial + ((size_t)first * p.HeadCount + head) * (D + 4);
-        size_t cstride = (size_t)p.HeadCount * (D + 4);
-        float m = 0; // the sink has logit 0 (softMax.Add(0), cpu_infer.cpp:444)
-        for (int c = 0; c < chunks; ++c) {
+        const size_t cstride = (size_t)p.HeadCount * (D + 4);
+        for (int c = tid; c < chunks; c += DEC_MERGE_THREADS) {
             m = fmaxf(m, base[c * cstride + D]);
         }
-        float l = exp2f(-m);
-        float acc = 0;
-        for (int c = 0; c < chunks; ++c) {
-            float f = exp2f(base[c * cstride + D] - m);
-            l += f * base[c * cstride + D + 1];
-            acc += f * base[c * cstride + x];
+        m = WarpMax(m);
+        if ((tid & 31) == 0) {
+            redMax[tid >> 5] = m;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < DEC_MERGE_THREADS / 32; ++w) {
+            m = fmaxf(m, redMax[w]);
+        }
+        float l = 0;
+        float4 acc = make_float4(0, 0, 0, 0);
+#pragma unroll 4
+        for (int c = group; c < chunks; c += GROUPS) {
+            const float *src = base + c * cstride;
+            const float2 ml = *reinterpret_cast<const float2 *>(src + D);
+            const float4 v = *reinterpret_cast<const float4 *>(src + 4 * sub);
+            const float f = exp2f(ml.x - m);
+            l = fmaf(f, ml.y, l);
+            acc.x = fmaf(f, v.x, acc.x);
+            acc.y = fmaf(f, v.y, acc.y);
+            acc.z = fmaf(f, v.z, acc.z);
+            acc.w = fmaf(f, v.w, acc.w);
+        }
+        sumAcc[group][sub] = acc;
+        if (sub == 0) {
+            sumL[group] = l;
+        }
+    }
+    __syncthreads();
+    const int x = tid;
+    if (x >= D) {
+        return;
+    }
+    float res = 0;
+    if (ctxLen > 0) {
+        float l = exp2f(-m), acc = 0;
+#pragma unroll
+        for (int gr = 0; gr < GROUPS; ++gr) {
+            l += sumL[gr];
+            acc += reinterpret_cast<const float *>(sumAcc[gr])[x];
         }
         res = acc / l;
     }
@@ -486,6 +541,8 @@ __global__ void __launch_bounds__(D) DecodeCombineKernel(TDecodeParams p)
 __global__ void KvAppendKernel(const tsa_kv_seq *seqs, int *ctxLens, int nSeq, int capacity, int rowBytes, int headCount, int scaleBytes,
     P2D<int8_t> kNew, P2D<char> kScaleNew, P2D<int8_t> vNew, P2D<char> vScaleNew, int *statusWord)
 {
+    PdlTrigger();
+    PdlWait();
     int seq = blockIdx.x;
     int pos = ctxLens[seq];
     if (pos >= capacity || pos < 0) {
@@ -575,16 +632,12 @@ int LaunchDecode(const tsa_decode_cfg *cfg, TDecodeParams p, int maxCtx, cudaStr
     dim3 grid(single ? (unsigned)p.NSeq : (unsigned)(slotBound < p.MaxSlots ? slotBound : p.MaxSlots));
     dim3 gridC(p.HeadCount, p.NSeq);
     void *args[] = {&p};
-    rc = CheckCuda(cudaLaunchKernel(kern, grid, dim3(DEC_WARPS * 32), args, 0, stream), "decode launch");
+    rc = CheckCuda(LaunchPdl(kern, grid, dim3(DEC_WARPS * 32), 0, stream, args), "decode launch");
     if (rc != TSA_OK || single) {
         return rc;
     }
-    if (cfg->head_dim == 128) {
-        DecodeCombineKernel<128><<<gridC, 128, 0, stream>>>(p);
-    } else {
-        DecodeCombineKernel<64><<<gridC, 64, 0, stream>>>(p);
-    }
-    return CheckCuda(cudaGetLastError(), "tsa_att_decode launch");
+    const void *merge = cfg->head_dim == 128 ? (const void *)DecodeCombineKernel<128> : (const void *)DecodeCombineKernel<64>;
+    return CheckCuda(LaunchPdl(merge, gridC, dim3(DEC_MERGE_THREADS), 0, stream, args), "tsa_att_decode launch");
 }
 
 } // namespace tsa
@@ -682,9 +735,11 @@ extern "C" __attribute__((visibility("default"))) int tsa_kv_append(const tsa_de
         "tsa_kv_append: kScaleNew/vScaleNew must be [nSeq][H]");
     TSA_REQUIRE((uintptr_t)kNew.data % 16 == 0 && kNew.stride_bytes % 16 == 0 && (uintptr_t)vNew.data % 16 == 0 && vNew.stride_bytes % 16 == 0,
         "tsa_kv_append: kNew/vNew must be 16-byte aligned");
-    KvAppendKernel<<<nSeq, 128, 0, (cudaStream_t)stream>>>(seqs, ctxLens, nSeq, capacity, rowBytes, headCount, DtypeSize(cfg->scale_dtype),
-        P2D<int8_t>(kNew), P2D<char>(kScaleNew), P2D<int8_t>(vNew), P2D<char>(vScaleNew), statusWord);
-    return CheckCuda(cudaGetLastError(), "tsa_kv_append launch");
+    int scaleBytes = DtypeSize(cfg->scale_dtype);
+    P2D<int8_t> k2(kNew), v2(vNew);
+    P2D<char> ks2(kScaleNew), vs2(vScaleNew);
+    void *args[] = {&seqs, &ctxLens, &nSeq, &capacity, &rowBytes, &headCount, &scaleBytes, &k2, &ks2, &v2, &vs2, &statusWord};
+    return CheckCuda(LaunchPdl((const void *)KvAppendKernel, dim3(nSeq), dim3(128), 0, (cudaStream_t)stream, args), "tsa_kv_append launch");
 }
 
 // ---- decode without any allocation -------------------------------------------------------------------

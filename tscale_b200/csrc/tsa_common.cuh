@@ -207,4 +207,32 @@ __device__ __forceinline__ float WarpSum(float x)
     return x;
 }
 
+// Programmatic dependent launch: a kernel launched with LaunchPdl may start while the kernel before it on the stream is still
+// running; it must call PdlWait() before its first access to memory that any earlier kernel writes or reads (the wait ends when
+// the kernel before it has finished and its stores are visible; that kernel has waited for the one before it in turn).
+// PdlTrigger() lets the next kernel start its own set-up early.  Both are no-ops in a kernel that was launched the usual way.
+__device__ __forceinline__ void PdlWait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void PdlTrigger()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+inline cudaError_t LaunchPdl(const void *kern, dim3 grid, dim3 block, size_t smemBytes, cudaStream_t stream, void **args)
+{
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid;
+    lc.blockDim = block;
+    lc.dynamicSmemBytes = smemBytes;
+    lc.stream = stream;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelExC(&lc, kern, args);
+}
+
 } // namespace tsa
