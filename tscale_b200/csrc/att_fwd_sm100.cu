@@ -147,44 +147,34 @@ struct TFwdSmem {
     static constexpr int TOTAL = MISC_OFF + (int)sizeof(TFwdMisc) + 1024; // + alignment slack
 };
 
-// tcgen05.wait::ld that names the registers an earlier tcgen05.ld fills, so that no use of them moves above the wait
-__device__ __forceinline__ void TmemWaitLdRegs(uint32_t *r)
+// 32 columns of this thread's lane, and the wait that names the registers the load fills so that no use of them moves above it.
+// Neither clobbers memory: the scale rows in shared memory that go with the scores may be read ahead of them (with the clobber
+// every group of 16 columns began with an exposed shared-memory read).
+__device__ __forceinline__ void TmemLoad32(uint32_t taddr, uint32_t *r)
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void TmemWait32(uint32_t *r)
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
                    "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
                    "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
-                   "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
-                 :
-                 : "memory");
+                   "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]));
 }
-
-__device__ __forceinline__ void TmemWaitLdRegs16(uint32_t *r)
+// eight columns of this thread's lane, without the memory clobber of TmemStN
+__device__ __forceinline__ void TmemStore8(uint32_t taddr, const uint32_t *r)
 {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-                 :
-                 : "memory");
-}
-
-// 2^x for a pair on the FMA / ALU pipes instead of the special-function unit: x = n + r with n = round(x),
-// |r| <= 0.5, 2^r by a cubic (relative error 7.5e-5, far below the e4m3 rounding of the weights), n added to the
-// exponent field.  x is clamped at -120 so the exponent cannot wrap; such weights are zero after the e4m3 pack.
-__device__ __forceinline__ float2 PolyExp2Pair(float2 x)
-{
-    const float kMagic = 12582912.0f; // 1.5 * 2^23: the sum's low mantissa bits hold round(x)
-    x.x = fmaxf(x.x, -120.0f);
-    x.y = fmaxf(x.y, -120.0f);
-    const float2 magic2 = make_float2(kMagic, kMagic);
-    float2 y = __fadd2_rn(x, magic2);
-    float2 r = __fadd2_rn(x, __fadd2_rn(make_float2(kMagic, kMagic), make_float2(-y.x, -y.y)));
-    float2 p = __ffma2_rn(r, make_float2(0.0551716685f, 0.0551716685f), make_float2(0.242611125f, 0.242611125f));
-    p = __ffma2_rn(p, r, make_float2(0.693260968f, 0.693260968f));
-    p = __ffma2_rn(p, r, make_float2(0.999928057f, 0.999928057f));
-    // the low 9 bits of the magic constant's pattern are zero, so (bits(y) << 23) is round(x) << 23
-    return make_float2(__uint_as_float(__float_as_uint(p.x) + (__float_as_uint(y.x) << 23)),
-        __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(y.y) << 23)));
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]));
 }
 
 // Slow path of the softmax: the row's reference moves up by d whole units, so what has been accumulated shrinks by
@@ -245,11 +235,6 @@ __device__ __forceinline__ int ValueScaleExponent(float x)
 #endif
 #ifndef TSA_FWD_SLEEP_SOFTMAX
 #define TSA_FWD_SLEEP_SOFTMAX 40
-#endif
-
-// number of register pairs out of every 8 whose exponentials go to the polynomial (0 = all on the SFU)
-#ifndef TSA_FWD_POLY_PAIRS
-#define TSA_FWD_POLY_PAIRS 0
 #endif
 
 // V_I8: the values are int8.  They reach the tensor cores exactly, as the sum of two e4m3 planes a pre-pass writes
@@ -928,7 +913,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                     for (int c0 = 0; c0 < TILE_N; c0 += 32) {
                         uint32_t s[32];
                         TmemLd32(tLane + c0, s);
-                        TmemWaitLdRegs(s);
+                        TmemWait32(s);
 #pragma unroll
                         for (int c = 0; c < 32; ++c) {
                             p.DumpScores[r * TILE_N + c0 + c] = (int32_t)s[c];
@@ -948,257 +933,152 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                 };
                 float eoff = rowOff - m + 7.0f;
 
-                // One key tile in chunks of W columns: logits in place of the scores and their maximum, a vote whether the
-                // row's reference has to move, then the weights.  The packed weights of the 32-key block b go to columns
-                // [32b, 32b + 8) and their residuals to [32b + 8, 32b + 16): inside the block's own score columns, which are
-                // in registers by then, so no store can hit scores that are still to be read.
-                // Unmasked tiles: W = 16, the next chunk's tcgen05.ld in flight while this one is worked on.
-                // Tiles the mask cuts through: W = 32, one buffer, residual term, chunks no row of the warp attends skipped.
-                auto processTile = [&](auto maskedTag) {
-                    constexpr bool MASKED = decltype(maskedTag)::value;
-                    constexpr int W = MASKED ? 32 : 16;
-                    int lsC = 0;
-                    unsigned spanW = TILE_N - 1;
-                    bool rowEmpty = false;
-                    unsigned act = 0xf; // 32-column chunks some row of the warp attends
-                    if (MASKED) {
-                        const int ls = spanS - j0, lf = spanF - j0; // span in tile-local columns
-                        lsC = max(ls, 0);
-                        const int lfC = min(lf, TILE_N - 1);
-                        rowEmpty = lsC > lfC;
-                        spanW = rowEmpty ? 0u : (unsigned)(lfC - lsC);
-                        act = 0;
+                // the reference moves up by d whole units: everything accumulated so far shrinks by 2^-d, and the W logits in s
+                // drop by d.  storedQuads: 16-key groups of this tile whose weights are in tensor memory.
+                auto raise = [&](float mxc, int storedQuads, uint32_t *s, auto widthTag, int withResidual) {
+                    constexpr int W = decltype(widthTag)::value;
+                    const float d = (mxc > headroom) ? floorf(mxc - 7.0f) : 0.0f;
+                    const float alpha = exp2f(-d);
+                    // the group voted on is the next one to be stored: it lies in half storedQuads / 4, whose earlier
+                    // quads are still this thread's; O holds something once a PV group of this item has been enabled,
+                    // and may be touched once the last enabled group has retired
+                    const int firstQuad = storedQuads & ~3;
+                    const bool oLive = hasO || firstQuad > 0;
+                    if (oLive && pvEnabled > 0) {
+                        // the last PV group enabled must have retired: the S = Q K^T group issued right behind it has
+                        // when its commit arrived (first half: the second half of this tile's S; second half: the
+                        // first half of the next tile's S)
+                        if (firstQuad == 0) {
+                            wait(&misc.BarS[1], sCount & 1, kDevTimeoutMma);
+                        } else {
+                            wait(&misc.BarS[0], (sCount + 1) & 1, kDevTimeoutMma);
+                        }
+                        TcFenceAfter();
+                    }
+                    ShrinkAccumulated<D>(tLane, alpha, oLive ? 1 : 0, firstQuad, storedQuads - firstQuad, withResidual);
+                    lacc2.x *= alpha;
+                    lacc2.y *= alpha;
+                    m += d;
+                    eoff -= d;
 #pragma unroll
-                        for (int ch = 0; ch < 4; ++ch) {
-                            if (__any_sync(0xffffffffu, !rowEmpty && lsC <= ch * 32 + 31 && lfC >= ch * 32)) {
-                                act |= 1u << ch;
-                            }
+                    for (int c = 0; c < W; ++c) {
+                        s[c] = __float_as_uint(__uint_as_float(s[c]) - d);
+                    }
+                };
+                // logits in place of the N scores s of the columns from cb on; returns their maximum
+                auto scaleGroup = [&](uint32_t *s, int cb, float mx, auto widthTag) {
+                    constexpr int W = decltype(widthTag)::value;
+                    const float2 eoff2 = make_float2(eoff, eoff);
+#pragma unroll
+                    for (int c = 0; c < W; c += 2) {
+                        const float2 tt = scalePair(s[c], s[c + 1], cb + c, eoff2);
+                        mx = Max3(mx, tt.x, tt.y);
+                        s[c] = __float_as_uint(tt.x);
+                        s[c + 1] = __float_as_uint(tt.y);
+                    }
+                    return mx;
+                };
+                // weights of four logits: added to the row sum, times the value scales of their columns
+                auto weighQuad = [&](const uint32_t *s, int col, float2 *e) {
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const float2 w = make_float2(FastExp2(__uint_as_float(s[2 * k])), FastExp2(__uint_as_float(s[2 * k + 1])));
+                        lacc2 = __fadd2_rn(lacc2, w);
+                        e[k] = HAS_VSCALE ? __fmul2_rn(w, *reinterpret_cast<const float2 *>(svBuf + col + 2 * k)) : w;
+                    }
+                };
+                using TW32 = std::integral_constant<int, 32>;
+                using TW64 = std::integral_constant<int, 64>;
+
+                // Tiles every row attends in full: a half (64 keys) at a time.  Its scores come in two tensor-memory loads (the
+                // second is in flight while the first is scaled), one vote says whether the row's reference has to move, then the
+                // weights.  One straight run of code per half keeps enough independent work in front of the scheduler; the other
+                // CTA's warp on the same scheduler fills what remains.
+                auto fullHalf = [&](int h) {
+                    uint32_t s[64], pk[16];
+                    const uint32_t cols = tLane + h * 64;
+                    TmemLoad32(cols, s);
+                    TmemWait32(s);
+                    TmemLoad32(cols + 32, s + 32);
+                    float mx = scaleGroup(s, h * 64, -INFINITY, TW32());
+                    TmemWait32(s + 32);
+                    mx = scaleGroup(s + 32, h * 64 + 32, mx, TW32());
+                    if (__any_sync(0xffffffffu, mx > headroom)) {
+                        raise(mx, h * 4, s, TW64(), 0);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 64; c += 4) {
+                        float2 e[2];
+                        weighQuad(s + c, h * 64 + c, e);
+                        pk[c >> 2] = PackE4M3x4(e[0].x, e[0].y, e[1].x, e[1].y);
+                        if (c == 28) {
+                            TmemStore8(cols, pk);
                         }
                     }
-                    // the reference moves up by d whole units: everything accumulated so far shrinks by 2^-d, and the
-                    // chunk's logits in s drop by d
-                    auto raise = [&](float mxc, int storedQuads, uint32_t *s) {
-                        const float d = (mxc > headroom) ? floorf(mxc - 7.0f) : 0.0f;
-                        const float alpha = exp2f(-d);
-                        // the chunk voted on is the next one to be stored: it lies in half storedQuads / 4, whose earlier
-                        // quads are still this thread's; O holds something once a PV group of this item has been enabled,
-                        // and may be touched once the last enabled group has retired
-                        const int firstQuad = storedQuads & ~3;
-                        const bool oLive = hasO || firstQuad > 0;
-                        if (oLive && pvEnabled > 0) {
-                            // the last PV group enabled must have retired: the S = Q K^T group issued right behind it has
-                            // when its commit arrived (first half: the second half of this tile's S; second half: the
-                            // first half of the next tile's S)
-                            if (firstQuad == 0) {
-                                wait(&misc.BarS[1], sCount & 1, kDevTimeoutMma);
-                            } else {
-                                wait(&misc.BarS[0], (sCount + 1) & 1, kDevTimeoutMma);
-                            }
-                            TcFenceAfter();
-                        }
-                        ShrinkAccumulated<D>(tLane, alpha, oLive ? 1 : 0, firstQuad, storedQuads - firstQuad, MASKED ? 1 : 0);
-                        lacc2.x *= alpha;
-                        lacc2.y *= alpha;
-                        m += d;
-                        eoff -= d;
-#pragma unroll
-                        for (int c = 0; c < W; ++c) {
-                            s[c] = __float_as_uint(__uint_as_float(s[c]) - d);
-                        }
-                    };
-                    // s: W scores of the columns from cb on; other: the buffer a tcgen05.ld may be filling meanwhile
-                    auto chunk = [&](uint32_t *s, uint32_t *other, int cb, uint32_t *pk, uint32_t *pl) {
-                        float mxc = -INFINITY;
-                        {
+                    TmemStore8(cols + 32, pk + 8);
+                };
+                // Tiles the mask cuts through (and every tile of the int8-value kernel): a block of 32 keys at a time, blocks
+                // no row of the warp attends skipped, weights as e4m3 plus an e4m3 residual.  A row's attended columns are a bit
+                // mask, so that masking a logit is one select on a predicate.
+                auto maskedTile = [&]() {
+                    const int ls = max(spanS - j0, 0), lf = min(spanF - j0, TILE_N - 1); // the row's span in tile columns
+#pragma unroll 1
+                    for (int blk = 0; blk < 4; ++blk) {
+                        const int lo = max(ls - blk * 32, 0), hi = min(lf - blk * 32, 31);
+                        const uint32_t bits = lo <= hi ? (0xffffffffu << lo) & (0xffffffffu >> (31 - hi)) : 0u;
+                        const uint32_t cols = tLane + blk * 32;
+                        uint32_t pk[8], pl[8];
+                        if (__any_sync(0xffffffffu, bits != 0)) {
+                            uint32_t s[32];
+                            TmemLoad32(cols, s);
+                            TmemWait32(s);
                             const float2 eoff2 = make_float2(eoff, eoff);
+                            float mx = -INFINITY;
 #pragma unroll
-                            for (int c = 0; c < W; c += 2) {
-                                float2 tt = scalePair(s[c], s[c + 1], cb + c, eoff2);
-                                if (MASKED) {
-                                    // unsigned compare folds both bounds: lsC <= col <= lfC
-                                    tt.x = ((unsigned)(cb + c - lsC) <= spanW) ? tt.x : -INFINITY;
-                                    tt.y = ((unsigned)(cb + c + 1 - lsC) <= spanW) ? tt.y : -INFINITY;
-                                }
-                                mxc = Max3(mxc, tt.x, tt.y);
+                            for (int c = 0; c < 32; c += 2) {
+                                float2 tt = scalePair(s[c], s[c + 1], blk * 32 + c, eoff2);
+                                tt.x = (bits & (1u << c)) ? tt.x : -INFINITY;
+                                tt.y = (bits & (2u << c)) ? tt.y : -INFINITY;
+                                mx = Max3(mx, tt.x, tt.y);
                                 s[c] = __float_as_uint(tt.x);
                                 s[c + 1] = __float_as_uint(tt.y);
                             }
-                        }
-                        if (MASKED && rowEmpty) {
-                            mxc = -INFINITY; // spanW = 0 would otherwise let column lsC through
-                        }
-                        if (__any_sync(0xffffffffu, mxc > headroom)) {
-                            if (!MASKED) {
-                                TmemWaitLdRegs16(other); // no load is in flight across the out-of-line call
+                            if (__any_sync(0xffffffffu, mx > headroom)) {
+                                raise(mx, blk * 2, s, TW32(), 1);
                             }
-                            raise(mxc, cb >> 4, s);
-                        }
-                        // an empty row gets -inf so that every weight is 0 whatever the compare let through
-                        const float kill = (MASKED && rowEmpty) ? -INFINITY : 0.0f;
 #pragma unroll
-                        for (int c = 0; c < W; c += 4) {
-                            float2 e[2];
-#pragma unroll
-                            for (int k = 0; k < 2; ++k) {
-                                const int cc = c + 2 * k;
-                                float2 tt = make_float2(__uint_as_float(s[cc]), __uint_as_float(s[cc + 1]));
-                                if (MASKED) {
-                                    tt.x += kill;
-                                    tt.y += kill;
-                                }
-                                float2 w;
-                                if (!MASKED && ((cc >> 1) & 7) < TSA_FWD_POLY_PAIRS) {
-                                    w = PolyExp2Pair(tt);
-                                } else {
-                                    w = make_float2(FastExp2(tt.x), FastExp2(tt.y));
-                                }
-                                lacc2 = __fadd2_rn(lacc2, w);
-                                if (HAS_VSCALE) {
-                                    e[k] = __fmul2_rn(w, *reinterpret_cast<const float2 *>(svBuf + cb + cc));
-                                } else {
-                                    e[k] = w;
-                                }
-                            }
-                            const uint32_t hi4 = PackE4M3x4(e[0].x, e[0].y, e[1].x, e[1].y);
-                            pk[c >> 2] = hi4;
-                            if (MASKED) {
+                            for (int c = 0; c < 32; c += 4) {
+                                float2 e[2];
+                                weighQuad(s + c, blk * 32 + c, e);
+                                const uint32_t hi4 = PackE4M3x4(e[0].x, e[0].y, e[1].x, e[1].y);
+                                pk[c >> 2] = hi4;
                                 pl[c >> 2] = ResidualE4M3x2(e[0].x, e[0].y, hi4 & 0xffff) | (ResidualE4M3x2(e[1].x, e[1].y, hi4 >> 16) << 16);
                             }
-                        }
-                    };
-                    if (MASKED) {
-#pragma unroll 1
-                        for (int ch = 0; ch < 4; ++ch) {
-                            uint32_t s[32], pk[8], pl[8];
-                            if (act & (1u << ch)) {
-                                TmemLd32(tLane + ch * 32, s);
-                                TmemWaitLdRegs(s);
-                                chunk(s, s, ch * 32, pk, pl);
-                            } else {
-#pragma unroll
-                                for (int k = 0; k < 8; ++k) {
-                                    pk[k] = 0;
-                                    pl[k] = 0;
-                                }
-                            }
-                            TmemStN<8>(tLane + ch * 32, pk);
-                            TmemStN<8>(tLane + ch * 32 + 8, pl);
-                            if (ch == 1) {
-                                handOver(0);
-                                waitSecondHalf();
-                            }
-                        }
-                    } else {
-                        // Software pipeline over the 8 chunks, interleaved at the source level: in step c the exponentials
-                        // of chunk c (special-function pipe) alternate with the scaling of chunk c + 1 (FMA pipe) inside one
-                        // loop body, while chunk c + 2 is on its way from tensor memory; the vote on chunk c + 1 closes
-                        // the step.  Raw scores of chunk k live in rawBuf[k & 1], logits in tBuf[k & 1].
-                        uint32_t tBuf[2][16], rawBuf[2][16], pk[4];
-                        float mxN = -INFINITY;
-                        // c: chunk that becomes weights (even: buffers 0, odd: buffers 1).  A loop over pairs of steps: fully
-                        // unrolled, the eight copies no longer fit the instruction cache and every head size got slower.
-                        // MODE 0: chunks c + 1 and c + 2 exist; 1: only c + 1; 2: neither (the last step); 3: decided at run
-                        // time, and the last step scales whatever the raw registers hold and ignores the result.  Head size
-                        // 128 runs the loop over steps 0-5 in mode 0 and steps 6, 7 in modes 1, 2 (four copies of the step),
-                        // head size 64 all eight steps in mode 3 (two copies): measured, each is the faster one for its size.
-                        auto step = [&](auto modeTag, auto oddTag, int c) {
-                            constexpr int MODE = decltype(modeTag)::value;
-                            constexpr int ODD = decltype(oddTag)::value;
-                            constexpr bool HAS_NEXT = MODE != 2;
-                            const bool LOAD = MODE == 0 || (MODE == 3 && c < 6);
-                            uint32_t *cur = tBuf[ODD], *nxt = tBuf[ODD ^ 1];
-                            uint32_t *rawCur = rawBuf[ODD ^ 1], *rawNxt = rawBuf[ODD];
-                            if (HAS_NEXT) {
-                                TmemWaitLdRegs16(rawCur);
-                            }
-                            if (LOAD) {
-                                if (c == 2) {
-                                    waitSecondHalf(); // chunk 4 is the first of the second half
-                                }
-                                TmemLd16(tLane + (c + 2) * 16, rawNxt);
-                            }
-                            const float2 eoff2 = make_float2(eoff, eoff);
-                            mxN = -INFINITY;
-#pragma unroll
-                            for (int k = 0; k < 16; k += 4) {
-                                float2 e[2];
-#pragma unroll
-                                for (int kk = 0; kk < 4; kk += 2) {
-                                    const int cc = k + kk;
-                                    if (HAS_NEXT) {
-                                        float2 tt = scalePair(rawCur[cc], rawCur[cc + 1], (c + 1) * 16 + cc, eoff2);
-                                        mxN = Max3(mxN, tt.x, tt.y);
-                                        nxt[cc] = __float_as_uint(tt.x);
-                                        nxt[cc + 1] = __float_as_uint(tt.y);
-                                    }
-                                    float2 x = make_float2(__uint_as_float(cur[cc]), __uint_as_float(cur[cc + 1]));
-                                    float2 w;
-                                    if (((cc >> 1) & 7) < TSA_FWD_POLY_PAIRS) {
-                                        w = PolyExp2Pair(x);
-                                    } else {
-                                        w = make_float2(FastExp2(x.x), FastExp2(x.y));
-                                    }
-                                    lacc2 = __fadd2_rn(lacc2, w);
-                                    if (HAS_VSCALE) {
-                                        e[kk >> 1] = __fmul2_rn(w, *reinterpret_cast<const float2 *>(svBuf + c * 16 + cc));
-                                    } else {
-                                        e[kk >> 1] = w;
-                                    }
-                                }
-                                pk[k >> 2] = PackE4M3x4(e[0].x, e[0].y, e[1].x, e[1].y);
-                            }
-                            TmemStN<4>(tLane + 32 * (c >> 1) + 4 * (c & 1), pk);
-                            if (c == 3) {
-                                handOver(0);
-                            }
-                            if (HAS_NEXT && __any_sync(0xffffffffu, (MODE != 3 || c < 7) && mxN > headroom)) {
-                                TmemWaitLdRegs16(rawNxt); // no load is in flight across the out-of-line call
-                                raise(mxN, c + 1, nxt);
-                            }
-                        };
-                        TmemLd16(tLane, rawBuf[0]);
-                        TmemWaitLdRegs16(rawBuf[0]);
-                        TmemLd16(tLane + 16, rawBuf[1]);
-                        {
-                            const float2 eoff2 = make_float2(eoff, eoff);
-#pragma unroll
-                            for (int cc = 0; cc < 16; cc += 2) {
-                                float2 tt = scalePair(rawBuf[0][cc], rawBuf[0][cc + 1], cc, eoff2);
-                                mxN = Max3(mxN, tt.x, tt.y);
-                                tBuf[0][cc] = __float_as_uint(tt.x);
-                                tBuf[0][cc + 1] = __float_as_uint(tt.y);
-                            }
-                        }
-                        if (__any_sync(0xffffffffu, mxN > headroom)) {
-                            TmemWaitLdRegs16(rawBuf[1]);
-                            raise(mxN, 0, tBuf[0]);
-                        }
-                        using TEven = std::integral_constant<int, 0>;
-                        using TOdd = std::integral_constant<int, 1>;
-                        if (D == 128) {
-#pragma unroll 1
-                            for (int c = 0; c < 6; c += 2) {
-                                step(std::integral_constant<int, 0>(), TEven(), c);
-                                step(std::integral_constant<int, 0>(), TOdd(), c + 1);
-                            }
-                            step(std::integral_constant<int, 1>(), TEven(), 6);
-                            step(std::integral_constant<int, 2>(), TOdd(), 7);
                         } else {
-#pragma unroll 1
-                            for (int c = 0; c < 8; c += 2) {
-                                step(std::integral_constant<int, 3>(), TEven(), c);
-                                step(std::integral_constant<int, 3>(), TOdd(), c + 1);
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                pk[k] = 0;
+                                pl[k] = 0;
                             }
+                        }
+                        TmemStore8(cols, pk);
+                        TmemStore8(cols + 8, pl);
+                        if (blk == 1) {
+                            handOver(0);
+                            waitSecondHalf();
                         }
                     }
                 };
-                if constexpr (V_I8) {
-                    processTile(std::true_type());
+                if (V_I8 || masked) {
+                    maskedTile();
                 } else {
-                    if (masked) {
-                        processTile(std::true_type());
-                    } else {
-                        processTile(std::false_type());
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+                        if (h == 1) {
+                            handOver(0);
+                            waitSecondHalf();
+                        }
+                        fullHalf(h);
                     }
                 }
                 handOver(1);
@@ -1273,7 +1153,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                     }
                     if (tilesInItem > 0) {
                         TmemLd32(tLane + TMEM_O_COL + c0, o);
-                        TmemWaitLdRegs(o);
+                        TmemWait32(o);
                     } else {
 #pragma unroll
                         for (int c = 0; c < 32; ++c) {
