@@ -12,7 +12,7 @@
 // reduced over the LPH lanes of a head with shuffles.  Each CTA keeps an online (max, sum, acc[D])
 // per head and writes it to the scratch buffer; a second kernel merges the chunks of a sequence and
 // adds the sink.  Algorithmic traffic per key: 2*D bytes + 2 scales per head.
-#include "tsa_common.cuh"
+#include "decode_device.cuh"
 #include <mutex>
 
 namespace tsa {
@@ -54,18 +54,6 @@ __device__ __forceinline__ int CtxLenOf(const TDecodeParams &p, int s)
 __device__ __forceinline__ float LoadScale(const void *base, size_t idx, int dt)
 {
     return dt == TSA_F16 ? __half2float(((const __half *)base)[idx]) : ((const float *)base)[idx];
-}
-
-__device__ __forceinline__ void KeyRange(int ctxLen, int window, int *j0, int *j1)
-{
-    int cur = ctxLen - 1;
-    if (window == 0) {
-        *j0 = cur;
-        *j1 = cur + 1;
-    } else {
-        *j0 = max(0, cur - window);
-        *j1 = cur;
-    }
 }
 
 constexpr int DEC_MIN_CHUNK = 16; // keys: short windows are spread over several CTAs of two batches rather than one CTA of eight
@@ -211,38 +199,6 @@ __device__ bool DecodePlan(const TDecodeParams &p, int slot, int *pSeq, int *pBe
     return found[0] >= 0;
 }
 
-template <bool F16>
-struct TScaleOf {
-    typedef __half T;
-};
-template <>
-struct TScaleOf<false> {
-    typedef float T;
-};
-__device__ __forceinline__ float LoadScaleT(const __half *p) { return __half2float(__ldg(p)); }
-__device__ __forceinline__ float LoadScaleT(const float *p) { return __ldg(p); }
-// sum of four (unsigned byte of a) x (signed byte of b) products, plus c
-__device__ __forceinline__ int Dp4aUS(uint32_t a, uint32_t b, int c)
-{
-    int d;
-    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-
-// two 16-bit x 8-bit products added to c: a = (w0 | w1 << 16) unsigned, b bytes signed; lo takes bytes 0 and 1 of b, hi bytes 2 and 3
-__device__ __forceinline__ int Dp2aLoUS(uint32_t a, uint32_t b, int c)
-{
-    int d;
-    asm("dp2a.lo.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-__device__ __forceinline__ int Dp2aHiUS(uint32_t a, uint32_t b, int c)
-{
-    int d;
-    asm("dp2a.hi.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-
 // One CTA = one chunk slot of the balanced plan, four warps, all heads.  Each lane keeps DEC_UNROLL tokens of K and
 // V (16 bytes each) in flight; four such CTAs are resident per SM.
 // FINAL: every sequence attends so few keys (a short window or short contexts, decided on the host from its bound) that
@@ -276,7 +232,6 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 4) DecodePartialKernel(TDecode
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane % LPH;             // 16-byte slice inside the head
     const int H = p.HeadCount;
-    const int rowInt4 = H * D / 16;          // int4 words per token row
     const tsa_kv_seq sq = p.Seqs[seq];
     typedef typename TScaleOf<SCALE_F16>::T TScale;
 
@@ -308,88 +263,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 4) DecodePartialKernel(TDecode
         for (int i = 0; i < 16; ++i) {
             acc[i] = 0;
         }
-        for (int tBase = tBeg; tBase < tEnd; tBase += DEC_UNROLL) {
-            int4 kv[DEC_UNROLL], vv[DEC_UNROLL];
-            float ks[DEC_UNROLL], vs[DEC_UNROLL];
-            const int cnt = tEnd - tBase; // tokens left, >= 1
-#pragma unroll
-            for (int u = 0; u < DEC_UNROLL; ++u) {
-                const int tt = u < cnt ? u : cnt - 1;
-                kv[u] = __ldg(kp + tt * rowInt4);
-                vv[u] = __ldg(vp + tt * rowInt4);
-                ks[u] = LoadScaleT(ksp + tt * H);
-                vs[u] = LoadScaleT(vsp + tt * H);
-            }
-            kp += DEC_UNROLL * rowInt4;
-            vp += DEC_UNROLL * rowInt4;
-            ksp += DEC_UNROLL * H;
-            vsp += DEC_UNROLL * H;
-            float z[DEC_UNROLL];
-            float cm = m;
-#pragma unroll
-            for (int u = 0; u < DEC_UNROLL; ++u) {
-                int dot = __dp4a(qv.x, kv[u].x, 0);
-                dot = __dp4a(qv.y, kv[u].y, dot);
-                dot = __dp4a(qv.z, kv[u].z, dot);
-                dot = __dp4a(qv.w, kv[u].w, dot);
-#pragma unroll
-                for (int o = LPH / 2; o > 0; o >>= 1) {
-                    dot += __shfl_xor_sync(0xffffffffu, dot, o);
-                }
-                // same association as the reference: ((dot * kScale) * attDotScale) * qScale - slope * dist
-                const float zz = (float)dot * ks[u] * logitMult - p.Slope * (float)(cur - (tBase + u));
-                z[u] = (u < cnt) ? zz : -1e30f;
-                cm = fmaxf(cm, z[u]);
-            }
-            if (cm != m) {
-                const float corr = exp2f(m - cm);
-                m = cm;
-                l *= corr;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    acc[i] *= corr;
-                }
-            }
-            // weights times value scales of the batch as 16-bit integers relative to the batch maximum (relative error of a
-            // weight at most 2^-17 of the largest one), so that the 8 x 16 byte products run as two-token integer dot
-            // products (dp2a) instead of a convert and a multiply-add per byte; one float update per batch
-            float wv[DEC_UNROLL];
-            float bmax = 0;
-#pragma unroll
-            for (int u = 0; u < DEC_UNROLL; ++u) {
-                const float w = exp2f(z[u] - m);
-                l += w;
-                wv[u] = w * vs[u];
-                bmax = fmaxf(bmax, wv[u]);
-            }
-            const float qScale = bmax > 0 ? 65535.0f / bmax : 0.0f;
-            int iacc[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                iacc[i] = 0;
-            }
-#pragma unroll
-            for (int u = 0; u < DEC_UNROLL; u += 2) {
-                const uint32_t wp = __float2uint_rn(wv[u] * qScale) | (__float2uint_rn(wv[u + 1] * qScale) << 16);
-                const uint32_t w0[4] = {(uint32_t)vv[u].x, (uint32_t)vv[u].y, (uint32_t)vv[u].z, (uint32_t)vv[u].w};
-                const uint32_t w1[4] = {(uint32_t)vv[u + 1].x, (uint32_t)vv[u + 1].y, (uint32_t)vv[u + 1].z, (uint32_t)vv[u + 1].w};
-#pragma unroll
-                for (int wi = 0; wi < 4; ++wi) {
-                    // bytes (t0 b0, t1 b0, t0 b1, t1 b1) and (t0 b2, t1 b2, t0 b3, t1 b3)
-                    const uint32_t lo = __byte_perm(w0[wi], w1[wi], 0x5140);
-                    const uint32_t hi = __byte_perm(w0[wi], w1[wi], 0x7362);
-                    iacc[wi * 4 + 0] = Dp2aLoUS(wp, lo, iacc[wi * 4 + 0]);
-                    iacc[wi * 4 + 1] = Dp2aHiUS(wp, lo, iacc[wi * 4 + 1]);
-                    iacc[wi * 4 + 2] = Dp2aLoUS(wp, hi, iacc[wi * 4 + 2]);
-                    iacc[wi * 4 + 3] = Dp2aHiUS(wp, hi, iacc[wi * 4 + 3]);
-                }
-            }
-            const float deq = bmax * (1.0f / 65535.0f);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                acc[i] = fmaf((float)iacc[i], deq, acc[i]);
-            }
-        }
+        AttendTokens<D, DEC_UNROLL, false>(qv, logitMult, p.Slope, cur, kp, vp, ksp, vsp, H, tBeg, tEnd, m, l, acc);
         if (split > 1) {
             float *mine = mergeBuf[warp][lane];
             mine[0] = m;

@@ -1,0 +1,54 @@
+// Shared by the files of the token step: constants and scalar helpers in the reference's rounding order.
+#pragma once
+#include "tsa_common.cuh"
+
+namespace tsa {
+
+constexpr float INF_VEC_SCALE = 1.0f / 24; // VEC_SCALE, cpu_infer.cpp:16
+constexpr int INF_NORM_TILE = 128;         // STATE_NORM_TILE, model_dim.h:23
+constexpr int INF_MAX_SEQ = 64;            // sequences per step
+
+// ConvertToInt8 (cpu_infer.cpp:88-92): round to nearest even, clamp to +-127
+__device__ __forceinline__ int ToInt8Clamp127(float x)
+{
+    return max(-127, min(127, __float2int_rn(x)));
+}
+
+// discrScale and 1 / discrScale of NormalizeState (cpu_infer.cpp:381-383); both 0 for an all-zero group
+__device__ __forceinline__ void NormScales(float sum2, int n, float *discr, float *mult)
+{
+    if (sum2 == 0) {
+        *discr = 0;
+        *mult = 0;
+    } else {
+        const float sko = __fsqrt_rn(__fdiv_rn(sum2, (float)n));
+        *discr = __fmul_rn(sko, INF_VEC_SCALE);
+        *mult = __fdiv_rn(1.0f, *discr);
+    }
+}
+
+// adds the squares of four consecutive elements in index order, one rounding per product and per sum
+__device__ __forceinline__ float AddSquares(float sum2, float4 v)
+{
+    sum2 = __fadd_rn(sum2, __fmul_rn(v.x, v.x));
+    sum2 = __fadd_rn(sum2, __fmul_rn(v.y, v.y));
+    sum2 = __fadd_rn(sum2, __fmul_rn(v.z, v.z));
+    return __fadd_rn(sum2, __fmul_rn(v.w, v.w));
+}
+
+struct TInferBuffers {
+    float *StateA, *StateB, *Logits, *SoftmaxPart, *Partial;
+    int *Sync;      // grid barrier and the attention chunks' counters, then the int32 sums: zeroed before every step
+    size_t SyncInts, ZeroBytes;
+    int *Proj, *Comb, *Expand, *Contract;
+    int8_t *NormState, *K8, *Kv8;
+    size_t Total;
+};
+
+TInferBuffers CarveInferBuffers(const tsa_infer_model *m, int nSeq, void *base);
+
+// all layers of the step: embedding to the normalised int8 state in b.NormState, caches appended and counted
+int InferLayersPersistent(const tsa_infer_model *model, const tsa_kv_seq *const *layerSeqs, int *ctxLens, int capacity, const int *labels, int labelsPerSeq,
+    int nSeq, int maxCtx, const TInferBuffers &b, int *statusWord, cudaStream_t stream);
+
+} // namespace tsa

@@ -1,0 +1,923 @@
+// The layers of a token step as ONE persistent kernel: a cooperative launch with one CTA per SM whose phases are separated by
+// grid-wide barriers.  What it computes is described in infer.cu; this file is about how.
+//
+// As separate launches the step was bound by launches and by latency, not by bytes: seven kernels per layer of 6 to 10 us each
+// for matrices of 1 to 2 MB (680 us per token for one sequence, twelve layers; the weights stream in 20 us).  Here a layer is five
+// phases
+//     P  proj      += W_qk|qv|k|v * norm(state)         int32 sums, exact
+//     A  attention     rope, per-head normalise, append to the caches, softmax(q K) V, times the combiner key -> int8
+//     C  comb      += W_combiner * A
+//     E  expand    += W_expand * norm(state + comb)
+//     T  contract  += W_contract * relu(norm(expand))
+// and a grid barrier (1.5 us) behind each.  A matrix product is cut into items of one 128-row tile and some 128-column chunks, as
+// many items as there are SMs, so that a 768 x 768 matrix uses the whole GPU; the items' int32 partial tiles are added in L2
+// (red.add: exact, the order does not matter).  The consumer of a product forms its own input from those sums: every item of
+// the next product normalises the 128-column chunk it multiplies with (a chunk is one STATE_NORM_TILE; the scalar loop's
+// order of operations, so the codes are bit-identical to the CPU's), which costs each of them a few hundred nanoseconds and
+// saves a phase and its barrier.  The weights do not depend on anything: every CTA keeps the tiles of its next items, across
+// phases and layers, in flight in a ring of shared memory (cp.async), so that their DRAM latency is never on the path.
+//
+// Measured on B200, twelve layers, dim 768, 12 heads x 64, one token: see InferLayersPersistent below.
+#include "att_sm100_common.cuh"
+#include "decode_device.cuh"
+#include "infer_internal.cuh"
+#include <stddef.h>
+
+namespace tsa {
+
+constexpr int PS_THREADS = 512, PS_GROUPS = 4; // attention works in groups of four warps
+constexpr int PS_RING = 8;                     // weight tiles in flight or in use per CTA
+constexpr int PS_TILE = 128 * 128;             // bytes of a weight tile: 128 rows x 128 columns
+constexpr int PS_B_BYTES = INF_MAX_SEQ * 128;  // the chunk's vectors, one row of 128 int8 per sequence
+constexpr int PS_F_PITCH = 132;                // floats per row of the fp32 chunk: 16-byte rows that fall into different banks
+constexpr int PS_MERGE_PITCH = 19;
+constexpr int PS_LAYERS = 32;                  // layers per launch
+constexpr int PS_MAX_SLOTS = 1024;             // attention chunks whose partials the workspace holds, at least
+constexpr int PS_MIN_CHUNK = 64;               // keys: two batches of eight for each of a group's four warps
+constexpr long long PS_WAIT_CYCLES = 1ll << 31;
+
+enum { PH_PROJ = 0, PH_COMB = 1, PH_EXPAND = 2, PH_CONTRACT = 3, PH_FINAL = 4 };
+enum { SRC_EMBED = 0, SRC_SUM = 1, SRC_STATE = 2 }; // where the first product of a launch gets the state from
+
+struct TStepLayer {
+    const int8_t *W[7]; // qk, qv, k, v, combiner, expand, contract
+    const tsa_kv_seq *Seqs;
+    int *CtxLens;
+    float QvMult, CombScale, ContractScale, Slope;
+    int Window;
+};
+
+struct TStepShape {
+    int Tiles, Chunks; // 128-row tiles, 128-column chunks of the phase's matrices
+    int Per, Splits;   // chunks per item, items per tile
+};
+
+struct TStepParams {
+    TStepLayer Layers[PS_LAYERS];
+    TStepShape Shape[4];
+    int LayerCount, FirstSource;
+    int NSeq, Dim, Heads, HeadSize, ReluDim, Capacity, MaxCtx, RopeLen;
+    const int *Labels;
+    int LabelsPerSeq, LabelCount;
+    const int8_t *Embed;
+    float EmbedScale;
+    const float *Rope;
+    float DotScale;
+    int *Barrier;                 // zero at launch
+    int *Arrived;                 // [nSeq][head groups] attention chunks done, zero between uses
+    int *Proj, *Comb, *Expand, *Contract; // int32 sums, zero at launch
+    float *StateA, *StateB;
+    int8_t *K8, *Kv8, *NormState;
+    float *Partial;
+    int *Status;
+};
+
+struct alignas(16) TAttGroupSmem {
+    float Rot[4][8 * 65];         // a head group's four projected vectors (8 x 64 or 4 x 128), rotated; pitch D + 1 per head
+    float Mult[4][8];
+    int8_t Q8[512], K8[512];
+    float Merge[4][32][PS_MERGE_PITCH];
+    int Last;
+};
+
+struct TStepSmem {
+    uint8_t Ring[PS_RING][PS_TILE];
+    uint8_t B[PS_B_BYTES];
+    union {
+        struct {
+            float F[INF_MAX_SEQ][PS_F_PITCH];
+            float Mult[INF_MAX_SEQ];
+        };
+        TAttGroupSmem Att[PS_GROUPS];
+    };
+    uint64_t MmaDone;
+    uint32_t TmemBase;
+    int Failed;
+};
+
+static_assert(sizeof(TAttGroupSmem) % 16 == 0 && offsetof(TAttGroupSmem, Q8) % 16 == 0 && offsetof(TStepSmem, F) % 16 == 0 && offsetof(TStepSmem, B) % 1024 == 0,
+    "16-byte accesses and swizzled operand tiles");
+
+__device__ __forceinline__ void CpAsync16(void *dst, const void *src, int bytes)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(SmemAddr(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void CpAsyncCommit()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void CpAsyncWait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void GroupSync(int group)
+{
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+}
+
+// Barrier of the whole grid.  Bounded: returns false in every thread of a CTA that has waited about a second.
+__device__ __forceinline__ bool GridSync(const TStepParams &p, TStepSmem &sm, int &passed)
+{
+    __syncthreads();
+    passed += gridDim.x;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p.Barrier) : "memory");
+        const long long t0 = clock64();
+        int seen;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(p.Barrier) : "memory");
+            if (seen >= passed) {
+                break;
+            }
+            if (clock64() - t0 > PS_WAIT_CYCLES) {
+                sm.Failed = 1;
+                if (p.Status) {
+                    atomicOr(p.Status, kDevTimeoutMma);
+                }
+                break;
+            }
+        }
+    }
+    __syncthreads();
+    return sm.Failed == 0;
+}
+
+// The CTA's weight tiles in the order it will use them: all items of all phases of all layers.
+struct TTileCursor {
+    int Layer, Phase, Item, Chunk;
+
+    __device__ __forceinline__ void Settle(const TStepParams &p)
+    {
+        while (Layer < p.LayerCount && Item >= p.Shape[Phase].Tiles * p.Shape[Phase].Splits) {
+            Item = blockIdx.x;
+            Chunk = 0;
+            if (++Phase == 4) {
+                Phase = 0;
+                ++Layer;
+            }
+        }
+    }
+    __device__ __forceinline__ void Next(const TStepParams &p)
+    {
+        if (Layer >= p.LayerCount) {
+            return;
+        }
+        const TStepShape &s = p.Shape[Phase];
+        const int first = (Item % s.Splits) * s.Per;
+        if (++Chunk >= min(s.Per, s.Chunks - first)) {
+            Chunk = 0;
+            Item += gridDim.x;
+            Settle(p);
+        }
+    }
+};
+
+// requests the cursor's tile (nothing past the last one) and closes the cp.async group; rows past the matrix read as zeros
+__device__ __forceinline__ void RequestTile(const TStepParams &p, const TTileCursor &c, uint8_t *dst)
+{
+    if (c.Layer < p.LayerCount) {
+        const TStepLayer &layer = p.Layers[c.Layer];
+        const TStepShape &s = p.Shape[c.Phase];
+        int tile = c.Item / s.Splits;
+        const int chunk = (c.Item - tile * s.Splits) * s.Per + c.Chunk;
+        int rows = c.Phase == PH_EXPAND ? p.ReluDim : p.Dim;
+        const int8_t *w = layer.W[c.Phase + 3];
+        if (c.Phase == PH_PROJ) {
+            const int perMatrix = s.Tiles / 4, m = tile / perMatrix;
+            tile -= m * perMatrix;
+            rows = p.Heads * p.HeadSize;
+            w = layer.W[m];
+        }
+        const int pitch = s.Chunks * 128;
+#pragma unroll
+        for (int k = 0; k < PS_TILE / 16 / PS_THREADS; ++k) {
+            const int idx = threadIdx.x + k * PS_THREADS, row = idx >> 3, c16 = idx & 7;
+            const bool ok = tile * 128 + row < rows;
+            CpAsync16(dst + row * 128 + ((c16 ^ (row & 7)) << 4), w + (ok ? (size_t)(tile * 128 + row) * pitch + chunk * 128 + c16 * 16 : 0), ok ? 16 : 0);
+        }
+    }
+    CpAsyncCommit();
+}
+
+// one 16-byte piece (columns c16 * 16 ..) of row s of the operand tile, 128-byte swizzle
+__device__ __forceinline__ void StoreCodes(uint8_t *tile, int s, int c16, int4 v)
+{
+    *reinterpret_cast<int4 *>(tile + s * 128 + ((c16 ^ (s & 7)) << 4)) = v;
+}
+
+// columns [128 chunk, +128) of the state after the last update, in sm.F: source 0 = embedding, 1 = state + sums * scale, 2 = state.
+// The writer also stores them to dst.  Ends with a barrier.
+__device__ void StageState(const TStepParams &p, TStepSmem &sm, int chunk, int source, const float *state, const int *sums, float scale, float *dst)
+{
+    for (int i = threadIdx.x; i < p.NSeq * 32; i += PS_THREADS) {
+        const int s = i >> 5, x = (i & 31) * 4, col = chunk * 128 + x;
+        float v[4];
+        if (source == SRC_EMBED) {
+            v[0] = v[1] = v[2] = v[3] = 0;
+            for (int k = 0; k < p.LabelsPerSeq; ++k) {
+                const int label = p.Labels[s * p.LabelsPerSeq + k];
+                if (label < 0 || label >= p.LabelCount) {
+                    if (col == 0 && dst && p.Status) {
+                        atomicOr(p.Status, kDevBadSpan);
+                    }
+                    continue;
+                }
+                const char4 e = *reinterpret_cast<const char4 *>(p.Embed + (size_t)label * p.Dim + col);
+                v[0] = __fadd_rn(v[0], __fmul_rn((float)e.x, p.EmbedScale));
+                v[1] = __fadd_rn(v[1], __fmul_rn((float)e.y, p.EmbedScale));
+                v[2] = __fadd_rn(v[2], __fmul_rn((float)e.z, p.EmbedScale));
+                v[3] = __fadd_rn(v[3], __fmul_rn((float)e.w, p.EmbedScale));
+            }
+        } else {
+            const float4 old = __ldcg(reinterpret_cast<const float4 *>(state + (size_t)s * p.Dim + col));
+            v[0] = old.x, v[1] = old.y, v[2] = old.z, v[3] = old.w;
+            if (source == SRC_SUM) {
+                const int4 a = __ldcg(reinterpret_cast<const int4 *>(sums + (size_t)s * p.Dim + col));
+                v[0] = __fadd_rn(v[0], __fmul_rn((float)a.x, scale)); // AddScaled, cpu_infer.cpp:296-303
+                v[1] = __fadd_rn(v[1], __fmul_rn((float)a.y, scale));
+                v[2] = __fadd_rn(v[2], __fmul_rn((float)a.z, scale));
+                v[3] = __fadd_rn(v[3], __fmul_rn((float)a.w, scale));
+            }
+        }
+        const float4 out = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4 *>(&sm.F[s][x]) = out;
+        if (dst) {
+            *reinterpret_cast<float4 *>(dst + (size_t)s * p.Dim + col) = out;
+        }
+    }
+    __syncthreads();
+}
+
+// int8 codes of the staged columns [x0, x0 + 16 pieces * 16) under sm.Mult, into the operand tile
+__device__ __forceinline__ void QuantiseStaged(const TStepParams &p, TStepSmem &sm, int piece0, int pieces, bool relu)
+{
+    for (int i = threadIdx.x; i < p.NSeq * pieces; i += PS_THREADS) {
+        const int s = i / pieces, c16 = piece0 + i - s * pieces;
+        const float mult = sm.Mult[s];
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float4 v = *reinterpret_cast<const float4 *>(&sm.F[s][c16 * 16 + k * 4]);
+            int q[4] = {ToInt8Clamp127(__fmul_rn(v.x, mult)), ToInt8Clamp127(__fmul_rn(v.y, mult)), ToInt8Clamp127(__fmul_rn(v.z, mult)),
+                ToInt8Clamp127(__fmul_rn(v.w, mult))};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                q[j] = relu ? max(q[j], 0) : q[j];
+            }
+            w[k] = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
+        }
+        StoreCodes(sm.B, s, c16, make_int4((int)w[0], (int)w[1], (int)w[2], (int)w[3]));
+    }
+}
+
+// NormalizeState of the staged chunk (one STATE_NORM_TILE): one thread per sequence adds the squares in index order
+__device__ void NormaliseStaged(const TStepParams &p, TStepSmem &sm)
+{
+    const int s = threadIdx.x;
+    if (s < p.NSeq) {
+        float sum2 = 0;
+#pragma unroll 8
+        for (int x = 0; x < 128; x += 4) {
+            sum2 = AddSquares(sum2, *reinterpret_cast<const float4 *>(&sm.F[s][x]));
+        }
+        float discr, mult;
+        NormScales(sum2, 128, &discr, &mult);
+        sm.Mult[s] = mult;
+    }
+    __syncthreads();
+    QuantiseStaged(p, sm, 0, 8, false);
+}
+
+// The contract product's input: relu of the expand sums normalised per head (groups of ReluDim / Heads columns).  A group that lies
+// inside the chunk is summed from shared memory, one that reaches beyond it from L2.
+__device__ void NormaliseRelu(const TStepParams &p, TStepSmem &sm, int chunk)
+{
+    for (int i = threadIdx.x; i < p.NSeq * 32; i += PS_THREADS) {
+        const int s = i >> 5, x = (i & 31) * 4;
+        const int4 a = __ldcg(reinterpret_cast<const int4 *>(p.Expand + (size_t)s * p.ReluDim + chunk * 128 + x));
+        *reinterpret_cast<float4 *>(&sm.F[s][x]) = make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w);
+    }
+    __syncthreads();
+    const int group = p.ReluDim / p.Heads, c0 = chunk * 128;
+    if (group % 16 != 0) {
+        // head sizes no model of the family has: a thread per 16 columns adds up the groups they belong to by itself
+        for (int i = threadIdx.x; i < p.NSeq * 8; i += PS_THREADS) {
+            const int s = i >> 3, c16 = i & 7;
+            const int *src = p.Expand + (size_t)s * p.ReluDim;
+            uint32_t w[4] = {0, 0, 0, 0};
+            int cur = -1;
+            float mult = 0;
+            for (int k = 0; k < 16; ++k) {
+                const int col = c0 + c16 * 16 + k;
+                if (col / group != cur) {
+                    cur = col / group;
+                    float sum2 = 0, discr;
+                    for (int x = cur * group; x < (cur + 1) * group; ++x) {
+                        const float a = (float)__ldcg(src + x);
+                        sum2 = __fadd_rn(sum2, __fmul_rn(a, a));
+                    }
+                    NormScales(sum2, group, &discr, &mult);
+                }
+                w[k >> 2] |= (uint32_t)(max(ToInt8Clamp127(__fmul_rn(sm.F[s][c16 * 16 + k], mult)), 0) & 0xff) << (8 * (k & 3));
+            }
+            StoreCodes(sm.B, s, c16, make_int4((int)w[0], (int)w[1], (int)w[2], (int)w[3]));
+        }
+        return;
+    }
+    for (int g = c0 / group; g * group < c0 + 128; ++g) {
+        const int g0 = g * group, g1 = g0 + group;
+        const int s = threadIdx.x;
+        if (s < p.NSeq) {
+            float sum2 = 0;
+            if (g0 >= c0 && g1 <= c0 + 128) {
+#pragma unroll 8
+                for (int x = g0 - c0; x < g1 - c0; x += 4) {
+                    sum2 = AddSquares(sum2, *reinterpret_cast<const float4 *>(&sm.F[s][x]));
+                }
+            } else {
+                const int4 *src = reinterpret_cast<const int4 *>(p.Expand + (size_t)s * p.ReluDim + g0);
+#pragma unroll 8
+                for (int x = 0; x < group / 4; ++x) {
+                    const int4 a = __ldcg(src + x);
+                    sum2 = AddSquares(sum2, make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w));
+                }
+            }
+            float discr, mult;
+            NormScales(sum2, group, &discr, &mult);
+            sm.Mult[s] = mult;
+        }
+        __syncthreads();
+        const int lo = max(g0, c0) - c0, hi = min(g1, c0 + 128) - c0;
+        QuantiseStaged(p, sm, lo / 16, (hi - lo) / 16, true);
+        __syncthreads(); // the next group overwrites sm.Mult
+    }
+}
+
+// All of this CTA's items of one matrix product.  Returns false when a bounded wait ran out.
+__device__ bool ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int phase, TTileCursor &cursor, int &tileCount, int &mmaCount)
+{
+    const TStepShape &s = p.Shape[phase];
+    const TStepLayer &layer = p.Layers[l];
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int hs = p.Heads * p.HeadSize;
+    const int nCols = (p.NSeq + 15) & ~15; // accumulator columns
+    const uint32_t idesc = MakeInstrDesc(2, 1, 1, 0, 0, 128, nCols);
+    for (int item = blockIdx.x; item < s.Tiles * s.Splits; item += gridDim.x) {
+        int tile = item / s.Splits;
+        const int first = (item - tile * s.Splits) * s.Per, chunks = min(s.Per, s.Chunks - first);
+        for (int c = 0; c < chunks; ++c) {
+            const int chunk = first + c;
+            if (phase == PH_PROJ) {
+                const int source = l > 0 ? SRC_SUM : p.FirstSource;
+                StageState(p, sm, chunk, source, source == SRC_STATE ? p.StateA : p.StateB, p.Contract, l > 0 ? p.Layers[l - 1].ContractScale : 0.0f,
+                    tile == 0 && source != SRC_STATE ? p.StateA : nullptr);
+                NormaliseStaged(p, sm);
+            } else if (phase == PH_COMB) {
+                for (int i = tid; i < p.NSeq * 8; i += PS_THREADS) {
+                    StoreCodes(sm.B, i >> 3, i & 7, __ldcg(reinterpret_cast<const int4 *>(p.Kv8 + (size_t)(i >> 3) * 4 * hs + chunk * 128 + (i & 7) * 16)));
+                }
+            } else if (phase == PH_EXPAND) {
+                StageState(p, sm, chunk, SRC_SUM, p.StateA, p.Comb, layer.CombScale, tile == 0 ? p.StateB : nullptr);
+                NormaliseStaged(p, sm);
+            } else {
+                NormaliseRelu(p, sm, chunk);
+            }
+            CpAsyncWait<PS_RING - 2>(); // this thread's part of the tile has landed (one group per tile, PS_RING - 1 requested ahead)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            TcFenceBefore();
+            __syncthreads();
+            TcFenceAfter();
+            if (warp == 0 && ElectOne()) {
+                const uint32_t sA = SmemAddr(sm.Ring[tileCount % PS_RING]), sB = SmemAddr(sm.B);
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) {
+                    MmaI8SS(sm.TmemBase, MakeSmemDesc(sA + ks * 32, 16, 1024, 128), MakeSmemDesc(sB + ks * 32, 16, 1024, 128), idesc,
+                        (c > 0 || ks > 0) ? 1u : 0u);
+                }
+                MmaCommit(&sm.MmaDone);
+            }
+            // the next tile goes into the slot of the tile before this one, whose products were waited for below
+            RequestTile(p, cursor, sm.Ring[(tileCount + PS_RING - 1) % PS_RING]);
+            cursor.Next(p);
+            if (!WaitBar(&sm.MmaDone, mmaCount & 1)) {
+                sm.Failed = 1;
+                if (p.Status) {
+                    atomicOr(p.Status, kDevTimeoutMma);
+                }
+            }
+            ++tileCount;
+            ++mmaCount;
+        }
+        TcFenceAfter();
+        // 128 rows x 16 sequences per warp: the item's sums join the others' in L2
+        int *out;
+        int rows, pitch;
+        if (phase == PH_PROJ) {
+            const int perMatrix = s.Tiles / 4, m = tile / perMatrix;
+            tile -= m * perMatrix;
+            out = p.Proj + m * hs;
+            rows = hs;
+            pitch = 4 * hs;
+        } else {
+            out = phase == PH_COMB ? p.Comb : phase == PH_EXPAND ? p.Expand : p.Contract;
+            rows = pitch = phase == PH_EXPAND ? p.ReluDim : p.Dim;
+        }
+        const int quad = warp & 3, s0 = (warp >> 2) * 16, row = tile * 128 + quad * 32 + (tid & 31);
+        if (s0 < nCols) {
+            uint32_t acc[16];
+            TmemLd16(sm.TmemBase + ((uint32_t)(quad * 32) << 16) + s0, acc);
+            TmemWaitLd();
+            if (row < rows) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (s0 + j < p.NSeq) {
+                        atomicAdd(out + (size_t)(s0 + j) * pitch + row, (int)acc[j]);
+                    }
+                }
+            }
+        }
+        TcFenceBefore();
+        __syncthreads();
+        if (sm.Failed) {
+            return false;
+        }
+    }
+    return true;
+}
+
+// ---- attention -----------------------------------------------------------------------------------------------------
+// A unit = one sequence x one head group (the heads a warp-wide 16-byte load covers: 8 of 64 or 4 of 128) x one chunk of keys,
+// taken by a group of four warps that split the chunk's keys.  All chunks have the same size, the smallest multiple of 32 (at least
+// PS_MIN_CHUNK) whose units all fit the resident groups of the grid in one wave; the plan is a bisection every warp does for itself.
+struct TAttPlan {
+    int Chunk;        // keys per unit
+    int Units;        // of all sequences
+    int Base0, Base1; // first unit of sequences lane and lane + 32
+    int Keys0, Keys1; // their keys
+};
+
+__device__ __forceinline__ int StepKeys(const TStepParams &p, const TStepLayer &layer, int s)
+{
+    if (s >= p.NSeq) {
+        return 0;
+    }
+    const int pos = layer.CtxLens[s];
+    if (pos < 0 || pos >= p.RopeLen || pos >= p.Capacity) {
+        return 0; // reported by the unit that would append
+    }
+    int j0, j1;
+    KeyRange(pos + 1, layer.Window, &j0, &j1);
+    return j1 - j0;
+}
+
+__device__ TAttPlan MakeAttPlan(const TStepParams &p, const TStepLayer &layer, int headGroups)
+{
+    const int lane = threadIdx.x & 31;
+    const int slots = max((int)gridDim.x * PS_GROUPS, p.NSeq * headGroups);
+    TAttPlan pl;
+    pl.Keys0 = StepKeys(p, layer, lane);
+    pl.Keys1 = StepKeys(p, layer, lane + 32);
+    const bool on0 = lane < p.NSeq, on1 = lane + 32 < p.NSeq;
+    // every sequence has at least one unit per head group: it appends the new token
+    auto units = [&](int keys, bool on, int chunk) { return on ? headGroups * max(1, (keys + chunk - 1) / chunk) : 0; };
+    const int total = __reduce_add_sync(0xffffffffu, pl.Keys0 + pl.Keys1), most = __reduce_max_sync(0xffffffffu, max(pl.Keys0, pl.Keys1));
+    int lo = max(PS_MIN_CHUNK / 32, (int)(((long long)total * headGroups / slots) / 32)), hi = max((most + 31) / 32, lo);
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        const int n = __reduce_add_sync(0xffffffffu, units(pl.Keys0, on0, mid * 32) + units(pl.Keys1, on1, mid * 32));
+        if (n <= slots) {
+            hi = mid;
+        } else {
+            lo = mid + 1;
+        }
+    }
+    pl.Chunk = lo * 32;
+    const int u0 = units(pl.Keys0, on0, pl.Chunk), u1 = units(pl.Keys1, on1, pl.Chunk);
+    int i0 = u0, i1 = u1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, i0, o), b = __shfl_up_sync(0xffffffffu, i1, o);
+        i0 += lane >= o ? a : 0;
+        i1 += lane >= o ? b : 0;
+    }
+    const int sum0 = __shfl_sync(0xffffffffu, i0, 31);
+    pl.Base0 = i0 - u0;
+    pl.Base1 = sum0 + i1 - u1;
+    pl.Units = sum0 + __shfl_sync(0xffffffffu, i1, 31);
+    return pl;
+}
+
+// The combiner input of four consecutive columns z .. z + 3 of a head: kv[blk][z] = int8(key[z ^ blk] * val[z]) (KVProduct,
+// cpu_infer.cpp:318-337); z ^ blk stays among the four.
+__device__ __forceinline__ void StoreKvProduct(int8_t *kv, int headSize, int z, char4 key, const float *val)
+{
+    const int k[4] = {key.x, key.y, key.z, key.w};
+#pragma unroll
+    for (int blk = 0; blk < 4; ++blk) {
+        uint32_t w = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            w |= (uint32_t)(ToInt8Clamp127(__fmul_rn((float)k[i ^ blk], val[i])) & 0xff) << (8 * i);
+        }
+        *reinterpret_cast<uint32_t *>(kv + blk * headSize + z) = w;
+    }
+}
+
+// One matrix (m: qk, qv, k, v) of a head group of one sequence, by one warp: rope on qk and qv (ReferenceApplyRope,
+// code/gpt/att/rope.cpp:28-46), NormalizeState per head, codes into shared memory (qk, k) or the sequence's cache (qv, v).
+template <int D>
+__device__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAttGroupSmem &g, int m, int seq, int head0, int heads, int pos)
+{
+    const int lane = threadIdx.x & 31, hs = p.Heads * D;
+    const int *src = p.Proj + (size_t)seq * 4 * hs + m * hs + head0 * D;
+    float *rot = g.Rot[m];
+#pragma unroll 4
+    for (int b = 0; b < heads * D / 64; ++b) {
+        const float v0 = (float)__ldcg(src + b * 64 + lane), v1 = (float)__ldcg(src + b * 64 + lane + 32);
+        float r0 = v0, r1 = v1;
+        const int in = (b * 64) & (D - 1);
+        if (m < 2) {
+            const float *rp = p.Rope + (size_t)pos * D + in;
+            const float c = __ldg(rp + lane), sn = __ldg(rp + lane + 32);
+            r0 = __fsub_rn(__fmul_rn(v0, c), __fmul_rn(v1, sn));
+            r1 = __fadd_rn(__fmul_rn(v0, sn), __fmul_rn(v1, c));
+        }
+        float *w = rot + (b * 64 / D) * (D + 1) + in;
+        w[lane] = r0;
+        w[lane + 32] = r1;
+    }
+    __syncwarp();
+    const tsa_kv_seq sq = layer.Seqs[seq];
+    if (lane < heads) {
+        const float *w = rot + lane * (D + 1);
+        float sum2 = 0;
+#pragma unroll 16
+        for (int x = 0; x < D; ++x) {
+            sum2 = __fadd_rn(sum2, __fmul_rn(w[x], w[x]));
+        }
+        float discr, mult;
+        NormScales(sum2, D, &discr, &mult);
+        g.Mult[m][lane] = mult;
+        if (m == 1) {
+            ((float *)sq.kScale)[(size_t)pos * p.Heads + head0 + lane] = __fmul_rn(discr, layer.QvMult);
+        } else if (m == 3) {
+            ((float *)sq.vScale)[(size_t)pos * p.Heads + head0 + lane] = INF_VEC_SCALE;
+        }
+    }
+    __syncwarp();
+    // four columns per lane and step
+    for (int i = lane * 4; i < heads * D; i += 128) {
+        const int h = i / D;
+        const float *w = rot + h * (D + 1) + (i & (D - 1));
+        const float mult = g.Mult[m][h];
+        char4 q;
+        q.x = (char)ToInt8Clamp127(__fmul_rn(w[0], mult));
+        q.y = (char)ToInt8Clamp127(__fmul_rn(w[1], mult));
+        q.z = (char)ToInt8Clamp127(__fmul_rn(w[2], mult));
+        q.w = (char)ToInt8Clamp127(__fmul_rn(w[3], mult));
+        if (m == 0) {
+            *reinterpret_cast<char4 *>(g.Q8 + i) = q;
+        } else if (m == 2) {
+            *reinterpret_cast<char4 *>(p.K8 + (size_t)seq * hs + head0 * D + i) = q;
+        } else {
+            *reinterpret_cast<char4 *>((int8_t *)(m == 1 ? sq.k : sq.v) + (size_t)pos * hs + head0 * D + i) = q;
+        }
+    }
+}
+
+template <int D>
+__device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
+{
+    constexpr int LPH = D / 16, HPW = 32 / LPH; // lanes per head, heads per warp-wide load
+    const TStepLayer &layer = p.Layers[l];
+    const int tid = threadIdx.x, lane = tid & 31, group = tid >> 7, w = (tid >> 5) & 3;
+    const int hs = p.Heads * D, headGroups = (p.Heads + HPW - 1) / HPW;
+    TAttGroupSmem &g = sm.Att[group];
+    const TAttPlan plan = MakeAttPlan(p, layer, headGroups);
+    const int head = lane / LPH, sub = lane % LPH; // head inside the group, 16-byte slice of it
+    for (int unit = group * gridDim.x + blockIdx.x; unit < plan.Units; unit += PS_GROUPS * gridDim.x) {
+        // the sequence whose units contain this one: the last with Base <= unit
+        const unsigned at0 = __ballot_sync(0xffffffffu, lane < p.NSeq && plan.Base0 <= unit), at1 = __ballot_sync(0xffffffffu, lane + 32 < p.NSeq && plan.Base1 <= unit);
+        const int seq = at1 ? 63 - __clz(at1) : 31 - __clz(at0);
+        const int keysA = __shfl_sync(0xffffffffu, plan.Keys0, seq & 31), keysB = __shfl_sync(0xffffffffu, plan.Keys1, seq & 31);
+        const int baseA = __shfl_sync(0xffffffffu, plan.Base0, seq & 31), baseB = __shfl_sync(0xffffffffu, plan.Base1, seq & 31);
+        const int keys = seq < 32 ? keysA : keysB, rel = unit - (seq < 32 ? baseA : baseB);
+        const int chunks = max(1, (keys + plan.Chunk - 1) / plan.Chunk);
+        const int hg = rel / chunks, chunk = rel - hg * chunks;
+        const int head0 = hg * HPW, heads = min(HPW, p.Heads - head0);
+        const int pos = layer.CtxLens[seq];
+        const bool posOk = pos >= 0 && pos < p.RopeLen && pos < p.Capacity;
+        if (tid % 128 == 0 && p.Status && (!posOk || pos + 1 > p.MaxCtx)) {
+            atomicOr(p.Status, kDevBadSpan); // the cache or the rope table is full, or longer than the caller's bound
+        }
+        if (posOk && (chunk == 0 || w == 0)) {
+            // the first chunk's unit also appends the token and leaves the combiner key
+            ProjectHeads<D>(p, layer, g, w, seq, head0, heads, pos);
+        }
+        GroupSync(group);
+        float m = -1e30f, lsum = 0, acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            acc[i] = 0;
+        }
+        const int headC = min(head, heads - 1);
+        int j0, j1;
+        KeyRange(pos + 1, layer.Window, &j0, &j1);
+        const int cBeg = j0 + chunk * plan.Chunk, cEnd = min(cBeg + plan.Chunk, j1);
+        const int part = (((cEnd - cBeg) + 3) / 4 + 7) & ~7;
+        const int tBeg = cBeg + w * part, tEnd = min(tBeg + part, cEnd);
+        if (posOk && tBeg < tEnd) {
+            const tsa_kv_seq sq = layer.Seqs[seq];
+            const int4 qv = *reinterpret_cast<const int4 *>(g.Q8 + headC * D + sub * 16);
+            const size_t off = (size_t)tBeg * hs + (head0 + headC) * D + sub * 16, soff = (size_t)tBeg * p.Heads + head0 + headC;
+            AttendTokens<D, 8, true>(qv, p.DotScale * INF_VEC_SCALE, layer.Slope, pos, reinterpret_cast<const int4 *>((const int8_t *)sq.k + off),
+                reinterpret_cast<const int4 *>((const int8_t *)sq.v + off), (const float *)sq.kScale + soff, (const float *)sq.vScale + soff, p.Heads, tBeg, tEnd, m,
+                lsum, acc);
+        }
+        {
+            float *mine = g.Merge[w][lane];
+            mine[0] = m;
+            mine[1] = lsum;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                mine[2 + i] = acc[i];
+            }
+        }
+        GroupSync(group);
+        // the four warps' shares of the chunk; warp w goes on with columns 4 w .. 4 w + 3 of every lane's slice
+        float mAll = g.Merge[0][lane][0];
+#pragma unroll
+        for (int k = 1; k < 4; ++k) {
+            mAll = fmaxf(mAll, g.Merge[k][lane][0]);
+        }
+        float lAll = 0, val[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float *other = g.Merge[k][lane];
+            const float f = exp2f(other[0] - mAll);
+            lAll = fmaf(f, other[1], lAll);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                val[i] = fmaf(f, other[2 + 4 * w + i], val[i]);
+            }
+        }
+        const int z = sub * 16 + 4 * w;
+        bool finish = true;
+        if (chunks > 1) {
+            // partials to L2; the unit that arrives last merges all of the row's
+            constexpr int PITCH = D + 4;
+            float *dst = p.Partial + ((size_t)unit * HPW + head) * PITCH;
+            __stcg(reinterpret_cast<float4 *>(dst + z), make_float4(val[0], val[1], val[2], val[3]));
+            if (z == 0) {
+                __stcg(reinterpret_cast<float2 *>(dst + D), make_float2(mAll, lAll));
+            }
+            __threadfence();
+            GroupSync(group);
+            if (tid % 128 == 0) {
+                const int done = atomicAdd(p.Arrived + seq * headGroups + hg, 1);
+                g.Last = done == chunks - 1;
+                __threadfence();
+            }
+            GroupSync(group);
+            finish = g.Last != 0;
+            if (finish) {
+                if (tid % 128 == 0) {
+                    p.Arrived[seq * headGroups + hg] = 0; // for the next layer
+                }
+                const float *src = p.Partial + ((size_t)(unit - chunk) * HPW + head) * PITCH;
+                mAll = -1e30f;
+#pragma unroll 4
+                for (int c = 0; c < chunks; ++c) {
+                    mAll = fmaxf(mAll, __ldcg(src + (size_t)c * HPW * PITCH + D));
+                }
+                lAll = 0;
+                val[0] = val[1] = val[2] = val[3] = 0;
+#pragma unroll 4
+                for (int c = 0; c < chunks; ++c) {
+                    const float *q = src + (size_t)c * HPW * PITCH;
+                    const float2 ml = __ldcg(reinterpret_cast<const float2 *>(q + D));
+                    const float4 v = __ldcg(reinterpret_cast<const float4 *>(q + z));
+                    const float f = exp2f(ml.x - mAll);
+                    lAll = fmaf(f, ml.y, lAll);
+                    val[0] = fmaf(f, v.x, val[0]);
+                    val[1] = fmaf(f, v.y, val[1]);
+                    val[2] = fmaf(f, v.z, val[2]);
+                    val[3] = fmaf(f, v.w, val[3]);
+                }
+            }
+        }
+        if (finish && head < heads) {
+            // the sink has logit 0 (softMax.Add(0), cpu_infer.cpp:444)
+            const float mF = fmaxf(mAll, 0.0f), f = exp2f(mAll - mF), lF = exp2f(-mF) + f * lAll;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                val[i] = posOk ? (f * val[i]) / lF : 0.0f;
+            }
+            char4 key = make_char4(0, 0, 0, 0);
+            if (posOk) {
+                const int packed = __ldcg(reinterpret_cast<const int *>(p.K8 + (size_t)seq * hs + (head0 + head) * D + z));
+                key = *reinterpret_cast<const char4 *>(&packed);
+            }
+            StoreKvProduct(p.Kv8 + ((size_t)seq * hs + (head0 + head) * D) * 4, D, z, key, val);
+        }
+        GroupSync(group); // the group's shared memory is used again by its next unit
+    }
+}
+
+__device__ __forceinline__ void ZeroSums(int *sums, int n)
+{
+    for (int i = blockIdx.x * PS_THREADS + threadIdx.x; i < n / 4; i += gridDim.x * PS_THREADS) {
+        reinterpret_cast<int4 *>(sums)[i] = make_int4(0, 0, 0, 0);
+    }
+}
+
+template <int D>
+__device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
+{
+    const int tid = threadIdx.x, hs = p.Heads * D;
+    TTileCursor cursor = {0, 0, (int)blockIdx.x, 0};
+    cursor.Settle(p);
+    for (int i = 0; i < PS_RING - 1; ++i) {
+        RequestTile(p, cursor, sm.Ring[i]);
+        cursor.Next(p);
+    }
+    int tileCount = 0, mmaCount = 0, passed = 0;
+    // Sums are cleared a phase or more after their last reader has passed a barrier and a phase or more before their next writer.
+    for (int l = 0; l < p.LayerCount; ++l) {
+        if (l > 0) {
+            ZeroSums(p.Expand, p.NSeq * p.ReluDim);
+        }
+        if (!ProductPhase(p, sm, l, PH_PROJ, cursor, tileCount, mmaCount) || !GridSync(p, sm, passed)) {
+            return;
+        }
+        if (l > 0) {
+            ZeroSums(p.Contract, p.NSeq * p.Dim);
+        }
+        AttentionPhase<D>(p, sm, l);
+        if (!GridSync(p, sm, passed)) {
+            return;
+        }
+        ZeroSums(p.Proj, p.NSeq * 4 * hs);
+        if (blockIdx.x == gridDim.x - 1 && tid < p.NSeq) {
+            p.Layers[l].CtxLens[tid] += 1; // the token is in every sequence's cache of this layer
+        }
+        if (!ProductPhase(p, sm, l, PH_COMB, cursor, tileCount, mmaCount) || !GridSync(p, sm, passed)) {
+            return;
+        }
+        if (!ProductPhase(p, sm, l, PH_EXPAND, cursor, tileCount, mmaCount) || !GridSync(p, sm, passed)) {
+            return;
+        }
+        ZeroSums(p.Comb, p.NSeq * p.Dim);
+        if (!ProductPhase(p, sm, l, PH_CONTRACT, cursor, tileCount, mmaCount) || !GridSync(p, sm, passed)) {
+            return;
+        }
+    }
+    // the state after the last layer: fp32 for a launch that continues from here, its int8 form for the final product
+    for (int chunk = blockIdx.x; chunk < p.Dim / 128; chunk += gridDim.x) {
+        StageState(p, sm, chunk, p.LayerCount > 0 ? SRC_SUM : p.FirstSource, p.StateB, p.Contract, p.LayerCount > 0 ? p.Layers[p.LayerCount - 1].ContractScale : 0.0f,
+            p.StateA);
+        NormaliseStaged(p, sm);
+        __syncthreads();
+        for (int i = tid; i < p.NSeq * 8; i += PS_THREADS) {
+            const int s = i >> 3, c16 = i & 7;
+            *reinterpret_cast<int4 *>(p.NormState + (size_t)s * p.Dim + chunk * 128 + c16 * 16) = *reinterpret_cast<const int4 *>(sm.B + s * 128 + ((c16 ^ (s & 7)) << 4));
+        }
+        __syncthreads();
+    }
+}
+
+// PS_THREADS x 128 registers and 213 KB of shared memory: one CTA per SM.
+template <int D>
+__global__ void __launch_bounds__(PS_THREADS, 1) InferLayersKernel(const __grid_constant__ TStepParams p)
+{
+    extern __shared__ uint8_t stepSmemRaw[];
+    TStepSmem &sm = *reinterpret_cast<TStepSmem *>(((uintptr_t)stepSmemRaw + 1023) & ~(uintptr_t)1023); // operand tiles: 128-byte swizzle
+    const int tid = threadIdx.x;
+    PdlWait();
+    if (tid == 0) {
+        MbarInit(&sm.MmaDone, 1);
+        FenceBarrierInit();
+        sm.Failed = 0;
+    }
+    if (tid < 32) {
+        TmemAlloc(&sm.TmemBase, 64);
+        TmemRelinquish();
+    }
+    for (int i = tid; i < PS_B_BYTES / 16; i += PS_THREADS) {
+        reinterpret_cast<int4 *>(sm.B)[i] = make_int4(0, 0, 0, 0); // rows past the batch stay zero
+    }
+    TcFenceBefore();
+    __syncthreads();
+    TcFenceAfter();
+    RunLayers<D>(p, sm);
+    CpAsyncWait<0>();
+    TcFenceBefore();
+    __syncthreads();
+    PdlTrigger();
+    if (tid < 32) {
+        TmemDealloc(sm.TmemBase, 64);
+    }
+}
+
+// Measured on B200 (dim 768, 12 heads x 64, twelve layers, three of four with a 64-key window), per token:
+// see the table in the class of the step's launches in infer.cu.
+int InferLayersPersistent(const tsa_infer_model *model, const tsa_kv_seq *const *layerSeqs, int *ctxLens, int capacity, const int *labels, int labelsPerSeq,
+    int nSeq, int maxCtx, const TInferBuffers &b, int *statusWord, cudaStream_t stream)
+{
+    const tsa_infer_dims &d = model->dims;
+    const int hs = d.head_count * d.head_dim, D = d.head_dim;
+    int dev = 0, sms = 0;
+    int rc = CheckCuda(cudaGetDevice(&dev), "cudaGetDevice");
+    if (rc == TSA_OK) {
+        rc = CheckCuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+    }
+    const void *kern = D == 64 ? (const void *)InferLayersKernel<64> : (const void *)InferLayersKernel<128>;
+    const int smemBytes = (int)sizeof(TStepSmem) + 1024;
+    if (rc == TSA_OK) {
+        rc = CheckCuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes), "cudaFuncSetAttribute(inference layers)");
+    }
+    if (rc != TSA_OK) {
+        return rc;
+    }
+    sms = sms < PS_MAX_SLOTS / PS_GROUPS ? sms : PS_MAX_SLOTS / PS_GROUPS;
+    TStepParams p;
+    auto shape = [&](int tiles, int columns) {
+        // as many items as SMs, each with the same number of column chunks
+        TStepShape s;
+        s.Tiles = tiles;
+        s.Chunks = columns / 128;
+        int splits = sms / tiles;
+        splits = splits < 1 ? 1 : splits > s.Chunks ? s.Chunks : splits;
+        s.Per = (s.Chunks + splits - 1) / splits;
+        s.Splits = (s.Chunks + s.Per - 1) / s.Per;
+        return s;
+    };
+    p.Shape[PH_PROJ] = shape(4 * ((hs + 127) / 128), d.dim);
+    p.Shape[PH_COMB] = shape(d.dim / 128, 4 * hs);
+    p.Shape[PH_EXPAND] = shape(d.relu_dim / 128, d.dim);
+    p.Shape[PH_CONTRACT] = shape(d.dim / 128, d.relu_dim);
+    p.NSeq = nSeq;
+    p.Dim = d.dim;
+    p.Heads = d.head_count;
+    p.HeadSize = D;
+    p.ReluDim = d.relu_dim;
+    p.Capacity = capacity;
+    p.MaxCtx = maxCtx + 1;
+    p.RopeLen = model->rope_len;
+    p.Labels = labels;
+    p.LabelsPerSeq = labelsPerSeq;
+    p.LabelCount = d.label_count;
+    p.Embed = model->label_embed;
+    p.EmbedScale = model->label_embed_scale;
+    p.Rope = model->rope;
+    p.DotScale = HostAttDotScale(D);
+    p.Barrier = b.Sync;
+    p.Arrived = b.Sync + 64;
+    p.Proj = b.Proj;
+    p.Comb = b.Comb;
+    p.Expand = b.Expand;
+    p.Contract = b.Contract;
+    p.StateA = b.StateA;
+    p.StateB = b.StateB;
+    p.K8 = b.K8;
+    p.Kv8 = b.Kv8;
+    p.NormState = b.NormState;
+    p.Partial = b.Partial;
+    p.Status = statusWord;
+    for (int l = 0; l < d.layer_count; ++l) {
+        const tsa_infer_layer &layer = model->layers[l];
+        TSA_REQUIRE(layer.qk && layer.qv && layer.k && layer.v && layer.combiner && layer.expand && layer.contract && layerSeqs[l],
+            "tsa_infer_step: layer %d has a null matrix or cache", l);
+    }
+    int done = 0;
+    do {
+        p.LayerCount = d.layer_count - done < PS_LAYERS ? d.layer_count - done : PS_LAYERS;
+        p.FirstSource = done == 0 ? SRC_EMBED : SRC_STATE;
+        for (int i = 0; i < p.LayerCount; ++i) {
+            const tsa_infer_layer &layer = model->layers[done + i];
+            TStepLayer &t = p.Layers[i];
+            const int8_t *w[7] = {layer.qk, layer.qv, layer.k, layer.v, layer.combiner, layer.expand, layer.contract};
+            for (int k = 0; k < 7; ++k) {
+                t.W[k] = w[k];
+            }
+            t.Seqs = layerSeqs[done + i];
+            t.CtxLens = ctxLens + (size_t)(done + i) * nSeq;
+            // same association as cpu_infer.cpp:504: qvScale *= (QVScale * VEC_SCALE) * dotScale(dim)
+            t.QvMult = layer.qv_scale * INF_VEC_SCALE * sqrtf(1.0f / d.dim);
+            t.CombScale = layer.combiner_scale * INF_VEC_SCALE * sqrtf(1.0f / (hs * 4));
+            t.ContractScale = layer.contract_scale * INF_VEC_SCALE * sqrtf(1.0f / d.relu_dim);
+            t.Slope = layer.alibi_slope;
+            t.Window = layer.attention_width;
+        }
+        rc = CheckCuda(cudaMemsetAsync(b.Sync, 0, b.ZeroBytes, stream), "clearing the inference sums");
+        if (rc == TSA_OK) {
+            void *args[] = {&p};
+            rc = CheckCuda(cudaLaunchCooperativeKernel(kern, dim3(sms), dim3(PS_THREADS), args, smemBytes, stream), "inference layers launch");
+        }
+        done += p.LayerCount;
+    } while (rc == TSA_OK && done < d.layer_count);
+    return rc;
+}
+
+} // namespace tsa
