@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(128, 2) InferGemmI8Kernel(const __grid_constan
 // SoftMax of the final layer (cpu_infer.cpp:340-354): base 2, the maximum starts at 0 (TSoftMaxBuf::Clear).
 // Two kernels over (sequence, slice of the vocabulary) so that a batch of 64 sequences fills the GPU: the first leaves
 // each slice's maximum and sum of 2^(w - max), the second merges the slices' pairs and writes the probabilities.
-constexpr int INF_SOFTMAX_SLICES = 8;
+constexpr int INF_SOFTMAX_SLICES = 64;
 
 __device__ __forceinline__ float BlockReduce(float v, bool isMax, float *red)
 {
@@ -218,16 +218,12 @@ __global__ void __launch_bounds__(256) InferSoftmaxKernel(const float *logits, c
     const int b = blockIdx.y, slice = blockIdx.x;
     const int per = (vocab + INF_SOFTMAX_SLICES - 1) / INF_SOFTMAX_SLICES;
     const int x0 = slice * per, x1 = min(x0 + per, vocab);
-    float mx = 0;
-#pragma unroll
-    for (int s = 0; s < INF_SOFTMAX_SLICES; ++s) {
-        mx = fmaxf(mx, part[(b * INF_SOFTMAX_SLICES + s) * 2]);
-    }
-    float sum = 0;
-#pragma unroll
-    for (int s = 0; s < INF_SOFTMAX_SLICES; ++s) {
-        sum += part[(b * INF_SOFTMAX_SLICES + s) * 2 + 1] * exp2f(part[(b * INF_SOFTMAX_SLICES + s) * 2] - mx);
-    }
+    // the slices' pairs, one per thread
+    __shared__ float red[8];
+    const bool has = threadIdx.x < INF_SOFTMAX_SLICES;
+    const float2 pair = has ? *reinterpret_cast<const float2 *>(part + (b * INF_SOFTMAX_SLICES + threadIdx.x) * 2) : make_float2(0.0f, 0.0f);
+    const float mx = BlockReduce(pair.x, true, red);
+    const float sum = BlockReduce(has ? pair.y * exp2f(pair.x - mx) : 0.0f, false, red);
     const float inv = 1.0f / sum;
     const float *l = logits + (size_t)b * vocab;
     float *out = prediction + (size_t)b * vocab;

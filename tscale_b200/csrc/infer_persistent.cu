@@ -25,7 +25,9 @@
 
 namespace tsa {
 
-constexpr int PS_THREADS = 512, PS_GROUPS = 4; // attention works in groups of four warps
+// Attention works in groups of four warps; three of them leave the key / value loop (64 registers of loads in flight) the 160-odd
+// registers it wants, with a fourth it spilled.
+constexpr int PS_THREADS = 384, PS_GROUPS = 3;
 constexpr int PS_RING = 8;                     // weight tiles in flight or in use per CTA
 constexpr int PS_TILE = 128 * 128;             // bytes of a weight tile: 128 rows x 128 columns
 constexpr int PS_B_BYTES = INF_MAX_SEQ * 128;  // the chunk's vectors, one row of 128 int8 per sequence
@@ -116,13 +118,20 @@ __device__ __forceinline__ void GroupSync(int group)
     asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
 }
 
-// Barrier of the whole grid.  Bounded: returns false in every thread of a CTA that has waited about a second.
-__device__ __forceinline__ bool GridSync(const TStepParams &p, TStepSmem &sm, int &passed)
+// Barrier of the whole grid in two parts, so that what does not depend on the other CTAs runs between them.  One counter and one
+// polling thread per CTA: 0.75 us when all arrive together (a flag per CTA polled by 148 threads took 3.1 us, eight counters 1.3).
+// Bounded: the wait returns false in every thread of a CTA that has waited about a second.
+__device__ __forceinline__ void GridArrive(const TStepParams &p, int &passed)
 {
     __syncthreads();
     passed += gridDim.x;
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p.Barrier) : "memory");
+    }
+}
+__device__ __forceinline__ bool GridWait(const TStepParams &p, TStepSmem &sm, int passed)
+{
+    if (threadIdx.x == 0) {
         const long long t0 = clock64();
         int seen;
         for (;;) {
@@ -191,13 +200,26 @@ __device__ __forceinline__ void RequestTile(const TStepParams &p, const TTileCur
         }
         const int pitch = s.Chunks * 128;
 #pragma unroll
-        for (int k = 0; k < PS_TILE / 16 / PS_THREADS; ++k) {
+        for (int k = 0; k < (PS_TILE / 16 + PS_THREADS - 1) / PS_THREADS; ++k) {
             const int idx = threadIdx.x + k * PS_THREADS, row = idx >> 3, c16 = idx & 7;
+            if (idx >= PS_TILE / 16) {
+                break;
+            }
             const bool ok = tile * 128 + row < rows;
             CpAsync16(dst + row * 128 + ((c16 ^ (row & 7)) << 4), w + (ok ? (size_t)(tile * 128 + row) * pitch + chunk * 128 + c16 * 16 : 0), ok ? 16 : 0);
         }
     }
     CpAsyncCommit();
+}
+
+// tiles for every free slot of the ring; the tiles before tileCount have been used up
+__device__ __forceinline__ void RefillRing(const TStepParams &p, TStepSmem &sm, TTileCursor &cursor, int tileCount, int &requested)
+{
+    while (requested - tileCount < PS_RING - 1) {
+        RequestTile(p, cursor, sm.Ring[requested % PS_RING]);
+        cursor.Next(p);
+        ++requested;
+    }
 }
 
 // one 16-byte piece (columns c16 * 16 ..) of row s of the operand tile, 128-byte swizzle
@@ -206,44 +228,73 @@ __device__ __forceinline__ void StoreCodes(uint8_t *tile, int s, int c16, int4 v
     *reinterpret_cast<int4 *>(tile + s * 128 + ((c16 ^ (s & 7)) << 4)) = v;
 }
 
+// four columns of the sum of a token's label embeddings (cpu_infer.cpp:536-543)
+__device__ float4 EmbedColumns(const TStepParams &p, int s, int col, bool report)
+{
+    float4 v = make_float4(0, 0, 0, 0);
+    for (int k = 0; k < p.LabelsPerSeq; ++k) {
+        const int label = p.Labels[s * p.LabelsPerSeq + k];
+        if (label < 0 || label >= p.LabelCount) {
+            if (col == 0 && report && p.Status) {
+                atomicOr(p.Status, kDevBadSpan);
+            }
+            continue;
+        }
+        const char4 e = *reinterpret_cast<const char4 *>(p.Embed + (size_t)label * p.Dim + col);
+        v.x = __fadd_rn(v.x, __fmul_rn((float)e.x, p.EmbedScale));
+        v.y = __fadd_rn(v.y, __fmul_rn((float)e.y, p.EmbedScale));
+        v.z = __fadd_rn(v.z, __fmul_rn((float)e.z, p.EmbedScale));
+        v.w = __fadd_rn(v.w, __fmul_rn((float)e.w, p.EmbedScale));
+    }
+    return v;
+}
+
 // columns [128 chunk, +128) of the state after the last update, in sm.F: source 0 = embedding, 1 = state + sums * scale, 2 = state.
 // The writer also stores them to dst.  Ends with a barrier.
 __device__ void StageState(const TStepParams &p, TStepSmem &sm, int chunk, int source, const float *state, const int *sums, float scale, float *dst)
 {
-    for (int i = threadIdx.x; i < p.NSeq * 32; i += PS_THREADS) {
-        const int s = i >> 5, x = (i & 31) * 4, col = chunk * 128 + x;
-        float v[4];
-        if (source == SRC_EMBED) {
-            v[0] = v[1] = v[2] = v[3] = 0;
-            for (int k = 0; k < p.LabelsPerSeq; ++k) {
-                const int label = p.Labels[s * p.LabelsPerSeq + k];
-                if (label < 0 || label >= p.LabelCount) {
-                    if (col == 0 && dst && p.Status) {
-                        atomicOr(p.Status, kDevBadSpan);
-                    }
-                    continue;
-                }
-                const char4 e = *reinterpret_cast<const char4 *>(p.Embed + (size_t)label * p.Dim + col);
-                v[0] = __fadd_rn(v[0], __fmul_rn((float)e.x, p.EmbedScale));
-                v[1] = __fadd_rn(v[1], __fmul_rn((float)e.y, p.EmbedScale));
-                v[2] = __fadd_rn(v[2], __fmul_rn((float)e.z, p.EmbedScale));
-                v[3] = __fadd_rn(v[3], __fmul_rn((float)e.w, p.EmbedScale));
-            }
-        } else {
-            const float4 old = __ldcg(reinterpret_cast<const float4 *>(state + (size_t)s * p.Dim + col));
-            v[0] = old.x, v[1] = old.y, v[2] = old.z, v[3] = old.w;
-            if (source == SRC_SUM) {
-                const int4 a = __ldcg(reinterpret_cast<const int4 *>(sums + (size_t)s * p.Dim + col));
-                v[0] = __fadd_rn(v[0], __fmul_rn((float)a.x, scale)); // AddScaled, cpu_infer.cpp:296-303
-                v[1] = __fadd_rn(v[1], __fmul_rn((float)a.y, scale));
-                v[2] = __fadd_rn(v[2], __fmul_rn((float)a.z, scale));
-                v[3] = __fadd_rn(v[3], __fmul_rn((float)a.w, scale));
+    if (source == SRC_EMBED) {
+        for (int i = threadIdx.x; i < p.NSeq * 32; i += PS_THREADS) {
+            const int s = i >> 5, x = (i & 31) * 4;
+            const float4 e = EmbedColumns(p, s, chunk * 128 + x, dst != nullptr);
+            *reinterpret_cast<float4 *>(&sm.F[s][x]) = e;
+            if (dst) {
+                *reinterpret_cast<float4 *>(dst + (size_t)s * p.Dim + chunk * 128 + x) = e;
             }
         }
-        const float4 out = make_float4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<float4 *>(&sm.F[s][x]) = out;
-        if (dst) {
-            *reinterpret_cast<float4 *>(dst + (size_t)s * p.Dim + col) = out;
+        __syncthreads();
+        return;
+    }
+    // two quads of columns per thread and step, their loads before the first use (all of a thread's quads at once took the registers
+    // the attention loop needs)
+    for (int base = threadIdx.x; base < p.NSeq * 32; base += 2 * PS_THREADS) {
+        float4 v[2];
+        int4 add[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int i = base + k * PS_THREADS, s = i >> 5, col = chunk * 128 + (i & 31) * 4;
+            if (i < p.NSeq * 32) {
+                v[k] = __ldcg(reinterpret_cast<const float4 *>(state + (size_t)s * p.Dim + col));
+                if (source == SRC_SUM) {
+                    add[k] = __ldcg(reinterpret_cast<const int4 *>(sums + (size_t)s * p.Dim + col));
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int i = base + k * PS_THREADS, s = i >> 5, x = (i & 31) * 4;
+            if (i < p.NSeq * 32) {
+                if (source == SRC_SUM) { // AddScaled, cpu_infer.cpp:296-303
+                    v[k].x = __fadd_rn(v[k].x, __fmul_rn((float)add[k].x, scale));
+                    v[k].y = __fadd_rn(v[k].y, __fmul_rn((float)add[k].y, scale));
+                    v[k].z = __fadd_rn(v[k].z, __fmul_rn((float)add[k].z, scale));
+                    v[k].w = __fadd_rn(v[k].w, __fmul_rn((float)add[k].w, scale));
+                }
+                *reinterpret_cast<float4 *>(&sm.F[s][x]) = v[k];
+                if (dst) {
+                    *reinterpret_cast<float4 *>(dst + (size_t)s * p.Dim + chunk * 128 + x) = v[k];
+                }
+            }
         }
     }
     __syncthreads();
@@ -293,6 +344,7 @@ __device__ void NormaliseStaged(const TStepParams &p, TStepSmem &sm)
 // inside the chunk is summed from shared memory, one that reaches beyond it from L2.
 __device__ void NormaliseRelu(const TStepParams &p, TStepSmem &sm, int chunk)
 {
+#pragma unroll 4
     for (int i = threadIdx.x; i < p.NSeq * 32; i += PS_THREADS) {
         const int s = i >> 5, x = (i & 31) * 4;
         const int4 a = __ldcg(reinterpret_cast<const int4 *>(p.Expand + (size_t)s * p.ReluDim + chunk * 128 + x));
@@ -354,8 +406,8 @@ __device__ void NormaliseRelu(const TStepParams &p, TStepSmem &sm, int chunk)
     }
 }
 
-// All of this CTA's items of one matrix product.  Returns false when a bounded wait ran out.
-__device__ bool ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int phase, TTileCursor &cursor, int &tileCount, int &mmaCount)
+// All of this CTA's items of one matrix product.
+__device__ void ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int phase, TTileCursor &cursor, int &tileCount, int &requested)
 {
     const TStepShape &s = p.Shape[phase];
     const TStepLayer &layer = p.Layers[l];
@@ -383,7 +435,13 @@ __device__ bool ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int pha
             } else {
                 NormaliseRelu(p, sm, chunk);
             }
-            CpAsyncWait<PS_RING - 2>(); // this thread's part of the tile has landed (one group per tile, PS_RING - 1 requested ahead)
+            // this thread's part of the tile has landed: the groups requested behind it (one per tile, at most PS_RING - 1 tiles are
+            // requested and not used up) may still be on their way
+            if (requested - tileCount == PS_RING - 1) {
+                CpAsyncWait<PS_RING - 2>();
+            } else {
+                CpAsyncWait<0>();
+            }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             TcFenceBefore();
             __syncthreads();
@@ -397,17 +455,16 @@ __device__ bool ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int pha
                 }
                 MmaCommit(&sm.MmaDone);
             }
-            // the next tile goes into the slot of the tile before this one, whose products were waited for below
-            RequestTile(p, cursor, sm.Ring[(tileCount + PS_RING - 1) % PS_RING]);
-            cursor.Next(p);
-            if (!WaitBar(&sm.MmaDone, mmaCount & 1)) {
+            if (!WaitBar(&sm.MmaDone, tileCount & 1)) {
                 sm.Failed = 1;
                 if (p.Status) {
                     atomicOr(p.Status, kDevTimeoutMma);
                 }
             }
             ++tileCount;
-            ++mmaCount;
+            if (requested - tileCount < PS_RING / 2) {
+                RefillRing(p, sm, cursor, tileCount, requested); // a phase with many tiles for one CTA: do not wait for its end
+            }
         }
         TcFenceAfter();
         // 128 rows x 16 sequences per warp: the item's sums join the others' in L2
@@ -423,8 +480,8 @@ __device__ bool ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int pha
             out = phase == PH_COMB ? p.Comb : phase == PH_EXPAND ? p.Expand : p.Contract;
             rows = pitch = phase == PH_EXPAND ? p.ReluDim : p.Dim;
         }
-        const int quad = warp & 3, s0 = (warp >> 2) * 16, row = tile * 128 + quad * 32 + (tid & 31);
-        if (s0 < nCols) {
+        const int quad = warp & 3, row = tile * 128 + quad * 32 + (tid & 31);
+        for (int s0 = (warp >> 2) * 16; s0 < nCols; s0 += PS_GROUPS * 16) {
             uint32_t acc[16];
             TmemLd16(sm.TmemBase + ((uint32_t)(quad * 32) << 16) + s0, acc);
             TmemWaitLd();
@@ -438,12 +495,10 @@ __device__ bool ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int pha
             }
         }
         TcFenceBefore();
-        __syncthreads();
-        if (sm.Failed) {
-            return false;
+        if (item + gridDim.x < s.Tiles * s.Splits) {
+            __syncthreads(); // the accumulators have been read
         }
     }
-    return true;
 }
 
 // ---- attention -----------------------------------------------------------------------------------------------------
@@ -586,15 +641,34 @@ __device__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAtt
     }
 }
 
+// this lane's share of a range of tokens, into the merge buffer
 template <int D>
-__device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
+__device__ __forceinline__ void AttendRange(const int4 qv, float logitMult, float slope, int pos, const int8_t *k, const int8_t *v, const float *ks, const float *vs,
+    int heads, int tBeg, int tEnd, float *mine)
+{
+    float m = -1e30f, l = 0, acc[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        acc[i] = 0;
+    }
+    AttendTokens<D, 8, true>(qv, logitMult, slope, pos, reinterpret_cast<const int4 *>(k), reinterpret_cast<const int4 *>(v), ks, vs, heads, tBeg, tEnd, m, l, acc);
+    mine[0] = m;
+    mine[1] = l;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        mine[2 + i] = acc[i];
+    }
+}
+
+template <int D>
+__device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l, const TAttPlan &plan)
 {
     constexpr int LPH = D / 16, HPW = 32 / LPH; // lanes per head, heads per warp-wide load
     const TStepLayer &layer = p.Layers[l];
     const int tid = threadIdx.x, lane = tid & 31, group = tid >> 7, w = (tid >> 5) & 3;
-    const int hs = p.Heads * D, headGroups = (p.Heads + HPW - 1) / HPW;
+    // head groups of even size: a group of a few left-over heads would take as long as a full one
+    const int hs = p.Heads * D, headGroups = (p.Heads + HPW - 1) / HPW, perGroup = (p.Heads + headGroups - 1) / headGroups;
     TAttGroupSmem &g = sm.Att[group];
-    const TAttPlan plan = MakeAttPlan(p, layer, headGroups);
     const int head = lane / LPH, sub = lane % LPH; // head inside the group, 16-byte slice of it
     for (int unit = group * gridDim.x + blockIdx.x; unit < plan.Units; unit += PS_GROUPS * gridDim.x) {
         // the sequence whose units contain this one: the last with Base <= unit
@@ -605,7 +679,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
         const int keys = seq < 32 ? keysA : keysB, rel = unit - (seq < 32 ? baseA : baseB);
         const int chunks = max(1, (keys + plan.Chunk - 1) / plan.Chunk);
         const int hg = rel / chunks, chunk = rel - hg * chunks;
-        const int head0 = hg * HPW, heads = min(HPW, p.Heads - head0);
+        const int head0 = hg * perGroup, heads = min(perGroup, p.Heads - head0);
         const int pos = layer.CtxLens[seq];
         const bool posOk = pos >= 0 && pos < p.RopeLen && pos < p.Capacity;
         if (tid % 128 == 0 && p.Status && (!posOk || pos + 1 > p.MaxCtx)) {
@@ -616,11 +690,6 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
             ProjectHeads<D>(p, layer, g, w, seq, head0, heads, pos);
         }
         GroupSync(group);
-        float m = -1e30f, lsum = 0, acc[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            acc[i] = 0;
-        }
         const int headC = min(head, heads - 1);
         int j0, j1;
         KeyRange(pos + 1, layer.Window, &j0, &j1);
@@ -631,17 +700,14 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
             const tsa_kv_seq sq = layer.Seqs[seq];
             const int4 qv = *reinterpret_cast<const int4 *>(g.Q8 + headC * D + sub * 16);
             const size_t off = (size_t)tBeg * hs + (head0 + headC) * D + sub * 16, soff = (size_t)tBeg * p.Heads + head0 + headC;
-            AttendTokens<D, 8, true>(qv, p.DotScale * INF_VEC_SCALE, layer.Slope, pos, reinterpret_cast<const int4 *>((const int8_t *)sq.k + off),
-                reinterpret_cast<const int4 *>((const int8_t *)sq.v + off), (const float *)sq.kScale + soff, (const float *)sq.vScale + soff, p.Heads, tBeg, tEnd, m,
-                lsum, acc);
-        }
-        {
+            AttendRange<D>(qv, p.DotScale * INF_VEC_SCALE, layer.Slope, pos, (const int8_t *)sq.k + off, (const int8_t *)sq.v + off, (const float *)sq.kScale + soff,
+                (const float *)sq.vScale + soff, p.Heads, tBeg, tEnd, g.Merge[w][lane]);
+        } else {
             float *mine = g.Merge[w][lane];
-            mine[0] = m;
-            mine[1] = lsum;
+            mine[0] = -1e30f;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                mine[2 + i] = acc[i];
+            for (int i = 1; i < 18; ++i) {
+                mine[i] = 0;
             }
         }
         GroupSync(group);
@@ -736,41 +802,45 @@ template <int D>
 __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
 {
     const int tid = threadIdx.x, hs = p.Heads * D;
+    const int headGroups = (p.Heads * D + 511) / 512;
     TTileCursor cursor = {0, 0, (int)blockIdx.x, 0};
     cursor.Settle(p);
-    for (int i = 0; i < PS_RING - 1; ++i) {
-        RequestTile(p, cursor, sm.Ring[i]);
-        cursor.Next(p);
-    }
-    int tileCount = 0, mmaCount = 0, passed = 0;
+    int tileCount = 0, requested = 0, passed = 0;
+    RefillRing(p, sm, cursor, tileCount, requested);
     // Sums are cleared a phase or more after their last reader has passed a barrier and a phase or more before their next writer.
     for (int l = 0; l < p.LayerCount; ++l) {
         if (l > 0) {
             ZeroSums(p.Expand, p.NSeq * p.ReluDim);
         }
-        if (!ProductPhase(p, sm, l, PH_PROJ, cursor, tileCount, mmaCount) || !GridSync(p, sm, passed)) {
+        ProductPhase(p, sm, l, PH_PROJ, cursor, tileCount, requested);
+        GridArrive(p, passed);
+        RefillRing(p, sm, cursor, tileCount, requested);
+        const TAttPlan plan = MakeAttPlan(p, p.Layers[l], headGroups);
+        if (!GridWait(p, sm, passed)) {
             return;
         }
         if (l > 0) {
             ZeroSums(p.Contract, p.NSeq * p.Dim);
         }
-        AttentionPhase<D>(p, sm, l);
-        if (!GridSync(p, sm, passed)) {
+        AttentionPhase<D>(p, sm, l, plan);
+        GridArrive(p, passed);
+        if (!GridWait(p, sm, passed)) {
             return;
         }
         ZeroSums(p.Proj, p.NSeq * 4 * hs);
         if (blockIdx.x == gridDim.x - 1 && tid < p.NSeq) {
             p.Layers[l].CtxLens[tid] += 1; // the token is in every sequence's cache of this layer
         }
-        if (!ProductPhase(p, sm, l, PH_COMB, cursor, tileCount, mmaCount) || !GridSync(p, sm, passed)) {
-            return;
-        }
-        if (!ProductPhase(p, sm, l, PH_EXPAND, cursor, tileCount, mmaCount) || !GridSync(p, sm, passed)) {
-            return;
-        }
-        ZeroSums(p.Comb, p.NSeq * p.Dim);
-        if (!ProductPhase(p, sm, l, PH_CONTRACT, cursor, tileCount, mmaCount) || !GridSync(p, sm, passed)) {
-            return;
+        for (int phase = PH_COMB; phase <= PH_CONTRACT; ++phase) {
+            if (phase == PH_CONTRACT) {
+                ZeroSums(p.Comb, p.NSeq * p.Dim);
+            }
+            ProductPhase(p, sm, l, phase, cursor, tileCount, requested);
+            GridArrive(p, passed);
+            RefillRing(p, sm, cursor, tileCount, requested);
+            if (!GridWait(p, sm, passed)) {
+                return;
+            }
         }
     }
     // the state after the last layer: fp32 for a launch that continues from here, its int8 form for the final product
@@ -787,7 +857,7 @@ __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
     }
 }
 
-// PS_THREADS x 128 registers and 213 KB of shared memory: one CTA per SM.
+// PS_THREADS x 168 registers and 195 KB of shared memory: one CTA per SM.
 template <int D>
 __global__ void __launch_bounds__(PS_THREADS, 1) InferLayersKernel(const __grid_constant__ TStepParams p)
 {
