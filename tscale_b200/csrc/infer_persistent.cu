@@ -28,6 +28,7 @@ namespace tsa {
 // Attention works in groups of four warps; three of them leave the key / value loop (64 registers of loads in flight) the 160-odd
 // registers it wants, with a fourth it spilled.
 constexpr int PS_THREADS = 384, PS_GROUPS = 3;
+constexpr int PS_LOADERS = PS_THREADS - 32; // threads that request weight tiles: all but the warp whose first lane polls the grid barrier
 constexpr int PS_RING = 8;                     // weight tiles in flight or in use per CTA
 constexpr int PS_TILE = 128 * 128;             // bytes of a weight tile: 128 rows x 128 columns
 constexpr int PS_B_BYTES = INF_MAX_SEQ * 128;  // the chunk's vectors, one row of 128 int8 per sequence
@@ -79,7 +80,15 @@ struct alignas(16) TAttGroupSmem {
     float Mult[4][8];
     int8_t Q8[512], K8[512];
     float Merge[4][32][PS_MERGE_PITCH];
+    tsa_kv_seq Seq;               // the group's unit: its sequence's cache, position of the new token,
+    int Pos, SeqIndex, HeadGroup, Chunk, Chunks; // which unit it is
     int Last;
+};
+
+// Chunks of the attention of one layer (see MakeAttPlan).
+struct TAttPlan {
+    int Window, Chunk, Units;
+    int Base[INF_MAX_SEQ], Keys[INF_MAX_SEQ]; // first unit and keys of each sequence
 };
 
 struct TStepSmem {
@@ -90,8 +99,9 @@ struct TStepSmem {
             float F[INF_MAX_SEQ][PS_F_PITCH];
             float Mult[INF_MAX_SEQ];
         };
-        TAttGroupSmem Att[PS_GROUPS];
+        TAttGroupSmem Att[PS_GROUPS]; // from the barrier in front of an attention to its end
     };
+    TAttPlan Plan[2];             // of the last two windows: the layers of a model alternate between two or so
     uint64_t MmaDone;
     uint32_t TmemBase;
     int Failed;
@@ -200,10 +210,10 @@ __device__ __forceinline__ void RequestTile(const TStepParams &p, const TTileCur
         }
         const int pitch = s.Chunks * 128;
 #pragma unroll
-        for (int k = 0; k < (PS_TILE / 16 + PS_THREADS - 1) / PS_THREADS; ++k) {
-            const int idx = threadIdx.x + k * PS_THREADS, row = idx >> 3, c16 = idx & 7;
-            if (idx >= PS_TILE / 16) {
-                break;
+        for (int k = 0; k < (PS_TILE / 16 + PS_LOADERS - 1) / PS_LOADERS; ++k) {
+            const int idx = (int)threadIdx.x - 32 + k * PS_LOADERS, row = idx >> 3, c16 = idx & 7;
+            if (idx < 0 || idx >= PS_TILE / 16) {
+                continue;
             }
             const bool ok = tile * 128 + row < rows;
             CpAsync16(dst + row * 128 + ((c16 ^ (row & 7)) << 4), w + (ok ? (size_t)(tile * 128 + row) * pitch + chunk * 128 + c16 * 16 : 0), ok ? 16 : 0);
@@ -212,14 +222,15 @@ __device__ __forceinline__ void RequestTile(const TStepParams &p, const TTileCur
     CpAsyncCommit();
 }
 
-// tiles for every free slot of the ring; the tiles before tileCount have been used up
-__device__ __forceinline__ void RefillRing(const TStepParams &p, TStepSmem &sm, TTileCursor &cursor, int tileCount, int &requested)
+// requests the cursor's next n tiles into the ring slots from `slot` on and returns the cursor behind them
+__device__ __noinline__ TTileCursor RefillRing(const TStepParams &p, TStepSmem &sm, TTileCursor cursor, int slot, int n)
 {
-    while (requested - tileCount < PS_RING - 1) {
-        RequestTile(p, cursor, sm.Ring[requested % PS_RING]);
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+        RequestTile(p, cursor, sm.Ring[(slot + i) % PS_RING]);
         cursor.Next(p);
-        ++requested;
     }
+    return cursor;
 }
 
 // one 16-byte piece (columns c16 * 16 ..) of row s of the operand tile, 128-byte swizzle
@@ -229,7 +240,7 @@ __device__ __forceinline__ void StoreCodes(uint8_t *tile, int s, int c16, int4 v
 }
 
 // four columns of the sum of a token's label embeddings (cpu_infer.cpp:536-543)
-__device__ float4 EmbedColumns(const TStepParams &p, int s, int col, bool report)
+__device__ __noinline__ float4 EmbedColumns(const TStepParams &p, int s, int col, bool report)
 {
     float4 v = make_float4(0, 0, 0, 0);
     for (int k = 0; k < p.LabelsPerSeq; ++k) {
@@ -251,7 +262,7 @@ __device__ float4 EmbedColumns(const TStepParams &p, int s, int col, bool report
 
 // columns [128 chunk, +128) of the state after the last update, in sm.F: source 0 = embedding, 1 = state + sums * scale, 2 = state.
 // The writer also stores them to dst.  Ends with a barrier.
-__device__ void StageState(const TStepParams &p, TStepSmem &sm, int chunk, int source, const float *state, const int *sums, float scale, float *dst)
+__device__ __forceinline__ void StageState(const TStepParams &p, TStepSmem &sm, int chunk, int source, const float *state, const int *sums, float scale, float *dst)
 {
     if (source == SRC_EMBED) {
         for (int i = threadIdx.x; i < p.NSeq * 32; i += PS_THREADS) {
@@ -323,7 +334,7 @@ __device__ __forceinline__ void QuantiseStaged(const TStepParams &p, TStepSmem &
 }
 
 // NormalizeState of the staged chunk (one STATE_NORM_TILE): one thread per sequence adds the squares in index order
-__device__ void NormaliseStaged(const TStepParams &p, TStepSmem &sm)
+__device__ __forceinline__ void NormaliseStaged(const TStepParams &p, TStepSmem &sm)
 {
     const int s = threadIdx.x;
     if (s < p.NSeq) {
@@ -342,9 +353,9 @@ __device__ void NormaliseStaged(const TStepParams &p, TStepSmem &sm)
 
 // The contract product's input: relu of the expand sums normalised per head (groups of ReluDim / Heads columns).  A group that lies
 // inside the chunk is summed from shared memory, one that reaches beyond it from L2.
-__device__ void NormaliseRelu(const TStepParams &p, TStepSmem &sm, int chunk)
+__device__ __forceinline__ void NormaliseRelu(const TStepParams &p, TStepSmem &sm, int chunk)
 {
-#pragma unroll 4
+#pragma unroll 8
     for (int i = threadIdx.x; i < p.NSeq * 32; i += PS_THREADS) {
         const int s = i >> 5, x = (i & 31) * 4;
         const int4 a = __ldcg(reinterpret_cast<const int4 *>(p.Expand + (size_t)s * p.ReluDim + chunk * 128 + x));
@@ -402,12 +413,14 @@ __device__ void NormaliseRelu(const TStepParams &p, TStepSmem &sm, int chunk)
         __syncthreads();
         const int lo = max(g0, c0) - c0, hi = min(g1, c0 + 128) - c0;
         QuantiseStaged(p, sm, lo / 16, (hi - lo) / 16, true);
-        __syncthreads(); // the next group overwrites sm.Mult
+        if (g1 < c0 + 128) {
+            __syncthreads(); // the next group overwrites sm.Mult
+        }
     }
 }
 
 // All of this CTA's items of one matrix product.
-__device__ void ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int phase, TTileCursor &cursor, int &tileCount, int &requested)
+__device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int phase, TTileCursor &cursor, int &tileCount, int &requested)
 {
     const TStepShape &s = p.Shape[phase];
     const TStepLayer &layer = p.Layers[l];
@@ -420,18 +433,17 @@ __device__ void ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int pha
         const int first = (item - tile * s.Splits) * s.Per, chunks = min(s.Per, s.Chunks - first);
         for (int c = 0; c < chunks; ++c) {
             const int chunk = first + c;
-            if (phase == PH_PROJ) {
-                const int source = l > 0 ? SRC_SUM : p.FirstSource;
-                StageState(p, sm, chunk, source, source == SRC_STATE ? p.StateA : p.StateB, p.Contract, l > 0 ? p.Layers[l - 1].ContractScale : 0.0f,
-                    tile == 0 && source != SRC_STATE ? p.StateA : nullptr);
+            if (phase == PH_PROJ || phase == PH_EXPAND) {
+                // StateA and StateB take turns: the first holds the state in front of the attention block, the second behind it
+                const bool proj = phase == PH_PROJ;
+                const int source = proj && l == 0 ? p.FirstSource : SRC_SUM;
+                StageState(p, sm, chunk, source, proj == (source == SRC_SUM) ? p.StateB : p.StateA, proj ? p.Contract : p.Comb,
+                    proj ? (l > 0 ? p.Layers[l - 1].ContractScale : 0.0f) : layer.CombScale, tile != 0 || source == SRC_STATE ? nullptr : proj ? p.StateA : p.StateB);
                 NormaliseStaged(p, sm);
             } else if (phase == PH_COMB) {
                 for (int i = tid; i < p.NSeq * 8; i += PS_THREADS) {
                     StoreCodes(sm.B, i >> 3, i & 7, __ldcg(reinterpret_cast<const int4 *>(p.Kv8 + (size_t)(i >> 3) * 4 * hs + chunk * 128 + (i & 7) * 16)));
                 }
-            } else if (phase == PH_EXPAND) {
-                StageState(p, sm, chunk, SRC_SUM, p.StateA, p.Comb, layer.CombScale, tile == 0 ? p.StateB : nullptr);
-                NormaliseStaged(p, sm);
             } else {
                 NormaliseRelu(p, sm, chunk);
             }
@@ -463,7 +475,9 @@ __device__ void ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int pha
             }
             ++tileCount;
             if (requested - tileCount < PS_RING / 2) {
-                RefillRing(p, sm, cursor, tileCount, requested); // a phase with many tiles for one CTA: do not wait for its end
+                // a phase with many tiles for one CTA: do not wait for its end
+                cursor = RefillRing(p, sm, cursor, requested, PS_RING - 1 - (requested - tileCount));
+                requested = tileCount + PS_RING - 1;
             }
         }
         TcFenceAfter();
@@ -505,13 +519,6 @@ __device__ void ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int pha
 // A unit = one sequence x one head group (the heads a warp-wide 16-byte load covers: 8 of 64 or 4 of 128) x one chunk of keys,
 // taken by a group of four warps that split the chunk's keys.  All chunks have the same size, the smallest multiple of 32 (at least
 // PS_MIN_CHUNK) whose units all fit the resident groups of the grid in one wave; the plan is a bisection every warp does for itself.
-struct TAttPlan {
-    int Chunk;        // keys per unit
-    int Units;        // of all sequences
-    int Base0, Base1; // first unit of sequences lane and lane + 32
-    int Keys0, Keys1; // their keys
-};
-
 __device__ __forceinline__ int StepKeys(const TStepParams &p, const TStepLayer &layer, int s)
 {
     if (s >= p.NSeq) {
@@ -526,29 +533,27 @@ __device__ __forceinline__ int StepKeys(const TStepParams &p, const TStepLayer &
     return j1 - j0;
 }
 
-__device__ TAttPlan MakeAttPlan(const TStepParams &p, const TStepLayer &layer, int headGroups)
+// by one warp, into shared memory
+__device__ __noinline__ void MakeAttPlan(const TStepParams &p, const TStepLayer &layer, int headGroups, TAttPlan &plan)
 {
     const int lane = threadIdx.x & 31;
     const int slots = max((int)gridDim.x * PS_GROUPS, p.NSeq * headGroups);
-    TAttPlan pl;
-    pl.Keys0 = StepKeys(p, layer, lane);
-    pl.Keys1 = StepKeys(p, layer, lane + 32);
+    const int keys0 = StepKeys(p, layer, lane), keys1 = StepKeys(p, layer, lane + 32);
     const bool on0 = lane < p.NSeq, on1 = lane + 32 < p.NSeq;
     // every sequence has at least one unit per head group: it appends the new token
     auto units = [&](int keys, bool on, int chunk) { return on ? headGroups * max(1, (keys + chunk - 1) / chunk) : 0; };
-    const int total = __reduce_add_sync(0xffffffffu, pl.Keys0 + pl.Keys1), most = __reduce_max_sync(0xffffffffu, max(pl.Keys0, pl.Keys1));
+    const int total = __reduce_add_sync(0xffffffffu, keys0 + keys1), most = __reduce_max_sync(0xffffffffu, max(keys0, keys1));
     int lo = max(PS_MIN_CHUNK / 32, (int)(((long long)total * headGroups / slots) / 32)), hi = max((most + 31) / 32, lo);
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        const int n = __reduce_add_sync(0xffffffffu, units(pl.Keys0, on0, mid * 32) + units(pl.Keys1, on1, mid * 32));
+        const int n = __reduce_add_sync(0xffffffffu, units(keys0, on0, mid * 32) + units(keys1, on1, mid * 32));
         if (n <= slots) {
             hi = mid;
         } else {
             lo = mid + 1;
         }
     }
-    pl.Chunk = lo * 32;
-    const int u0 = units(pl.Keys0, on0, pl.Chunk), u1 = units(pl.Keys1, on1, pl.Chunk);
+    const int u0 = units(keys0, on0, lo * 32), u1 = units(keys1, on1, lo * 32);
     int i0 = u0, i1 = u1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -557,10 +562,77 @@ __device__ TAttPlan MakeAttPlan(const TStepParams &p, const TStepLayer &layer, i
         i1 += lane >= o ? b : 0;
     }
     const int sum0 = __shfl_sync(0xffffffffu, i0, 31);
-    pl.Base0 = i0 - u0;
-    pl.Base1 = sum0 + i1 - u1;
-    pl.Units = sum0 + __shfl_sync(0xffffffffu, i1, 31);
-    return pl;
+    plan.Base[lane] = i0 - u0;
+    plan.Base[lane + 32] = sum0 + i1 - u1;
+    plan.Keys[lane] = keys0;
+    plan.Keys[lane + 32] = keys1;
+    if (lane == 31) {
+        plan.Chunk = lo * 32;
+        plan.Units = sum0 + i1;
+        plan.Window = layer.Window;
+    }
+    __syncwarp();
+}
+
+// which unit is number `unit`, and its sequence's cache, into the group's shared memory (one warp)
+__device__ __noinline__ void LocateUnit(const TStepParams &p, const TStepLayer &layer, const TAttPlan &plan, int unit, TAttGroupSmem &g)
+{
+    const int lane = threadIdx.x & 31;
+    // the sequence whose units contain this one: the last with Base <= unit
+    const unsigned at0 = __ballot_sync(0xffffffffu, lane < p.NSeq && plan.Base[lane] <= unit);
+    const unsigned at1 = __ballot_sync(0xffffffffu, lane + 32 < p.NSeq && plan.Base[lane + 32] <= unit);
+    const int seq = at1 ? 63 - __clz(at1) : 31 - __clz(at0);
+    const int chunks = max(1, (plan.Keys[seq] + plan.Chunk - 1) / plan.Chunk), rel = unit - plan.Base[seq], hg = rel / chunks;
+    if (lane == 0) {
+        g.Pos = layer.CtxLens[seq];
+        g.Seq = layer.Seqs[seq];
+        g.SeqIndex = seq;
+        g.HeadGroup = hg;
+        g.Chunk = rel - hg * chunks;
+        g.Chunks = chunks;
+    }
+    __syncwarp();
+}
+
+// The group's first unit of layer l, while the grid barrier in front of the attention is waited for: the second warp of each group
+// looks up the unit and requests its first keys and values into L2 (neither depends on this step's products).
+__device__ __noinline__ void PrepareAttention(const TStepParams &p, TStepSmem &sm, int l, int headGroups, int perGroup)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = warp >> 2;
+    if ((warp & 3) != 1) {
+        return;
+    }
+    const TStepLayer &layer = p.Layers[l];
+    int slot = sm.Plan[0].Window == layer.Window ? 0 : 1;
+    if (sm.Plan[slot].Window != layer.Window) {
+        return; // a window not seen lately: planned behind the barrier
+    }
+    const TAttPlan &plan = sm.Plan[slot];
+    TAttGroupSmem &g = sm.Att[group];
+    const int unit = group * gridDim.x + blockIdx.x;
+    if (unit >= plan.Units) {
+        return;
+    }
+    LocateUnit(p, layer, plan, unit, g);
+    const int pos = g.Pos, rowBytes = p.Heads * p.HeadSize, headBytes = perGroup * p.HeadSize;
+    if (pos < 0 || pos >= p.Capacity) {
+        return;
+    }
+    int j0, j1;
+    KeyRange(pos + 1, layer.Window, &j0, &j1);
+    const int beg = j0 + g.Chunk * plan.Chunk, end = min(beg + min(plan.Chunk, PS_MIN_CHUNK), j1);
+    const int lines = (headBytes + 127) / 128; // of one token's rows, per matrix
+    for (int i = lane; i < (end - beg) * 2 * lines; i += 32) {
+        const int t = i / (2 * lines), r = i - t * 2 * lines, col = g.HeadGroup * headBytes + (r % lines) * 128;
+        if (col < rowBytes) {
+            const int8_t *row = (const int8_t *)(r < lines ? g.Seq.k : g.Seq.v) + (size_t)(beg + t) * rowBytes + col;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(row));
+        }
+    }
+    for (int i = lane; i * 32 < (end - beg) * p.Heads; i += 32) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"((const float *)g.Seq.kScale + (size_t)beg * p.Heads + i * 32));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"((const float *)g.Seq.vScale + (size_t)beg * p.Heads + i * 32));
+    }
 }
 
 // The combiner input of four consecutive columns z .. z + 3 of a head: kv[blk][z] = int8(key[z ^ blk] * val[z]) (KVProduct,
@@ -587,7 +659,7 @@ __device__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAtt
     const int lane = threadIdx.x & 31, hs = p.Heads * D;
     const int *src = p.Proj + (size_t)seq * 4 * hs + m * hs + head0 * D;
     float *rot = g.Rot[m];
-#pragma unroll 4
+#pragma unroll 8
     for (int b = 0; b < heads * D / 64; ++b) {
         const float v0 = (float)__ldcg(src + b * 64 + lane), v1 = (float)__ldcg(src + b * 64 + lane + 32);
         float r0 = v0, r1 = v1;
@@ -603,7 +675,7 @@ __device__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAtt
         w[lane + 32] = r1;
     }
     __syncwarp();
-    const tsa_kv_seq sq = layer.Seqs[seq];
+    const tsa_kv_seq sq = g.Seq;
     if (lane < heads) {
         const float *w = rot + lane * (D + 1);
         float sum2 = 0;
@@ -634,6 +706,7 @@ __device__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAtt
         if (m == 0) {
             *reinterpret_cast<char4 *>(g.Q8 + i) = q;
         } else if (m == 2) {
+            *reinterpret_cast<char4 *>(g.K8 + i) = q;
             *reinterpret_cast<char4 *>(p.K8 + (size_t)seq * hs + head0 * D + i) = q;
         } else {
             *reinterpret_cast<char4 *>((int8_t *)(m == 1 ? sq.k : sq.v) + (size_t)pos * hs + head0 * D + i) = q;
@@ -661,26 +734,38 @@ __device__ __forceinline__ void AttendRange(const int4 qv, float logitMult, floa
 }
 
 template <int D>
-__device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l, const TAttPlan &plan)
+__device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l, int headGroups, int perGroup)
 {
     constexpr int LPH = D / 16, HPW = 32 / LPH; // lanes per head, heads per warp-wide load
     const TStepLayer &layer = p.Layers[l];
     const int tid = threadIdx.x, lane = tid & 31, group = tid >> 7, w = (tid >> 5) & 3;
-    // head groups of even size: a group of a few left-over heads would take as long as a full one
-    const int hs = p.Heads * D, headGroups = (p.Heads + HPW - 1) / HPW, perGroup = (p.Heads + headGroups - 1) / headGroups;
+    const int hs = p.Heads * D;
     TAttGroupSmem &g = sm.Att[group];
+    int slot = sm.Plan[0].Window == layer.Window ? 0 : 1;
+    bool located = true;
+    if (sm.Plan[slot].Window != layer.Window) {
+        // not among the last two windows (the same for the whole CTA: the plans change only here)
+        __syncthreads();
+        slot = sm.Plan[0].Window < 0 ? 0 : sm.Plan[1].Window < 0 ? 1 : l & 1;
+        __syncthreads();
+        if (tid < 32) {
+            MakeAttPlan(p, layer, headGroups, sm.Plan[slot]);
+        }
+        __syncthreads();
+        located = false;
+    }
+    const TAttPlan &plan = sm.Plan[slot];
     const int head = lane / LPH, sub = lane % LPH; // head inside the group, 16-byte slice of it
     for (int unit = group * gridDim.x + blockIdx.x; unit < plan.Units; unit += PS_GROUPS * gridDim.x) {
-        // the sequence whose units contain this one: the last with Base <= unit
-        const unsigned at0 = __ballot_sync(0xffffffffu, lane < p.NSeq && plan.Base0 <= unit), at1 = __ballot_sync(0xffffffffu, lane + 32 < p.NSeq && plan.Base1 <= unit);
-        const int seq = at1 ? 63 - __clz(at1) : 31 - __clz(at0);
-        const int keysA = __shfl_sync(0xffffffffu, plan.Keys0, seq & 31), keysB = __shfl_sync(0xffffffffu, plan.Keys1, seq & 31);
-        const int baseA = __shfl_sync(0xffffffffu, plan.Base0, seq & 31), baseB = __shfl_sync(0xffffffffu, plan.Base1, seq & 31);
-        const int keys = seq < 32 ? keysA : keysB, rel = unit - (seq < 32 ? baseA : baseB);
-        const int chunks = max(1, (keys + plan.Chunk - 1) / plan.Chunk);
-        const int hg = rel / chunks, chunk = rel - hg * chunks;
+        if (!located) {
+            if (w == 1) {
+                LocateUnit(p, layer, plan, unit, g);
+            }
+            GroupSync(group);
+        }
+        located = false; // the next unit was not looked up in advance
+        const int seq = g.SeqIndex, hg = g.HeadGroup, chunk = g.Chunk, chunks = g.Chunks, pos = g.Pos;
         const int head0 = hg * perGroup, heads = min(perGroup, p.Heads - head0);
-        const int pos = layer.CtxLens[seq];
         const bool posOk = pos >= 0 && pos < p.RopeLen && pos < p.Capacity;
         if (tid % 128 == 0 && p.Status && (!posOk || pos + 1 > p.MaxCtx)) {
             atomicOr(p.Status, kDevBadSpan); // the cache or the rope table is full, or longer than the caller's bound
@@ -697,7 +782,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l, const
         const int part = (((cEnd - cBeg) + 3) / 4 + 7) & ~7;
         const int tBeg = cBeg + w * part, tEnd = min(tBeg + part, cEnd);
         if (posOk && tBeg < tEnd) {
-            const tsa_kv_seq sq = layer.Seqs[seq];
+            const tsa_kv_seq &sq = g.Seq;
             const int4 qv = *reinterpret_cast<const int4 *>(g.Q8 + headC * D + sub * 16);
             const size_t off = (size_t)tBeg * hs + (head0 + headC) * D + sub * 16, soff = (size_t)tBeg * p.Heads + head0 + headC;
             AttendRange<D>(qv, p.DotScale * INF_VEC_SCALE, layer.Slope, pos, (const int8_t *)sq.k + off, (const int8_t *)sq.v + off, (const float *)sq.kScale + soff,
@@ -753,13 +838,13 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l, const
                 }
                 const float *src = p.Partial + ((size_t)(unit - chunk) * HPW + head) * PITCH;
                 mAll = -1e30f;
-#pragma unroll 4
+#pragma unroll 8
                 for (int c = 0; c < chunks; ++c) {
                     mAll = fmaxf(mAll, __ldcg(src + (size_t)c * HPW * PITCH + D));
                 }
                 lAll = 0;
                 val[0] = val[1] = val[2] = val[3] = 0;
-#pragma unroll 4
+#pragma unroll 8
                 for (int c = 0; c < chunks; ++c) {
                     const float *q = src + (size_t)c * HPW * PITCH;
                     const float2 ml = __ldcg(reinterpret_cast<const float2 *>(q + D));
@@ -781,7 +866,9 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l, const
                 val[i] = posOk ? (f * val[i]) / lF : 0.0f;
             }
             char4 key = make_char4(0, 0, 0, 0);
-            if (posOk) {
+            if (posOk && chunks == 1) {
+                key = *reinterpret_cast<const char4 *>(g.K8 + head * D + z);
+            } else if (posOk) {
                 const int packed = __ldcg(reinterpret_cast<const int *>(p.K8 + (size_t)seq * hs + (head0 + head) * D + z));
                 key = *reinterpret_cast<const char4 *>(&packed);
             }
@@ -802,45 +889,52 @@ template <int D>
 __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
 {
     const int tid = threadIdx.x, hs = p.Heads * D;
-    const int headGroups = (p.Heads * D + 511) / 512;
+    // a head group is what a warp-wide 16-byte load covers, 512 columns at most; groups of even size, because a group of a few
+    // left-over heads would take as long as a full one
+    const int headGroups = (p.Heads * D + 511) / 512, perGroup = (p.Heads + headGroups - 1) / headGroups;
     TTileCursor cursor = {0, 0, (int)blockIdx.x, 0};
     cursor.Settle(p);
-    int tileCount = 0, requested = 0, passed = 0;
-    RefillRing(p, sm, cursor, tileCount, requested);
+    int tileCount = 0, requested = PS_RING - 1, passed = 0;
+    cursor = RefillRing(p, sm, cursor, 0, requested);
+    // One loop over all phases, so that every piece of code exists once: the kernel's loop has to fit the SM's instruction cache
+    // (with the phases written out one after another a quarter of the instruction fetches missed it).
     // Sums are cleared a phase or more after their last reader has passed a barrier and a phase or more before their next writer.
-    for (int l = 0; l < p.LayerCount; ++l) {
-        if (l > 0) {
-            ZeroSums(p.Expand, p.NSeq * p.ReluDim);
-        }
-        ProductPhase(p, sm, l, PH_PROJ, cursor, tileCount, requested);
-        GridArrive(p, passed);
-        RefillRing(p, sm, cursor, tileCount, requested);
-        const TAttPlan plan = MakeAttPlan(p, p.Layers[l], headGroups);
-        if (!GridWait(p, sm, passed)) {
-            return;
-        }
-        if (l > 0) {
-            ZeroSums(p.Contract, p.NSeq * p.Dim);
-        }
-        AttentionPhase<D>(p, sm, l, plan);
-        GridArrive(p, passed);
-        if (!GridWait(p, sm, passed)) {
-            return;
-        }
-        ZeroSums(p.Proj, p.NSeq * 4 * hs);
-        if (blockIdx.x == gridDim.x - 1 && tid < p.NSeq) {
-            p.Layers[l].CtxLens[tid] += 1; // the token is in every sequence's cache of this layer
-        }
-        for (int phase = PH_COMB; phase <= PH_CONTRACT; ++phase) {
-            if (phase == PH_CONTRACT) {
-                ZeroSums(p.Comb, p.NSeq * p.Dim);
+    int l = 0, phase = PH_PROJ;
+    bool attention = false; // the attention follows PH_PROJ
+#pragma unroll 1
+    while (l < p.LayerCount) {
+        if (attention) {
+            ZeroSums(l > 0 ? p.Contract : p.Comb, p.NSeq * p.Dim);
+            AttentionPhase<D>(p, sm, l, headGroups, perGroup);
+        } else {
+            int *done = phase == PH_PROJ ? p.Expand : phase == PH_COMB ? p.Proj : p.Comb;
+            const int doneInts = p.NSeq * (phase == PH_PROJ ? p.ReluDim : phase == PH_COMB ? 4 * hs : p.Dim);
+            if (phase != PH_EXPAND && (phase != PH_PROJ || l > 0)) {
+                ZeroSums(done, doneInts);
+            }
+            if (phase == PH_COMB && blockIdx.x == gridDim.x - 1 && tid < p.NSeq) {
+                p.Layers[l].CtxLens[tid] += 1; // the token is in every sequence's cache of this layer
             }
             ProductPhase(p, sm, l, phase, cursor, tileCount, requested);
-            GridArrive(p, passed);
-            RefillRing(p, sm, cursor, tileCount, requested);
-            if (!GridWait(p, sm, passed)) {
-                return;
+        }
+        GridArrive(p, passed);
+        const int refill = PS_RING - 1 - (requested - tileCount);
+        if (refill > 0) {
+            cursor = RefillRing(p, sm, cursor, requested, refill);
+            requested += refill;
+        }
+        if (!attention && phase == PH_PROJ) {
+            PrepareAttention(p, sm, l, headGroups, perGroup);
+            attention = true;
+        } else {
+            attention = false;
+            if (++phase == 4) {
+                phase = PH_PROJ;
+                ++l;
             }
+        }
+        if (!GridWait(p, sm, passed)) {
+            return;
         }
     }
     // the state after the last layer: fp32 for a launch that continues from here, its int8 form for the final product
@@ -869,6 +963,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) InferLayersKernel(const __grid_
         MbarInit(&sm.MmaDone, 1);
         FenceBarrierInit();
         sm.Failed = 0;
+        sm.Plan[0].Window = sm.Plan[1].Window = -1;
     }
     if (tid < 32) {
         TmemAlloc(&sm.TmemBase, 64);
@@ -959,6 +1054,7 @@ int InferLayersPersistent(const tsa_infer_model *model, const tsa_kv_seq *const 
         const tsa_infer_layer &layer = model->layers[l];
         TSA_REQUIRE(layer.qk && layer.qv && layer.k && layer.v && layer.combiner && layer.expand && layer.contract && layerSeqs[l],
             "tsa_infer_step: layer %d has a null matrix or cache", l);
+        TSA_REQUIRE(layer.attention_width >= 0, "tsa_infer_step: layer %d has a negative attention width", l);
     }
     int done = 0;
     do {
