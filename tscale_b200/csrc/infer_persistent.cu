@@ -60,6 +60,7 @@ struct TStepParams {
     TStepShape Shape[4];
     int LayerCount, FirstSource;
     int NSeq, Dim, Heads, HeadSize, ReluDim, Capacity, MaxCtx, RopeLen;
+    int HeadGroups, PerGroup;     // groups of heads the attention works in, heads of a group (the last may have fewer)
     const int *Labels;
     int LabelsPerSeq, LabelCount;
     const int8_t *Embed;
@@ -76,7 +77,7 @@ struct TStepParams {
 };
 
 struct alignas(16) TAttGroupSmem {
-    float Rot[4][8 * 65];         // a head group's four projected vectors (8 x 64 or 4 x 128), rotated; pitch D + 1 per head
+    float Rot[4][8 * 68];         // a head group's four projected vectors (8 x 64 or 4 x 128), rotated; pitch D + 4 per head
     float Mult[4][8];
     int8_t Q8[512], K8[512];
     float Merge[4][32][PS_MERGE_PITCH];
@@ -91,6 +92,15 @@ struct TAttPlan {
     int Base[INF_MAX_SEQ], Keys[INF_MAX_SEQ]; // first unit and keys of each sequence
 };
 
+// one 128 x 128 weight tile of the CTA's share of a layer
+enum { TILE_FIRST = 1, TILE_LAST = 2 }; // of its item
+struct TWeightTile {
+    uint8_t Matrix, Flags; // index into TStepLayer::W
+    uint16_t Chunk;
+    int Tile;
+};
+constexpr int PS_TABLE = 512; // tiles per CTA and layer kept in shared memory (1.2 GB of weights in one layer); beyond it they are computed
+
 struct TStepSmem {
     uint8_t Ring[PS_RING][PS_TILE];
     uint8_t B[PS_B_BYTES];
@@ -99,12 +109,15 @@ struct TStepSmem {
             float F[INF_MAX_SEQ][PS_F_PITCH];
             float Mult[INF_MAX_SEQ];
         };
-        TAttGroupSmem Att[PS_GROUPS]; // from the barrier in front of an attention to its end
+        TAttGroupSmem Att[PS_GROUPS];
     };
+    TWeightTile Table[PS_TABLE];
+    int PhaseBegin[5];            // first tile of each phase, and their number
     TAttPlan Plan[2];             // of the last two windows: the layers of a model alternate between two or so
     uint64_t MmaDone;
     uint32_t TmemBase;
     int Failed;
+    int Passed;                   // arrivals at the grid barrier that complete its present phase
 };
 
 static_assert(sizeof(TAttGroupSmem) % 16 == 0 && offsetof(TAttGroupSmem, Q8) % 16 == 0 && offsetof(TStepSmem, F) % 16 == 0 && offsetof(TStepSmem, B) % 1024 == 0,
@@ -131,17 +144,17 @@ __device__ __forceinline__ void GroupSync(int group)
 // Barrier of the whole grid in two parts, so that what does not depend on the other CTAs runs between them.  One counter and one
 // polling thread per CTA: 0.75 us when all arrive together (a flag per CTA polled by 148 threads took 3.1 us, eight counters 1.3).
 // Bounded: the wait returns false in every thread of a CTA that has waited about a second.
-__device__ __forceinline__ void GridArrive(const TStepParams &p, int &passed)
+__device__ __forceinline__ void GridArrive(const TStepParams &p)
 {
     __syncthreads();
-    passed += gridDim.x;
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p.Barrier) : "memory");
     }
 }
-__device__ __forceinline__ bool GridWait(const TStepParams &p, TStepSmem &sm, int passed)
+__device__ __forceinline__ bool GridWait(const TStepParams &p, TStepSmem &sm)
 {
     if (threadIdx.x == 0) {
+        const int passed = sm.Passed += gridDim.x;
         const long long t0 = clock64();
         int seen;
         for (;;) {
@@ -162,75 +175,78 @@ __device__ __forceinline__ bool GridWait(const TStepParams &p, TStepSmem &sm, in
     return sm.Failed == 0;
 }
 
-// The CTA's weight tiles in the order it will use them: all items of all phases of all layers.
-struct TTileCursor {
-    int Layer, Phase, Item, Chunk;
-
-    __device__ __forceinline__ void Settle(const TStepParams &p)
-    {
-        while (Layer < p.LayerCount && Item >= p.Shape[Phase].Tiles * p.Shape[Phase].Splits) {
-            Item = blockIdx.x;
-            Chunk = 0;
-            if (++Phase == 4) {
-                Phase = 0;
-                ++Layer;
-            }
-        }
-    }
-    __device__ __forceinline__ void Next(const TStepParams &p)
-    {
-        if (Layer >= p.LayerCount) {
-            return;
-        }
-        const TStepShape &s = p.Shape[Phase];
-        const int first = (Item % s.Splits) * s.Per;
-        if (++Chunk >= min(s.Per, s.Chunks - first)) {
-            Chunk = 0;
-            Item += gridDim.x;
-            Settle(p);
-        }
-    }
-};
-
-// requests the cursor's tile (nothing past the last one) and closes the cp.async group; rows past the matrix read as zeros
-__device__ __forceinline__ void RequestTile(const TStepParams &p, const TTileCursor &c, uint8_t *dst)
+// The CTA's weight tiles of one layer in the order it uses them, tile number `index`: item blockIdx.x, blockIdx.x + gridDim.x, ... of
+// every phase, an item's chunks one after another.
+__device__ __noinline__ TWeightTile ComputeTile(const TStepParams &p, int index)
 {
-    if (c.Layer < p.LayerCount) {
-        const TStepLayer &layer = p.Layers[c.Layer];
-        const TStepShape &s = p.Shape[c.Phase];
-        int tile = c.Item / s.Splits;
-        const int chunk = (c.Item - tile * s.Splits) * s.Per + c.Chunk;
-        int rows = c.Phase == PH_EXPAND ? p.ReluDim : p.Dim;
-        const int8_t *w = layer.W[c.Phase + 3];
-        if (c.Phase == PH_PROJ) {
-            const int perMatrix = s.Tiles / 4, m = tile / perMatrix;
-            tile -= m * perMatrix;
-            rows = p.Heads * p.HeadSize;
-            w = layer.W[m];
+    TWeightTile t = {};
+    for (int phase = 0; phase < 4; ++phase) {
+        const TStepShape &s = p.Shape[phase];
+        for (int item = blockIdx.x; item < s.Tiles * s.Splits; item += gridDim.x) {
+            const int tile = item / s.Splits, first = (item - tile * s.Splits) * s.Per, chunks = min(s.Per, s.Chunks - first);
+            if (index < chunks) {
+                const int perMatrix = phase == PH_PROJ ? s.Tiles / 4 : s.Tiles;
+                t.Matrix = (uint8_t)(phase == PH_PROJ ? tile / perMatrix : phase + 3);
+                t.Tile = tile % perMatrix;
+                t.Chunk = first + index;
+                t.Flags = (uint8_t)((index == 0 ? TILE_FIRST : 0) | (index == chunks - 1 ? TILE_LAST : 0));
+                return t;
+            }
+            index -= chunks;
         }
+    }
+    return t;
+}
+__device__ __forceinline__ TWeightTile TileAt(const TStepParams &p, const TStepSmem &sm, int index)
+{
+    return index < PS_TABLE ? sm.Table[index] : ComputeTile(p, index);
+}
+
+// requests tile number `index` of layer l (nothing past the last layer) and closes the cp.async group; rows past the matrix read as
+// zeros.  All warps but the first, whose lane polls the grid barrier meanwhile.
+__device__ __forceinline__ void RequestTile(const TStepParams &p, const TStepSmem &sm, int l, int index, uint8_t *dst)
+{
+    if (l < p.LayerCount) {
+        const TWeightTile t = TileAt(p, sm, index);
+        const int8_t *w = p.Layers[l].W[t.Matrix];
+        const TStepShape &s = p.Shape[t.Matrix < 4 ? PH_PROJ : t.Matrix - 3];
+        const int rows = t.Matrix < 4 ? p.Heads * p.HeadSize : t.Matrix - 3 == PH_EXPAND ? p.ReluDim : p.Dim;
         const int pitch = s.Chunks * 128;
+        w += (size_t)t.Tile * 128 * pitch + t.Chunk * 128;
 #pragma unroll
         for (int k = 0; k < (PS_TILE / 16 + PS_LOADERS - 1) / PS_LOADERS; ++k) {
             const int idx = (int)threadIdx.x - 32 + k * PS_LOADERS, row = idx >> 3, c16 = idx & 7;
-            if (idx < 0 || idx >= PS_TILE / 16) {
-                continue;
+            if (idx < PS_TILE / 16) {
+                const bool ok = t.Tile * 128 + row < rows;
+                CpAsync16(dst + row * 128 + ((c16 ^ (row & 7)) << 4), ok ? w + (size_t)row * pitch + c16 * 16 : p.Layers[l].W[t.Matrix], ok ? 16 : 0);
             }
-            const bool ok = tile * 128 + row < rows;
-            CpAsync16(dst + row * 128 + ((c16 ^ (row & 7)) << 4), w + (ok ? (size_t)(tile * 128 + row) * pitch + chunk * 128 + c16 * 16 : 0), ok ? 16 : 0);
         }
     }
     CpAsyncCommit();
 }
 
-// requests the cursor's next n tiles into the ring slots from `slot` on and returns the cursor behind them
-__device__ __noinline__ TTileCursor RefillRing(const TStepParams &p, TStepSmem &sm, TTileCursor cursor, int slot, int n)
+// Where the CTA stands in its sequence of weight tiles.
+struct TTileCursor {
+    int Used, Requested;      // tiles used up / requested so far, over all layers
+    int NextLayer, NextIndex; // the next tile to request
+};
+
+// requests tiles until PS_RING - 1 of them are on their way or waiting (the slot of the tile used last is free again)
+__device__ __noinline__ void RefillRing(const TStepParams &p, TStepSmem &sm, TTileCursor *cursor)
 {
+    TTileCursor c = *cursor;
 #pragma unroll 1
-    for (int i = 0; i < n; ++i) {
-        RequestTile(p, cursor, sm.Ring[(slot + i) % PS_RING]);
-        cursor.Next(p);
+    while (c.Requested - c.Used < PS_RING - 1) {
+        if (threadIdx.x >= 32) {
+            RequestTile(p, sm, c.NextLayer, c.NextIndex, sm.Ring[c.Requested % PS_RING]);
+        }
+        ++c.Requested;
+        if (++c.NextIndex >= sm.PhaseBegin[4]) {
+            c.NextIndex = 0;
+            ++c.NextLayer;
+        }
     }
-    return cursor;
+    *cursor = c;
 }
 
 // one 16-byte piece (columns c16 * 16 ..) of row s of the operand tile, 128-byte swizzle
@@ -420,19 +436,18 @@ __device__ __forceinline__ void NormaliseRelu(const TStepParams &p, TStepSmem &s
 }
 
 // All of this CTA's items of one matrix product.
-__device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int phase, TTileCursor &cursor, int &tileCount, int &requested)
+__device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int phase, TTileCursor &cursor)
 {
-    const TStepShape &s = p.Shape[phase];
     const TStepLayer &layer = p.Layers[l];
     const int tid = threadIdx.x, warp = tid >> 5;
     const int hs = p.Heads * p.HeadSize;
     const int nCols = (p.NSeq + 15) & ~15; // accumulator columns
     const uint32_t idesc = MakeInstrDesc(2, 1, 1, 0, 0, 128, nCols);
-    for (int item = blockIdx.x; item < s.Tiles * s.Splits; item += gridDim.x) {
-        int tile = item / s.Splits;
-        const int first = (item - tile * s.Splits) * s.Per, chunks = min(s.Per, s.Chunks - first);
-        for (int c = 0; c < chunks; ++c) {
-            const int chunk = first + c;
+    const int end = sm.PhaseBegin[phase + 1];
+    for (int index = sm.PhaseBegin[phase]; index < end; ++index) {
+        const TWeightTile t = TileAt(p, sm, index);
+        const int chunk = t.Chunk, tile = t.Matrix == 0 || t.Matrix > 3 ? t.Tile : -1; // tile 0 of the phase also keeps the new state
+        {
             if (phase == PH_PROJ || phase == PH_EXPAND) {
                 // StateA and StateB take turns: the first holds the state in front of the attention block, the second behind it
                 const bool proj = phase == PH_PROJ;
@@ -449,7 +464,7 @@ __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm
             }
             // this thread's part of the tile has landed: the groups requested behind it (one per tile, at most PS_RING - 1 tiles are
             // requested and not used up) may still be on their way
-            if (requested - tileCount == PS_RING - 1) {
+            if (cursor.Requested - cursor.Used == PS_RING - 1) {
                 CpAsyncWait<PS_RING - 2>();
             } else {
                 CpAsyncWait<0>();
@@ -459,42 +474,33 @@ __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm
             __syncthreads();
             TcFenceAfter();
             if (warp == 0 && ElectOne()) {
-                const uint32_t sA = SmemAddr(sm.Ring[tileCount % PS_RING]), sB = SmemAddr(sm.B);
+                const uint32_t sA = SmemAddr(sm.Ring[cursor.Used % PS_RING]), sB = SmemAddr(sm.B);
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
                     MmaI8SS(sm.TmemBase, MakeSmemDesc(sA + ks * 32, 16, 1024, 128), MakeSmemDesc(sB + ks * 32, 16, 1024, 128), idesc,
-                        (c > 0 || ks > 0) ? 1u : 0u);
+                        (!(t.Flags & TILE_FIRST) || ks > 0) ? 1u : 0u);
                 }
                 MmaCommit(&sm.MmaDone);
             }
-            if (!WaitBar(&sm.MmaDone, tileCount & 1)) {
+            if (!WaitBar(&sm.MmaDone, cursor.Used & 1)) {
                 sm.Failed = 1;
                 if (p.Status) {
                     atomicOr(p.Status, kDevTimeoutMma);
                 }
             }
-            ++tileCount;
-            if (requested - tileCount < PS_RING / 2) {
-                // a phase with many tiles for one CTA: do not wait for its end
-                cursor = RefillRing(p, sm, cursor, requested, PS_RING - 1 - (requested - tileCount));
-                requested = tileCount + PS_RING - 1;
+            ++cursor.Used;
+            if (cursor.Requested - cursor.Used < PS_RING / 2) {
+                RefillRing(p, sm, &cursor); // a phase with many tiles for one CTA: do not wait for its end
             }
+        }
+        if (!(t.Flags & TILE_LAST)) {
+            continue;
         }
         TcFenceAfter();
         // 128 rows x 16 sequences per warp: the item's sums join the others' in L2
-        int *out;
-        int rows, pitch;
-        if (phase == PH_PROJ) {
-            const int perMatrix = s.Tiles / 4, m = tile / perMatrix;
-            tile -= m * perMatrix;
-            out = p.Proj + m * hs;
-            rows = hs;
-            pitch = 4 * hs;
-        } else {
-            out = phase == PH_COMB ? p.Comb : phase == PH_EXPAND ? p.Expand : p.Contract;
-            rows = pitch = phase == PH_EXPAND ? p.ReluDim : p.Dim;
-        }
-        const int quad = warp & 3, row = tile * 128 + quad * 32 + (tid & 31);
+        int *out = phase == PH_PROJ ? p.Proj + t.Matrix * hs : phase == PH_COMB ? p.Comb : phase == PH_EXPAND ? p.Expand : p.Contract;
+        const int rows = phase == PH_PROJ ? hs : phase == PH_EXPAND ? p.ReluDim : p.Dim, pitch = phase == PH_PROJ ? 4 * hs : rows;
+        const int quad = warp & 3, row = t.Tile * 128 + quad * 32 + (tid & 31);
         for (int s0 = (warp >> 2) * 16; s0 < nCols; s0 += PS_GROUPS * 16) {
             uint32_t acc[16];
             TmemLd16(sm.TmemBase + ((uint32_t)(quad * 32) << 16) + s0, acc);
@@ -509,7 +515,7 @@ __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm
             }
         }
         TcFenceBefore();
-        if (item + gridDim.x < s.Tiles * s.Splits) {
+        if (index + 1 < end) {
             __syncthreads(); // the accumulators have been read
         }
     }
@@ -534,16 +540,16 @@ __device__ __forceinline__ int StepKeys(const TStepParams &p, const TStepLayer &
 }
 
 // by one warp, into shared memory
-__device__ __noinline__ void MakeAttPlan(const TStepParams &p, const TStepLayer &layer, int headGroups, TAttPlan &plan)
+__device__ __noinline__ void MakeAttPlan(const TStepParams &p, const TStepLayer &layer, TAttPlan &plan)
 {
     const int lane = threadIdx.x & 31;
-    const int slots = max((int)gridDim.x * PS_GROUPS, p.NSeq * headGroups);
+    const int slots = max((int)gridDim.x * PS_GROUPS, p.NSeq * p.HeadGroups);
     const int keys0 = StepKeys(p, layer, lane), keys1 = StepKeys(p, layer, lane + 32);
     const bool on0 = lane < p.NSeq, on1 = lane + 32 < p.NSeq;
     // every sequence has at least one unit per head group: it appends the new token
-    auto units = [&](int keys, bool on, int chunk) { return on ? headGroups * max(1, (keys + chunk - 1) / chunk) : 0; };
+    auto units = [&](int keys, bool on, int chunk) { return on ? p.HeadGroups * max(1, (keys + chunk - 1) / chunk) : 0; };
     const int total = __reduce_add_sync(0xffffffffu, keys0 + keys1), most = __reduce_max_sync(0xffffffffu, max(keys0, keys1));
-    int lo = max(PS_MIN_CHUNK / 32, (int)(((long long)total * headGroups / slots) / 32)), hi = max((most + 31) / 32, lo);
+    int lo = max(PS_MIN_CHUNK / 32, (int)(((long long)total * p.HeadGroups / slots) / 32)), hi = max((most + 31) / 32, lo);
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
         const int n = __reduce_add_sync(0xffffffffu, units(keys0, on0, mid * 32) + units(keys1, on1, mid * 32));
@@ -594,47 +600,6 @@ __device__ __noinline__ void LocateUnit(const TStepParams &p, const TStepLayer &
     __syncwarp();
 }
 
-// The group's first unit of layer l, while the grid barrier in front of the attention is waited for: the second warp of each group
-// looks up the unit and requests its first keys and values into L2 (neither depends on this step's products).
-__device__ __noinline__ void PrepareAttention(const TStepParams &p, TStepSmem &sm, int l, int headGroups, int perGroup)
-{
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = warp >> 2;
-    if ((warp & 3) != 1) {
-        return;
-    }
-    const TStepLayer &layer = p.Layers[l];
-    int slot = sm.Plan[0].Window == layer.Window ? 0 : 1;
-    if (sm.Plan[slot].Window != layer.Window) {
-        return; // a window not seen lately: planned behind the barrier
-    }
-    const TAttPlan &plan = sm.Plan[slot];
-    TAttGroupSmem &g = sm.Att[group];
-    const int unit = group * gridDim.x + blockIdx.x;
-    if (unit >= plan.Units) {
-        return;
-    }
-    LocateUnit(p, layer, plan, unit, g);
-    const int pos = g.Pos, rowBytes = p.Heads * p.HeadSize, headBytes = perGroup * p.HeadSize;
-    if (pos < 0 || pos >= p.Capacity) {
-        return;
-    }
-    int j0, j1;
-    KeyRange(pos + 1, layer.Window, &j0, &j1);
-    const int beg = j0 + g.Chunk * plan.Chunk, end = min(beg + min(plan.Chunk, PS_MIN_CHUNK), j1);
-    const int lines = (headBytes + 127) / 128; // of one token's rows, per matrix
-    for (int i = lane; i < (end - beg) * 2 * lines; i += 32) {
-        const int t = i / (2 * lines), r = i - t * 2 * lines, col = g.HeadGroup * headBytes + (r % lines) * 128;
-        if (col < rowBytes) {
-            const int8_t *row = (const int8_t *)(r < lines ? g.Seq.k : g.Seq.v) + (size_t)(beg + t) * rowBytes + col;
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(row));
-        }
-    }
-    for (int i = lane; i * 32 < (end - beg) * p.Heads; i += 32) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"((const float *)g.Seq.kScale + (size_t)beg * p.Heads + i * 32));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"((const float *)g.Seq.vScale + (size_t)beg * p.Heads + i * 32));
-    }
-}
-
 // The combiner input of four consecutive columns z .. z + 3 of a head: kv[blk][z] = int8(key[z ^ blk] * val[z]) (KVProduct,
 // cpu_infer.cpp:318-337); z ^ blk stays among the four.
 __device__ __forceinline__ void StoreKvProduct(int8_t *kv, int headSize, int z, char4 key, const float *val)
@@ -659,29 +624,48 @@ __device__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAtt
     const int lane = threadIdx.x & 31, hs = p.Heads * D;
     const int *src = p.Proj + (size_t)seq * 4 * hs + m * hs + head0 * D;
     float *rot = g.Rot[m];
-#pragma unroll 8
-    for (int b = 0; b < heads * D / 64; ++b) {
-        const float v0 = (float)__ldcg(src + b * 64 + lane), v1 = (float)__ldcg(src + b * 64 + lane + 32);
-        float r0 = v0, r1 = v1;
-        const int in = (b * 64) & (D - 1);
-        if (m < 2) {
-            const float *rp = p.Rope + (size_t)pos * D + in;
-            const float c = __ldg(rp + lane), sn = __ldg(rp + lane + 32);
-            r0 = __fsub_rn(__fmul_rn(v0, c), __fmul_rn(v1, sn));
-            r1 = __fadd_rn(__fmul_rn(v0, sn), __fmul_rn(v1, c));
+    // up to eight blocks of 64 columns, all loads in flight at once
+    constexpr int PER_HEAD = D / 64;
+    const int blocks = heads * PER_HEAD;
+    float cs[PER_HEAD], sn[PER_HEAD];
+    int v0[8], v1[8];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        if (b < blocks) {
+            v0[b] = __ldcg(src + b * 64 + lane);
+            v1[b] = __ldcg(src + b * 64 + lane + 32);
         }
-        float *w = rot + (b * 64 / D) * (D + 1) + in;
-        w[lane] = r0;
-        w[lane + 32] = r1;
+    }
+    if (m < 2) {
+        const float *rp = p.Rope + (size_t)pos * D;
+#pragma unroll
+        for (int b = 0; b < PER_HEAD; ++b) {
+            cs[b] = __ldg(rp + b * 64 + lane);
+            sn[b] = __ldg(rp + b * 64 + lane + 32);
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        if (b < blocks) {
+            float r0 = (float)v0[b], r1 = (float)v1[b];
+            if (m < 2) {
+                const float x0 = r0, x1 = r1, c = cs[b % PER_HEAD], s = sn[b % PER_HEAD];
+                r0 = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
+                r1 = __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c));
+            }
+            float *w = rot + (b / PER_HEAD) * (D + 4) + (b % PER_HEAD) * 64;
+            w[lane] = r0;
+            w[lane + 32] = r1;
+        }
     }
     __syncwarp();
     const tsa_kv_seq sq = g.Seq;
     if (lane < heads) {
-        const float *w = rot + lane * (D + 1);
+        const float *w = rot + lane * (D + 4);
         float sum2 = 0;
 #pragma unroll 16
-        for (int x = 0; x < D; ++x) {
-            sum2 = __fadd_rn(sum2, __fmul_rn(w[x], w[x]));
+        for (int x = 0; x < D; x += 4) {
+            sum2 = AddSquares(sum2, *reinterpret_cast<const float4 *>(w + x));
         }
         float discr, mult;
         NormScales(sum2, D, &discr, &mult);
@@ -696,13 +680,13 @@ __device__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAtt
     // four columns per lane and step
     for (int i = lane * 4; i < heads * D; i += 128) {
         const int h = i / D;
-        const float *w = rot + h * (D + 1) + (i & (D - 1));
+        const float4 w = *reinterpret_cast<const float4 *>(rot + h * (D + 4) + (i & (D - 1)));
         const float mult = g.Mult[m][h];
         char4 q;
-        q.x = (char)ToInt8Clamp127(__fmul_rn(w[0], mult));
-        q.y = (char)ToInt8Clamp127(__fmul_rn(w[1], mult));
-        q.z = (char)ToInt8Clamp127(__fmul_rn(w[2], mult));
-        q.w = (char)ToInt8Clamp127(__fmul_rn(w[3], mult));
+        q.x = (char)ToInt8Clamp127(__fmul_rn(w.x, mult));
+        q.y = (char)ToInt8Clamp127(__fmul_rn(w.y, mult));
+        q.z = (char)ToInt8Clamp127(__fmul_rn(w.z, mult));
+        q.w = (char)ToInt8Clamp127(__fmul_rn(w.w, mult));
         if (m == 0) {
             *reinterpret_cast<char4 *>(g.Q8 + i) = q;
         } else if (m == 2) {
@@ -734,7 +718,7 @@ __device__ __forceinline__ void AttendRange(const int4 qv, float logitMult, floa
 }
 
 template <int D>
-__device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l, int headGroups, int perGroup)
+__device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
 {
     constexpr int LPH = D / 16, HPW = 32 / LPH; // lanes per head, heads per warp-wide load
     const TStepLayer &layer = p.Layers[l];
@@ -742,60 +726,60 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l, int h
     const int hs = p.Heads * D;
     TAttGroupSmem &g = sm.Att[group];
     int slot = sm.Plan[0].Window == layer.Window ? 0 : 1;
-    bool located = true;
     if (sm.Plan[slot].Window != layer.Window) {
         // not among the last two windows (the same for the whole CTA: the plans change only here)
         __syncthreads();
         slot = sm.Plan[0].Window < 0 ? 0 : sm.Plan[1].Window < 0 ? 1 : l & 1;
         __syncthreads();
         if (tid < 32) {
-            MakeAttPlan(p, layer, headGroups, sm.Plan[slot]);
+            MakeAttPlan(p, layer, sm.Plan[slot]);
         }
         __syncthreads();
-        located = false;
     }
     const TAttPlan &plan = sm.Plan[slot];
     const int head = lane / LPH, sub = lane % LPH; // head inside the group, 16-byte slice of it
     for (int unit = group * gridDim.x + blockIdx.x; unit < plan.Units; unit += PS_GROUPS * gridDim.x) {
-        if (!located) {
-            if (w == 1) {
-                LocateUnit(p, layer, plan, unit, g);
+        if (w == 0) {
+            LocateUnit(p, layer, plan, unit, g);
+        }
+        GroupSync(group);
+        {
+            const int chunk = g.Chunk, pos = g.Pos, head0 = g.HeadGroup * p.PerGroup, heads = min(p.PerGroup, p.Heads - head0);
+            const bool posOk = pos >= 0 && pos < p.RopeLen && pos < p.Capacity;
+            if (tid % 128 == 0 && p.Status && (!posOk || pos + 1 > p.MaxCtx)) {
+                atomicOr(p.Status, kDevBadSpan); // the cache or the rope table is full, or longer than the caller's bound
+            }
+            if (posOk && (chunk == 0 || w == 0)) {
+                // the first chunk's unit also appends the token and leaves the combiner key
+                ProjectHeads<D>(p, layer, g, w, g.SeqIndex, head0, heads, pos);
             }
             GroupSync(group);
-        }
-        located = false; // the next unit was not looked up in advance
-        const int seq = g.SeqIndex, hg = g.HeadGroup, chunk = g.Chunk, chunks = g.Chunks, pos = g.Pos;
-        const int head0 = hg * perGroup, heads = min(perGroup, p.Heads - head0);
-        const bool posOk = pos >= 0 && pos < p.RopeLen && pos < p.Capacity;
-        if (tid % 128 == 0 && p.Status && (!posOk || pos + 1 > p.MaxCtx)) {
-            atomicOr(p.Status, kDevBadSpan); // the cache or the rope table is full, or longer than the caller's bound
-        }
-        if (posOk && (chunk == 0 || w == 0)) {
-            // the first chunk's unit also appends the token and leaves the combiner key
-            ProjectHeads<D>(p, layer, g, w, seq, head0, heads, pos);
-        }
-        GroupSync(group);
-        const int headC = min(head, heads - 1);
-        int j0, j1;
-        KeyRange(pos + 1, layer.Window, &j0, &j1);
-        const int cBeg = j0 + chunk * plan.Chunk, cEnd = min(cBeg + plan.Chunk, j1);
-        const int part = (((cEnd - cBeg) + 3) / 4 + 7) & ~7;
-        const int tBeg = cBeg + w * part, tEnd = min(tBeg + part, cEnd);
-        if (posOk && tBeg < tEnd) {
-            const tsa_kv_seq &sq = g.Seq;
-            const int4 qv = *reinterpret_cast<const int4 *>(g.Q8 + headC * D + sub * 16);
-            const size_t off = (size_t)tBeg * hs + (head0 + headC) * D + sub * 16, soff = (size_t)tBeg * p.Heads + head0 + headC;
-            AttendRange<D>(qv, p.DotScale * INF_VEC_SCALE, layer.Slope, pos, (const int8_t *)sq.k + off, (const int8_t *)sq.v + off, (const float *)sq.kScale + soff,
-                (const float *)sq.vScale + soff, p.Heads, tBeg, tEnd, g.Merge[w][lane]);
-        } else {
+            const int headC = head0 + min(head, heads - 1);
+            int j0, j1;
+            KeyRange(pos + 1, layer.Window, &j0, &j1);
+            const int cBeg = j0 + chunk * plan.Chunk, cEnd = min(cBeg + plan.Chunk, j1);
+            const int part = (((cEnd - cBeg) + 3) / 4 + 7) & ~7;
+            const int tBeg = cBeg + w * part, tEnd = min(tBeg + part, cEnd);
             float *mine = g.Merge[w][lane];
-            mine[0] = -1e30f;
+            if (posOk && tBeg < tEnd) {
+                const int4 qv = *reinterpret_cast<const int4 *>(g.Q8 + (headC - head0) * D + sub * 16);
+                const size_t off = (size_t)tBeg * hs + headC * D + sub * 16, soff = (size_t)tBeg * p.Heads + headC;
+                AttendRange<D>(qv, p.DotScale * INF_VEC_SCALE, layer.Slope, pos, (const int8_t *)g.Seq.k + off, (const int8_t *)g.Seq.v + off,
+                    (const float *)g.Seq.kScale + soff, (const float *)g.Seq.vScale + soff, p.Heads, tBeg, tEnd, mine);
+            } else {
+                mine[0] = -1e30f;
 #pragma unroll
-            for (int i = 1; i < 18; ++i) {
-                mine[i] = 0;
+                for (int i = 1; i < 18; ++i) {
+                    mine[i] = 0;
+                }
             }
         }
         GroupSync(group);
+        // which unit this was, read again: the key loop needs the registers
+        const volatile TAttGroupSmem &vg = g;
+        const int seq = vg.SeqIndex, hg = vg.HeadGroup, chunk = vg.Chunk, chunks = vg.Chunks, pos = vg.Pos;
+        const int head0 = hg * p.PerGroup, heads = min(p.PerGroup, p.Heads - head0);
+        const bool posOk = pos >= 0 && pos < p.RopeLen && pos < p.Capacity;
         // the four warps' shares of the chunk; warp w goes on with columns 4 w .. 4 w + 3 of every lane's slice
         float mAll = g.Merge[0][lane][0];
 #pragma unroll
@@ -826,7 +810,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l, int h
             __threadfence();
             GroupSync(group);
             if (tid % 128 == 0) {
-                const int done = atomicAdd(p.Arrived + seq * headGroups + hg, 1);
+                const int done = atomicAdd(p.Arrived + seq * p.HeadGroups + hg, 1);
                 g.Last = done == chunks - 1;
                 __threadfence();
             }
@@ -834,7 +818,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l, int h
             finish = g.Last != 0;
             if (finish) {
                 if (tid % 128 == 0) {
-                    p.Arrived[seq * headGroups + hg] = 0; // for the next layer
+                    p.Arrived[seq * p.HeadGroups + hg] = 0; // for the next layer
                 }
                 const float *src = p.Partial + ((size_t)(unit - chunk) * HPW + head) * PITCH;
                 mAll = -1e30f;
@@ -889,13 +873,23 @@ template <int D>
 __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
 {
     const int tid = threadIdx.x, hs = p.Heads * D;
-    // a head group is what a warp-wide 16-byte load covers, 512 columns at most; groups of even size, because a group of a few
-    // left-over heads would take as long as a full one
-    const int headGroups = (p.Heads * D + 511) / 512, perGroup = (p.Heads + headGroups - 1) / headGroups;
-    TTileCursor cursor = {0, 0, (int)blockIdx.x, 0};
-    cursor.Settle(p);
-    int tileCount = 0, requested = PS_RING - 1, passed = 0;
-    cursor = RefillRing(p, sm, cursor, 0, requested);
+    if (tid < 5) {
+        int n = 0;
+        for (int phase = 0; phase < tid; ++phase) {
+            const TStepShape &s = p.Shape[phase];
+            for (int item = blockIdx.x; item < s.Tiles * s.Splits; item += gridDim.x) {
+                n += min(s.Per, s.Chunks - (item % s.Splits) * s.Per);
+            }
+        }
+        sm.PhaseBegin[tid] = n;
+    }
+    __syncthreads();
+    for (int i = tid; i < sm.PhaseBegin[4] && i < PS_TABLE; i += PS_THREADS) {
+        sm.Table[i] = ComputeTile(p, i);
+    }
+    __syncthreads();
+    TTileCursor cursor = {0, 0, sm.PhaseBegin[4] > 0 ? 0 : p.LayerCount, 0};
+    RefillRing(p, sm, &cursor);
     // One loop over all phases, so that every piece of code exists once: the kernel's loop has to fit the SM's instruction cache
     // (with the phases written out one after another a quarter of the instruction fetches missed it).
     // Sums are cleared a phase or more after their last reader has passed a barrier and a phase or more before their next writer.
@@ -905,7 +899,7 @@ __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
     while (l < p.LayerCount) {
         if (attention) {
             ZeroSums(l > 0 ? p.Contract : p.Comb, p.NSeq * p.Dim);
-            AttentionPhase<D>(p, sm, l, headGroups, perGroup);
+            AttentionPhase<D>(p, sm, l);
         } else {
             int *done = phase == PH_PROJ ? p.Expand : phase == PH_COMB ? p.Proj : p.Comb;
             const int doneInts = p.NSeq * (phase == PH_PROJ ? p.ReluDim : phase == PH_COMB ? 4 * hs : p.Dim);
@@ -915,16 +909,11 @@ __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
             if (phase == PH_COMB && blockIdx.x == gridDim.x - 1 && tid < p.NSeq) {
                 p.Layers[l].CtxLens[tid] += 1; // the token is in every sequence's cache of this layer
             }
-            ProductPhase(p, sm, l, phase, cursor, tileCount, requested);
+            ProductPhase(p, sm, l, phase, cursor);
         }
-        GridArrive(p, passed);
-        const int refill = PS_RING - 1 - (requested - tileCount);
-        if (refill > 0) {
-            cursor = RefillRing(p, sm, cursor, requested, refill);
-            requested += refill;
-        }
+        GridArrive(p);
+        RefillRing(p, sm, &cursor);
         if (!attention && phase == PH_PROJ) {
-            PrepareAttention(p, sm, l, headGroups, perGroup);
             attention = true;
         } else {
             attention = false;
@@ -933,7 +922,7 @@ __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
                 ++l;
             }
         }
-        if (!GridWait(p, sm, passed)) {
+        if (!GridWait(p, sm)) {
             return;
         }
     }
@@ -963,6 +952,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) InferLayersKernel(const __grid_
         MbarInit(&sm.MmaDone, 1);
         FenceBarrierInit();
         sm.Failed = 0;
+        sm.Passed = 0;
         sm.Plan[0].Window = sm.Plan[1].Window = -1;
     }
     if (tid < 32) {
@@ -1026,6 +1016,10 @@ int InferLayersPersistent(const tsa_infer_model *model, const tsa_kv_seq *const 
     p.Dim = d.dim;
     p.Heads = d.head_count;
     p.HeadSize = D;
+    // a head group is what a warp-wide 16-byte load covers, 512 columns at most; groups of even size, because a group of a few
+    // left-over heads would take as long as a full one
+    p.HeadGroups = (hs + 511) / 512;
+    p.PerGroup = (d.head_count + p.HeadGroups - 1) / p.HeadGroups;
     p.ReluDim = d.relu_dim;
     p.Capacity = capacity;
     p.MaxCtx = maxCtx + 1;
