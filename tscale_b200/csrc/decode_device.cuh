@@ -64,29 +64,31 @@ __device__ __forceinline__ int Dp2aHiUS(uint32_t a, uint32_t b, int c)
 }
 
 // Tokens [tBeg, tEnd) for this lane's 16-byte slice of its head: kp, vp, ksp, vsp point at token tBeg, qv is the query's slice.
-// Keeps UNROLL tokens of K and V in flight; online softmax in (m, l, acc).
+// Keeps UNROLL tokens of K and V in flight; online softmax in (m, l, acc).  A warp whose heads take no more than half of its lanes
+// works on `perLoad` tokens at a time: this lane takes token `tokenOff` of each such group, and the lanes' results are merged by the
+// caller (a lane that saw no token keeps m = -1e30).
 template <int D, int UNROLL, bool COHERENT, class TScale>
 __device__ __forceinline__ void AttendTokens(const int4 qv, float logitMult, float slope, int cur, const int4 *kp, const int4 *vp, const TScale *ksp,
-    const TScale *vsp, int H, int tBeg, int tEnd, float &m, float &l, float (&acc)[16])
+    const TScale *vsp, int H, int tBeg, int tEnd, int perLoad, int tokenOff, float &m, float &l, float (&acc)[16])
 {
     constexpr int LPH = D / 16;     // lanes per head
     const int rowInt4 = H * D / 16; // int4 words per token row
-    for (int tBase = tBeg; tBase < tEnd; tBase += UNROLL) {
+    for (int tBase = tBeg; tBase < tEnd; tBase += UNROLL * perLoad) {
         int4 kv[UNROLL], vv[UNROLL];
         float ks[UNROLL], vs[UNROLL];
         const int cnt = tEnd - tBase; // tokens left, >= 1
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
-            const int tt = u < cnt ? u : cnt - 1;
+            const int tt = min(u * perLoad + tokenOff, cnt - 1);
             kv[u] = LoadRow<COHERENT>(kp + tt * rowInt4);
             vv[u] = LoadRow<COHERENT>(vp + tt * rowInt4);
             ks[u] = LoadScaleT<COHERENT>(ksp + tt * H);
             vs[u] = LoadScaleT<COHERENT>(vsp + tt * H);
         }
-        kp += UNROLL * rowInt4;
-        vp += UNROLL * rowInt4;
-        ksp += UNROLL * H;
-        vsp += UNROLL * H;
+        kp += UNROLL * perLoad * rowInt4;
+        vp += UNROLL * perLoad * rowInt4;
+        ksp += UNROLL * perLoad * H;
+        vsp += UNROLL * perLoad * H;
         float z[UNROLL];
         float cm = m;
 #pragma unroll
@@ -100,8 +102,8 @@ __device__ __forceinline__ void AttendTokens(const int4 qv, float logitMult, flo
                 dot += __shfl_xor_sync(0xffffffffu, dot, o);
             }
             // same association as the reference: ((dot * kScale) * attDotScale) * qScale - slope * dist
-            const float zz = (float)dot * ks[u] * logitMult - slope * (float)(cur - (tBase + u));
-            z[u] = (u < cnt) ? zz : -1e30f;
+            const float zz = (float)dot * ks[u] * logitMult - slope * (float)(cur - (tBase + u * perLoad + tokenOff));
+            z[u] = (u * perLoad + tokenOff < cnt) ? zz : -1e30f;
             cm = fmaxf(cm, z[u]);
         }
         if (cm != m) {

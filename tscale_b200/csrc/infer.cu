@@ -261,7 +261,7 @@ TInferBuffers CarveInferBuffers(const tsa_infer_model *m, int nSeq, void *base)
 {
     const tsa_infer_dims &d = m->dims;
     const size_t hs = (size_t)d.head_count * d.head_dim;
-    const int perGroup = 512 / d.head_dim, headGroups = (d.head_count + perGroup - 1) / perGroup; // heads of a warp-wide 16-byte load
+    const int perGroup = AttGroupHeads(d.head_count, d.head_dim), headGroups = (d.head_count + perGroup - 1) / perGroup;
     TInferBuffers b;
     size_t off = 0;
     auto take = [&](size_t bytes) {

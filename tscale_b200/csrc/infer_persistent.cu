@@ -61,6 +61,7 @@ struct TStepParams {
     int LayerCount, FirstSource;
     int NSeq, Dim, Heads, HeadSize, ReluDim, Capacity, MaxCtx, RopeLen;
     int HeadGroups, PerGroup;     // groups of heads the attention works in, heads of a group (the last may have fewer)
+    int PerLoad;                  // tokens a warp-wide load covers
     const int *Labels;
     int LabelsPerSeq, LabelCount;
     const int8_t *Embed;
@@ -588,13 +589,13 @@ __device__ __noinline__ void LocateUnit(const TStepParams &p, const TStepLayer &
     const unsigned at0 = __ballot_sync(0xffffffffu, lane < p.NSeq && plan.Base[lane] <= unit);
     const unsigned at1 = __ballot_sync(0xffffffffu, lane + 32 < p.NSeq && plan.Base[lane + 32] <= unit);
     const int seq = at1 ? 63 - __clz(at1) : 31 - __clz(at0);
-    const int chunks = max(1, (plan.Keys[seq] + plan.Chunk - 1) / plan.Chunk), rel = unit - plan.Base[seq], hg = rel / chunks;
+    const int chunks = max(1, (plan.Keys[seq] + plan.Chunk - 1) / plan.Chunk), rel = unit - plan.Base[seq], chunk = rel / p.HeadGroups;
     if (lane == 0) {
         g.Pos = layer.CtxLens[seq];
         g.Seq = layer.Seqs[seq];
         g.SeqIndex = seq;
-        g.HeadGroup = hg;
-        g.Chunk = rel - hg * chunks;
+        g.HeadGroup = rel - chunk * p.HeadGroups;
+        g.Chunk = chunk;
         g.Chunks = chunks;
     }
     __syncwarp();
@@ -619,7 +620,7 @@ __device__ __forceinline__ void StoreKvProduct(int8_t *kv, int headSize, int z, 
 // One matrix (m: qk, qv, k, v) of a head group of one sequence, by one warp: rope on qk and qv (ReferenceApplyRope,
 // code/gpt/att/rope.cpp:28-46), NormalizeState per head, codes into shared memory (qk, k) or the sequence's cache (qv, v).
 template <int D>
-__device__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAttGroupSmem &g, int m, int seq, int head0, int heads, int pos)
+__device__ __noinline__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAttGroupSmem &g, int m, int seq, int head0, int heads, int pos)
 {
     const int lane = threadIdx.x & 31, hs = p.Heads * D;
     const int *src = p.Proj + (size_t)seq * 4 * hs + m * hs + head0 * D;
@@ -701,14 +702,14 @@ __device__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAtt
 // this lane's share of a range of tokens, into the merge buffer
 template <int D>
 __device__ __forceinline__ void AttendRange(const int4 qv, float logitMult, float slope, int pos, const int8_t *k, const int8_t *v, const float *ks, const float *vs,
-    int heads, int tBeg, int tEnd, float *mine)
+    int heads, int tBeg, int tEnd, int perLoad, int tokenOff, float *mine)
 {
     float m = -1e30f, l = 0, acc[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         acc[i] = 0;
     }
-    AttendTokens<D, 8, true>(qv, logitMult, slope, pos, reinterpret_cast<const int4 *>(k), reinterpret_cast<const int4 *>(v), ks, vs, heads, tBeg, tEnd, m, l, acc);
+    AttendTokens<D, 8, true>(qv, logitMult, slope, pos, reinterpret_cast<const int4 *>(k), reinterpret_cast<const int4 *>(v), ks, vs, heads, tBeg, tEnd, perLoad, tokenOff, m, l, acc);
     mine[0] = m;
     mine[1] = l;
 #pragma unroll
@@ -720,7 +721,7 @@ __device__ __forceinline__ void AttendRange(const int4 qv, float logitMult, floa
 template <int D>
 __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
 {
-    constexpr int LPH = D / 16, HPW = 32 / LPH; // lanes per head, heads per warp-wide load
+    constexpr int LPH = D / 16; // lanes per head
     const TStepLayer &layer = p.Layers[l];
     const int tid = threadIdx.x, lane = tid & 31, group = tid >> 7, w = (tid >> 5) & 3;
     const int hs = p.Heads * D;
@@ -737,7 +738,10 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
         __syncthreads();
     }
     const TAttPlan &plan = sm.Plan[slot];
-    const int head = lane / LPH, sub = lane % LPH; // head inside the group, 16-byte slice of it
+    // this lane's token of a load, head inside the group, 16-byte slice of the head; lanes past the last token repeat the first's
+    const int tokenLanes = p.PerGroup * LPH;
+    const int tokenOff = lane / tokenLanes < p.PerLoad ? lane / tokenLanes : 0;
+    const int head = lane % tokenLanes / LPH, sub = lane % LPH;
     for (int unit = group * gridDim.x + blockIdx.x; unit < plan.Units; unit += PS_GROUPS * gridDim.x) {
         if (w == 0) {
             LocateUnit(p, layer, plan, unit, g);
@@ -758,14 +762,14 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
             int j0, j1;
             KeyRange(pos + 1, layer.Window, &j0, &j1);
             const int cBeg = j0 + chunk * plan.Chunk, cEnd = min(cBeg + plan.Chunk, j1);
-            const int part = (((cEnd - cBeg) + 3) / 4 + 7) & ~7;
+            const int round = 8 * p.PerLoad - 1, part = (((cEnd - cBeg) + 3) / 4 + round) & ~round;
             const int tBeg = cBeg + w * part, tEnd = min(tBeg + part, cEnd);
             float *mine = g.Merge[w][lane];
             if (posOk && tBeg < tEnd) {
                 const int4 qv = *reinterpret_cast<const int4 *>(g.Q8 + (headC - head0) * D + sub * 16);
                 const size_t off = (size_t)tBeg * hs + headC * D + sub * 16, soff = (size_t)tBeg * p.Heads + headC;
                 AttendRange<D>(qv, p.DotScale * INF_VEC_SCALE, layer.Slope, pos, (const int8_t *)g.Seq.k + off, (const int8_t *)g.Seq.v + off,
-                    (const float *)g.Seq.kScale + soff, (const float *)g.Seq.vScale + soff, p.Heads, tBeg, tEnd, mine);
+                    (const float *)g.Seq.kScale + soff, (const float *)g.Seq.vScale + soff, p.Heads, tBeg, tEnd, p.PerLoad, tokenOff, mine);
             } else {
                 mine[0] = -1e30f;
 #pragma unroll
@@ -780,16 +784,18 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
         const int seq = vg.SeqIndex, hg = vg.HeadGroup, chunk = vg.Chunk, chunks = vg.Chunks, pos = vg.Pos;
         const int head0 = hg * p.PerGroup, heads = min(p.PerGroup, p.Heads - head0);
         const bool posOk = pos >= 0 && pos < p.RopeLen && pos < p.Capacity;
-        // the four warps' shares of the chunk; warp w goes on with columns 4 w .. 4 w + 3 of every lane's slice
-        float mAll = g.Merge[0][lane][0];
-#pragma unroll
-        for (int k = 1; k < 4; ++k) {
-            mAll = fmaxf(mAll, g.Merge[k][lane][0]);
+        // the shares of the chunk of the four warps and of the tokens of a load; warp w goes on with columns 4 w .. 4 w + 3 of every
+        // lane's slice
+        const int first = lane % tokenLanes, shares = 4 * p.PerLoad;
+        auto shareOf = [&](int k) { return (const float *)g.Merge[k & 3][first + (k >> 2) * tokenLanes]; };
+        float mAll = -1e30f;
+        for (int k = 0; k < shares; k += 4) {
+            mAll = fmaxf(fmaxf(mAll, fmaxf(shareOf(k)[0], shareOf(k + 1)[0])), fmaxf(shareOf(k + 2)[0], shareOf(k + 3)[0]));
         }
         float lAll = 0, val[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float *other = g.Merge[k][lane];
+#pragma unroll 4
+        for (int k = 0; k < shares; ++k) {
+            const float *other = shareOf(k);
             const float f = exp2f(other[0] - mAll);
             lAll = fmaf(f, other[1], lAll);
 #pragma unroll
@@ -802,9 +808,11 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
         if (chunks > 1) {
             // partials to L2; the unit that arrives last merges all of the row's
             constexpr int PITCH = D + 4;
-            float *dst = p.Partial + ((size_t)unit * HPW + head) * PITCH;
-            __stcg(reinterpret_cast<float4 *>(dst + z), make_float4(val[0], val[1], val[2], val[3]));
-            if (z == 0) {
+            float *dst = p.Partial + ((size_t)unit * p.PerGroup + head) * PITCH;
+            if (lane < tokenLanes) {
+                __stcg(reinterpret_cast<float4 *>(dst + z), make_float4(val[0], val[1], val[2], val[3]));
+            }
+            if (z == 0 && lane < tokenLanes) {
                 __stcg(reinterpret_cast<float2 *>(dst + D), make_float2(mAll, lAll));
             }
             __threadfence();
@@ -820,17 +828,18 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
                 if (tid % 128 == 0) {
                     p.Arrived[seq * p.HeadGroups + hg] = 0; // for the next layer
                 }
-                const float *src = p.Partial + ((size_t)(unit - chunk) * HPW + head) * PITCH;
+                const float *src = p.Partial + ((size_t)(unit - chunk * p.HeadGroups) * p.PerGroup + head) * PITCH;
+                const size_t step = (size_t)p.HeadGroups * p.PerGroup * PITCH;
                 mAll = -1e30f;
 #pragma unroll 8
                 for (int c = 0; c < chunks; ++c) {
-                    mAll = fmaxf(mAll, __ldcg(src + (size_t)c * HPW * PITCH + D));
+                    mAll = fmaxf(mAll, __ldcg(src + c * step + D));
                 }
                 lAll = 0;
                 val[0] = val[1] = val[2] = val[3] = 0;
 #pragma unroll 8
                 for (int c = 0; c < chunks; ++c) {
-                    const float *q = src + (size_t)c * HPW * PITCH;
+                    const float *q = src + c * step;
                     const float2 ml = __ldcg(reinterpret_cast<const float2 *>(q + D));
                     const float4 v = __ldcg(reinterpret_cast<const float4 *>(q + z));
                     const float f = exp2f(ml.x - mAll);
@@ -842,7 +851,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
                 }
             }
         }
-        if (finish && head < heads) {
+        if (finish && head < heads && lane < tokenLanes) {
             // the sink has logit 0 (softMax.Add(0), cpu_infer.cpp:444)
             const float mF = fmaxf(mAll, 0.0f), f = exp2f(mAll - mF), lF = exp2f(-mF) + f * lAll;
 #pragma unroll
@@ -1016,10 +1025,9 @@ int InferLayersPersistent(const tsa_infer_model *model, const tsa_kv_seq *const 
     p.Dim = d.dim;
     p.Heads = d.head_count;
     p.HeadSize = D;
-    // a head group is what a warp-wide 16-byte load covers, 512 columns at most; groups of even size, because a group of a few
-    // left-over heads would take as long as a full one
-    p.HeadGroups = (hs + 511) / 512;
-    p.PerGroup = (d.head_count + p.HeadGroups - 1) / p.HeadGroups;
+    p.PerGroup = AttGroupHeads(d.head_count, D);
+    p.HeadGroups = (d.head_count + p.PerGroup - 1) / p.PerGroup;
+    p.PerLoad = 512 / D / p.PerGroup;
     p.ReluDim = d.relu_dim;
     p.Capacity = capacity;
     p.MaxCtx = maxCtx + 1;
