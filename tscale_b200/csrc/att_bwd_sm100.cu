@@ -10,10 +10,10 @@
 // vectors are first widened to bf16 (exact: every int8 and e4m3 value is a bf16 number) into scratch, dO is taken
 // as bf16, and all GEMMs run as kind::f16 with dS and P handed to the tensor core as bf16: one pass, no row maximum.
 //
-// One kernel, two modes, the same tile engine:
-//   mode dQ     : CTA = head x 128 query rows (R1 = Q, R2 = dO), loop over key tiles (C1 = K, C2 = V) of the row
+// One kernel, two modes, the same tile engine; a work item is a head and 128 rows:
+//   mode dQ     : item = head x 128 query rows (R1 = Q, R2 = dO), loop over key tiles (C1 = K, C2 = V) of the row
 //                 spans:  S = R1 C1^T, dP = R2 C2^T, A1 = dS * sk_j,                  dQ  += A1 C1
-//   mode dK,dV  : CTA = head x 128 key rows  (R1 = K, R2 = V ), loop over query tiles (C1 = Q, C2 = dO) of the
+//   mode dK,dV  : item = head x 128 key rows (R1 = K, R2 = V ), loop over query tiles (C1 = Q, C2 = dO) of the
 //                 transposed spans:  S^T = R1 C1^T, dP^T = R2 C2^T, A1 = dS * sq_i, A2 = P,  dK += A1 C1, dV += A2 C2
 // Tensor memory (512 columns): [0,128) S, [128,256) dP, [256,256+D) first output, [256+D,256+2D) second output.
 // A1 / A2 (bf16, two per column) are written back over the S / dP columns the writing thread has already consumed.
@@ -24,7 +24,13 @@
 // half (its output products, then its S / dP of the next tile) run.  Each half has its own MMA-issuing warp (an elected
 // lane of a converged warp issues, in grouped asm blocks); the two take turns block by block, so one does its waits
 // while the other issues and the accumulation order is fixed; one more warp issues the TMA copies.  Row tiles stay in shared memory; column tiles stream through a ring of
-// half stages (64 rows of C1 and C2), freed per half.  All waits are bounded; a failed wait is carried to the
+// half stages (64 rows of C1 and C2), freed per half.
+//
+// Persistent: one CTA per SM (all of its tensor memory and most of its shared memory) takes items from a counter, long ones first,
+// and the pipelines run on across items: the next item's row tiles are loaded when the present one's last score products have retired,
+// its first scores run while the arithmetic warps still drain the outputs, and those warps look up the next item's spans while the
+// last output products run.  With a CTA per item every item paid 4.4 K clocks of start-up and 7 K from its last weights to the end
+// of the CTA, half of the 22 K that an item of a window-256 layer took.  All waits are bounded; a failed wait is carried to the
 // arithmetic threads' next named barrier so they leave together.
 #include "att_sm100_common.cuh"
 
@@ -36,15 +42,6 @@ constexpr int BWD_LOAD_WARP = BWD_CTRL_WARP + 2;
 constexpr int BWD_THREADS = BWD_ARITH_THREADS + 96;
 constexpr uint32_t BWD_TMEM_COLS = 512;
 constexpr uint32_t BWD_S_COL = 0, BWD_DP_COL = 128, BWD_OUT_COL = 256;
-
-// Phase trace for profiling builds (-DTSA_BWD_TRACE): clock64() per tile from lane 0 of the first warp of each half
-// and of the control warp of one CTA; tsa_debug_trace_bwd copies the buffer out.
-#ifdef TSA_BWD_TRACE
-__device__ long long g_traceBwd[4096];
-#define TRB(T, e) do { if (traceOn && (T) < 64) g_traceBwd[(T) * 16 + (e)] = clock64(); } while (0)
-#else
-#define TRB(T, e) do { } while (0)
-#endif
 
 struct TBwdParams {
     int HeadCount;
@@ -60,7 +57,11 @@ struct TBwdParams {
     float Slope;
     float GradMult;
     P2D<char> Out1, Out2;
+    int WideStores;   // the outputs' rows are 32-byte aligned
     int GradDtype;
+    int Items;        // row tiles x heads
+    int Ascending;    // order of the row tiles: the long ones come first
+    int *Counter;     // work-item counter, zero at launch
     int *Status;
 };
 
@@ -85,12 +86,16 @@ struct TBwdMisc {
     float ColB[2][TILE_ROWS]; // dQ: sv_j c ln2;  dK/dV: -delta_i c ln2
     int Abort;
     int Turn;                 // issue blocks handed to the tensor pipe so far: control warp h issues the blocks with index = h (mod 2)
+    uint64_t ItemFull[2];     // loader -> all: Item[] holds the next work item (-1: none left)
+    uint64_t ItemEmpty[2];    // all -> loader: the record has been read
+    int Item[2];
     uint64_t BarR;            // TMA: row tiles landed
+    uint64_t BarREmpty;       // MMA warps -> loader: the item's last score products have retired
     uint64_t BarFull[8];      // TMA: half stage (64 rows of C1 and C2) landed
     uint64_t BarEmpty[8];     // MMA warp -> loader: the half stage's output products have retired
     uint64_t BarS[2];         // control -> half h: S and dP columns of the half ready
     uint64_t BarP[2];         // half h -> control: A1 / A2 of the half written (8 warp arrivals)
-    uint64_t BarDone;         // control -> all: every output product has retired
+    uint64_t BarOut;          // MMA warps -> arithmetic: every output product of the item has retired
     uint32_t TmemBase;
 };
 static_assert(sizeof(TBwdMisc) <= 8192, "misc block");
@@ -125,8 +130,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
     TBwdMisc &misc = *reinterpret_cast<TBwdMisc *>(smem + SM::MISC_OFF);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int head = blockIdx.y;
-    const int rowTile = gridDim.x - 1 - blockIdx.x;
+    // item -> row tile and head: heads side by side, long row tiles first (the late ones of the mask, the early ones of its transpose)
+    auto locate = [&](int item, int &rowTile, int &head) {
+        const int k = item / p.HeadCount;
+        head = item - k * p.HeadCount;
+        rowTile = p.Ascending ? k : p.Items / p.HeadCount - 1 - k;
+    };
 
     if ((SmemAddr(smem) & 1023u) != 0) {
         if (tid == 0 && p.Status) {
@@ -135,7 +144,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
         return;
     }
     if (tid == 0) {
+        for (int s = 0; s < 2; ++s) {
+            MbarInit(&misc.ItemFull[s], 1);
+            MbarInit(&misc.ItemEmpty[s], BWD_ARITH_THREADS / 32 + 2);
+        }
         MbarInit(&misc.BarR, 1);
+        MbarInit(&misc.BarREmpty, 2);
         for (int s = 0; s < HSTAGES; ++s) {
             MbarInit(&misc.BarFull[s], 1);
             MbarInit(&misc.BarEmpty[s], 1);
@@ -144,7 +158,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
             MbarInit(&misc.BarS[h], 1);
             MbarInit(&misc.BarP[h], BWD_ARITH_THREADS / 32);
         }
-        MbarInit(&misc.BarDone, 2);
+        MbarInit(&misc.BarOut, 2);
         misc.Abort = 0;
         misc.Turn = 0;
         FenceBarrierInit();
@@ -158,67 +172,94 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
     TcFenceAfter();
     const uint32_t tmem = misc.TmemBase;
     const int *abortFlag = &misc.Abort;
-#ifdef TSA_BWD_TRACE
-    const bool traceOn = blockIdx.x == 40 && blockIdx.y == 3 && lane == 0 && (warp == 0 || warp == 8 || warp == BWD_CTRL_WARP || warp == BWD_CTRL_WARP + 1);
-#endif
-
-    // The row tiles depend only on the CTA's coordinates: their copies start before the span lookup (two dependent global
-    // loads) instead of behind it.
-    if (warp == BWD_LOAD_WARP && lane == 0) {
-        PrefetchTensorMap(&tmR1);
-        PrefetchTensorMap(&tmR2);
-        // every tensor map has boxes of 64 rows x 64 elements (128 bytes): a row tile is two boxes per block
-        auto loadTile = [&](uint8_t *dst, const CUtensorMap *tm, int rowBase, uint64_t *bar) {
-#pragma unroll
-            for (int kb = 0; kb < KBLOCKS; ++kb) {
-                TmaLoad2D(dst + kb * BLOCK_BYTES, tm, head * D + kb * 64, rowBase, bar);
-                TmaLoad2D(dst + kb * BLOCK_BYTES + HALF_BLOCK_BYTES, tm, head * D + kb * 64, rowBase + 64, bar);
-            }
-        };
-        MbarExpectTx(&misc.BarR, 2 * SM::TILE_BYTES);
-        loadTile(sR1, &tmR1, rowTile * TILE_ROWS, &misc.BarR);
-        loadTile(sR2, &tmR2, rowTile * TILE_ROWS, &misc.BarR);
+    // The dK/dV pass reads nothing that the dQ pass in front of it writes: its CTAs move in as the dQ pass's leave.  They start only
+    // when every dQ CTA has passed the wait here, so what the kernels before that wrote is complete and visible; the wait at the end
+    // keeps the order for whatever comes behind.
+    if (!MODE_DKV) {
+        PdlWait();
     }
-
-    TTileIter cur;
-    cur.Init(p.Spans, p.SpanPtr, p.LenAttTiles, rowTile, p.Rows);
+    PdlTrigger();
 
     if (warp == BWD_LOAD_WARP) {
-        // ---------------------------------------------------------------- loader warp: every TMA copy
-        if (lane == 0 && !cur.Valid) {
-            WaitBar(&misc.BarR, 0); // a CTA without column tiles: the row tiles must have landed before it ends
-        }
-        if (lane == 0 && cur.Valid) {
+        // ---------------------------------------------------------------- loader warp: the work items and every TMA copy
+        if (lane == 0) {
+            PrefetchTensorMap(&tmR1);
+            PrefetchTensorMap(&tmR2);
             PrefetchTensorMap(&tmC1);
             PrefetchTensorMap(&tmC2);
-            auto loadHalf = [&](uint8_t *dst, const CUtensorMap *tm, int rowBase, uint64_t *bar) {
-#pragma unroll
-                for (int kb = 0; kb < KBLOCKS; ++kb) {
-                    TmaLoad2D(dst + kb * HALF_BLOCK_BYTES, tm, head * D + kb * 64, rowBase, bar);
-                }
-            };
-            int g = 0; // half stages requested
+            int g = 0, rCount = 0; // half stages / row tiles requested
             bool failed = false;
-            for (TTileIter prod = cur; prod.Valid && !failed; prod.Advance()) {
-#pragma unroll 1
-                for (int h = 0; h < 2; ++h, ++g) {
-                    const int slot = g % HSTAGES;
-                    if (g >= HSTAGES && !WaitBarA(&misc.BarEmpty[slot], ((g / HSTAGES) - 1) & 1, abortFlag)) {
-                        failed = true;
-                        *(volatile int *)&misc.Abort = 1;
-                        if (p.Status) {
-                            atomicOr(p.Status, kDevTimeoutMma);
-                        }
-                        break;
+            auto wait = [&](uint64_t *bar, uint32_t parity) {
+                if (!WaitBarA(bar, parity, abortFlag)) {
+                    failed = true;
+                    *(volatile int *)&misc.Abort = 1;
+                    if (p.Status) {
+                        atomicOr(p.Status, kDevTimeoutMma);
                     }
-                    MbarExpectTx(&misc.BarFull[slot], 2 * SM::HALF_TILE_BYTES);
-                    loadHalf(sC + slot * 2 * SM::HALF_TILE_BYTES, &tmC1, prod.J0 + 64 * h, &misc.BarFull[slot]);
-                    loadHalf(sC + slot * 2 * SM::HALF_TILE_BYTES + SM::HALF_TILE_BYTES, &tmC2, prod.J0 + 64 * h, &misc.BarFull[slot]);
+                }
+                return !failed;
+            };
+            int item = blockIdx.x;
+            for (int n = 0;; ++n) {
+                if (n >= 2 && !wait(&misc.ItemEmpty[n & 1], ((n >> 1) - 1) & 1)) {
+                    break;
+                }
+                *(volatile int *)&misc.Item[n & 1] = item < p.Items ? item : -1;
+                MbarArrive(&misc.ItemFull[n & 1]);
+                if (item >= p.Items) {
+                    break;
+                }
+                const int next = gridDim.x + atomicAdd(p.Counter, 1); // in flight while this item is set up
+                int rowTile, head;
+                locate(item, rowTile, head);
+                item = next;
+                TTileIter prod;
+                prod.Init(p.Spans, p.SpanPtr, p.LenAttTiles, rowTile, p.Rows);
+                if (!prod.Valid) {
+                    continue;
+                }
+                if (rCount > 0 && !wait(&misc.BarREmpty, (rCount - 1) & 1)) {
+                    break;
+                }
+                // every tensor map has boxes of 64 rows x 64 elements (128 bytes): a row tile is two boxes per block
+                auto loadTile = [&](uint8_t *dst, const CUtensorMap *tm) {
+#pragma unroll
+                    for (int kb = 0; kb < KBLOCKS; ++kb) {
+                        TmaLoad2D(dst + kb * BLOCK_BYTES, tm, head * D + kb * 64, rowTile * TILE_ROWS, &misc.BarR);
+                        TmaLoad2D(dst + kb * BLOCK_BYTES + HALF_BLOCK_BYTES, tm, head * D + kb * 64, rowTile * TILE_ROWS + 64, &misc.BarR);
+                    }
+                };
+                MbarExpectTx(&misc.BarR, 2 * SM::TILE_BYTES);
+                loadTile(sR1, &tmR1);
+                loadTile(sR2, &tmR2);
+                ++rCount;
+                auto loadHalf = [&](uint8_t *dst, const CUtensorMap *tm, int rowBase, uint64_t *bar) {
+#pragma unroll
+                    for (int kb = 0; kb < KBLOCKS; ++kb) {
+                        TmaLoad2D(dst + kb * HALF_BLOCK_BYTES, tm, head * D + kb * 64, rowBase, bar);
+                    }
+                };
+                for (; prod.Valid && !failed; prod.Advance()) {
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h, ++g) {
+                        const int slot = g % HSTAGES;
+                        if (g >= HSTAGES && !wait(&misc.BarEmpty[slot], ((g / HSTAGES) - 1) & 1)) {
+                            break;
+                        }
+                        MbarExpectTx(&misc.BarFull[slot], 2 * SM::HALF_TILE_BYTES);
+                        loadHalf(sC + slot * 2 * SM::HALF_TILE_BYTES, &tmC1, prod.J0 + 64 * h, &misc.BarFull[slot]);
+                        loadHalf(sC + slot * 2 * SM::HALF_TILE_BYTES + SM::HALF_TILE_BYTES, &tmC2, prod.J0 + 64 * h, &misc.BarFull[slot]);
+                    }
+                }
+                if (failed) {
+                    break;
                 }
             }
-            if (*(volatile int *)&misc.Abort) {
+            if (failed || *(volatile int *)&misc.Abort) {
                 // drain copies that were requested, so none lands after the CTA is gone
-                WaitBar(&misc.BarR, 0);
+                if (rCount > 0) {
+                    WaitBar(&misc.BarR, (rCount - 1) & 1);
+                }
                 for (int t = max(0, g - HSTAGES); t < g; ++t) {
                     WaitBar(&misc.BarFull[t % HSTAGES], (t / HSTAGES) & 1);
                 }
@@ -232,7 +273,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
         // clear before their first hand-over so that every output product accumulates, whichever warp comes first; while
         // one warp is between two issue blocks (waits, votes, loop code) the other keeps the tensor pipe fed.
         const int h = warp - BWD_CTRL_WARP;
-        if (cur.Valid) {
+        {
             const uint32_t sR1a = SmemAddr(sR1), sR2a = SmemAddr(sR2), sCa = SmemAddr(sC);
             bool failed = false;
             // descriptors of a K-major tile and of an MN-major half column tile without the address (added per use, in
@@ -264,9 +305,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                     }
                 }
             };
-            if (!__all_sync(0xffffffffu, WaitBarA(&misc.BarR, 0, abortFlag))) {
-                fail(kDevTimeoutTma);
-            }
             // Order inside a half: out(h, it-1) then scores(h, it): the outputs read the half's A columns before the next
             // scores overwrite them, and a thread's products run in order.  The warp never waits for its own MMAs; the
             // loader refills a half stage when the commit made after its output products completes.  Half (it, h) lives
@@ -299,44 +337,77 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                     *(volatile int *)&misc.Turn = index + 1;
                 }
             };
-            int it = 0;
-            TTileIter ctl = cur;
-            for (; ctl.Valid && !failed; ++it, ctl.Advance()) {
-                const int g = 2 * it + h;
-                const int slot = g % HSTAGES, prevSlot = (g - 2 + HSTAGES) % HSTAGES;
-                TRB(it, 8 + 4 * h);
-                if (!__all_sync(0xffffffffu, WaitBarA(&misc.BarFull[slot], (g / HSTAGES) & 1, abortFlag))) {
+            int it = 0, items = 0; // tiles and items with tiles so far
+            bool prevLast = false; // the tile whose output products are still to come is its item's last
+            for (int n = 0; !failed; ++n) {
+                if (!__all_sync(0xffffffffu, WaitBarA(&misc.ItemFull[n & 1], (n >> 1) & 1, abortFlag))) {
                     fail(kDevTimeoutTma);
                     break;
                 }
-                if (it > 0) {
-                    if (!__all_sync(0xffffffffu, WaitBarSleep<20>(&misc.BarP[h], (it - 1) & 1, abortFlag))) {
+                const int item = *(volatile int *)&misc.Item[n & 1];
+                __syncwarp();
+                if (lane == 0) {
+                    MbarArrive(&misc.ItemEmpty[n & 1]);
+                }
+                if (item < 0) {
+                    break;
+                }
+                int rowTile, head;
+                locate(item, rowTile, head);
+                TTileIter ctl;
+                ctl.Init(p.Spans, p.SpanPtr, p.LenAttTiles, rowTile, p.Rows);
+                if (!ctl.Valid) {
+                    continue;
+                }
+                if (!__all_sync(0xffffffffu, WaitBarA(&misc.BarR, items & 1, abortFlag))) {
+                    fail(kDevTimeoutTma);
+                    break;
+                }
+                ++items;
+                for (; ctl.Valid && !failed; ++it) {
+                    const int g = 2 * it + h;
+                    const int slot = g % HSTAGES, prevSlot = (g - 2 + HSTAGES) % HSTAGES;
+                    ctl.Advance();
+                    const bool last = !ctl.Valid;
+                    if (!__all_sync(0xffffffffu, WaitBarA(&misc.BarFull[slot], (g / HSTAGES) & 1, abortFlag))) {
+                        fail(kDevTimeoutTma);
+                        break;
+                    }
+                    if (it > 0) {
+                        if (!__all_sync(0xffffffffu, WaitBarSleep<20>(&misc.BarP[h], (it - 1) & 1, abortFlag))) {
+                            fail(kDevTimeoutMma);
+                            break;
+                        }
+                    }
+                    if (!__all_sync(0xffffffffu, takeTurn(g))) {
                         fail(kDevTimeoutMma);
                         break;
                     }
-                }
-                if (!__all_sync(0xffffffffu, takeTurn(g))) {
-                    fail(kDevTimeoutMma);
-                    break;
-                }
-                TcFenceAfter();
-                TRB(it, 9 + 4 * h);
-                if (ElectOne()) {
-                    if (it > 0) {
-                        issueOutputs(prevSlot, h);
-                        MmaCommit(&misc.BarEmpty[prevSlot]);
+                    TcFenceAfter();
+                    if (ElectOne()) {
+                        if (it > 0) {
+                            issueOutputs(prevSlot, h);
+                            MmaCommit(&misc.BarEmpty[prevSlot]);
+                            if (prevLast) {
+                                MmaCommit(&misc.BarOut);
+                            }
+                        }
+                        issueScores(slot, h);
+                        MmaCommit(&misc.BarS[h]);
+                        if (last) {
+                            MmaCommit(&misc.BarREmpty);
+                        }
                     }
-                    issueScores(slot, h);
-                    MmaCommit(&misc.BarS[h]);
+                    passTurn(g);
+                    prevLast = last;
                 }
-                passTurn(g);
-                TRB(it, 10 + 4 * h);
             }
             if (!failed && it > 0) {
                 if (__all_sync(0xffffffffu, WaitBarSleep<20>(&misc.BarP[h], (it - 1) & 1, abortFlag) && takeTurn(2 * it + h))) {
                     TcFenceAfter();
                     if (ElectOne()) {
                         issueOutputs((2 * (it - 1) + h) % HSTAGES, h);
+                        MmaCommit(&misc.BarOut);
                     }
                     passTurn(2 * it + h);
                 } else {
@@ -344,38 +415,20 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                 }
             }
             __syncwarp();
-            if (ElectOne()) {
-                MmaCommit(&misc.BarDone);
-            }
         }
         __syncwarp();
     } else {
         // ---------------------------------------------------------------- arithmetic warps
         const int quarter = tid >> 7;          // 16-column block of each 64-column half
         const int r = tid & (TILE_ROWS - 1);
-        const int row = rowTile * TILE_ROWS + r;
         const uint32_t tLane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-        const bool rowOk = row < p.Rows;
         const float g = p.GlobalScale ? *p.GlobalScale : 1.0f;
         const float cg = p.C * g;
         const float dsMult = cg * kLog2;
+        int rowTile = 0, head = 0, row = 0;
+        TTileIter cur;
         // per-row constants.  dQ pass: the row is a query (scale sq, lse, delta); dK/dV pass: the row is a key (sk, sv)
-        float rowScale = 0, rowLse = 0, rowDelta = 0, rowSv = 0;
-        if (rowOk) {
-            if (!MODE_DKV) {
-                rowScale = p.QScale.Valid() ? p.QScale.Row(head)[row] : p.QkVecScale;
-                rowLse = p.Lse.Row(head)[row];
-                rowDelta = p.DScale.Row(head)[row];
-            } else {
-                rowScale = p.KScale.Row(head)[row];
-                rowSv = p.VScale.Valid() ? p.VScale.Row(head)[row] : p.VVecScale;
-            }
-        }
-        const float rowMult = rowScale * cg;
-        const float2 rowMult2 = make_float2(rowMult, rowMult);
-        const float2 rowSvM2 = make_float2(rowSv * dsMult, rowSv * dsMult);
-        const float2 negDeltaM2 = make_float2(-rowDelta * dsMult, -rowDelta * dsMult);
-
+        float rowMult = 0, rowLse = 0, rowOther = 0; // rowOther: sv c ln2 or -delta c ln2
         int spanS = 1, spanF = 0, spanRound = -1;
         // the tile's 128 column factors are staged by the first 128 threads, one tile ahead
         float pfA = 0, pfT = 0, pfB = 0;
@@ -396,9 +449,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                 }
             }
         };
-        if (cur.Valid) {
-            fetchCols(cur.J0);
-            // clear this thread's quarter of the output accumulators: every output product accumulates
+        // clears this thread's quarter of the output accumulators: every output product accumulates
+        auto clearOutputs = [&]() {
             uint32_t zero[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
@@ -413,145 +465,190 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
             }
             TmemWaitSt();
             TcFenceBefore();
-        }
+        };
         bool failed = false;
-        int it = 0;
-        while (cur.Valid) {
-            if (cur.Round != spanRound) {
-                spanS = 1;
-                spanF = 0;
-                const tsa_span_group *gp = (r < 64) ? cur.G0 : cur.G1;
-                const int n = (r < 64) ? cur.N0 : cur.N1;
-                if (cur.Round < n) {
-                    spanS = gp[cur.Round].SpanStart[r & 63];
-                    spanF = gp[cur.Round].SpanFinish[r & 63];
+        // The next work item (-1: none).  False, in all threads alike, when a wait has run out somewhere: the arithmetic threads
+        // leave together, none of them waits alone at a named barrier.
+        auto takeItem = [&](int n, int &item) {
+            const bool ok = WaitBarA(&misc.ItemFull[n & 1], (n >> 1) & 1, abortFlag);
+            item = *(volatile int *)&misc.Item[n & 1];
+            if (BarRedOr(BAR_ARITH, BWD_ARITH_THREADS, failed || !ok)) {
+                return false;
+            }
+            if (lane == 0) {
+                MbarArrive(&misc.ItemEmpty[n & 1]);
+            }
+            return true;
+        };
+        auto setUp = [&](int item) {
+            locate(item, rowTile, head);
+            row = rowTile * TILE_ROWS + r;
+            cur.Init(p.Spans, p.SpanPtr, p.LenAttTiles, rowTile, p.Rows);
+            rowMult = 0;
+            rowLse = 0;
+            rowOther = 0;
+            if (row < p.Rows) {
+                if (!MODE_DKV) {
+                    rowMult = (p.QScale.Valid() ? p.QScale.Row(head)[row] : p.QkVecScale) * cg;
+                    rowLse = p.Lse.Row(head)[row];
+                    rowOther = -p.DScale.Row(head)[row] * dsMult;
+                } else {
+                    rowMult = p.KScale.Row(head)[row] * cg;
+                    rowOther = (p.VScale.Valid() ? p.VScale.Row(head)[row] : p.VVecScale) * dsMult;
                 }
-                spanRound = cur.Round;
             }
-            TRB(it, 0);
-            const int buf = it & 1;
-            if (tid < TILE_ROWS) {
-                misc.ColA[buf][tid] = pfA;
-                misc.ColT[buf][tid] = pfT;
-                misc.ColB[buf][tid] = pfB;
+            spanRound = -1;
+            if (cur.Valid) {
+                fetchCols(cur.J0);
             }
-            const int c0 = cur.J0;
-            const int ls = spanS - c0, lf = min(spanF, p.Rows - 1) - c0; // span in tile-local columns
-            const bool rowFull = ls <= 0 && lf >= TILE_ROWS - 1;
-            const bool warpMasked = !__all_sync(0xffffffffu, rowFull);
-            // publishes the staged columns; a failed wait is carried here so the arithmetic threads leave together
-            if (BarRedOr(BAR_ARITH, BWD_ARITH_THREADS, failed || (*(volatile int *)&misc.Abort != 0))) {
-                failed = true;
+        };
+        int it = 0, outCount = 0; // tiles, items with tiles
+        int item = 0;
+        bool alive = takeItem(0, item);
+        if (alive && item >= 0) {
+            setUp(item);
+            clearOutputs();
+        }
+        for (int n = 1; alive && item >= 0; ++n) {
+            const bool hasTiles = cur.Valid;
+            while (cur.Valid) {
+                if (cur.Round != spanRound) {
+                    spanS = 1;
+                    spanF = 0;
+                    const tsa_span_group *gp = (r < 64) ? cur.G0 : cur.G1;
+                    const int n = (r < 64) ? cur.N0 : cur.N1;
+                    if (cur.Round < n) {
+                        spanS = gp[cur.Round].SpanStart[r & 63];
+                        spanF = gp[cur.Round].SpanFinish[r & 63];
+                    }
+                    spanRound = cur.Round;
+                }
+                const int buf = it & 1;
+                if (tid < TILE_ROWS) {
+                    misc.ColA[buf][tid] = pfA;
+                    misc.ColT[buf][tid] = pfT;
+                    misc.ColB[buf][tid] = pfB;
+                }
+                const int c0 = cur.J0;
+                const int ls = spanS - c0, lf = min(spanF, p.Rows - 1) - c0; // span in tile-local columns
+                const bool rowFull = ls <= 0 && lf >= TILE_ROWS - 1;
+                const bool warpMasked = !__all_sync(0xffffffffu, rowFull);
+                // publishes the staged columns; a failed wait is carried here so the arithmetic threads leave together
+                if (BarRedOr(BAR_ARITH, BWD_ARITH_THREADS, failed || (*(volatile int *)&misc.Abort != 0))) {
+                    failed = true;
+                    break;
+                }
+                {
+                    TTileIter nxt = cur;
+                    nxt.Advance();
+                    if (nxt.Valid) {
+                        fetchCols(nxt.J0);
+                    }
+                }
+                // exponent = u * rowMult + (ColT + rowConst):  dQ: ALiBi + rowOff - lse_i;  dK/dV: -lse_i - ALiBi with the sign of the
+                // transposed tile
+                const float2 rowMult2 = make_float2(rowMult, rowMult), rowOther2 = make_float2(rowOther, rowOther);
+                const float rowOff = -p.Slope * (float)(row - c0);
+                const float rowConst = MODE_DKV ? -rowOff : rowOff - rowLse;
+                const float2 rowConst2 = make_float2(rowConst, rowConst);
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h) {
+                    if (!WaitBarA(&misc.BarS[h], it & 1, abortFlag)) {
+                        failed = true;
+                        *(volatile int *)&misc.Abort = 1;
+                        if (p.Status) {
+                            atomicOr(p.Status, kDevTimeoutMma);
+                        }
+                        break; // to the next barrier of the arithmetic threads
+                    }
+                    TcFenceAfter();
+                    const int cb = h * 64 + quarter * 16; // first tile column of this thread's block in the half
+                    // span clipped to this block, block-local: (unsigned)(c - lsQ) <= spanW  <=>  inside the span
+                    const int lsC = max(ls, cb), lfC = min(lf, cb + 15);
+                    const bool rowEmpty = lsC > lfC;
+                    const int lsQ = lsC - cb;
+                    const unsigned spanW = rowEmpty ? 0u : (unsigned)(lfC - lsC);
+                    const bool anyCh = !warpMasked || __any_sync(0xffffffffu, !rowEmpty);
+                    uint32_t a1[8], a2[8];
+                    if (anyCh) {
+                        float2 s[8], d[8];
+                        TmemLd16x2Pairs(tLane + BWD_S_COL + cb, tLane + BWD_DP_COL + cb, s, d);
+                        const float4 *A4 = reinterpret_cast<const float4 *>(misc.ColA[buf] + cb);
+                        const float4 *T4 = reinterpret_cast<const float4 *>(misc.ColT[buf] + cb);
+                        const float4 *B4 = reinterpret_cast<const float4 *>(misc.ColB[buf] + cb);
+#pragma unroll
+                        for (int c = 0; c < 16; c += 4) {
+                            const float4 a4 = A4[c >> 2], t4 = T4[c >> 2], b4 = B4[c >> 2];
+#pragma unroll
+                            for (int k = 0; k < 2; ++k) {
+                                const int i = (c >> 1) + k;
+                                const float2 ca = k ? make_float2(a4.z, a4.w) : make_float2(a4.x, a4.y);
+                                const float2 ct = k ? make_float2(t4.z, t4.w) : make_float2(t4.x, t4.y);
+                                const float2 cbv = k ? make_float2(b4.z, b4.w) : make_float2(b4.x, b4.y);
+                                const float2 u = __fmul2_rn(s[i], ca);
+                                const float2 e = __ffma2_rn(u, rowMult2, __fadd2_rn(ct, rowConst2));
+                                float2 pij = FastExp2Pair(e);
+                                if (warpMasked) {
+                                    pij.x = (!rowEmpty && (unsigned)(c + 2 * k - lsQ) <= spanW) ? pij.x : 0.0f;
+                                    pij.y = (!rowEmpty && (unsigned)(c + 2 * k + 1 - lsQ) <= spanW) ? pij.y : 0.0f;
+                                }
+                                const float2 dpv = MODE_DKV ? __ffma2_rn(d[i], rowOther2, cbv) : __ffma2_rn(d[i], cbv, rowOther2);
+                                const float2 ds = __fmul2_rn(__fmul2_rn(pij, dpv), ca);
+                                a1[i] = PackBf16x2(ds.x, ds.y);
+                                a2[i] = PackBf16x2(pij.x, pij.y);
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            a1[k] = 0;
+                            a2[k] = 0;
+                        }
+                    }
+                    // 16 bf16 values = 8 columns, written over the first half of the 16 columns this thread has just read
+                    TmemStN<8>(tLane + BWD_S_COL + cb, a1);
+                    if (MODE_DKV) {
+                        TmemStN<8>(tLane + BWD_DP_COL + cb, a2);
+                    }
+                    TmemWaitSt();
+                    TcFenceBefore();
+                    __syncwarp();
+                    if (lane == 0) {
+                        MbarArrive(&misc.BarP[h]);
+                    }
+                }
+                cur.Advance();
+                ++it;
+            }
+
+            // The next item's spans, row constants and first column factors are looked up while this one's last output products run.
+            const int doneRow = row, doneHead = head;
+            alive = takeItem(n, item);
+            if (!alive) {
                 break;
             }
-            TRB(it, 1);
-            {
-                TTileIter nxt = cur;
-                nxt.Advance();
-                if (nxt.Valid) {
-                    fetchCols(nxt.J0);
-                }
+            if (item >= 0) {
+                setUp(item);
             }
-            // exponent = u * rowMult + (ColT + rowConst):  dQ: ALiBi + rowOff - lse_i;  dK/dV: -lse_i - ALiBi with the sign of the
-            // transposed tile
-            const float rowOff = -p.Slope * (float)(row - c0);
-            const float rowConst = MODE_DKV ? -rowOff : rowOff - rowLse;
-            const float2 rowConst2 = make_float2(rowConst, rowConst);
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                if (!WaitBarA(&misc.BarS[h], it & 1, abortFlag)) {
-                    failed = true;
+            if (hasTiles) {
+                if (!__all_sync(0xffffffffu, WaitBarA(&misc.BarOut, outCount & 1, abortFlag))) {
+                    failed = true; // carried to the next item's barrier; without one the thread just leaves
                     *(volatile int *)&misc.Abort = 1;
                     if (p.Status) {
                         atomicOr(p.Status, kDevTimeoutMma);
                     }
-                    break; // to the next barrier of the arithmetic threads
+                    continue;
                 }
+                ++outCount;
                 TcFenceAfter();
-                TRB(it, 4 * h + 2);
-                const int cb = h * 64 + quarter * 16; // first tile column of this thread's block in the half
-                // span clipped to this block, block-local: (unsigned)(c - lsQ) <= spanW  <=>  inside the span
-                const int lsC = max(ls, cb), lfC = min(lf, cb + 15);
-                const bool rowEmpty = lsC > lfC;
-                const int lsQ = lsC - cb;
-                const unsigned spanW = rowEmpty ? 0u : (unsigned)(lfC - lsC);
-                const bool anyCh = !warpMasked || __any_sync(0xffffffffu, !rowEmpty);
-                uint32_t a1[8], a2[8];
-                if (anyCh) {
-                    float2 s[8], d[8];
-                    TmemLd16x2Pairs(tLane + BWD_S_COL + cb, tLane + BWD_DP_COL + cb, s, d);
-                    const float4 *A4 = reinterpret_cast<const float4 *>(misc.ColA[buf] + cb);
-                    const float4 *T4 = reinterpret_cast<const float4 *>(misc.ColT[buf] + cb);
-                    const float4 *B4 = reinterpret_cast<const float4 *>(misc.ColB[buf] + cb);
-#pragma unroll
-                    for (int c = 0; c < 16; c += 4) {
-                        const float4 a4 = A4[c >> 2], t4 = T4[c >> 2], b4 = B4[c >> 2];
-#pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            const int i = (c >> 1) + k;
-                            const float2 ca = k ? make_float2(a4.z, a4.w) : make_float2(a4.x, a4.y);
-                            const float2 ct = k ? make_float2(t4.z, t4.w) : make_float2(t4.x, t4.y);
-                            const float2 cbv = k ? make_float2(b4.z, b4.w) : make_float2(b4.x, b4.y);
-                            const float2 u = __fmul2_rn(s[i], ca);
-                            const float2 e = __ffma2_rn(u, rowMult2, __fadd2_rn(ct, rowConst2));
-                            float2 pij = FastExp2Pair(e);
-                            if (warpMasked) {
-                                pij.x = (!rowEmpty && (unsigned)(c + 2 * k - lsQ) <= spanW) ? pij.x : 0.0f;
-                                pij.y = (!rowEmpty && (unsigned)(c + 2 * k + 1 - lsQ) <= spanW) ? pij.y : 0.0f;
-                            }
-                            const float2 dpv = MODE_DKV ? __ffma2_rn(d[i], rowSvM2, cbv) : __ffma2_rn(d[i], cbv, negDeltaM2);
-                            const float2 ds = __fmul2_rn(__fmul2_rn(pij, dpv), ca);
-                            a1[i] = PackBf16x2(ds.x, ds.y);
-                            a2[i] = PackBf16x2(pij.x, pij.y);
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        a1[k] = 0;
-                        a2[k] = 0;
-                    }
-                }
-                // 16 bf16 values = 8 columns, written over the first half of the 16 columns this thread has just read
-                TmemStN<8>(tLane + BWD_S_COL + cb, a1);
-                if (MODE_DKV) {
-                    TmemStN<8>(tLane + BWD_DP_COL + cb, a2);
-                }
-                TmemWaitSt();
-                TcFenceBefore();
-                __syncwarp();
-                if (lane == 0) {
-                    MbarArrive(&misc.BarP[h]);
-                }
-                TRB(it, 4 * h + 3);
             }
-            cur.Advance();
-            ++it;
-        }
-
-        const int tiles = it;
-        if (!failed && tiles > 0) {
-            if (!WaitBarA(&misc.BarDone, 0, abortFlag)) {
-                failed = true;
-                if (p.Status) {
-                    atomicOr(p.Status, kDevTimeoutMma);
-                }
-            }
-            TcFenceAfter();
-        }
-        // Outputs: tensor memory -> registers -> shared memory -> global memory in whole rows.  A thread holds a quarter of
-        // one row, so stores straight from the registers would put 32 different rows into every store instruction (32
-        // sectors each, serialised in the load/store unit: 4 K clocks per CTA); staged through shared memory (the tile
-        // buffers are idle by now; row pitch padded by 16 bytes against bank conflicts) a warp writes two whole rows per
-        // instruction.  The vote makes the staging barrier safe when some thread has given up.
-        if (!BarRedOr(BAR_ARITH, BWD_ARITH_THREADS, failed)) {
+            // Outputs straight from the registers, 32 bytes (a whole sector) per store where the rows allow it: a thread holds a quarter
+            // of one row.  The stores drain while the next item's score products run.
             const int esz = (p.GradDtype == TSA_F32) ? 4 : 2;
-            const int rowBytes = D * esz, pitch = rowBytes + 16;
-            constexpr int STAGE_BYTES = TILE_ROWS * (D * 4 + 16);
 #pragma unroll
             for (int o = 0; o < OUTPUTS; ++o) {
                 uint32_t v[QUARTER_D];
-                if (tiles > 0) {
+                if (hasTiles) {
                     if (QUARTER_D == 32) {
                         TmemLd32(tLane + BWD_OUT_COL + o * D + quarter * QUARTER_D, v);
                     } else {
@@ -564,44 +661,49 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                         v[c] = 0;
                     }
                 }
-                uint8_t *dstS = smem + o * STAGE_BYTES + r * pitch + quarter * QUARTER_D * esz;
-                if (p.GradDtype == TSA_F32) {
-                    float4 *dst = reinterpret_cast<float4 *>(dstS);
-#pragma unroll
-                    for (int c = 0; c < QUARTER_D; c += 4) {
-                        dst[c >> 2] = make_float4(__uint_as_float(v[c]) * p.GradMult, __uint_as_float(v[c + 1]) * p.GradMult,
-                            __uint_as_float(v[c + 2]) * p.GradMult, __uint_as_float(v[c + 3]) * p.GradMult);
-                    }
-                } else {
-                    uint4 *dst = reinterpret_cast<uint4 *>(dstS);
-#pragma unroll
-                    for (int c = 0; c < QUARTER_D; c += 8) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const float a = __uint_as_float(v[c + 2 * k]) * p.GradMult, b = __uint_as_float(v[c + 2 * k + 1]) * p.GradMult;
-                            w[k] = (p.GradDtype == TSA_BF16) ? PackBf16x2(a, b) : PackHalf2(a, b);
+                if (doneRow < p.Rows) {
+                    const P2D<char> &outp = (o == 0) ? p.Out1 : p.Out2;
+                    char *dst = outp.Row(doneRow) + (size_t)(doneHead * D + quarter * QUARTER_D) * esz;
+                    auto put = [&](const uint32_t *w) { // 32 bytes
+                        if (p.WideStores) {
+                            StGlobal256(dst, w);
+                        } else {
+                            reinterpret_cast<uint4 *>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                            reinterpret_cast<uint4 *>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
                         }
-                        dst[c >> 3] = make_uint4(w[0], w[1], w[2], w[3]);
+                        dst += 32;
+                    };
+                    if (p.GradDtype == TSA_F32) {
+#pragma unroll
+                        for (int c = 0; c < QUARTER_D; c += 8) {
+                            uint32_t w[8];
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                w[k] = __float_as_uint(__uint_as_float(v[c + k]) * p.GradMult);
+                            }
+                            put(w);
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < QUARTER_D; c += 16) {
+                            uint32_t w[8];
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                const float a = __uint_as_float(v[c + 2 * k]) * p.GradMult, b = __uint_as_float(v[c + 2 * k + 1]) * p.GradMult;
+                                w[k] = (p.GradDtype == TSA_BF16) ? PackBf16x2(a, b) : PackHalf2(a, b);
+                            }
+                            put(w);
+                        }
                     }
                 }
             }
-            BarRedOr(BAR_ARITH, BWD_ARITH_THREADS, false);
-            const int chunksPerRow = rowBytes >> 4;
-#pragma unroll
-            for (int o = 0; o < OUTPUTS; ++o) {
-                const P2D<char> &outp = (o == 0) ? p.Out1 : p.Out2;
-                const uint8_t *stage = smem + o * STAGE_BYTES;
-                for (int id = tid; id < TILE_ROWS * chunksPerRow; id += BWD_ARITH_THREADS) {
-                    const int rr = id / chunksPerRow, cc = id - rr * chunksPerRow;
-                    const int grow = rowTile * TILE_ROWS + rr;
-                    if (grow < p.Rows) {
-                        *reinterpret_cast<uint4 *>(outp.Row(grow) + (size_t)head * D * esz + cc * 16) =
-                            *reinterpret_cast<const uint4 *>(stage + rr * pitch + cc * 16);
-                    }
-                }
+            if (hasTiles && item >= 0) {
+                clearOutputs();
             }
         }
+    }
+    if (MODE_DKV) {
+        PdlWait();
     }
     TcFenceBefore();
     __syncthreads();
@@ -635,6 +737,7 @@ struct TWiden3 {
     int Stride[3];
     int Dtype[3];
     __nv_bfloat16 *Dst[3];
+    int *Counters; // of the backward kernels that follow: set to zero
 };
 
 __device__ __forceinline__ uint32_t Widen2(uint32_t w, int shift, int dtype)
@@ -652,7 +755,12 @@ __device__ __forceinline__ uint32_t Widen2(uint32_t w, int shift, int dtype)
 
 __global__ void __launch_bounds__(256) Widen8x3Kernel(TWiden3 t, int rows, int cols)
 {
+    PdlTrigger();
+    PdlWait();
     const int m = blockIdx.y;
+    if (blockIdx.x == 0 && m == 0 && threadIdx.x < 2) {
+        t.Counters[threadIdx.x] = 0;
+    }
     const char *src = t.Src[m];
     const int stride = t.Stride[m], dtype = t.Dtype[m];
     __nv_bfloat16 *dst = t.Dst[m];
@@ -704,11 +812,11 @@ bool Sm100BwdSupports(const tsa_att_cfg *cfg, int headCount)
 size_t Sm100BwdWorkspaceBytes(int headCount, int headDim, int rows)
 {
     const size_t mat = ((size_t)rows * headCount * headDim * 2 + 255) / 256 * 256;
-    return 4 * mat; // Q, K, V, dO as bf16
+    return 256 + 4 * mat; // work-item counters of the two passes; Q, K, V, dO as bf16
 }
 
 template <int D, bool MODE_DKV>
-static int LaunchBwdT(const CUtensorMap &r1, const CUtensorMap &r2, const CUtensorMap &c1, const CUtensorMap &c2, const TBwdParams &bp,
+static int LaunchBwdT(const CUtensorMap &r1, const CUtensorMap &r2, const CUtensorMap &c1, const CUtensorMap &c2, TBwdParams bp,
     int rowTiles, cudaStream_t stream)
 {
     auto kern = BwdSm100Kernel<D, MODE_DKV>;
@@ -717,9 +825,17 @@ static int LaunchBwdT(const CUtensorMap &r1, const CUtensorMap &r2, const CUtens
     if (rc != TSA_OK) {
         return rc;
     }
-    dim3 grid(rowTiles, bp.HeadCount);
-    kern<<<grid, BWD_THREADS, smemBytes, stream>>>(r1, r2, c1, c2, bp);
-    return CheckCuda(cudaGetLastError(), "tcgen05 backward launch");
+    int dev = 0, sms = 0;
+    rc = CheckCuda(cudaGetDevice(&dev), "cudaGetDevice");
+    if (rc == TSA_OK) {
+        rc = CheckCuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+    }
+    if (rc != TSA_OK) {
+        return rc;
+    }
+    bp.Items = rowTiles * bp.HeadCount;
+    void *args[] = {(void *)&r1, (void *)&r2, (void *)&c1, (void *)&c2, &bp};
+    return CheckCuda(LaunchPdl((const void *)kern, dim3(bp.Items < sms ? bp.Items : sms), dim3(BWD_THREADS), smemBytes, stream, args), "tcgen05 backward launch");
 }
 
 int LaunchSm100Bwd(const tsa_att_cfg *cfg, const TGenParams &p, tsa_ptr2d qk, tsa_ptr2d qv, tsa_ptr2d v, tsa_ptr2d dOut,
@@ -729,6 +845,8 @@ int LaunchSm100Bwd(const tsa_att_cfg *cfg, const TGenParams &p, tsa_ptr2d qk, ts
     const int rows = p.Len;
     const int cols = p.HeadCount * D;
     const size_t mat = ((size_t)rows * cols * 2 + 255) / 256 * 256;
+    int *counters = (int *)workspace;
+    workspace = (char *)workspace + 256;
     __nv_bfloat16 *qb = (__nv_bfloat16 *)workspace;
     __nv_bfloat16 *kb = (__nv_bfloat16 *)((char *)workspace + mat);
     __nv_bfloat16 *vb = (__nv_bfloat16 *)((char *)workspace + 2 * mat);
@@ -748,8 +866,18 @@ int LaunchSm100Bwd(const tsa_att_cfg *cfg, const TGenParams &p, tsa_ptr2d qk, ts
         }
         const long long g16 = (long long)rows * (cols / 16);
         const int b16 = (int)((g16 + 255) / 256 < 148 * 8 ? (g16 + 255) / 256 : 148 * 8);
-        Widen8x3Kernel<<<dim3(b16, 3), 256, 0, stream>>>(t, rows, cols);
+        t.Counters = counters;
+        int r = rows, c = cols;
+        void *args[] = {&t, &r, &c};
+        const int rc = CheckCuda(LaunchPdl((const void *)Widen8x3Kernel, dim3(b16, 3), dim3(256), 0, stream, args), "bf16 widening launch");
+        if (rc != TSA_OK) {
+            return rc;
+        }
     } else {
+        const int rc = CheckCuda(cudaMemsetAsync(counters, 0, 256, stream), "clearing the backward counters");
+        if (rc != TSA_OK) {
+            return rc;
+        }
         ToBf16Kernel<<<blocks, 256, 0, stream>>>(cfg->qk_dtype, P2D<char>(qk), rows, cols, qb);
         ToBf16Kernel<<<blocks, 256, 0, stream>>>(cfg->qk_dtype, P2D<char>(qv), rows, cols, kb);
         ToBf16Kernel<<<blocks, 256, 0, stream>>>(cfg->v_dtype, P2D<char>(v), rows, cols, vb);
@@ -809,6 +937,10 @@ int LaunchSm100Bwd(const tsa_att_cfg *cfg, const TGenParams &p, tsa_ptr2d qk, ts
     bp.SpanPtr = p.SpanPtr;
     bp.Out1 = p.DQ;
     bp.Out2 = p.DQ;
+    auto wide = [](const P2D<char> &a) { return (((uintptr_t)a.Data | (uintptr_t)a.Stride) & 31) == 0; };
+    bp.WideStores = wide(p.DQ);
+    bp.Ascending = 0;
+    bp.Counter = counters;
     rc = (D == 128) ? LaunchBwdT<128, false>(mq, mdo, mk, mv, bp, rowTiles, stream) : LaunchBwdT<64, false>(mq, mdo, mk, mv, bp, rowTiles, stream);
     if (rc != TSA_OK) {
         return rc;
@@ -818,14 +950,10 @@ int LaunchSm100Bwd(const tsa_att_cfg *cfg, const TGenParams &p, tsa_ptr2d qk, ts
     bp.SpanPtr = p.RevSpanPtr;
     bp.Out1 = p.DK;
     bp.Out2 = p.DV;
+    bp.WideStores = wide(p.DK) && wide(p.DV);
+    bp.Ascending = 1;
+    bp.Counter = counters + 1;
     return (D == 128) ? LaunchBwdT<128, true>(mk, mv, mq, mdo, bp, rowTiles, stream) : LaunchBwdT<64, true>(mk, mv, mq, mdo, bp, rowTiles, stream);
 }
 
 } // namespace tsa
-
-#ifdef TSA_BWD_TRACE
-extern "C" __attribute__((visibility("default"))) int tsa_debug_trace_bwd(long long *dst, int n)
-{
-    return (int)cudaMemcpyFromSymbol(dst, tsa::g_traceBwd, n * sizeof(long long));
-}
-#endif
