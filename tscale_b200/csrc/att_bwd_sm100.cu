@@ -218,6 +218,14 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                 if (!prod.Valid) {
                     continue;
                 }
+                // the row tiles' buffers are in use for a while yet: bring the tiles as far as L2 meanwhile
+#pragma unroll
+                for (int kb = 0; kb < KBLOCKS; ++kb) {
+                    TmaPrefetch2D(&tmR1, head * D + kb * 64, rowTile * TILE_ROWS);
+                    TmaPrefetch2D(&tmR1, head * D + kb * 64, rowTile * TILE_ROWS + 64);
+                    TmaPrefetch2D(&tmR2, head * D + kb * 64, rowTile * TILE_ROWS);
+                    TmaPrefetch2D(&tmR2, head * D + kb * 64, rowTile * TILE_ROWS + 64);
+                }
                 if (rCount > 0 && !wait(&misc.BarREmpty, (rCount - 1) & 1)) {
                     break;
                 }
@@ -428,26 +436,39 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
         int rowTile = 0, head = 0, row = 0;
         TTileIter cur;
         // per-row constants.  dQ pass: the row is a query (scale sq, lse, delta); dK/dV pass: the row is a key (sk, sv)
-        float rowMult = 0, rowLse = 0, rowOther = 0; // rowOther: sv c ln2 or -delta c ln2
+        // (kept as loaded until an item's first tile, so that their latency passes behind the previous item's outputs)
+        float rowScale = 0, rowLse = 0, rowOther = 0;
+        float rowMult = 0;
         int spanS = 1, spanF = 0, spanRound = -1;
-        // the tile's 128 column factors are staged by the first 128 threads, one tile ahead
+        // the tile's 128 column factors are staged by the first 128 threads, one tile ahead, and worked on when they are staged
         float pfA = 0, pfT = 0, pfB = 0;
         auto fetchCols = [&](int c0) {
+            const int c = c0 + tid;
+            const bool ok = tid < TILE_ROWS && c < p.Rows;
             pfA = 0;
             pfT = 0;
             pfB = 0;
-            const int c = c0 + tid;
-            if (tid < TILE_ROWS && c < p.Rows) {
+            if (ok) {
                 if (!MODE_DKV) {
                     pfA = p.KScale.Row(head)[c];
-                    pfT = p.Slope * (float)tid;
-                    pfB = (p.VScale.Valid() ? p.VScale.Row(head)[c] : p.VVecScale) * dsMult;
+                    pfB = p.VScale.Valid() ? p.VScale.Row(head)[c] : p.VVecScale;
                 } else {
                     pfA = p.QScale.Valid() ? p.QScale.Row(head)[c] : p.QkVecScale;
-                    pfT = -p.Lse.Row(head)[c] - p.Slope * (float)tid;
-                    pfB = -p.DScale.Row(head)[c] * dsMult;
+                    pfT = p.Lse.Row(head)[c];
+                    pfB = p.DScale.Row(head)[c];
                 }
             }
+        };
+        auto fetchSpans = [&]() {
+            spanS = 1;
+            spanF = 0;
+            const tsa_span_group *gp = (r < 64) ? cur.G0 : cur.G1;
+            const int n = (r < 64) ? cur.N0 : cur.N1;
+            if (cur.Round < n) {
+                spanS = gp[cur.Round].SpanStart[r & 63];
+                spanF = gp[cur.Round].SpanFinish[r & 63];
+            }
+            spanRound = cur.Round;
         };
         // clears this thread's quarter of the output accumulators: every output product accumulates
         auto clearOutputs = [&]() {
@@ -484,22 +505,22 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
             locate(item, rowTile, head);
             row = rowTile * TILE_ROWS + r;
             cur.Init(p.Spans, p.SpanPtr, p.LenAttTiles, rowTile, p.Rows);
-            rowMult = 0;
+            rowScale = 0;
             rowLse = 0;
             rowOther = 0;
             if (row < p.Rows) {
                 if (!MODE_DKV) {
-                    rowMult = (p.QScale.Valid() ? p.QScale.Row(head)[row] : p.QkVecScale) * cg;
+                    rowScale = p.QScale.Valid() ? p.QScale.Row(head)[row] : p.QkVecScale;
                     rowLse = p.Lse.Row(head)[row];
-                    rowOther = -p.DScale.Row(head)[row] * dsMult;
+                    rowOther = p.DScale.Row(head)[row];
                 } else {
-                    rowMult = p.KScale.Row(head)[row] * cg;
-                    rowOther = (p.VScale.Valid() ? p.VScale.Row(head)[row] : p.VVecScale) * dsMult;
+                    rowScale = p.KScale.Row(head)[row];
+                    rowOther = p.VScale.Valid() ? p.VScale.Row(head)[row] : p.VVecScale;
                 }
             }
-            spanRound = -1;
             if (cur.Valid) {
                 fetchCols(cur.J0);
+                fetchSpans();
             }
         };
         int it = 0, outCount = 0; // tiles, items with tiles
@@ -511,23 +532,17 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
         }
         for (int n = 1; alive && item >= 0; ++n) {
             const bool hasTiles = cur.Valid;
+            rowMult = rowScale * cg;
+            rowOther *= MODE_DKV ? dsMult : -dsMult;
             while (cur.Valid) {
                 if (cur.Round != spanRound) {
-                    spanS = 1;
-                    spanF = 0;
-                    const tsa_span_group *gp = (r < 64) ? cur.G0 : cur.G1;
-                    const int n = (r < 64) ? cur.N0 : cur.N1;
-                    if (cur.Round < n) {
-                        spanS = gp[cur.Round].SpanStart[r & 63];
-                        spanF = gp[cur.Round].SpanFinish[r & 63];
-                    }
-                    spanRound = cur.Round;
+                    fetchSpans();
                 }
                 const int buf = it & 1;
                 if (tid < TILE_ROWS) {
                     misc.ColA[buf][tid] = pfA;
-                    misc.ColT[buf][tid] = pfT;
-                    misc.ColB[buf][tid] = pfB;
+                    misc.ColT[buf][tid] = MODE_DKV ? -pfT - p.Slope * (float)tid : p.Slope * (float)tid;
+                    misc.ColB[buf][tid] = MODE_DKV ? -pfB * dsMult : pfB * dsMult;
                 }
                 const int c0 = cur.J0;
                 const int ls = spanS - c0, lf = min(spanF, p.Rows - 1) - c0; // span in tile-local columns

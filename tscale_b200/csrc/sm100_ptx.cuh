@@ -99,6 +99,11 @@ __device__ __forceinline__ void TmaLoad2D(void *smemDst, const void *tensorMap, 
         : "r"(SmemAddr(smemDst)), "l"(tensorMap), "r"(x), "r"(y), "r"(SmemAddr(bar))
         : "memory");
 }
+// the same tile into L2 only
+__device__ __forceinline__ void TmaPrefetch2D(const void *tensorMap, int x, int y)
+{
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(tensorMap), "r"(x), "r"(y) : "memory");
+}
 // untiled bulk copy global -> shared: both addresses 16-byte aligned, size a multiple of 16 bytes
 __device__ __forceinline__ void BulkLoad(void *smemDst, const void *gsrc, uint32_t bytes, uint64_t *bar)
 {
