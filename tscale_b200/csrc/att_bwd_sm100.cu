@@ -86,9 +86,12 @@ struct TBwdMisc {
     float ColB[2][TILE_ROWS]; // dQ: sv_j c ln2;  dK/dV: -delta_i c ln2
     int Abort;
     int Turn;                 // issue blocks handed to the tensor pipe so far: control warp h issues the blocks with index = h (mod 2)
-    uint64_t ItemFull[2];     // loader -> all: Item[] holds the next work item (-1: none left)
+    uint64_t ItemFull[2];     // loader -> all: Item[] holds the next work item
     uint64_t ItemEmpty[2];    // all -> loader: the record has been read
-    int Item[2];
+    struct {
+        int RowTile, Head; // RowTile < 0: no items left
+        TTileIter First;   // at the item's first column tile
+    } Item[2];
     uint64_t BarR;            // TMA: row tiles landed
     uint64_t BarREmpty;       // MMA warps -> loader: the item's last score products have retired
     uint64_t BarFull[8];      // TMA: half stage (64 rows of C1 and C2) landed
@@ -204,9 +207,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                 if (n >= 2 && !wait(&misc.ItemEmpty[n & 1], ((n >> 1) - 1) & 1)) {
                     break;
                 }
-                *(volatile int *)&misc.Item[n & 1] = item < p.Items ? item : -1;
-                MbarArrive(&misc.ItemFull[n & 1]);
                 if (item >= p.Items) {
+                    misc.Item[n & 1].RowTile = -1;
+                    MbarArrive(&misc.ItemFull[n & 1]);
                     break;
                 }
                 const int next = gridDim.x + atomicAdd(p.Counter, 1); // in flight while this item is set up
@@ -215,6 +218,10 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                 item = next;
                 TTileIter prod;
                 prod.Init(p.Spans, p.SpanPtr, p.LenAttTiles, rowTile, p.Rows);
+                misc.Item[n & 1].RowTile = rowTile;
+                misc.Item[n & 1].Head = head;
+                misc.Item[n & 1].First = prod;
+                MbarArrive(&misc.ItemFull[n & 1]);
                 if (!prod.Valid) {
                     continue;
                 }
@@ -345,25 +352,22 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                     *(volatile int *)&misc.Turn = index + 1;
                 }
             };
-            int it = 0, items = 0; // tiles and items with tiles so far
-            bool prevLast = false; // the tile whose output products are still to come is its item's last
+            // An item's last output products are an issue block of their own, so that they do not wait for the next item's row tiles.
+            int it = 0, items = 0, block = 0; // tiles, items with tiles and issue blocks so far
             for (int n = 0; !failed; ++n) {
                 if (!__all_sync(0xffffffffu, WaitBarA(&misc.ItemFull[n & 1], (n >> 1) & 1, abortFlag))) {
                     fail(kDevTimeoutTma);
                     break;
                 }
-                const int item = *(volatile int *)&misc.Item[n & 1];
+                const bool none = misc.Item[n & 1].RowTile < 0;
+                TTileIter ctl = misc.Item[n & 1].First;
                 __syncwarp();
                 if (lane == 0) {
                     MbarArrive(&misc.ItemEmpty[n & 1]);
                 }
-                if (item < 0) {
+                if (none) {
                     break;
                 }
-                int rowTile, head;
-                locate(item, rowTile, head);
-                TTileIter ctl;
-                ctl.Init(p.Spans, p.SpanPtr, p.LenAttTiles, rowTile, p.Rows);
                 if (!ctl.Valid) {
                     continue;
                 }
@@ -372,54 +376,47 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                     break;
                 }
                 ++items;
-                for (; ctl.Valid && !failed; ++it) {
+                for (bool first = true;; first = false) {
+                    const bool more = ctl.Valid; // a tile's scores behind the previous tile's outputs, or the item's last outputs
                     const int g = 2 * it + h;
                     const int slot = g % HSTAGES, prevSlot = (g - 2 + HSTAGES) % HSTAGES;
-                    ctl.Advance();
-                    const bool last = !ctl.Valid;
-                    if (!__all_sync(0xffffffffu, WaitBarA(&misc.BarFull[slot], (g / HSTAGES) & 1, abortFlag))) {
-                        fail(kDevTimeoutTma);
-                        break;
-                    }
-                    if (it > 0) {
-                        if (!__all_sync(0xffffffffu, WaitBarSleep<20>(&misc.BarP[h], (it - 1) & 1, abortFlag))) {
-                            fail(kDevTimeoutMma);
+                    if (more) {
+                        ctl.Advance();
+                        if (!__all_sync(0xffffffffu, WaitBarA(&misc.BarFull[slot], (g / HSTAGES) & 1, abortFlag))) {
+                            fail(kDevTimeoutTma);
                             break;
                         }
                     }
-                    if (!__all_sync(0xffffffffu, takeTurn(g))) {
+                    if (!first && !__all_sync(0xffffffffu, WaitBarSleep<20>(&misc.BarP[h], (it - 1) & 1, abortFlag))) {
+                        fail(kDevTimeoutMma);
+                        break;
+                    }
+                    if (!__all_sync(0xffffffffu, takeTurn(2 * block + h))) {
                         fail(kDevTimeoutMma);
                         break;
                     }
                     TcFenceAfter();
                     if (ElectOne()) {
-                        if (it > 0) {
+                        if (!first) {
                             issueOutputs(prevSlot, h);
                             MmaCommit(&misc.BarEmpty[prevSlot]);
-                            if (prevLast) {
-                                MmaCommit(&misc.BarOut);
+                        }
+                        if (more) {
+                            issueScores(slot, h);
+                            MmaCommit(&misc.BarS[h]);
+                            if (!ctl.Valid) {
+                                MmaCommit(&misc.BarREmpty);
                             }
-                        }
-                        issueScores(slot, h);
-                        MmaCommit(&misc.BarS[h]);
-                        if (last) {
-                            MmaCommit(&misc.BarREmpty);
+                        } else {
+                            MmaCommit(&misc.BarOut);
                         }
                     }
-                    passTurn(g);
-                    prevLast = last;
-                }
-            }
-            if (!failed && it > 0) {
-                if (__all_sync(0xffffffffu, WaitBarSleep<20>(&misc.BarP[h], (it - 1) & 1, abortFlag) && takeTurn(2 * it + h))) {
-                    TcFenceAfter();
-                    if (ElectOne()) {
-                        issueOutputs((2 * (it - 1) + h) % HSTAGES, h);
-                        MmaCommit(&misc.BarOut);
+                    passTurn(2 * block + h);
+                    ++block;
+                    if (!more) {
+                        break;
                     }
-                    passTurn(2 * it + h);
-                } else {
-                    fail(kDevTimeoutMma);
+                    ++it;
                 }
             }
             __syncwarp();
@@ -488,11 +485,13 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
             TcFenceBefore();
         };
         bool failed = false;
-        // The next work item (-1: none).  False, in all threads alike, when a wait has run out somewhere: the arithmetic threads
+        // The next work item into (rowTile, head, cur); rowTile < 0: none.  False, in all threads alike, when a wait has run out somewhere: the arithmetic threads
         // leave together, none of them waits alone at a named barrier.
-        auto takeItem = [&](int n, int &item) {
+        auto takeItem = [&](int n) {
             const bool ok = WaitBarA(&misc.ItemFull[n & 1], (n >> 1) & 1, abortFlag);
-            item = *(volatile int *)&misc.Item[n & 1];
+            rowTile = misc.Item[n & 1].RowTile;
+            head = misc.Item[n & 1].Head;
+            cur = misc.Item[n & 1].First;
             if (BarRedOr(BAR_ARITH, BWD_ARITH_THREADS, failed || !ok)) {
                 return false;
             }
@@ -501,10 +500,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
             }
             return true;
         };
-        auto setUp = [&](int item) {
-            locate(item, rowTile, head);
+        auto setUp = [&]() {
             row = rowTile * TILE_ROWS + r;
-            cur.Init(p.Spans, p.SpanPtr, p.LenAttTiles, rowTile, p.Rows);
             rowScale = 0;
             rowLse = 0;
             rowOther = 0;
@@ -524,13 +521,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
             }
         };
         int it = 0, outCount = 0; // tiles, items with tiles
-        int item = 0;
-        bool alive = takeItem(0, item);
-        if (alive && item >= 0) {
-            setUp(item);
+        bool alive = takeItem(0);
+        if (alive && rowTile >= 0) {
+            setUp();
             clearOutputs();
         }
-        for (int n = 1; alive && item >= 0; ++n) {
+        for (int n = 1; alive && rowTile >= 0; ++n) {
             const bool hasTiles = cur.Valid;
             rowMult = rowScale * cg;
             rowOther *= MODE_DKV ? dsMult : -dsMult;
@@ -638,12 +634,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
 
             // The next item's spans, row constants and first column factors are looked up while this one's last output products run.
             const int doneRow = row, doneHead = head;
-            alive = takeItem(n, item);
+            alive = takeItem(n);
             if (!alive) {
                 break;
             }
-            if (item >= 0) {
-                setUp(item);
+            if (rowTile >= 0) {
+                setUp();
             }
             if (hasTiles) {
                 if (!__all_sync(0xffffffffu, WaitBarA(&misc.BarOut, outCount & 1, abortFlag))) {
@@ -712,7 +708,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                     }
                 }
             }
-            if (hasTiles && item >= 0) {
+            if (hasTiles && rowTile >= 0) {
                 clearOutputs();
             }
         }
