@@ -727,6 +727,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
 // src: [rows][cols] of i8 / e4m3 / f16 / bf16 / f32 -> dst bf16 [rows][cols] (dense); 8 elements per thread
 __global__ void __launch_bounds__(256) ToBf16Kernel(int srcDtype, P2D<char> src, int rows, int cols, __nv_bfloat16 *dst)
 {
+    PdlTrigger();
+    PdlWait();
     const long long groups = (long long)rows * (cols / 8);
     for (long long gidx = blockIdx.x * (long long)blockDim.x + threadIdx.x; gidx < groups; gidx += (long long)gridDim.x * blockDim.x) {
         const int rowIdx = (int)(gidx / (cols / 8));
@@ -889,14 +891,14 @@ int LaunchSm100Bwd(const tsa_att_cfg *cfg, const TGenParams &p, tsa_ptr2d qk, ts
         if (rc != TSA_OK) {
             return rc;
         }
-        ToBf16Kernel<<<blocks, 256, 0, stream>>>(cfg->qk_dtype, P2D<char>(qk), rows, cols, qb);
-        ToBf16Kernel<<<blocks, 256, 0, stream>>>(cfg->qk_dtype, P2D<char>(qv), rows, cols, kb);
-        ToBf16Kernel<<<blocks, 256, 0, stream>>>(cfg->v_dtype, P2D<char>(v), rows, cols, vb);
+        LaunchPdlArgs(ToBf16Kernel, dim3(blocks), dim3(256), 0, stream, cfg->qk_dtype, P2D<char>(qk), rows, cols, qb);
+        LaunchPdlArgs(ToBf16Kernel, dim3(blocks), dim3(256), 0, stream, cfg->qk_dtype, P2D<char>(qv), rows, cols, kb);
+        LaunchPdlArgs(ToBf16Kernel, dim3(blocks), dim3(256), 0, stream, cfg->v_dtype, P2D<char>(v), rows, cols, vb);
     }
     // dO that already is bf16 in a TMA-compatible layout is read where it lies
     const bool dOutInPlace = cfg->grad_dtype == TSA_BF16 && (uintptr_t)dOut.data % 16 == 0 && dOut.stride_bytes % 16 == 0 && dOut.xsize >= cols;
     if (!dOutInPlace) {
-        ToBf16Kernel<<<blocks, 256, 0, stream>>>(cfg->grad_dtype, P2D<char>(dOut), rows, cols, dob);
+        LaunchPdlArgs(ToBf16Kernel, dim3(blocks), dim3(256), 0, stream, cfg->grad_dtype, P2D<char>(dOut), rows, cols, dob);
     }
     int rc = CheckCuda(cudaGetLastError(), "bf16 widening launch");
     if (rc != TSA_OK) {

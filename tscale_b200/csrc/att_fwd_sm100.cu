@@ -317,6 +317,8 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
     __syncthreads();
     TcFenceAfter();
     const uint32_t tmem = misc.TmemBase;
+    PdlTrigger(); // behind the allocation: a CTA of the next kernel may hold tensor memory of this SM from here on
+    PdlWait();
     const int *abortFlag = &misc.Abort;
     auto fail = [&](int code) {
         *(volatile int *)&misc.Abort = 1;
@@ -1251,6 +1253,8 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
 // One thread per 16 bytes of a row; rows are rowBytes wide (a multiple of 16), planes have the pitch `pitch`.
 __global__ void __launch_bounds__(256) SplitI8ValuesKernel(P2D<uint8_t> v, int rows, int rowBytes, uint8_t *va, uint8_t *vb, int pitch)
 {
+    PdlTrigger();
+    PdlWait();
     const int perRow = rowBytes / 16;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)rows * perRow) {
@@ -1282,6 +1286,8 @@ __global__ void __launch_bounds__(256) SplitI8ValuesKernel(P2D<uint8_t> v, int r
 constexpr int VREF_CHUNK = 2048;
 __global__ void __launch_bounds__(256) VRefKernel(P2D<float> vScale, int keyRows, float *vRef)
 {
+    PdlTrigger();
+    PdlWait();
     int head = blockIdx.y;
     const float *rowp = vScale.Row(head);
     int t0 = blockIdx.x * VREF_CHUNK;
@@ -1305,6 +1311,8 @@ __global__ void __launch_bounds__(256) VRefKernel(P2D<float> vScale, int keyRows
 constexpr int VREF_ONE_CTA_ROWS = 1 << 18;
 __global__ void __launch_bounds__(1024) VRefHeadKernel(P2D<float> vScale, int keyRows, float *vRef, int *counter)
 {
+    PdlTrigger();
+    PdlWait();
     __shared__ float part[32];
     const int head = blockIdx.x, tid = threadIdx.x;
     const float *rowp = vScale.Row(head);
@@ -1516,7 +1524,7 @@ static int LaunchFwdT2(const CUtensorMap &mq, const CUtensorMap &mk, const CUten
     if (ctas > fp.TotalItems) {
         ctas = fp.TotalItems;
     }
-    kern<<<ctas, FORWARD ? FW_THREADS_FORWARD : FW_THREADS, smemBytes, stream>>>(mq, mk, mv, mv2, fp);
+    LaunchPdlArgs(kern, dim3(ctas), dim3(FORWARD ? FW_THREADS_FORWARD : FW_THREADS), smemBytes, stream, mq, mk, mv, mv2, fp);
     return CheckCuda(cudaGetLastError(), "tcgen05 forward launch");
 }
 
@@ -1570,7 +1578,7 @@ int LaunchSm100Fwd(const tsa_att_cfg *cfg, const TGenParams &p, tsa_ptr2d qk, ts
         }
         if (rc == TSA_OK) {
             const long long items = (long long)keyRows * (rowBytes / 16);
-            SplitI8ValuesKernel<<<(unsigned)((items + 255) / 256), 256, 0, stream>>>(p.V, keyRows, rowBytes, va, vb, pitch);
+            LaunchPdlArgs(SplitI8ValuesKernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, stream, p.V, keyRows, rowBytes, va, vb, pitch);
             rc = CheckCuda(cudaGetLastError(), "int8 value split launch");
         }
     }
@@ -1632,7 +1640,7 @@ int LaunchSm100Fwd(const tsa_att_cfg *cfg, const TGenParams &p, tsa_ptr2d qk, ts
     fp.WithholdTile = g_dump.WithholdTile;
     if (hasVs && keyRows <= VREF_ONE_CTA_ROWS) {
         // one launch writes the per-head maxima and zeroes the counter
-        VRefHeadKernel<<<p.HeadCount, 1024, 0, stream>>>(p.VScale, keyRows, (float *)workspace, fp.Counter);
+        LaunchPdlArgs(VRefHeadKernel, dim3(p.HeadCount), dim3(1024), 0, stream, p.VScale, keyRows, (float *)workspace, fp.Counter);
         rc = CheckCuda(cudaGetLastError(), "value-scale maximum launch");
         if (rc != TSA_OK) {
             return rc;
@@ -1645,7 +1653,7 @@ int LaunchSm100Fwd(const tsa_att_cfg *cfg, const TGenParams &p, tsa_ptr2d qk, ts
         }
         if (hasVs) {
             dim3 vgrid((keyRows + VREF_CHUNK - 1) / VREF_CHUNK, p.HeadCount);
-            VRefKernel<<<vgrid, 256, 0, stream>>>(p.VScale, keyRows, (float *)workspace);
+            LaunchPdlArgs(VRefKernel, vgrid, dim3(256), 0, stream, p.VScale, keyRows, (float *)workspace);
         }
     }
     const bool i8 = cfg->qk_dtype == TSA_I8;

@@ -64,6 +64,8 @@ template <class TIn, class TOut>
 __global__ void __launch_bounds__(256) KvProductKernel(int len, int headCount, int headDim, float kvMult, P2D<typename TIn::T> k,
     P2D<typename TIn::T> val, P2D<typename TOut::T> kv)
 {
+    PdlTrigger();
+    PdlWait();
     const int width = headCount * headDim;
     const int groups = width / 8;
     const long long total = (long long)len * groups;
@@ -92,6 +94,8 @@ template <class TIn, class TGrad>
 __global__ void __launch_bounds__(256) KvProductBwdKernel(int len, int headCount, int headDim, P2D<typename TIn::T> k, P2D<typename TIn::T> val,
     P2D<typename TGrad::T> dkv, P2D<typename TGrad::T> dK, P2D<typename TGrad::T> dVal, P2D<float> dScale)
 {
+    PdlTrigger();
+    PdlWait();
     const int width = headCount * headDim;
     const int groups = width / 8;
     const long long total = (long long)len * groups;
@@ -170,7 +174,7 @@ extern "C" __attribute__((visibility("default"))) int tsa_kv_product(int inDtype
     }
     cudaStream_t s = (cudaStream_t)stream;
     const int grid = CombinerGrid((long long)len * (width / 8));
-#define TSA_KVP(TI, TO) KvProductKernel<TI, TO><<<grid, 256, 0, s>>>(len, headCount, headDim, kvMult, P2D<typename TI::T>(k), P2D<typename TI::T>(valLookup), P2D<typename TO::T>(kv))
+#define TSA_KVP(TI, TO) LaunchPdlArgs(KvProductKernel<TI, TO>, dim3(grid), dim3(256), 0, s, len, headCount, headDim, kvMult, P2D<typename TI::T>(k), P2D<typename TI::T>(valLookup), P2D<typename TO::T>(kv))
     if (inDtype == TSA_F32 && outDtype == TSA_F32) {
         TSA_KVP(TagF32, TagF32);
     } else if (inDtype == TSA_BF16 && outDtype == TSA_BF16) {
@@ -207,7 +211,7 @@ extern "C" __attribute__((visibility("default"))) int tsa_kv_product_bwd(int inD
     }
     cudaStream_t s = (cudaStream_t)stream;
     const int grid = CombinerGrid((long long)len * (width / 8));
-#define TSA_KVB(TI, TG) KvProductBwdKernel<TI, TG><<<grid, 256, 0, s>>>(len, headCount, headDim, P2D<typename TI::T>(k), P2D<typename TI::T>(valLookup), \
+#define TSA_KVB(TI, TG) LaunchPdlArgs(KvProductBwdKernel<TI, TG>, dim3(grid), dim3(256), 0, s, len, headCount, headDim, P2D<typename TI::T>(k), P2D<typename TI::T>(valLookup), \
     P2D<typename TG::T>(dkv), P2D<typename TG::T>(dK), P2D<typename TG::T>(dValLookup), P2D<float>(dScale))
     if (inDtype == TSA_F32 && gradDtype == TSA_F32) {
         TSA_KVB(TagF32, TagF32);

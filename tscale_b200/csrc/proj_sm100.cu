@@ -86,6 +86,8 @@ __global__ void __launch_bounds__(256, 2) ProjNormRopeKernel(const __grid_consta
     TcFenceAfter();
     const uint32_t tmem = misc.TmemBase;
     bool failed = false;
+    PdlTrigger(); // behind the allocation: a CTA of the next kernel may hold tensor memory of this SM from here on
+    PdlWait();
     if (tid == 0) {
         PrefetchTensorMap(&tmX);
         PrefetchTensorMap(&tmW);
@@ -361,5 +363,5 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
         return rc;
     }
     void *args[] = {&mx, &mw, &a, &statusWord};
-    return CheckCuda(cudaLaunchKernel(kern, grid, dim3(256), args, PROJ_SMEM_BYTES, (cudaStream_t)stream), "tsa_matmul_norm_rope_quant launch");
+    return CheckCuda(LaunchPdl(kern, grid, dim3(256), PROJ_SMEM_BYTES, (cudaStream_t)stream, args), "tsa_matmul_norm_rope_quant launch");
 }

@@ -79,6 +79,8 @@ template <class TSrc, bool DST_E4M3, int VEC>
 __global__ void __launch_bounds__(256) QuantRowsKernel(int kind, float vecScale, int len, int rows, int tileCount, int tile,
     P2D<typename TSrc::T> src, P2D<uint8_t> dst, P2D<float> scale)
 {
+    PdlTrigger();
+    PdlWait();
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (warp >= rows * tileCount) {
@@ -167,9 +169,9 @@ static int LaunchQuant(int kind, float vecScale, tsa_ptr2d src, tsa_ptr2d dst, t
     P2D<float> sc(scale);
     bool aligned = ((uintptr_t)src.data % 16 == 0) && (src.stride_bytes % 16 == 0) && ((uintptr_t)dst.data % 4 == 0) && (dst.stride_bytes % 4 == 0);
     if (tile % 128 == 0 && aligned) {
-        QuantRowsKernel<TSrc, DST_E4M3, 4><<<blocks, 256, 0, stream>>>(kind, vecScale, len, rows, tileCount, tile, s, d, sc);
+        LaunchPdlArgs(QuantRowsKernel<TSrc, DST_E4M3, 4>, dim3(blocks), dim3(256), 0, stream, kind, vecScale, len, rows, tileCount, tile, s, d, sc);
     } else {
-        QuantRowsKernel<TSrc, DST_E4M3, 1><<<blocks, 256, 0, stream>>>(kind, vecScale, len, rows, tileCount, tile, s, d, sc);
+        LaunchPdlArgs(QuantRowsKernel<TSrc, DST_E4M3, 1>, dim3(blocks), dim3(256), 0, stream, kind, vecScale, len, rows, tileCount, tile, s, d, sc);
     }
     return CheckCuda(cudaGetLastError(), "tsa_quant_rows launch");
 }
@@ -184,6 +186,8 @@ template <class TSrc, class TRope, bool DST_E4M3, int EPL, int ITEMS, int STEPS>
 __global__ void __launch_bounds__(256) NormRopeQuantKernel(float vecScale, float ropeDir, int len, int rows, int headCount, int headShift,
     P2D<typename TSrc::T> src, P2D<typename TRope::T> rope, P2D<uint8_t> dst, P2D<float> scale)
 {
+    PdlTrigger();
+    PdlWait();
     constexpr int LPB = 32 / EPL;                                   // lanes per 64-element block
     constexpr int STEP_ELEMS = 64 * EPL;                            // elements of a warp step
     const int headDim = 1 << headShift;
@@ -337,7 +341,7 @@ static int LaunchNormRope(bool e4, float vecScale, float ropeDir, tsa_ptr2d src,
     {                                                                                                                           \
         const long long warps = (items + ITEMS - 1) / ITEMS;                                                                    \
         const int blocks = (int)((warps * 32 + 255) / 256);                                                                     \
-        NormRopeQuantKernel<TSrc, TRope, E4, EPL, ITEMS, STEPS><<<blocks, 256, 0, stream>>>(vecScale, ropeDir, len, rows, headCount, headShift, s, r, d, sc); \
+        LaunchPdlArgs(NormRopeQuantKernel<TSrc, TRope, E4, EPL, ITEMS, STEPS>, dim3(blocks), dim3(256), 0, stream, vecScale, ropeDir, len, rows, headCount, headShift, s, r, d, sc); \
     }
     if (steps == 1) {
         if (e4) TSA_NRQ_LAUNCH(true, 2, 1) else TSA_NRQ_LAUNCH(false, 2, 1)
@@ -385,6 +389,8 @@ template <class TSrc, class TGrad, class TRope, int EPL, int STEPS>
 __global__ void __launch_bounds__(256) RopeNormBwdKernel(float ropeDir, int len, int headCount, int headShift,
     P2D<typename TSrc::T> src, P2D<typename TGrad::T> grad, P2D<typename TRope::T> rope, P2D<typename TGrad::T> out)
 {
+    PdlTrigger();
+    PdlWait();
     constexpr int LPB = 32 / EPL;
     constexpr int STEP_ELEMS = 64 * EPL;
     const int headDim = 1 << headShift;
@@ -480,9 +486,9 @@ static int LaunchRopeNormBwd(float ropeDir, tsa_ptr2d src, tsa_ptr2d grad, tsa_p
     P2D<typename TGrad::T> g(grad), o(out);
     P2D<typename TRope::T> r(rope);
     if (steps == 1) {
-        RopeNormBwdKernel<TSrc, TGrad, TRope, EPL, 1><<<blocks, 256, 0, stream>>>(ropeDir, len, headCount, headShift, s, g, r, o);
+        LaunchPdlArgs(RopeNormBwdKernel<TSrc, TGrad, TRope, EPL, 1>, dim3(blocks), dim3(256), 0, stream, ropeDir, len, headCount, headShift, s, g, r, o);
     } else {
-        RopeNormBwdKernel<TSrc, TGrad, TRope, EPL, 2><<<blocks, 256, 0, stream>>>(ropeDir, len, headCount, headShift, s, g, r, o);
+        LaunchPdlArgs(RopeNormBwdKernel<TSrc, TGrad, TRope, EPL, 2>, dim3(blocks), dim3(256), 0, stream, ropeDir, len, headCount, headShift, s, g, r, o);
     }
     return CheckCuda(cudaGetLastError(), "tsa_rope_norm_bwd launch");
 }
@@ -491,6 +497,8 @@ static int LaunchRopeNormBwd(float ropeDir, tsa_ptr2d src, tsa_ptr2d grad, tsa_p
 __global__ void __launch_bounds__(256) DScaleKernel(int outDt, int gradDt, int len, int headCount, int headDim,
     P2D<char> out, P2D<char> dOut, P2D<float> dScale)
 {
+    PdlTrigger();
+    PdlWait();
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (warp >= len * headCount) {
@@ -517,6 +525,8 @@ template <class T16>
 __global__ void __launch_bounds__(256) DScaleVecKernel(int len, int headCount, int headDim, int chunksPerRow,
     P2D<char> out, P2D<char> dOut, P2D<float> dScale)
 {
+    PdlTrigger();
+    PdlWait();
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= (long long)len * chunksPerRow) {
@@ -567,14 +577,14 @@ int LaunchDScale(int outDtype, int gradDtype, tsa_ptr2d out, tsa_ptr2d dOut, tsa
         const long long vecWarps = (long long)len * chunksPerRow;
         const int vblocks = (int)((vecWarps * 32 + 255) / 256);
         if (outDtype == TSA_F16) {
-            DScaleVecKernel<__half><<<vblocks, 256, 0, stream>>>(len, headCount, headDimV, chunksPerRow, P2D<char>(out), P2D<char>(dOut), P2D<float>(dScale));
+            LaunchPdlArgs(DScaleVecKernel<__half>, dim3(vblocks), dim3(256), 0, stream, len, headCount, headDimV, chunksPerRow, P2D<char>(out), P2D<char>(dOut), P2D<float>(dScale));
         } else {
-            DScaleVecKernel<__nv_bfloat16><<<vblocks, 256, 0, stream>>>(len, headCount, headDimV, chunksPerRow, P2D<char>(out), P2D<char>(dOut), P2D<float>(dScale));
+            LaunchPdlArgs(DScaleVecKernel<__nv_bfloat16>, dim3(vblocks), dim3(256), 0, stream, len, headCount, headDimV, chunksPerRow, P2D<char>(out), P2D<char>(dOut), P2D<float>(dScale));
         }
         return CheckCuda(cudaGetLastError(), "tsa_calc_dscale launch");
     }
     int blocks = (int)((warps * 32 + 255) / 256);
-    DScaleKernel<<<blocks, 256, 0, stream>>>(outDtype, gradDtype, len, headCount, headDimV, P2D<char>(out), P2D<char>(dOut), P2D<float>(dScale));
+    LaunchPdlArgs(DScaleKernel, dim3(blocks), dim3(256), 0, stream, outDtype, gradDtype, len, headCount, headDimV, P2D<char>(out), P2D<char>(dOut), P2D<float>(dScale));
     return CheckCuda(cudaGetLastError(), "tsa_calc_dscale launch");
 }
 

@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include <tuple>
 #include "tsa.h"
 
 namespace tsa {
@@ -233,6 +234,17 @@ inline cudaError_t LaunchPdl(const void *kern, dim3 grid, dim3 block, size_t sme
     lc.attrs = attr;
     lc.numAttrs = 1;
     return cudaLaunchKernelExC(&lc, kern, args);
+}
+
+// the same with the kernel's own argument list
+template <class... P, class... A>
+inline cudaError_t LaunchPdlArgs(void (*kern)(P...), dim3 grid, dim3 block, size_t smemBytes, cudaStream_t stream, A... values)
+{
+    std::tuple<P...> list(values...);
+    return std::apply([&](P &...p) {
+        void *args[] = {(void *)&p...};
+        return LaunchPdl((const void *)kern, grid, block, smemBytes, stream, args);
+    }, list);
 }
 
 } // namespace tsa
