@@ -8,42 +8,39 @@
 //   per head: discr = sqrt(sum y^2 / D) * vecScale;  z = y / discr;  rope (elements k and k + 32 of a 64-block);
 //             dst = quantise(z) (int8 or e4m3);  scale[head][t] = discr
 //
-// One CTA = 128 rows of x times 256 output columns (4 heads of 64 or 2 of 128): tcgen05.mma kind::i8, M = 128, N = 256,
-// exact int32 accumulators in 256 tensor-memory columns; thread 0 streams both operands through a TMA ring of 64-column
-// chunks and issues the MMAs.  In the epilogue a row belongs to two threads (256 per CTA), each with half of the tile's
-// heads, so a head's sum of squares, the rotation partners
-// and the 64 output bytes of a block are all in one thread: no exchange between threads, sums in the scalar loop's
-// order (bit-identical to the stand-alone normalise + rope + quantise of the CPU code on the same projection).
+// Persistent: one CTA per SM takes tiles of 128 rows of x times 256 output columns (4 heads of 64 or 2 of 128), tcgen05.mma kind::i8,
+// M = 128, N = 256, exact int32 accumulators in 256 tensor-memory columns, two such sets in turn.  One warp streams both operands
+// through a TMA ring of 64-column chunks that runs on across tiles, one issues the MMAs, and eight work on the epilogue of the tile
+// before: a row belongs to two threads, each with half of the tile's heads, so a head's sum of squares, the rotation partners and the
+// 64 output bytes of a block are all in one thread: no exchange between threads, sums in the scalar loop's order (bit-identical to
+// the stand-alone normalise + rope + quantise of the CPU code on the same projection).  A CTA's tiles are neighbours along the
+// columns, so its rows of x stay in L2 and its rows of the rope table in shared memory.
+// Bound by the operand stream out of L2 (24 KB per 256 clocks of MMA, more than the 64 bytes per clock an SM gets) and the epilogue's
+// issue slots.  Before, two CTAs per SM each ran load, multiply and epilogue in sequence with two chunks in flight: the tensor cores
+// waited for the latency of every chunk.  MEASURED
 #include "att_sm100_common.cuh"
 
 namespace tsa {
 
-// 64-column chunks (64-byte swizzle) keep a CTA's ring at 96 KB, so two CTAs share an SM (2 x 256 tensor-memory
-// columns) and one's epilogue overlaps the other's loads and MMAs
-constexpr int PROJ_STAGES = 4;
+constexpr int PROJ_MAX_STAGES = 9;
 constexpr int PROJ_M = 128, PROJ_N = 256, PROJ_KB = 64;
 constexpr int PROJ_STAGE_BYTES = (PROJ_M + PROJ_N) * PROJ_KB;
-constexpr int PROJ_SMEM_BYTES = PROJ_STAGES * PROJ_STAGE_BYTES + 1024 /* barriers */ + 1024 /* alignment */;
-
-// bounded barrier wait of this kernel: about 20 ms, then the caller records which wait gave up
-__device__ __forceinline__ bool ProjWait(uint64_t *bar, uint32_t parity)
-{
-    const long long t0 = clock64();
-    for (;;) {
-        if (MbarWaitBounded(bar, parity, 16)) {
-            return true;
-        }
-        if (clock64() - t0 > (1ll << 25)) {
-            return false;
-        }
-    }
-}
-constexpr int kProjEmptyTimeout = 0x100, kProjFullTimeout = 0x200, kProjDoneTimeout = 0x400;
+constexpr int PROJ_LOAD_WARP = 0, PROJ_MMA_WARP = 1, PROJ_EPI_WARPS = 8;
+constexpr int PROJ_EPI_THREADS = PROJ_EPI_WARPS * 32, PROJ_THREADS = PROJ_EPI_THREADS + 64;
+constexpr int PROJ_SMEM_MAX = 227 * 1024;
 
 struct TProjMisc {
-    uint64_t Full[PROJ_STAGES], Empty[PROJ_STAGES], Done;
+    uint64_t Full[PROJ_MAX_STAGES], Empty[PROJ_MAX_STAGES]; // ring: copies landed / MMAs that read them retired
+    uint64_t AccFull[2], AccEmpty[2];                        // accumulator set complete / read out (one arrival per epilogue warp)
     uint32_t TmemBase;
+    int Abort; // a bounded wait ran out somewhere in the CTA
 };
+
+__device__ __forceinline__ uint32_t PackBf16(float lo, float hi)
+{
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
 
 struct TProjArgs {
     P2D<float> Rope;  // [len][D] f32, may be absent
@@ -51,243 +48,290 @@ struct TProjArgs {
     P2D<float> Scale; // [H][rows], may be absent
     float VecScale, SrcScale, RopeDir;
     int Len, Rows, HeadCount, Chunks;
+    int ColTiles, Items; // tiles along the output columns, and all of them
+    int Stages;          // of the ring
 };
 
 // X_E4M3: both operands are e4m3 bytes (MulForwardFp8, gpt_cuda.cu:488-491), products accumulate in f32 on the tensor
 // cores (kind::f8f6f4); otherwise int8 x int8 with exact int32 accumulators (kind::i8).
 // DST: TSA_I8, TSA_E4M3 (quantised) or TSA_F16 / TSA_BF16 (the normalised, rotated values themselves: the reference's K16).
 template <int D, int DST, bool X_E4M3>
-__global__ void __launch_bounds__(256, 2) ProjNormRopeKernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, TProjArgs a, int *status)
+__global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, TProjArgs a,
+    int *status)
 {
     // s32 accumulators, s8 x s8 -- or f32 accumulators, e4m3 x e4m3; both operands K-major
     constexpr uint32_t IDESC = X_E4M3 ? MakeInstrDesc(1, 0, 0, 0, 0, PROJ_M, PROJ_N) : MakeInstrDesc(2, 1, 1, 0, 0, PROJ_M, PROJ_N);
     auto accValue = [](uint32_t bits) { return X_E4M3 ? __uint_as_float(bits) : (float)(int32_t)bits; };
-    constexpr int HPC = PROJ_N / D;                                          // heads per CTA
+    constexpr int HPC = PROJ_N / D;                                          // heads per tile
     extern __shared__ uint8_t projSmemRaw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)projSmemRaw + 1023) & ~(uintptr_t)1023);
-    TProjMisc &misc = *reinterpret_cast<TProjMisc *>(smem + PROJ_STAGES * PROJ_STAGE_BYTES);
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int rowBase = blockIdx.x * PROJ_M, colBase = blockIdx.y * PROJ_N;
+    TProjMisc &misc = *reinterpret_cast<TProjMisc *>(smem + a.Stages * PROJ_STAGE_BYTES);
+    float *ropeTile = reinterpret_cast<float *>(smem + a.Stages * PROJ_STAGE_BYTES + 1024);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
-#pragma unroll
-        for (int s = 0; s < PROJ_STAGES; ++s) {
+        for (int s = 0; s < a.Stages; ++s) {
             MbarInit(&misc.Full[s], 1);
             MbarInit(&misc.Empty[s], 1);
         }
-        MbarInit(&misc.Done, 1);
+        for (int b = 0; b < 2; ++b) {
+            MbarInit(&misc.AccFull[b], 1);
+            MbarInit(&misc.AccEmpty[b], PROJ_EPI_WARPS);
+        }
+        misc.Abort = 0;
         FenceBarrierInit();
     }
-    if (warp == 0) {
-        TmemAlloc(&misc.TmemBase, PROJ_N);
+    if (warp == PROJ_MMA_WARP) {
+        TmemAlloc(&misc.TmemBase, 2 * PROJ_N);
         TmemRelinquish();
     }
     TcFenceBefore();
     __syncthreads();
     TcFenceAfter();
     const uint32_t tmem = misc.TmemBase;
-    bool failed = false;
     PdlTrigger(); // behind the allocation: a CTA of the next kernel may hold tensor memory of this SM from here on
     PdlWait();
-    if (tid == 0) {
-        PrefetchTensorMap(&tmX);
-        PrefetchTensorMap(&tmW);
-        auto load = [&](int chunk) {
-            const int s = chunk % PROJ_STAGES;
-            uint8_t *sA = smem + s * PROJ_STAGE_BYTES, *sB = sA + PROJ_M * PROJ_KB;
-            MbarExpectTx(&misc.Full[s], PROJ_STAGE_BYTES);
-            TmaLoad2D(sA, &tmX, chunk * PROJ_KB, rowBase, &misc.Full[s]);
-            TmaLoad2D(sB, &tmW, chunk * PROJ_KB, colBase, &misc.Full[s]);
-        };
-        // PROJ_AHEAD chunks in flight; a stage is refilled once the MMAs of two iterations ago have released it
-        constexpr int PROJ_AHEAD = PROJ_STAGES - 2;
-        const int chunks = a.Chunks;
-        int issued = 0, landed = 0; // chunks requested / chunks whose copies were seen to arrive
-        for (int c = 0; c < PROJ_AHEAD && c < chunks; ++c) {
-            load(c);
-            ++issued;
+    const int *abortFlag = &misc.Abort;
+    auto fail = [&](int code) {
+        *(volatile int *)&misc.Abort = 1;
+        if (status) {
+            atomicOr(status, code);
         }
-        for (int c = 0; c < chunks; ++c) {
-            const int ahead = c + PROJ_AHEAD;
-            if (ahead < chunks) {
-                if (ahead >= PROJ_STAGES && !ProjWait(&misc.Empty[ahead % PROJ_STAGES], (uint32_t)((ahead / PROJ_STAGES - 1) & 1))) {
-                    failed = true;
-                    if (status) {
-                        atomicOr(status, kDevTimeoutMma | kProjEmptyTimeout);
+    };
+    const int itemBegin = (int)((long long)a.Items * blockIdx.x / gridDim.x), itemEnd = (int)((long long)a.Items * (blockIdx.x + 1) / gridDim.x);
+    if (warp == PROJ_LOAD_WARP) {
+        if (lane == 0) {
+            PrefetchTensorMap(&tmX);
+            PrefetchTensorMap(&tmW);
+            int s = 0, phase = 0, requested = 0; // ring slot, its parity, chunks requested
+            bool failed = false;
+            for (int item = itemBegin; item < itemEnd && !failed; ++item) {
+                const int rowBase = item / a.ColTiles * PROJ_M, colBase = item % a.ColTiles * PROJ_N;
+                for (int c = 0; c < a.Chunks; ++c) {
+                    if (requested >= a.Stages && !WaitBarA(&misc.Empty[s], phase ^ 1, abortFlag)) {
+                        failed = true;
+                        fail(kDevTimeoutMma);
+                        break;
                     }
+                    uint8_t *sA = smem + s * PROJ_STAGE_BYTES;
+                    MbarExpectTx(&misc.Full[s], PROJ_STAGE_BYTES);
+                    TmaLoad2D(sA, &tmX, c * PROJ_KB, rowBase, &misc.Full[s]);
+                    TmaLoad2D(sA + PROJ_M * PROJ_KB, &tmW, c * PROJ_KB, colBase, &misc.Full[s]);
+                    ++requested;
+                    if (++s == a.Stages) {
+                        s = 0;
+                        phase ^= 1;
+                    }
+                }
+            }
+            if (failed || *(volatile int *)&misc.Abort) {
+                // copies that were requested but never consumed must not land after the CTA is gone: wait (bounded) for them
+                for (int k = max(0, requested - a.Stages); k < requested; ++k) {
+                    WaitBar(&misc.Full[k % a.Stages], (k / a.Stages) & 1);
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == PROJ_MMA_WARP) {
+        // the whole warp runs the loop and the waits, one elected lane issues (descriptors stay in uniform registers that way)
+        int s = 0, phase = 0, n = 0;
+        bool failed = false;
+        auto wait = [&](uint64_t *bar, uint32_t parity, int code) {
+            if (!__all_sync(0xffffffffu, WaitBarA(bar, parity, abortFlag))) {
+                failed = true;
+                if (lane == 0) {
+                    fail(code);
+                }
+            }
+            return !failed;
+        };
+        for (int item = itemBegin; item < itemEnd && !failed; ++item, ++n) {
+            const uint32_t acc = tmem + (n & 1) * PROJ_N;
+            if (n >= 2 && !wait(&misc.AccEmpty[n & 1], ((n >> 1) - 1) & 1, kDevTimeoutMma)) {
+                break;
+            }
+            for (int c = 0; c < a.Chunks; ++c) {
+                if (!wait(&misc.Full[s], phase, kDevTimeoutTma)) {
                     break;
                 }
-                load(ahead);
-                ++issued;
-            }
-            const int s = c % PROJ_STAGES;
-            if (!ProjWait(&misc.Full[s], (uint32_t)((c / PROJ_STAGES) & 1))) {
-                failed = true;
-                if (status) {
-                    atomicOr(status, kDevTimeoutTma | kProjFullTimeout);
-                }
-                break;
-            }
-            ++landed;
-            TcFenceAfter();
-            const uint32_t sA = SmemAddr(smem + s * PROJ_STAGE_BYTES), sB = sA + PROJ_M * PROJ_KB;
+                TcFenceAfter();
+                if (ElectOne()) {
+                    const uint32_t sA = SmemAddr(smem + s * PROJ_STAGE_BYTES), sB = sA + PROJ_M * PROJ_KB;
 #pragma unroll
-            for (int ks = 0; ks < PROJ_KB / 32; ++ks) {
-                const uint64_t aDesc = MakeSmemDesc(sA + ks * 32, 16, 8 * PROJ_KB, PROJ_KB);
-                const uint64_t bDesc = MakeSmemDesc(sB + ks * 32, 16, 8 * PROJ_KB, PROJ_KB);
-                if (X_E4M3) {
-                    MmaF8SS(tmem, aDesc, bDesc, IDESC, (c > 0 || ks > 0) ? 1u : 0u);
-                } else {
-                    MmaI8SS(tmem, aDesc, bDesc, IDESC, (c > 0 || ks > 0) ? 1u : 0u);
-                }
-            }
-            MmaCommit(&misc.Empty[s]);
-        }
-        if (failed) {
-            // copies that were requested but never consumed must not land after the CTA is gone: wait (bounded) for them
-            for (int t = landed; t < issued; ++t) {
-                ProjWait(&misc.Full[t % PROJ_STAGES], (uint32_t)((t / PROJ_STAGES) & 1));
-            }
-        }
-        MmaCommit(&misc.Done);
-    }
-    if (!ProjWait(&misc.Done, 0)) {
-        failed = true;
-        if (status) {
-            atomicOr(status, kDevTimeoutMma | kProjDoneTimeout);
-        }
-    }
-    TcFenceAfter();
-    failed = __syncthreads_or(failed ? 1 : 0) != 0;
-
-    // every thread of a warp takes part in the tensor-memory loads (they are warp-wide instructions): rows past the
-    // buffer only skip their global loads and stores
-    const int rowInTile = tid & (PROJ_M - 1), colHalf = tid >> 7; // two threads per row: each takes half of the tile's heads
-    const int t = rowBase + rowInTile;
-    const bool inBuf = t < a.Rows;
-    // the tile's rows of the rope table through shared memory (the ring is idle now): coalesced loads, and a row pitch
-    // of D + 1 words lets every thread walk its own row without bank conflicts
-    float *ropeTile = reinterpret_cast<float *>(smem);
-    const bool withRope = a.Rope.Valid();
-    if (!failed && withRope) {
-        for (int idx = tid; idx < PROJ_M * (D / 4); idx += 256) {
-            const int row = idx / (D / 4), c4 = idx - row * (D / 4);
-            float4 v = make_float4(0, 0, 0, 0);
-            if (rowBase + row < a.Len) {
-                v = *reinterpret_cast<const float4 *>(a.Rope.Row(rowBase + row) + c4 * 4);
-            }
-            float *dstRope = ropeTile + row * (D + 1) + c4 * 4;
-            dstRope[0] = v.x, dstRope[1] = v.y, dstRope[2] = v.z, dstRope[3] = v.w;
-        }
-        __syncthreads();
-    }
-    if (!failed) {
-        const uint32_t tLane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-        const bool live = t < a.Len;
-#pragma unroll 1
-        for (int hh = colHalf * (HPC / 2); hh < (colHalf + 1) * (HPC / 2); ++hh) {
-            const int head = blockIdx.y * HPC + hh;
-            if (head >= a.HeadCount) {
-                break;
-            }
-            // sum of squares of the head in column order, one rounding per product and per sum
-            float sum2 = 0;
-#pragma unroll 1
-            for (int c0 = 0; c0 < D; c0 += 32) {
-                uint32_t r[32];
-                TmemLd32(tLane + hh * D + c0, r);
-                TmemWaitLd();
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float y = __fmul_rn(accValue(r[i]), a.SrcScale);
-                    sum2 = __fadd_rn(sum2, __fmul_rn(y, y));
-                }
-            }
-            float discr = 0;
-            if (sum2 > 0 && live) {
-                discr = __fmul_rn(__fsqrt_rn(__fdiv_rn(sum2, (float)D)), a.VecScale);
-            }
-            const float mult = discr > 0 ? __fdiv_rn(1.0f, discr) : 0.0f;
-            constexpr int ES = (DST == TSA_F16 || DST == TSA_BF16) ? 2 : 1; // bytes per output element
-            uint8_t *dstRow = a.Dst.Row(inBuf ? t : 0) + head * D * ES;
-#pragma unroll 1
-            for (int blk = 0; blk < D; blk += 64) {
-                uint32_t lo[32], hi[32];
-                TmemLd32(tLane + hh * D + blk, lo);
-                TmemLd32(tLane + hh * D + blk + 32, hi);
-                TmemWaitLd();
-                uint32_t outLo[8], outHi[8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    float z0[4], z1[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int k = q * 4 + i;
-                        float y0 = __fmul_rn(__fmul_rn(accValue(lo[k]), a.SrcScale), mult);
-                        float y1 = __fmul_rn(__fmul_rn(accValue(hi[k]), a.SrcScale), mult);
-                        if (withRope && live) {
-                            const float cs = ropeTile[rowInTile * (D + 1) + blk + k];
-                            const float sn = __fmul_rn(ropeTile[rowInTile * (D + 1) + blk + k + 32], a.RopeDir);
-                            const float r0 = __fsub_rn(__fmul_rn(y0, cs), __fmul_rn(y1, sn));
-                            const float r1 = __fadd_rn(__fmul_rn(y0, sn), __fmul_rn(y1, cs));
-                            y0 = r0;
-                            y1 = r1;
-                        }
-                        z0[i] = y0;
-                        z1[i] = y1;
-                    }
-                    if (ES == 2) {
-                        uint2 w0, w1;
-                        if (DST == TSA_F16) {
-                            const __half2 a0 = __floats2half2_rn(z0[0], z0[1]), a1 = __floats2half2_rn(z0[2], z0[3]);
-                            const __half2 b0 = __floats2half2_rn(z1[0], z1[1]), b1 = __floats2half2_rn(z1[2], z1[3]);
-                            w0 = make_uint2(*reinterpret_cast<const uint32_t *>(&a0), *reinterpret_cast<const uint32_t *>(&a1));
-                            w1 = make_uint2(*reinterpret_cast<const uint32_t *>(&b0), *reinterpret_cast<const uint32_t *>(&b1));
+                    for (int ks = 0; ks < PROJ_KB / 32; ++ks) {
+                        const uint64_t aDesc = MakeSmemDesc(sA + ks * 32, 16, 8 * PROJ_KB, PROJ_KB);
+                        const uint64_t bDesc = MakeSmemDesc(sB + ks * 32, 16, 8 * PROJ_KB, PROJ_KB);
+                        if (X_E4M3) {
+                            MmaF8SS(acc, aDesc, bDesc, IDESC, (c > 0 || ks > 0) ? 1u : 0u);
                         } else {
-                            const __nv_bfloat162 a0 = __floats2bfloat162_rn(z0[0], z0[1]), a1 = __floats2bfloat162_rn(z0[2], z0[3]);
-                            const __nv_bfloat162 b0 = __floats2bfloat162_rn(z1[0], z1[1]), b1 = __floats2bfloat162_rn(z1[2], z1[3]);
-                            w0 = make_uint2(*reinterpret_cast<const uint32_t *>(&a0), *reinterpret_cast<const uint32_t *>(&a1));
-                            w1 = make_uint2(*reinterpret_cast<const uint32_t *>(&b0), *reinterpret_cast<const uint32_t *>(&b1));
-                        }
-                        if (inBuf) {
-                            *reinterpret_cast<uint2 *>(dstRow + (blk + q * 4) * 2) = w0;
-                            *reinterpret_cast<uint2 *>(dstRow + (blk + 32 + q * 4) * 2) = w1;
-                        }
-                    } else if (DST == TSA_E4M3) {
-                        outLo[q] = PackE4M3x4(z0[0], z0[1], z0[2], z0[3]);
-                        outHi[q] = PackE4M3x4(z1[0], z1[1], z1[2], z1[3]);
-                    } else {
-                        outLo[q] = 0;
-                        outHi[q] = 0;
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            outLo[q] |= (uint32_t)(FloatToI8Sat(z0[i]) & 0xff) << (8 * i);
-                            outHi[q] |= (uint32_t)(FloatToI8Sat(z1[i]) & 0xff) << (8 * i);
+                            MmaI8SS(acc, aDesc, bDesc, IDESC, (c > 0 || ks > 0) ? 1u : 0u);
                         }
                     }
+                    MmaCommit(&misc.Empty[s]);
+                    if (c == a.Chunks - 1) {
+                        MmaCommit(&misc.AccFull[n & 1]);
+                    }
                 }
-                if (inBuf && ES == 1) {
-                    if ((((uintptr_t)a.Dst.Data | (uintptr_t)a.Dst.Stride) & 31) == 0) {
-                        // two 32-byte stores: whole sectors from a thread that owns the row
-                        StGlobal256(dstRow + blk, outLo);
-                        StGlobal256(dstRow + blk + 32, outHi);
-                    } else {
-                        uint4 *d4 = reinterpret_cast<uint4 *>(dstRow + blk);
-                        d4[0] = make_uint4(outLo[0], outLo[1], outLo[2], outLo[3]);
-                        d4[1] = make_uint4(outLo[4], outLo[5], outLo[6], outLo[7]);
-                        d4[2] = make_uint4(outHi[0], outHi[1], outHi[2], outHi[3]);
-                        d4[3] = make_uint4(outHi[4], outHi[5], outHi[6], outHi[7]);
+                __syncwarp();
+                if (++s == a.Stages) {
+                    s = 0;
+                    phase ^= 1;
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        constexpr int BAR_EPI = 1;
+        const int quad = warp & 3, colHalf = (warp - 2) >> 2; // tensor-memory lanes of the warp; two threads per row: each takes half of the tile's heads
+        const int rowInTile = quad * 32 + lane;
+        const bool withRope = a.Rope.Valid();
+        // 32 bytes of a row: one store (a whole sector) where the rows allow it
+        const bool wideStores = (((uintptr_t)a.Dst.Data | (uintptr_t)a.Dst.Stride) & 31) == 0;
+        auto store32 = [&](uint8_t *dst, const uint32_t *w) {
+            if (wideStores) {
+                StGlobal256(dst, w);
+            } else {
+                reinterpret_cast<uint4 *>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                reinterpret_cast<uint4 *>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+            }
+        };
+        int ropeRow = -1, n = 0; // first row of the rope table's rows in shared memory
+        bool failed = false;
+        for (int item = itemBegin; item < itemEnd; ++item, ++n) {
+            const int rowBase = item / a.ColTiles * PROJ_M, headBase = item % a.ColTiles * HPC;
+            if (!WaitBarA(&misc.AccFull[n & 1], (n >> 1) & 1, abortFlag)) {
+                failed = true;
+                fail(kDevTimeoutMma);
+            }
+            // one vote of the epilogue threads per tile, so that they leave together; it also says that all of them are done with the rope
+            // rows of the tile before
+            if (BarRedOr(BAR_EPI, PROJ_EPI_THREADS, failed)) {
+                break;
+            }
+            TcFenceAfter();
+            // every thread of a warp takes part in the tensor-memory loads (they are warp-wide instructions): rows past the
+            // buffer only skip their global loads and stores
+            const int t = rowBase + rowInTile;
+            const bool inBuf = t < a.Rows;
+            // the rows of the rope table through shared memory: coalesced loads, and a row pitch of D + 1 words lets every thread walk its
+            // own row without bank conflicts
+            if (withRope && ropeRow != rowBase) {
+                ropeRow = rowBase;
+#pragma unroll 4
+                for (int idx = tid - 64; idx < PROJ_M * (D / 4); idx += PROJ_EPI_THREADS) {
+                    const int row = idx / (D / 4), c4 = idx - row * (D / 4);
+                    float4 v = make_float4(0, 0, 0, 0);
+                    if (rowBase + row < a.Len) {
+                        v = *reinterpret_cast<const float4 *>(a.Rope.Row(rowBase + row) + c4 * 4);
+                    }
+                    float *dstRope = ropeTile + row * (D + 1) + c4 * 4;
+                    dstRope[0] = v.x, dstRope[1] = v.y, dstRope[2] = v.z, dstRope[3] = v.w;
+                }
+                BarSync(BAR_EPI, PROJ_EPI_THREADS);
+            }
+            {
+                const uint32_t tLane = tmem + (n & 1) * PROJ_N + ((uint32_t)(quad * 32) << 16);
+                const bool live = t < a.Len;
+#pragma unroll 1
+                for (int hh = colHalf * (HPC / 2); hh < (colHalf + 1) * (HPC / 2); ++hh) {
+                    const int head = headBase + hh;
+                    if (head >= a.HeadCount) {
+                        break;
+                    }
+                    // sum of squares of the head in column order, one rounding per product and per sum
+                    float sum2 = 0;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < D; c0 += 32) {
+                        uint32_t r[32];
+                        TmemLd32(tLane + hh * D + c0, r);
+                        TmemWaitLd();
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            const float y = __fmul_rn(accValue(r[i]), a.SrcScale);
+                            sum2 = __fadd_rn(sum2, __fmul_rn(y, y));
+                        }
+                    }
+                    float discr = 0;
+                    if (sum2 > 0 && live) {
+                        discr = __fmul_rn(__fsqrt_rn(__fdiv_rn(sum2, (float)D)), a.VecScale);
+                    }
+                    const float mult = discr > 0 ? __fdiv_rn(1.0f, discr) : 0.0f;
+                    constexpr int ES = (DST == TSA_F16 || DST == TSA_BF16) ? 2 : 1; // bytes per output element
+                    uint8_t *dstRow = a.Dst.Row(inBuf ? t : 0) + head * D * ES;
+#pragma unroll 1
+                    for (int blk = 0; blk < D; blk += 64) {
+                        uint32_t lo[32], hi[32];
+                        TmemLd32(tLane + hh * D + blk, lo);
+                        TmemLd32(tLane + hh * D + blk + 32, hi);
+                        TmemWaitLd();
+                        uint32_t outLo[8], outHi[8];
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            float z0[4], z1[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const int k = q * 4 + i;
+                                float y0 = __fmul_rn(__fmul_rn(accValue(lo[k]), a.SrcScale), mult);
+                                float y1 = __fmul_rn(__fmul_rn(accValue(hi[k]), a.SrcScale), mult);
+                                if (withRope && live) {
+                                    const float cs = ropeTile[rowInTile * (D + 1) + blk + k];
+                                    const float sn = __fmul_rn(ropeTile[rowInTile * (D + 1) + blk + k + 32], a.RopeDir);
+                                    const float r0 = __fsub_rn(__fmul_rn(y0, cs), __fmul_rn(y1, sn));
+                                    const float r1 = __fadd_rn(__fmul_rn(y0, sn), __fmul_rn(y1, cs));
+                                    y0 = r0;
+                                    y1 = r1;
+                                }
+                                z0[i] = y0;
+                                z1[i] = y1;
+                            }
+                            if (ES == 2) {
+                                // eight words = 16 columns = 32 bytes at a time
+                                const int w0 = 2 * (q & 3);
+                                if (DST == TSA_F16) {
+                                    outLo[w0] = PackHalf2(z0[0], z0[1]), outLo[w0 + 1] = PackHalf2(z0[2], z0[3]);
+                                    outHi[w0] = PackHalf2(z1[0], z1[1]), outHi[w0 + 1] = PackHalf2(z1[2], z1[3]);
+                                } else {
+                                    outLo[w0] = PackBf16(z0[0], z0[1]), outLo[w0 + 1] = PackBf16(z0[2], z0[3]);
+                                    outHi[w0] = PackBf16(z1[0], z1[1]), outHi[w0 + 1] = PackBf16(z1[2], z1[3]);
+                                }
+                                if ((q & 3) == 3 && inBuf) {
+                                    store32(dstRow + (blk + (q - 3) * 4) * 2, outLo);
+                                    store32(dstRow + (blk + 32 + (q - 3) * 4) * 2, outHi);
+                                }
+                            } else if (DST == TSA_E4M3) {
+                                outLo[q] = PackE4M3x4(z0[0], z0[1], z0[2], z0[3]);
+                                outHi[q] = PackE4M3x4(z1[0], z1[1], z1[2], z1[3]);
+                            } else {
+                                outLo[q] = 0;
+                                outHi[q] = 0;
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    outLo[q] |= (uint32_t)(FloatToI8Sat(z0[i]) & 0xff) << (8 * i);
+                                    outHi[q] |= (uint32_t)(FloatToI8Sat(z1[i]) & 0xff) << (8 * i);
+                                }
+                            }
+                        }
+                        if (inBuf && ES == 1) {
+                            store32(dstRow + blk, outLo);
+                            store32(dstRow + blk + 32, outHi);
+                        }
+                    }
+                    if (a.Scale.Valid() && inBuf) {
+                        a.Scale.Row(head)[t] = discr;
                     }
                 }
             }
-            if (a.Scale.Valid() && inBuf) {
-                a.Scale.Row(head)[t] = discr;
+            // this warp has read the accumulators for the last time
+            TcFenceBefore();
+            __syncwarp();
+            if (lane == 0) {
+                MbarArrive(&misc.AccEmpty[n & 1]);
             }
         }
     }
     TcFenceBefore();
     __syncthreads();
-    if (warp == 0) {
-        TmemDealloc(tmem, PROJ_N);
+    if (warp == PROJ_MMA_WARP) {
+        TmemDealloc(tmem, 2 * PROJ_N);
     }
 }
 
@@ -344,7 +388,21 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     a.Rows = dst.ysize;
     a.HeadCount = headCount;
     a.Chunks = dim / PROJ_KB;
-    dim3 grid((dst.ysize + PROJ_M - 1) / PROJ_M, (outCols + PROJ_N - 1) / PROJ_N);
+    a.ColTiles = (outCols + PROJ_N - 1) / PROJ_N;
+    a.Items = (dst.ysize + PROJ_M - 1) / PROJ_M * a.ColTiles;
+    // as many ring stages as fit beside the rope rows
+    const int ropeBytes = rope.data ? PROJ_M * (headDim + 1) * (int)sizeof(float) : 0;
+    a.Stages = (PROJ_SMEM_MAX - 2048 - ropeBytes) / PROJ_STAGE_BYTES;
+    a.Stages = a.Stages < PROJ_MAX_STAGES ? a.Stages : PROJ_MAX_STAGES;
+    const int smemBytes = a.Stages * PROJ_STAGE_BYTES + 1024 /* barriers */ + 1024 /* alignment */ + ropeBytes;
+    int dev = 0, sms = 0;
+    rc = CheckCuda(cudaGetDevice(&dev), "cudaGetDevice");
+    if (rc == TSA_OK) {
+        rc = CheckCuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+    }
+    if (rc != TSA_OK) {
+        return rc;
+    }
     const bool x8 = srcDtype == TSA_E4M3;
     const void *kern = nullptr;
 #define TSA_PROJ_CASE(DD, DT, X8)                                       \
@@ -358,10 +416,10 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     TSA_PROJ_CASES(128, true)
 #undef TSA_PROJ_CASES
 #undef TSA_PROJ_CASE
-    rc = CheckCuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PROJ_SMEM_BYTES), "cudaFuncSetAttribute");
+    rc = CheckCuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes), "cudaFuncSetAttribute");
     if (rc != TSA_OK) {
         return rc;
     }
     void *args[] = {&mx, &mw, &a, &statusWord};
-    return CheckCuda(LaunchPdl(kern, grid, dim3(256), PROJ_SMEM_BYTES, (cudaStream_t)stream, args), "tsa_matmul_norm_rope_quant launch");
+    return CheckCuda(LaunchPdl(kern, dim3(a.Items < sms ? a.Items : sms), dim3(PROJ_THREADS), smemBytes, (cudaStream_t)stream, args), "tsa_matmul_norm_rope_quant launch");
 }
