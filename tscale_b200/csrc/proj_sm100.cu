@@ -17,7 +17,8 @@
 // columns, so its rows of x stay in L2 and its rows of the rope table in shared memory.
 // Bound by the operand stream out of L2 (24 KB per 256 clocks of MMA, more than the 64 bytes per clock an SM gets) and the epilogue's
 // issue slots.  Before, two CTAs per SM each ran load, multiply and epilogue in sequence with two chunks in flight: the tensor cores
-// waited for the latency of every chunk.  MEASURED
+// waited for the latency of every chunk.  12345 rows x 2048 -> 16 heads of 128: 82 us (66 to 96 with the variant) before, 67 to 74 now,
+// where 67 us is the 24-KB stages through L2 at 9 TB/s; the four projections and the attention of a block 752 -> 606 us.
 #include "att_sm100_common.cuh"
 
 namespace tsa {
