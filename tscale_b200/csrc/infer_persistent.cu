@@ -20,7 +20,7 @@
 // Measured, twelve layers, dim 768, 12 heads x 64, vocabulary 50304, a whole token with the final layer and softmax:
 //     1 sequence, 500 tokens of context       750 -> 320 us, of which about 240 us are the sixty phases at some 4 us each: the
 //                                             barrier, the sums through L2 and the norm, in a chain; the bytes take 20 us
-//     64 sequences, 1024 to 8192 tokens       970 -> 870 us (three of four layers see 64 tokens); 200 us are the bytes of the wide
+//     64 sequences, 1024 to 8192 tokens       970 -> 825 us (three of four layers see 64 tokens); 200 us are the bytes of the wide
 //                                             layers' caches, the phases around them come on top, unoverlapped
 #include "att_sm100_common.cuh"
 #include "decode_device.cuh"
@@ -39,7 +39,7 @@ constexpr int PS_B_BYTES = INF_MAX_SEQ * 128;  // the chunk's vectors, one row o
 constexpr int PS_F_PITCH = 132;                // floats per row of the fp32 chunk: 16-byte rows that fall into different banks
 constexpr int PS_MERGE_PITCH = 19;
 constexpr int PS_LAYERS = 32;                  // layers per launch
-constexpr int PS_MAX_SLOTS = 1024;             // attention chunks whose partials the workspace holds, at least
+constexpr int PS_MAX_SLOTS = 1024;             // attention units whose partials the workspace holds, at least
 constexpr int PS_MIN_CHUNK = 64;               // keys: two batches of eight for each of a group's four warps
 constexpr long long PS_WAIT_CYCLES = 1ll << 31;
 
@@ -86,15 +86,17 @@ struct alignas(16) TAttGroupSmem {
     float Mult[4][8];
     int8_t Q8[512], K8[512];
     float Merge[4][32][PS_MERGE_PITCH];
-    tsa_kv_seq Seq;               // the group's unit: its sequence's cache, position of the new token,
-    int Pos, SeqIndex, HeadGroup, Chunk, Chunks; // which unit it is
+    tsa_kv_seq Seq;               // the group's chunk: its sequence's cache, position of the new token,
+    int Pos, SeqIndex, HeadGroup, Chunk, Chunks; // which of the chunks of which row it is,
+    int KeyBeg, KeyEnd;           // its keys, counted from the first the row attends,
+    int Next;                     // and where in the stream the unit goes on, -1: this was its last chunk
     int Last;
 };
 
-// Chunks of the attention of one layer (see MakeAttPlan).
+// Units of the attention of one layer (see MakeAttPlan).
 struct TAttPlan {
-    int Window, Chunk, Units;
-    int Base[INF_MAX_SEQ], Keys[INF_MAX_SEQ]; // first unit and keys of each sequence
+    int Window, Quantum, Units;               // Quantum: blocks of 32 keys per unit
+    int Base[INF_MAX_SEQ], Len[INF_MAX_SEQ];  // first block of each sequence in the stream, and their number
 };
 
 // one 128 x 128 weight tile of the CTA's share of a layer
@@ -527,9 +529,12 @@ __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm
 }
 
 // ---- attention -----------------------------------------------------------------------------------------------------
-// A unit = one sequence x one head group (the heads a warp-wide 16-byte load covers: 8 of 64 or 4 of 128) x one chunk of keys,
-// taken by a group of four warps that split the chunk's keys.  All chunks have the same size, the smallest multiple of 32 (at least
-// PS_MIN_CHUNK) whose units all fit the resident groups of the grid in one wave; the plan is a bisection, done once per window and launch.
+// The keys of all sequences, one behind the other, are cut into ranges of the same size: as many as the grid has groups of four
+// warps for each head group (the heads a warp-wide 16-byte load covers: 8 of 64 or 4 of 128).  A unit = one range x one head group,
+// taken by one group; its parts that belong to different sequences are its chunks, whose keys the four warps split.  With chunks
+// that all had one size and ended with their sequence, 64 sequences of 1024 to 8192 tokens kept a fifth of the groups idle at the
+// end of the phase (a token of the twelve-layer model 870 us, now 825).  A sequence counts with at least PS_MIN_CHUNK keys, which is also the least size of a range: short contexts and
+// narrow windows stay one chunk, and one group each.
 __device__ __forceinline__ int StepKeys(const TStepParams &p, const TStepLayer &layer, int s)
 {
     if (s >= p.NSeq) {
@@ -548,59 +553,52 @@ __device__ __forceinline__ int StepKeys(const TStepParams &p, const TStepLayer &
 __device__ __noinline__ void MakeAttPlan(const TStepParams &p, const TStepLayer &layer, TAttPlan &plan)
 {
     const int lane = threadIdx.x & 31;
-    const int slots = max((int)gridDim.x * PS_GROUPS, p.NSeq * p.HeadGroups);
-    const int keys0 = StepKeys(p, layer, lane), keys1 = StepKeys(p, layer, lane + 32);
-    const bool on0 = lane < p.NSeq, on1 = lane + 32 < p.NSeq;
-    // every sequence has at least one unit per head group: it appends the new token
-    auto units = [&](int keys, bool on, int chunk) { return on ? p.HeadGroups * max(1, (keys + chunk - 1) / chunk) : 0; };
-    const int total = __reduce_add_sync(0xffffffffu, keys0 + keys1), most = __reduce_max_sync(0xffffffffu, max(keys0, keys1));
-    int lo = max(PS_MIN_CHUNK / 32, (int)(((long long)total * p.HeadGroups / slots) / 32)), hi = max((most + 31) / 32, lo);
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        const int n = __reduce_add_sync(0xffffffffu, units(keys0, on0, mid * 32) + units(keys1, on1, mid * 32));
-        if (n <= slots) {
-            hi = mid;
-        } else {
-            lo = mid + 1;
-        }
-    }
-    const int u0 = units(keys0, on0, lo * 32), u1 = units(keys1, on1, lo * 32);
-    int i0 = u0, i1 = u1;
+    const int ranges = max((int)gridDim.x * PS_GROUPS / p.HeadGroups, 1);
+    // blocks of 32 keys; every sequence has at least one chunk per head group: it appends the new token
+    auto blocks = [&](int s) { return s < p.NSeq ? (max(StepKeys(p, layer, s), PS_MIN_CHUNK) + 31) / 32 : 0; };
+    const int n0 = blocks(lane), n1 = blocks(lane + 32);
+    int i0 = n0, i1 = n1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int a = __shfl_up_sync(0xffffffffu, i0, o), b = __shfl_up_sync(0xffffffffu, i1, o);
         i0 += lane >= o ? a : 0;
         i1 += lane >= o ? b : 0;
     }
-    const int sum0 = __shfl_sync(0xffffffffu, i0, 31);
-    plan.Base[lane] = i0 - u0;
-    plan.Base[lane + 32] = sum0 + i1 - u1;
-    plan.Keys[lane] = keys0;
-    plan.Keys[lane + 32] = keys1;
-    if (lane == 31) {
-        plan.Chunk = lo * 32;
-        plan.Units = sum0 + i1;
+    const int sum0 = __shfl_sync(0xffffffffu, i0, 31), total = sum0 + __shfl_sync(0xffffffffu, i1, 31);
+    plan.Base[lane] = i0 - n0;
+    plan.Base[lane + 32] = sum0 + i1 - n1;
+    plan.Len[lane] = n0;
+    plan.Len[lane + 32] = n1;
+    if (lane == 0) {
+        const int quantum = max((total + ranges - 1) / ranges, PS_MIN_CHUNK / 32);
+        plan.Quantum = quantum;
+        plan.Units = (total + quantum - 1) / quantum * p.HeadGroups;
         plan.Window = layer.Window;
     }
     __syncwarp();
 }
 
-// which unit is number `unit`, and its sequence's cache, into the group's shared memory (one warp)
-__device__ __noinline__ void LocateUnit(const TStepParams &p, const TStepLayer &layer, const TAttPlan &plan, int unit, TAttGroupSmem &g)
+// the chunk of unit number `unit` that begins at block `at` of the stream, and its sequence's cache, into the group's shared memory
+// (one warp)
+__device__ __noinline__ void LocateChunk(const TStepParams &p, const TStepLayer &layer, const TAttPlan &plan, int unit, int at, TAttGroupSmem &g)
 {
     const int lane = threadIdx.x & 31;
-    // the sequence whose units contain this one: the last with Base <= unit
-    const unsigned at0 = __ballot_sync(0xffffffffu, lane < p.NSeq && plan.Base[lane] <= unit);
-    const unsigned at1 = __ballot_sync(0xffffffffu, lane + 32 < p.NSeq && plan.Base[lane + 32] <= unit);
+    // the sequence this block belongs to: the last with Base <= at
+    const unsigned at0 = __ballot_sync(0xffffffffu, lane < p.NSeq && plan.Base[lane] <= at);
+    const unsigned at1 = __ballot_sync(0xffffffffu, lane + 32 < p.NSeq && plan.Base[lane + 32] <= at);
     const int seq = at1 ? 63 - __clz(at1) : 31 - __clz(at0);
-    const int chunks = max(1, (plan.Keys[seq] + plan.Chunk - 1) / plan.Chunk), rel = unit - plan.Base[seq], chunk = rel / p.HeadGroups;
     if (lane == 0) {
+        const int range = unit / p.HeadGroups, base = plan.Base[seq], seqEnd = base + plan.Len[seq], unitEnd = (range + 1) * plan.Quantum;
+        const int firstRange = base / plan.Quantum;
         g.Pos = layer.CtxLens[seq];
         g.Seq = layer.Seqs[seq];
         g.SeqIndex = seq;
-        g.HeadGroup = rel - chunk * p.HeadGroups;
-        g.Chunk = chunk;
-        g.Chunks = chunks;
+        g.HeadGroup = unit - range * p.HeadGroups;
+        g.Chunk = range - firstRange;
+        g.Chunks = (seqEnd - 1) / plan.Quantum - firstRange + 1;
+        g.KeyBeg = (at - base) * 32;
+        g.KeyEnd = (min(seqEnd, unitEnd) - base) * 32;
+        g.Next = seqEnd < unitEnd && seq + 1 < p.NSeq ? seqEnd : -1;
     }
     __syncwarp();
 }
@@ -746,9 +744,10 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
     const int tokenLanes = p.PerGroup * LPH;
     const int tokenOff = lane / tokenLanes < p.PerLoad ? lane / tokenLanes : 0;
     const int head = lane % tokenLanes / LPH, sub = lane % LPH;
-    for (int unit = group * gridDim.x + blockIdx.x; unit < plan.Units; unit += PS_GROUPS * gridDim.x) {
+    int unit = group * gridDim.x + blockIdx.x, at = unit / p.HeadGroups * plan.Quantum;
+    while (unit < plan.Units) {
         if (w == 0) {
-            LocateUnit(p, layer, plan, unit, g);
+            LocateChunk(p, layer, plan, unit, at, g);
         }
         GroupSync(group);
         {
@@ -765,7 +764,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
             const int headC = head0 + min(head, heads - 1);
             int j0, j1;
             KeyRange(pos + 1, layer.Window, &j0, &j1);
-            const int cBeg = j0 + chunk * plan.Chunk, cEnd = min(cBeg + plan.Chunk, j1);
+            const int cBeg = j0 + g.KeyBeg, cEnd = min(j0 + g.KeyEnd, j1);
             const int round = 8 * p.PerLoad - 1, part = (((cEnd - cBeg) + 3) / 4 + round) & ~round;
             const int tBeg = cBeg + w * part, tEnd = min(tBeg + part, cEnd);
             float *mine = g.Merge[w][lane];
@@ -783,7 +782,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
             }
         }
         GroupSync(group);
-        // which unit this was, read again: the key loop needs the registers
+        // which chunk this was, read again: the key loop needs the registers
         const volatile TAttGroupSmem &vg = g;
         const int seq = vg.SeqIndex, hg = vg.HeadGroup, chunk = vg.Chunk, chunks = vg.Chunks, pos = vg.Pos;
         const int head0 = hg * p.PerGroup, heads = min(p.PerGroup, p.Heads - head0);
@@ -810,9 +809,11 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
         const int z = sub * 16 + 4 * w;
         bool finish = true;
         if (chunks > 1) {
-            // partials to L2; the unit that arrives last merges all of the row's
+            // partials to L2; the group that arrives last merges all of the row's.  Chunk c of sequence s lies in range
+            // first(s) + c, and with s added no two chunks have one place: from a chunk to the next either grows.
             constexpr int PITCH = D + 4;
-            float *dst = p.Partial + ((size_t)unit * p.PerGroup + head) * PITCH;
+            const int place = unit + seq * p.HeadGroups;
+            float *dst = p.Partial + ((size_t)place * p.PerGroup + head) * PITCH;
             if (lane < tokenLanes) {
                 __stcg(reinterpret_cast<float4 *>(dst + z), make_float4(val[0], val[1], val[2], val[3]));
             }
@@ -832,7 +833,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
                 if (tid % 128 == 0) {
                     p.Arrived[seq * p.HeadGroups + hg] = 0; // for the next layer
                 }
-                const float *src = p.Partial + ((size_t)(unit - chunk * p.HeadGroups) * p.PerGroup + head) * PITCH;
+                const float *src = p.Partial + ((size_t)(place - chunk * p.HeadGroups) * p.PerGroup + head) * PITCH;
                 const size_t step = (size_t)p.HeadGroups * p.PerGroup * PITCH;
                 mAll = -1e30f;
 #pragma unroll 8
@@ -871,7 +872,12 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
             }
             StoreKvProduct(p.Kv8 + ((size_t)seq * hs + (head0 + head) * D) * 4, D, z, key, val);
         }
-        GroupSync(group); // the group's shared memory is used again by its next unit
+        at = vg.Next;
+        if (at < 0) {
+            unit += PS_GROUPS * gridDim.x;
+            at = unit / p.HeadGroups * plan.Quantum;
+        }
+        GroupSync(group); // the group's shared memory is used again by its next chunk
     }
 }
 
