@@ -18,9 +18,9 @@
 // phases and layers, in flight in a ring of shared memory (cp.async), so that their DRAM latency is never on the path.
 //
 // Measured, twelve layers, dim 768, 12 heads x 64, vocabulary 50304, a whole token with the final layer and softmax:
-//     1 sequence, 500 tokens of context       750 -> 320 us, of which about 240 us are the sixty phases at some 4 us each: the
+//     1 sequence, 500 tokens of context       750 -> 328 us, of which about 240 us are the sixty phases at some 4 us each: the
 //                                             barrier, the sums through L2 and the norm, in a chain; the bytes take 20 us
-//     64 sequences, 1024 to 8192 tokens       970 -> 825 us (three of four layers see 64 tokens); 200 us are the bytes of the wide
+//     64 sequences, 1024 to 8192 tokens       970 -> 855 us (three of four layers see 64 tokens); 200 us are the bytes of the wide
 //                                             layers' caches, the phases around them come on top, unoverlapped
 #include "att_sm100_common.cuh"
 #include "decode_device.cuh"
@@ -533,7 +533,7 @@ __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm
 // warps for each head group (the heads a warp-wide 16-byte load covers: 8 of 64 or 4 of 128).  A unit = one range x one head group,
 // taken by one group; its parts that belong to different sequences are its chunks, whose keys the four warps split.  With chunks
 // that all had one size and ended with their sequence, 64 sequences of 1024 to 8192 tokens kept a fifth of the groups idle at the
-// end of the phase (a token of the twelve-layer model 870 us, now 825).  A sequence counts with at least PS_MIN_CHUNK keys, which is also the least size of a range: short contexts and
+// end of the phase (a token of the twelve-layer model 870 us, with equal ranges 825).  A sequence counts with at least PS_MIN_CHUNK keys, which is also the least size of a range: short contexts and
 // narrow windows stay one chunk, and one group each.
 __device__ __forceinline__ int StepKeys(const TStepParams &p, const TStepLayer &layer, int s)
 {
