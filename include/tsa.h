@@ -423,7 +423,10 @@ int tsa_matmul_norm_rope_quant(int srcDtype, int dstDtype, float vecScale, float
  * increments (all layers of a sequence hold the same count).  maxCtx: host-side upper bound of the counts before the
  * step.  labels: device int [nSeq][labelsPerSeq], the embedding rows summed for each sequence's new token.
  * prediction f32 [nSeq][vocab_size] (may be NULL) receives the distribution over the vocabulary, logits (may be NULL)
- * the exact int32 products of the final layer as floats.  Asynchronous on `stream`; allocates nothing. */
+ * the exact int32 products of the final layer as floats.  Asynchronous on `stream`; allocates nothing.
+ * The order in which a sequence's attention sums are formed depends on the size of the chunks its keys are cut into, which follows
+ * from the contexts of the whole batch: equal sequences of one batch get equal bits, whatever their slots; beside other
+ * sequences the last bits of a long context's sums, and with them single int8 roundings, can differ. */
 typedef struct {
     int dim;
     int head_dim;

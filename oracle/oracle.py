@@ -472,6 +472,12 @@ class InferOracle:
         if not use_ref:
             self._l.oracle_infer_set_exp(self._h, 0 if exp_mode == "poly" else 1)
 
+    def load(self, keys, key_scales, vals, val_scales):
+        """Caches [layer][tokens][H*D] int8 and their scales [layer][tokens][H] f32, as `tokens` steps would have left them."""
+        assert not self.use_ref
+        arrays = [_b(keys), _f(key_scales), _b(vals), _f(val_scales)]
+        self._l.oracle_infer_load(self._h, int(keys.shape[1]), *[p for _, p in arrays])
+
     def step(self, labels, want_logits=False):
         labels, lp = _i(labels)
         pred = np.zeros(self.vocab, dtype=np.float32)

@@ -838,6 +838,21 @@ extern "C" void oracle_infer_set_exp(void *handle, int expMode)
     ((TInferOracle *)handle)->ExpMode = expMode;
 }
 
+// the layers' caches as they are after `tokens` steps: keys, vals [layer][tokens][H * D], their scales [layer][tokens][H]
+extern "C" void oracle_infer_load(void *handle, int tokens, const int8_t *keys, const float *keyScales, const int8_t *vals, const float *valScales)
+{
+    TInferOracle &m = *(TInferOracle *)handle;
+    const size_t row = (size_t)tokens * m.HeadCount * m.HeadDim, scales = (size_t)tokens * m.HeadCount;
+    for (size_t d = 0; d < m.Layers.size(); ++d) {
+        TInferLayer &l = m.Layers[d];
+        l.KeyCache.assign(keys + d * row, keys + (d + 1) * row);
+        l.ValCache.assign(vals + d * row, vals + (d + 1) * row);
+        l.KeyScale.assign(keyScales + d * scales, keyScales + (d + 1) * scales);
+        l.ValScale.assign(valScales + d * scales, valScales + (d + 1) * scales);
+    }
+    m.T = tokens;
+}
+
 // prediction [vocab] (may be null); logits [vocab] (may be null) receives the int32 products of the final layer as floats
 extern "C" void oracle_infer_step(void *handle, const int *labels, int labelCount, float *prediction, float *logits)
 {

@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 4) DecodePartialKernel(TDecode
         for (int i = 0; i < 16; ++i) {
             acc[i] = 0;
         }
-        AttendTokens<D, DEC_UNROLL, false>(qv, logitMult, p.Slope, cur, kp, vp, ksp, vsp, H, tBeg, tEnd, 1, 0, m, l, acc);
+        AttendTokens<D, DEC_UNROLL, false>(qv, logitMult, p.Slope, cur, kp, vp, ksp, vsp, H, tBeg, tEnd, (tEnd - tBeg + DEC_UNROLL - 1) / DEC_UNROLL, m, l, acc);
         if (split > 1) {
             float *mine = mergeBuf[warp][lane];
             mine[0] = m;

@@ -64,32 +64,31 @@ __device__ __forceinline__ int Dp2aHiUS(uint32_t a, uint32_t b, int c)
 }
 
 // Tokens [tBeg, tEnd) for this lane's 16-byte slice of its head: kp, vp, ksp, vsp point at token tBeg, qv is the query's slice.
-// Keeps UNROLL tokens of K and V in flight; online softmax in (m, l, acc).  A warp whose heads take no more than half of its lanes
-// works on `perLoad` batches of UNROLL tokens at a time: this lane takes batch `tokenOff` of each such group, and the lanes' results
-// are merged by the caller (a lane that saw no token keeps m = -1e30).  A batch is UNROLL consecutive tokens from a multiple of UNROLL
-// behind tBeg whatever perLoad is, so that the batch's 16-bit weights, and with them the int8 codes that follow, do not depend on it.
+// Keeps UNROLL tokens of K and V in flight; online softmax in (m, l, acc), batch after batch.  The warp runs `batches` of them, enough
+// for every lane; a lane that has no tokens left repeats its last one (token tEnd - 1 has to be readable) with weight zero, which changes
+// none of its sums.  A lane that never had one keeps m = -1e30, and its l and acc mean nothing.
 template <int D, int UNROLL, bool COHERENT, class TScale>
 __device__ __forceinline__ void AttendTokens(const int4 qv, float logitMult, float slope, int cur, const int4 *kp, const int4 *vp, const TScale *ksp,
-    const TScale *vsp, int H, int tBeg, int tEnd, int perLoad, int tokenOff, float &m, float &l, float (&acc)[16])
+    const TScale *vsp, int H, int tBeg, int tEnd, int batches, float &m, float &l, float (&acc)[16])
 {
     constexpr int LPH = D / 16;     // lanes per head
     const int rowInt4 = H * D / 16; // int4 words per token row
-    for (int tBase = tBeg; tBase < tEnd; tBase += UNROLL * perLoad) {
+    for (int tBase = tBeg; batches > 0; --batches, tBase += UNROLL) {
         int4 kv[UNROLL], vv[UNROLL];
         float ks[UNROLL], vs[UNROLL];
-        const int cnt = tEnd - tBase; // tokens left, >= 1
+        const int cnt = tEnd - tBase; // tokens left
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
-            const int tt = min(tokenOff * UNROLL + u, cnt - 1);
+            const int tt = min(u, cnt - 1);
             kv[u] = LoadRow<COHERENT>(kp + tt * rowInt4);
             vv[u] = LoadRow<COHERENT>(vp + tt * rowInt4);
             ks[u] = LoadScaleT<COHERENT>(ksp + tt * H);
             vs[u] = LoadScaleT<COHERENT>(vsp + tt * H);
         }
-        kp += UNROLL * perLoad * rowInt4;
-        vp += UNROLL * perLoad * rowInt4;
-        ksp += UNROLL * perLoad * H;
-        vsp += UNROLL * perLoad * H;
+        kp += UNROLL * rowInt4;
+        vp += UNROLL * rowInt4;
+        ksp += UNROLL * H;
+        vsp += UNROLL * H;
         float z[UNROLL];
         float cm = m;
 #pragma unroll
@@ -103,8 +102,8 @@ __device__ __forceinline__ void AttendTokens(const int4 qv, float logitMult, flo
                 dot += __shfl_xor_sync(0xffffffffu, dot, o);
             }
             // same association as the reference: ((dot * kScale) * attDotScale) * qScale - slope * dist
-            const float zz = (float)dot * ks[u] * logitMult - slope * (float)(cur - (tBase + tokenOff * UNROLL + u));
-            z[u] = (tokenOff * UNROLL + u < cnt) ? zz : -1e30f;
+            const float zz = (float)dot * ks[u] * logitMult - slope * (float)(cur - (tBase + u));
+            z[u] = (u < cnt) ? zz : -1e30f;
             cm = fmaxf(cm, z[u]);
         }
         if (cm != m) {

@@ -283,9 +283,8 @@ TInferBuffers CarveInferBuffers(const tsa_infer_model *m, int nSeq, void *base)
     b.NormState = (int8_t *)take((size_t)nSeq * d.dim);
     b.K8 = (int8_t *)take((size_t)nSeq * hs);
     b.Kv8 = (int8_t *)take((size_t)nSeq * hs * 4);
-    // partials of the attention's chunks: one more per sequence than units, of which there are no more than groups of warps
-    const size_t units = (size_t)nSeq * headGroups + (headGroups > 1024 ? headGroups : 1024);
-    b.Partial = (float *)take(sizeof(float) * units * perGroup * (d.head_dim + 4));
+    // partials of the attention's chunks
+    b.Partial = (float *)take(sizeof(float) * ((size_t)INF_MAX_CHUNKS + nSeq) * d.head_count * (d.head_dim + 4));
     b.Total = off;
     return b;
 }

@@ -7,6 +7,7 @@ namespace tsa {
 constexpr float INF_VEC_SCALE = 1.0f / 24; // VEC_SCALE, cpu_infer.cpp:16
 constexpr int INF_NORM_TILE = 128;         // STATE_NORM_TILE, model_dim.h:23
 constexpr int INF_MAX_SEQ = 64;            // sequences per step
+constexpr int INF_MAX_CHUNKS = 1024;       // chunks the keys of a layer are cut into, beside one per sequence
 
 // ConvertToInt8 (cpu_infer.cpp:88-92): round to nearest even, clamp to +-127
 __device__ __forceinline__ int ToInt8Clamp127(float x)

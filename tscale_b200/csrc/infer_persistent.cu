@@ -9,19 +9,23 @@
 //     C  comb      += W_combiner * A
 //     E  expand    += W_expand * norm(state + comb)
 //     T  contract  += W_contract * relu(norm(expand))
-// and a grid barrier (0.75 us: one counter, arrival and wait apart) behind each.  A matrix product is cut into items of one 128-row tile and some 128-column chunks, as
-// many items as there are SMs, so that a 768 x 768 matrix uses the whole GPU; the items' int32 partial tiles are added in L2
+// and a grid barrier (0.75 us: one counter, arrival and wait apart) behind each.  A matrix product is cut into items of one 128-row
+// tile and some 128-column chunks, as many items as there are SMs, so that a 768 x 768 matrix uses the whole GPU; the items' int32 partial tiles are added in L2
 // (red.add: exact, the order does not matter).  The consumer of a product forms its own input from those sums: every item of
 // the next product normalises the 128-column chunk it multiplies with (a chunk is one STATE_NORM_TILE; the scalar loop's
 // order of operations, so the codes are bit-identical to the CPU's), which costs each of them a few hundred nanoseconds and
 // saves a phase and its barrier.  The weights do not depend on anything: every CTA keeps the tiles of its next items, across
 // phases and layers, in flight in a ring of shared memory (cp.async), so that their DRAM latency is never on the path.
 //
-// Measured, twelve layers, dim 768, 12 heads x 64, vocabulary 50304, a whole token with the final layer and softmax:
-//     1 sequence, 500 tokens of context       750 -> 328 us, of which about 240 us are the sixty phases at some 4 us each: the
-//                                             barrier, the sums through L2 and the norm, in a chain; the bytes take 20 us
-//     64 sequences, 1024 to 8192 tokens       970 -> 855 us (three of four layers see 64 tokens); 200 us are the bytes of the wide
-//                                             layers' caches, the phases around them come on top, unoverlapped
+// Measured, twelve layers, dim 768, 12 heads x 64, vocabulary 50304, a whole token with the final layer and softmax, launches / graph:
+//     1 sequence, 500 tokens of context       744 / 568 -> 334 / 328 us, of which 312 are there with windows of 64 tokens in all
+//                                             layers: sixty phases at some 5 us, the barrier, the sums through L2 and the norm, in a
+//                                             chain; the bytes take 20 us
+//     64 sequences, 1024 to 8192 tokens       968 / 801 -> 735 / 727 us (three of four layers see 64 tokens): 473 us with the short
+//                                             windows in all layers, and 85 us for every wide layer, whose keys and values then
+//                                             stream at 5.8 TB/s
+// Head counts whose chunks need a whole group of four warps leave a quarter of the groups a second unit: with 16 heads x 64 such a
+// batch takes 975 / 968 us, where separate launches, 16 warps per SM in the attention, took 1085 / 897.
 #include "att_sm100_common.cuh"
 #include "decode_device.cuh"
 #include "infer_internal.cuh"
@@ -29,8 +33,8 @@
 
 namespace tsa {
 
-// Attention works in groups of four warps; three of them leave the key / value loop (64 registers of loads in flight) the 160-odd
-// registers it wants, with a fourth it spilled.
+// Attention works in groups of four warps.  Three of them leave the loop over keys the 168 registers it wants (64 of loads in flight); with
+// a fourth, at 128, it spills and a token of 64 sequences takes 912 us where this takes 735.
 constexpr int PS_THREADS = 384, PS_GROUPS = 3;
 constexpr int PS_LOADERS = PS_THREADS - 32; // threads that request weight tiles: all but the warp whose first lane polls the grid barrier
 constexpr int PS_RING = 8;                     // weight tiles in flight or in use per CTA
@@ -39,8 +43,8 @@ constexpr int PS_B_BYTES = INF_MAX_SEQ * 128;  // the chunk's vectors, one row o
 constexpr int PS_F_PITCH = 132;                // floats per row of the fp32 chunk: 16-byte rows that fall into different banks
 constexpr int PS_MERGE_PITCH = 19;
 constexpr int PS_LAYERS = 32;                  // layers per launch
-constexpr int PS_MAX_SLOTS = 1024;             // attention units whose partials the workspace holds, at least
-constexpr int PS_MIN_CHUNK = 64;               // keys: two batches of eight for each of a group's four warps
+constexpr int PS_CHUNKS_PER_SM = 4;            // the keys of a layer are cut into no more chunks than this times the SMs
+constexpr int PS_MIN_CHUNK = 16;               // keys
 constexpr long long PS_WAIT_CYCLES = 1ll << 31;
 
 enum { PH_PROJ = 0, PH_COMB = 1, PH_EXPAND = 2, PH_CONTRACT = 3, PH_FINAL = 4 };
@@ -65,7 +69,8 @@ struct TStepParams {
     int LayerCount, FirstSource;
     int NSeq, Dim, Heads, HeadSize, ReluDim, Capacity, MaxCtx, RopeLen;
     int HeadGroups, PerGroup;     // groups of heads the attention works in, heads of a group (the last may have fewer)
-    int PerLoad;                  // tokens a warp-wide load covers
+    int PerLoadLog;               // log2 of the streams of keys a warp-wide load covers
+    int Split;                    // parts a chunk's keys are cut into, 1, 2 or 4
     const int *Labels;
     int LabelsPerSeq, LabelCount;
     const int8_t *Embed;
@@ -73,7 +78,7 @@ struct TStepParams {
     const float *Rope;
     float DotScale;
     int *Barrier;                 // zero at launch
-    int *Arrived;                 // [nSeq][head groups] attention chunks done, zero between uses
+    int *Arrived;                 // [nSeq][head groups] chunks done of the rows that several units share, zero between uses
     int *Proj, *Comb, *Expand, *Contract; // int32 sums, zero at launch
     float *StateA, *StateB;
     int8_t *K8, *Kv8, *NormState;
@@ -82,21 +87,24 @@ struct TStepParams {
 };
 
 struct alignas(16) TAttGroupSmem {
-    float Rot[4][8 * 68];         // a head group's four projected vectors (8 x 64 or 4 x 128), rotated; pitch D + 4 per head
+    union {
+        float Rot[4][8 * 68];     // projected vectors a warp works on (8 x 64 or 4 x 128), rotated; pitch D + 4 per head
+        float Merge[4][32][PS_MERGE_PITCH]; // maximum, sum and 16 columns of every lane's stream of keys
+    };
     float Mult[4][8];
-    int8_t Q8[512], K8[512];
-    float Merge[4][32][PS_MERGE_PITCH];
-    tsa_kv_seq Seq;               // the group's chunk: its sequence's cache, position of the new token,
-    int Pos, SeqIndex, HeadGroup, Chunk, Chunks; // which of the chunks of which row it is,
-    int KeyBeg, KeyEnd;           // its keys, counted from the first the row attends,
-    int Next;                     // and where in the stream the unit goes on, -1: this was its last chunk
-    int Last;
+    int8_t Q8[2048], K8[2048];    // codes of the queries and combiner keys, [sequence of the unit][heads of the group][D]
+    int Last[2];                  // this unit is the last of the row's: its first sequence, its last one
 };
 
 // Units of the attention of one layer (see MakeAttPlan).
 struct TAttPlan {
-    int Window, Quantum, Units;               // Quantum: blocks of 32 keys per unit
-    int Base[INF_MAX_SEQ], Len[INF_MAX_SEQ];  // first block of each sequence in the stream, and their number
+    int Window;                                // of the layer, -1: none yet
+    int Chunk, Parts;                          // keys of a chunk, streams of keys it is worked on in
+    int PerUnit, Slots;                        // chunks of a unit, and all of them
+    int UnitBegin, UnitEnd;                    // this CTA's units
+    int Pos[INF_MAX_SEQ];                      // position of each sequence's new token
+    int Base[INF_MAX_SEQ], Count[INF_MAX_SEQ]; // its first chunk and their number
+    uint8_t SeqOf[INF_MAX_CHUNKS + INF_MAX_SEQ]; // sequence of a chunk
 };
 
 // one 128 x 128 weight tile of the CTA's share of a layer
@@ -121,14 +129,17 @@ struct TStepSmem {
     TWeightTile Table[PS_TABLE];
     int PhaseBegin[5];            // first tile of each phase, and their number
     TAttPlan Plan[2];             // of the last two windows: the layers of a model alternate between two or so
+    int PlanOf;                   // which of them is the present layer's
+    tsa_kv_seq Seqs[INF_MAX_SEQ]; // the present layer's caches
     uint64_t MmaDone;
     uint32_t TmemBase;
     int Failed;
     int Passed;                   // arrivals at the grid barrier that complete its present phase
 };
 
-static_assert(sizeof(TAttGroupSmem) % 16 == 0 && offsetof(TAttGroupSmem, Q8) % 16 == 0 && offsetof(TStepSmem, F) % 16 == 0 && offsetof(TStepSmem, B) % 1024 == 0,
+static_assert(sizeof(TAttGroupSmem) % 16 == 0 && offsetof(TAttGroupSmem, Q8) % 16 == 0 && offsetof(TAttGroupSmem, K8) % 16 == 0 && offsetof(TStepSmem, F) % 16 == 0 && offsetof(TStepSmem, B) % 1024 == 0,
     "16-byte accesses and swizzled operand tiles");
+static_assert(sizeof(TStepSmem) + 1024 <= 227 * 1024, "shared memory of a CTA, with the slack that aligns the tiles");
 
 __device__ __forceinline__ void CpAsync16(void *dst, const void *src, int bytes)
 {
@@ -529,78 +540,128 @@ __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm
 }
 
 // ---- attention -----------------------------------------------------------------------------------------------------
-// The keys of all sequences, one behind the other, are cut into ranges of the same size: as many as the grid has groups of four
-// warps for each head group (the heads a warp-wide 16-byte load covers: 8 of 64 or 4 of 128).  A unit = one range x one head group,
-// taken by one group; its parts that belong to different sequences are its chunks, whose keys the four warps split.  With chunks
-// that all had one size and ended with their sequence, 64 sequences of 1024 to 8192 tokens kept a fifth of the groups idle at the
-// end of the phase (a token of the twelve-layer model 870 us, with equal ranges 825).  A sequence counts with at least PS_MIN_CHUNK keys, which is also the least size of a range: short contexts and
-// narrow windows stay one chunk, and one group each.
-__device__ __forceinline__ int StepKeys(const TStepParams &p, const TStepLayer &layer, int s)
+// Every sequence's keys are cut into chunks of one size, counted from the first key it attends: the smallest multiple of eight (at
+// least PS_MIN_CHUNK) that gives no more than PS_CHUNKS_PER_SM chunks per SM, the rule of the decode kernel (DecodePlan), and a
+// chunk into Split parts of whole batches of eight.  Sums are formed in that order and no other: keys of a part one batch after
+// another, parts of a chunk, chunks of a row.  So the bits of a sequence's result depend on the chunk size alone, not on its slot or
+// on which unit takes what, and are those of the decode kernel's chunks merged one after another.
+// A warp-wide 16-byte load covers a head group (AttGroupHeads) for one stream of keys or several; a stream is one part of one
+// chunk.  A unit = as many consecutive chunks as four warps have streams for x one head group, taken by a group of four warps.
+// Its chunks may belong to several sequences.
+__device__ __forceinline__ bool PosOk(const TStepParams &p, int pos)
 {
-    if (s >= p.NSeq) {
-        return 0;
-    }
-    const int pos = layer.CtxLens[s];
-    if (pos < 0 || pos >= p.RopeLen || pos >= p.Capacity) {
-        return 0; // reported by the unit that would append
-    }
-    int j0, j1;
-    KeyRange(pos + 1, layer.Window, &j0, &j1);
-    return j1 - j0;
+    return pos >= 0 && pos < p.RopeLen && pos < p.Capacity;
 }
 
-// by one warp, into shared memory
-__device__ __noinline__ void MakeAttPlan(const TStepParams &p, const TStepLayer &layer, TAttPlan &plan)
+// by one warp, into shared memory; pos: lane i has those of sequences i and i + 32
+__device__ __noinline__ void MakeAttPlan(const TStepParams &p, int window, int pos0, int pos1, TAttPlan &plan)
 {
     const int lane = threadIdx.x & 31;
-    const int ranges = max((int)gridDim.x * PS_GROUPS / p.HeadGroups, 1);
-    // blocks of 32 keys; every sequence has at least one chunk per head group: it appends the new token
-    auto blocks = [&](int s) { return s < p.NSeq ? (max(StepKeys(p, layer, s), PS_MIN_CHUNK) + 31) / 32 : 0; };
-    const int n0 = blocks(lane), n1 = blocks(lane + 32);
-    int i0 = n0, i1 = n1;
+    auto keysOf = [&](int s, int pos) {
+        int j0 = 0, j1 = 0;
+        if (s < p.NSeq && PosOk(p, pos)) {
+            KeyRange(pos + 1, window, &j0, &j1);
+        }
+        return j1 - j0;
+    };
+    auto warpSum = [](int v) { return (int)__reduce_add_sync(0xffffffffu, (unsigned)v); };
+    const int k0 = keysOf(lane, pos0), k1 = keysOf(lane + 32, pos1);
+    const int total = warpSum(k0 + k1), target = min((int)gridDim.x * PS_CHUNKS_PER_SM, INF_MAX_CHUNKS);
+    int chunk = max(((total + target - 1) / target + 7) & ~7, PS_MIN_CHUNK);
+    if (p.NSeq < target) {
+        // a sequence's last chunk is a partial one: the count falls as the size grows, total / (target - NSeq) is always enough
+        int lo = chunk / 8, hi = max(((total + (target - p.NSeq) - 1) / (target - p.NSeq) + 7) / 8, lo);
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (warpSum((k0 + mid * 8 - 1) / (mid * 8) + (k1 + mid * 8 - 1) / (mid * 8)) <= target) {
+                hi = mid;
+            } else {
+                lo = mid + 1;
+            }
+        }
+        chunk = lo * 8;
+    }
+    // a sequence without keys has a chunk too: the unit that takes it appends the new token
+    const int n0 = lane < p.NSeq ? max((k0 + chunk - 1) / chunk, 1) : 0, n1 = lane + 32 < p.NSeq ? max((k1 + chunk - 1) / chunk, 1) : 0;
+    const int parts = min(p.Split, chunk / 8), perUnit = (4 << p.PerLoadLog) / parts; // no part is shorter than a batch
+    // every sequence begins with a unit of its own where the groups of four warps suffice for that: rows that fit a unit then need no
+    // partials
+    const int w0 = (n0 + perUnit - 1) / perUnit, w1 = (n1 + perUnit - 1) / perUnit, whole = warpSum(w0 + w1);
+    const bool apart = whole * p.HeadGroups <= (int)gridDim.x * PS_GROUPS && whole * perUnit <= INF_MAX_CHUNKS;
+    const int t0 = apart ? w0 * perUnit : n0, t1 = apart ? w1 * perUnit : n1;
+    int i0 = t0, i1 = t1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int a = __shfl_up_sync(0xffffffffu, i0, o), b = __shfl_up_sync(0xffffffffu, i1, o);
         i0 += lane >= o ? a : 0;
         i1 += lane >= o ? b : 0;
     }
-    const int sum0 = __shfl_sync(0xffffffffu, i0, 31), total = sum0 + __shfl_sync(0xffffffffu, i1, 31);
-    plan.Base[lane] = i0 - n0;
-    plan.Base[lane + 32] = sum0 + i1 - n1;
-    plan.Len[lane] = n0;
-    plan.Len[lane + 32] = n1;
+    const int sum0 = __shfl_sync(0xffffffffu, i0, 31), slots = sum0 + __shfl_sync(0xffffffffu, i1, 31);
+    const int b0 = i0 - t0, b1 = sum0 + i1 - t1;
+    plan.Pos[lane] = pos0;
+    plan.Pos[lane + 32] = pos1;
+    plan.Base[lane] = b0;
+    plan.Base[lane + 32] = b1;
+    plan.Count[lane] = n0;
+    plan.Count[lane + 32] = n1;
+    for (int i = 0; i < t0; ++i) {
+        plan.SeqOf[b0 + i] = (uint8_t)lane;
+    }
+    for (int i = 0; i < t1; ++i) {
+        plan.SeqOf[b1 + i] = (uint8_t)(lane + 32);
+    }
     if (lane == 0) {
-        const int quantum = max((total + ranges - 1) / ranges, PS_MIN_CHUNK / 32);
-        plan.Quantum = quantum;
-        plan.Units = (total + quantum - 1) / quantum * p.HeadGroups;
-        plan.Window = layer.Window;
+        plan.Window = window;
+        plan.Chunk = chunk;
+        plan.Parts = parts;
+        plan.PerUnit = perUnit;
+        plan.Slots = slots;
+        // neighbouring units, the head groups of the same chunks, on one SM
+        const long long units = (slots + perUnit - 1) / perUnit * p.HeadGroups;
+        plan.UnitBegin = (int)(units * blockIdx.x / gridDim.x);
+        plan.UnitEnd = (int)(units * (blockIdx.x + 1) / gridDim.x);
     }
     __syncwarp();
 }
 
-// the chunk of unit number `unit` that begins at block `at` of the stream, and its sequence's cache, into the group's shared memory
-// (one warp)
-__device__ __noinline__ void LocateChunk(const TStepParams &p, const TStepLayer &layer, const TAttPlan &plan, int unit, int at, TAttGroupSmem &g)
+// What the attention of layer l needs besides the projections, while the CTA waits for them: the plan (warp 1; the one in shared
+// memory if window and positions are the same) and the table of the caches (warps 2 and 3).
+__device__ __noinline__ void PrepareAttention(const TStepParams &p, TStepSmem &sm, int l)
 {
-    const int lane = threadIdx.x & 31;
-    // the sequence this block belongs to: the last with Base <= at
-    const unsigned at0 = __ballot_sync(0xffffffffu, lane < p.NSeq && plan.Base[lane] <= at);
-    const unsigned at1 = __ballot_sync(0xffffffffu, lane + 32 < p.NSeq && plan.Base[lane + 32] <= at);
-    const int seq = at1 ? 63 - __clz(at1) : 31 - __clz(at0);
-    if (lane == 0) {
-        const int range = unit / p.HeadGroups, base = plan.Base[seq], seqEnd = base + plan.Len[seq], unitEnd = (range + 1) * plan.Quantum;
-        const int firstRange = base / plan.Quantum;
-        g.Pos = layer.CtxLens[seq];
-        g.Seq = layer.Seqs[seq];
-        g.SeqIndex = seq;
-        g.HeadGroup = unit - range * p.HeadGroups;
-        g.Chunk = range - firstRange;
-        g.Chunks = (seqEnd - 1) / plan.Quantum - firstRange + 1;
-        g.KeyBeg = (at - base) * 32;
-        g.KeyEnd = (min(seqEnd, unitEnd) - base) * 32;
-        g.Next = seqEnd < unitEnd && seq + 1 < p.NSeq ? seqEnd : -1;
+    const TStepLayer &layer = p.Layers[l];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 1) {
+        const int pos0 = lane < p.NSeq ? layer.CtxLens[lane] : 0, pos1 = lane + 32 < p.NSeq ? layer.CtxLens[lane + 32] : 0;
+        auto report = [&](int s, int pos) {
+            if (s < p.NSeq && (!PosOk(p, pos) || pos + 1 > p.MaxCtx) && p.Status) {
+                atomicOr(p.Status, kDevBadSpan); // the cache or the rope table is full, or longer than the caller's bound
+            }
+        };
+        if (blockIdx.x == 0) {
+            report(lane, pos0);
+            report(lane + 32, pos1);
+        }
+        int slot = -1;
+        for (int i = 0; i < 2; ++i) {
+            const TAttPlan &plan = sm.Plan[i];
+            if (plan.Window == layer.Window && __all_sync(0xffffffffu, plan.Pos[lane] == pos0 && plan.Pos[lane + 32] == pos1)) {
+                slot = i;
+            }
+        }
+        if (slot < 0) {
+            slot = sm.Plan[0].Window < 0 ? 0 : sm.Plan[1].Window < 0 ? 1 : sm.PlanOf ^ 1; // the one not used last
+            __syncwarp();
+            MakeAttPlan(p, layer.Window, pos0, pos1, sm.Plan[slot]);
+        }
+        if (lane == 0) {
+            sm.PlanOf = slot;
+        }
+    } else if (warp == 2 || warp == 3) {
+        const int s = (int)threadIdx.x - 64;
+        if (s < p.NSeq) {
+            sm.Seqs[s] = layer.Seqs[s];
+        }
     }
-    __syncwarp();
 }
 
 // The combiner input of four consecutive columns z .. z + 3 of a head: kv[blk][z] = int8(key[z ^ blk] * val[z]) (KVProduct,
@@ -620,13 +681,14 @@ __device__ __forceinline__ void StoreKvProduct(int8_t *kv, int headSize, int z, 
 }
 
 // One matrix (m: qk, qv, k, v) of a head group of one sequence, by one warp: rope on qk and qv (ReferenceApplyRope,
-// code/gpt/att/rope.cpp:28-46), NormalizeState per head, codes into shared memory (qk, k) or the sequence's cache (qv, v).
+// code/gpt/att/rope.cpp:28-46), NormalizeState per head, codes into shared memory (qk, k: at `codes`) or the sequence's cache (qv, v).
 template <int D>
-__device__ __noinline__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAttGroupSmem &g, int m, int seq, int head0, int heads, int pos)
+__device__ __noinline__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAttGroupSmem &g, const tsa_kv_seq &sq, int m, int seq, int codes,
+    int head0, int heads, int pos)
 {
-    const int lane = threadIdx.x & 31, hs = p.Heads * D;
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 3, hs = p.Heads * D;
     const int *src = p.Proj + (size_t)seq * 4 * hs + m * hs + head0 * D;
-    float *rot = g.Rot[m];
+    float *rot = g.Rot[warp];
     // up to eight blocks of 64 columns, all loads in flight at once
     constexpr int PER_HEAD = D / 64;
     const int blocks = heads * PER_HEAD;
@@ -662,7 +724,6 @@ __device__ __noinline__ void ProjectHeads(const TStepParams &p, const TStepLayer
         }
     }
     __syncwarp();
-    const tsa_kv_seq sq = g.Seq;
     if (lane < heads) {
         const float *w = rot + lane * (D + 4);
         float sum2 = 0;
@@ -672,7 +733,7 @@ __device__ __noinline__ void ProjectHeads(const TStepParams &p, const TStepLayer
         }
         float discr, mult;
         NormScales(sum2, D, &discr, &mult);
-        g.Mult[m][lane] = mult;
+        g.Mult[warp][lane] = mult;
         if (m == 1) {
             ((float *)sq.kScale)[(size_t)pos * p.Heads + head0 + lane] = __fmul_rn(discr, layer.QvMult);
         } else if (m == 3) {
@@ -684,200 +745,241 @@ __device__ __noinline__ void ProjectHeads(const TStepParams &p, const TStepLayer
     for (int i = lane * 4; i < heads * D; i += 128) {
         const int h = i / D;
         const float4 w = *reinterpret_cast<const float4 *>(rot + h * (D + 4) + (i & (D - 1)));
-        const float mult = g.Mult[m][h];
+        const float mult = g.Mult[warp][h];
         char4 q;
         q.x = (char)ToInt8Clamp127(__fmul_rn(w.x, mult));
         q.y = (char)ToInt8Clamp127(__fmul_rn(w.y, mult));
         q.z = (char)ToInt8Clamp127(__fmul_rn(w.z, mult));
         q.w = (char)ToInt8Clamp127(__fmul_rn(w.w, mult));
         if (m == 0) {
-            *reinterpret_cast<char4 *>(g.Q8 + i) = q;
+            *reinterpret_cast<char4 *>(g.Q8 + codes + i) = q;
         } else if (m == 2) {
-            *reinterpret_cast<char4 *>(g.K8 + i) = q;
+            *reinterpret_cast<char4 *>(g.K8 + codes + i) = q;
             *reinterpret_cast<char4 *>(p.K8 + (size_t)seq * hs + head0 * D + i) = q;
         } else {
             *reinterpret_cast<char4 *>((int8_t *)(m == 1 ? sq.k : sq.v) + (size_t)pos * hs + head0 * D + i) = q;
         }
     }
+    __syncwarp(); // the warp's buffers are used again for its next matrix
 }
 
-// this lane's share of a range of tokens, into the merge buffer
+// four columns of a row's result, times the combiner key (its codes in shared memory, or null: in L2), as codes for the combiner
+template <int D>
+__device__ __noinline__ void FinishColumns(const TStepParams &p, int pos, int seq, int head, int z, const int8_t *keyCodes, float sum, float4 acc)
+{
+    const size_t row = (size_t)seq * p.Heads * D;
+    char4 key = make_char4(0, 0, 0, 0);
+    float val[4] = {0, 0, 0, 0};
+    if (PosOk(p, pos)) {
+        const int packed = keyCodes ? *reinterpret_cast<const int *>(keyCodes) : __ldcg(reinterpret_cast<const int *>(p.K8 + row + head * D + z));
+        key = *reinterpret_cast<const char4 *>(&packed);
+        val[0] = acc.x / sum, val[1] = acc.y / sum, val[2] = acc.z / sum, val[3] = acc.w / sum;
+    }
+    StoreKvProduct(p.Kv8 + (row + head * D) * 4, D, z, key, val);
+}
+
+// all chunks of a row, their partials one step of all heads apart, and the sink
+template <int D>
+__device__ __noinline__ void MergePartials(const TStepParams &p, const float *src, int chunks, int z, float &sum, float (&val)[4])
+{
+    const size_t step = (size_t)p.Heads * (D + 4);
+    constexpr int LPH = D / 16;
+    float mAll = 0; // the sink has logit 0 (softMax.Add(0), cpu_infer.cpp:444)
+#pragma unroll 4
+    for (int c = (threadIdx.x & 31) % LPH; c < chunks; c += LPH) { // shared out among the lanes of the head
+        mAll = fmaxf(mAll, __ldcg(src + c * step + D));
+    }
+#pragma unroll
+    for (int o = LPH / 2; o > 0; o >>= 1) {
+        mAll = fmaxf(mAll, __shfl_xor_sync(0xffffffffu, mAll, o));
+    }
+    float sumAll = exp2f(-mAll);
+    float4 acc = make_float4(0, 0, 0, 0);
+#pragma unroll 4
+    for (int c = 0; c < chunks; ++c) {
+        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(src + c * step + D));
+        const float4 v = __ldcg(reinterpret_cast<const float4 *>(src + c * step + z));
+        const float f = exp2f(ml.x - mAll);
+        sumAll = fmaf(f, ml.y, sumAll);
+        acc.x = fmaf(f, v.x, acc.x);
+        acc.y = fmaf(f, v.y, acc.y);
+        acc.z = fmaf(f, v.z, acc.z);
+        acc.w = fmaf(f, v.w, acc.w);
+    }
+    sum = sumAll;
+    val[0] = acc.x, val[1] = acc.y, val[2] = acc.z, val[3] = acc.w;
+}
+
+// this lane's stream of keys, its maximum, sum and columns into the merge buffer
 template <int D>
 __device__ __forceinline__ void AttendRange(const int4 qv, float logitMult, float slope, int pos, const int8_t *k, const int8_t *v, const float *ks, const float *vs,
-    int heads, int tBeg, int tEnd, int perLoad, int tokenOff, float *mine)
+    int heads, int tBeg, int tEnd, int batches, float *mine)
 {
-    float m = -1e30f, l = 0, acc[16];
+    float m = -1e30f, sum = 0, acc[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         acc[i] = 0;
     }
-    AttendTokens<D, 8, true>(qv, logitMult, slope, pos, reinterpret_cast<const int4 *>(k), reinterpret_cast<const int4 *>(v), ks, vs, heads, tBeg, tEnd, perLoad, tokenOff, m, l, acc);
+    AttendTokens<D, 8, true>(qv, logitMult, slope, pos, reinterpret_cast<const int4 *>(k), reinterpret_cast<const int4 *>(v), ks, vs, heads, tBeg, tEnd, batches, m,
+        sum, acc);
+    const bool any = tBeg < tEnd;
     mine[0] = m;
-    mine[1] = l;
+    mine[1] = any ? sum : 0.0f;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-        mine[2 + i] = acc[i];
+        mine[2 + i] = any ? acc[i] : 0.0f;
     }
 }
 
 template <int D>
 __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
 {
-    constexpr int LPH = D / 16; // lanes per head
+    constexpr int LPH = D / 16;  // lanes per head
+    constexpr int PITCH = D + 4; // of a partial: columns, maximum, sum
     const TStepLayer &layer = p.Layers[l];
+    const TAttPlan &plan = sm.Plan[sm.PlanOf];
     const int tid = threadIdx.x, lane = tid & 31, group = tid >> 7, w = (tid >> 5) & 3;
     const int hs = p.Heads * D;
     TAttGroupSmem &g = sm.Att[group];
-    int slot = sm.Plan[0].Window == layer.Window ? 0 : 1;
-    if (sm.Plan[slot].Window != layer.Window) {
-        // not among the last two windows (the same for the whole CTA: the plans change only here)
-        __syncthreads();
-        slot = sm.Plan[0].Window < 0 ? 0 : sm.Plan[1].Window < 0 ? 1 : l & 1;
-        __syncthreads();
-        if (tid < 32) {
-            MakeAttPlan(p, layer, sm.Plan[slot]);
-        }
-        __syncthreads();
-    }
-    const TAttPlan &plan = sm.Plan[slot];
-    // this lane's token of a load, head inside the group, 16-byte slice of the head; lanes past the last token repeat the first's
-    const int tokenLanes = p.PerGroup * LPH;
-    const int tokenOff = lane / tokenLanes < p.PerLoad ? lane / tokenLanes : 0;
-    const int head = lane % tokenLanes / LPH, sub = lane % LPH;
-    int unit = group * gridDim.x + blockIdx.x, at = unit / p.HeadGroups * plan.Quantum;
-    while (unit < plan.Units) {
-        if (w == 0) {
-            LocateChunk(p, layer, plan, unit, at, g);
+    // this lane's stream among those of a load, head inside the group, 16-byte slice of the head; lanes past the last stream repeat the first's
+    const int streamLanes = p.PerGroup * LPH, perLoad = 1 << p.PerLoadLog;
+    const int streamOff = lane / streamLanes < perLoad ? lane / streamLanes : 0, first = lane % streamLanes;
+    const int head = first / LPH, sub = lane % LPH, z = sub * 16 + 4 * w;
+    for (int unit = plan.UnitBegin + group; unit < plan.UnitEnd; unit += PS_GROUPS) {
+        const int range = unit / p.HeadGroups, hg = unit - range * p.HeadGroups, head0 = hg * p.PerGroup, heads = min(p.PerGroup, p.Heads - head0);
+        const int slot0 = range * plan.PerUnit, slots = min(plan.PerUnit, plan.Slots - slot0);
+        const int seq0 = plan.SeqOf[slot0], seq1 = plan.SeqOf[slot0 + slots - 1];
+        // the four matrices of a sequence by the four warps; only the unit with its first chunk appends the token and leaves the combiner key
+        for (int seq = seq0; seq <= seq1; ++seq) {
+            const int m = (w + seq - seq0) & 3, pos = plan.Pos[seq];
+            if (PosOk(p, pos) && (m == 0 || plan.Base[seq] >= slot0)) {
+                ProjectHeads<D>(p, layer, g, sm.Seqs[seq], m, seq, (seq - seq0) * p.PerGroup * D, head0, heads, pos);
+            }
         }
         GroupSync(group);
         {
-            const int chunk = g.Chunk, pos = g.Pos, head0 = g.HeadGroup * p.PerGroup, heads = min(p.PerGroup, p.Heads - head0);
-            const bool posOk = pos >= 0 && pos < p.RopeLen && pos < p.Capacity;
-            if (tid % 128 == 0 && p.Status && (!posOk || pos + 1 > p.MaxCtx)) {
-                atomicOr(p.Status, kDevBadSpan); // the cache or the rope table is full, or longer than the caller's bound
-            }
-            if (posOk && (chunk == 0 || w == 0)) {
-                // the first chunk's unit also appends the token and leaves the combiner key
-                ProjectHeads<D>(p, layer, g, w, g.SeqIndex, head0, heads, pos);
-            }
-            GroupSync(group);
-            const int headC = head0 + min(head, heads - 1);
-            int j0, j1;
-            KeyRange(pos + 1, layer.Window, &j0, &j1);
-            const int cBeg = j0 + g.KeyBeg, cEnd = min(j0 + g.KeyEnd, j1);
-            const int round = 8 * p.PerLoad - 1, part = (((cEnd - cBeg) + 3) / 4 + round) & ~round;
-            const int tBeg = cBeg + w * part, tEnd = min(tBeg + part, cEnd);
-            float *mine = g.Merge[w][lane];
-            if (posOk && tBeg < tEnd) {
-                const int4 qv = *reinterpret_cast<const int4 *>(g.Q8 + (headC - head0) * D + sub * 16);
-                const size_t off = (size_t)tBeg * hs + headC * D + sub * 16, soff = (size_t)tBeg * p.Heads + headC;
-                AttendRange<D>(qv, p.DotScale * INF_VEC_SCALE, layer.Slope, pos, (const int8_t *)g.Seq.k + off, (const int8_t *)g.Seq.v + off,
-                    (const float *)g.Seq.kScale + soff, (const float *)g.Seq.vScale + soff, p.Heads, tBeg, tEnd, p.PerLoad, tokenOff, mine);
-            } else {
-                mine[0] = -1e30f;
-#pragma unroll
-                for (int i = 1; i < 18; ++i) {
-                    mine[i] = 0;
+            // this lane's stream: part `part` of chunk `chunk` of the unit
+            const int stream = (w << p.PerLoadLog) + streamOff, parts = plan.Parts;
+            const int chunk = parts == 3 ? stream / 3 : stream >> (parts >> 1), part = stream - chunk * parts;
+            int tBeg = 1, tEnd = 1, seq = seq0; // none: the lane reads the first key and takes nothing from it
+            if (chunk < slots) {
+                seq = plan.SeqOf[slot0 + chunk];
+                int j0, j1;
+                KeyRange(plan.Pos[seq] + 1, layer.Window, &j0, &j1);
+                const int cBeg = j0 + (slot0 + chunk - plan.Base[seq]) * plan.Chunk, cEnd = min(cBeg + plan.Chunk, j1);
+                const int perPart = (((cEnd - cBeg + p.Split - 1) >> (p.Split >> 1)) + 7) & ~7, beg = cBeg + part * perPart, end = min(beg + perPart, cEnd);
+                if (beg < end && PosOk(p, plan.Pos[seq])) {
+                    tBeg = beg;
+                    tEnd = end;
                 }
             }
+            const int batches = __reduce_max_sync(0xffffffffu, (unsigned)(tEnd - tBeg + 7) / 8);
+            const int headC = head0 + min(head, heads - 1);
+            const tsa_kv_seq &sq = sm.Seqs[seq];
+            const int4 qv = *reinterpret_cast<const int4 *>(g.Q8 + (seq - seq0) * p.PerGroup * D + (headC - head0) * D + sub * 16);
+            const size_t off = (size_t)tBeg * hs + headC * D + sub * 16, soff = (size_t)tBeg * p.Heads + headC;
+            AttendRange<D>(qv, p.DotScale * INF_VEC_SCALE, layer.Slope, plan.Pos[seq], (const int8_t *)sq.k + off, (const int8_t *)sq.v + off,
+                (const float *)sq.kScale + soff, (const float *)sq.vScale + soff, p.Heads, tBeg, tEnd, batches, g.Merge[w][lane]);
         }
         GroupSync(group);
-        // which chunk this was, read again: the key loop needs the registers
-        const volatile TAttGroupSmem &vg = g;
-        const int seq = vg.SeqIndex, hg = vg.HeadGroup, chunk = vg.Chunk, chunks = vg.Chunks, pos = vg.Pos;
-        const int head0 = hg * p.PerGroup, heads = min(p.PerGroup, p.Heads - head0);
-        const bool posOk = pos >= 0 && pos < p.RopeLen && pos < p.Capacity;
-        // the shares of the chunk of the four warps and of the tokens of a load; warp w goes on with columns 4 w .. 4 w + 3 of every
-        // lane's slice
-        const int first = lane % tokenLanes, shares = 4 * p.PerLoad;
-        auto shareOf = [&](int k) { return (const float *)g.Merge[k & 3][first + (k >> 2) * tokenLanes]; };
-        float mAll = -1e30f;
-        for (int k = 0; k < shares; k += 4) {
-            mAll = fmaxf(fmaxf(mAll, fmaxf(shareOf(k)[0], shareOf(k + 1)[0])), fmaxf(shareOf(k + 2)[0], shareOf(k + 3)[0]));
-        }
-        float lAll = 0, val[4] = {0, 0, 0, 0};
-#pragma unroll 4
-        for (int k = 0; k < shares; ++k) {
-            const float *other = shareOf(k);
-            const float f = exp2f(other[0] - mAll);
-            lAll = fmaf(f, other[1], lAll);
+        // Warp w goes on with columns 4 w .. 4 w + 3 of every slice.
+        auto shareOf = [&](int stream) { return (const float *)g.Merge[stream >> p.PerLoadLog][first + (stream & (perLoad - 1)) * streamLanes]; };
+        // the parts of a chunk
+        auto mergeChunk = [&](int chunk, float &m, float &sum, float (&val)[4]) {
+            const float *share = shareOf(chunk * plan.Parts);
+            m = share[0];
+            sum = share[1];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                val[i] = fmaf(f, other[2 + 4 * w + i], val[i]);
+                val[i] = share[2 + 4 * w + i];
             }
-        }
-        const int z = sub * 16 + 4 * w;
-        bool finish = true;
-        if (chunks > 1) {
-            // partials to L2; the group that arrives last merges all of the row's.  Chunk c of sequence s lies in range
-            // first(s) + c, and with s added no two chunks have one place: from a chunk to the next either grows.
-            constexpr int PITCH = D + 4;
-            const int place = unit + seq * p.HeadGroups;
-            float *dst = p.Partial + ((size_t)place * p.PerGroup + head) * PITCH;
-            if (lane < tokenLanes) {
-                __stcg(reinterpret_cast<float4 *>(dst + z), make_float4(val[0], val[1], val[2], val[3]));
-            }
-            if (z == 0 && lane < tokenLanes) {
-                __stcg(reinterpret_cast<float2 *>(dst + D), make_float2(mAll, lAll));
-            }
-            __threadfence();
-            GroupSync(group);
-            if (tid % 128 == 0) {
-                const int done = atomicAdd(p.Arrived + seq * p.HeadGroups + hg, 1);
-                g.Last = done == chunks - 1;
-                __threadfence();
-            }
-            GroupSync(group);
-            finish = g.Last != 0;
-            if (finish) {
-                if (tid % 128 == 0) {
-                    p.Arrived[seq * p.HeadGroups + hg] = 0; // for the next layer
-                }
-                const float *src = p.Partial + ((size_t)(place - chunk * p.HeadGroups) * p.PerGroup + head) * PITCH;
-                const size_t step = (size_t)p.HeadGroups * p.PerGroup * PITCH;
-                mAll = -1e30f;
-#pragma unroll 8
-                for (int c = 0; c < chunks; ++c) {
-                    mAll = fmaxf(mAll, __ldcg(src + c * step + D));
-                }
-                lAll = 0;
-                val[0] = val[1] = val[2] = val[3] = 0;
-#pragma unroll 8
-                for (int c = 0; c < chunks; ++c) {
-                    const float *q = src + c * step;
-                    const float2 ml = __ldcg(reinterpret_cast<const float2 *>(q + D));
-                    const float4 v = __ldcg(reinterpret_cast<const float4 *>(q + z));
-                    const float f = exp2f(ml.x - mAll);
-                    lAll = fmaf(f, ml.y, lAll);
-                    val[0] = fmaf(f, v.x, val[0]);
-                    val[1] = fmaf(f, v.y, val[1]);
-                    val[2] = fmaf(f, v.z, val[2]);
-                    val[3] = fmaf(f, v.w, val[3]);
-                }
-            }
-        }
-        if (finish && head < heads && lane < tokenLanes) {
-            // the sink has logit 0 (softMax.Add(0), cpu_infer.cpp:444)
-            const float mF = fmaxf(mAll, 0.0f), f = exp2f(mAll - mF), lF = exp2f(-mF) + f * lAll;
+            for (int k = 1; k < plan.Parts; ++k) {
+                const float *other = shareOf(chunk * plan.Parts + k);
+                const float mAll = fmaxf(m, other[0]);
+                const float c1 = exp2f(m - mAll), c2 = exp2f(other[0] - mAll);
+                sum = sum * c1 + other[1] * c2;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                val[i] = posOk ? (f * val[i]) / lF : 0.0f;
+                for (int i = 0; i < 4; ++i) {
+                    val[i] = val[i] * c1 + other[2 + 4 * w + i] * c2;
+                }
+                m = mAll;
             }
-            char4 key = make_char4(0, 0, 0, 0);
-            if (posOk && chunks == 1) {
-                key = *reinterpret_cast<const char4 *>(g.K8 + head * D + z);
-            } else if (posOk) {
-                const int packed = __ldcg(reinterpret_cast<const int *>(p.K8 + (size_t)seq * hs + (head0 + head) * D + z));
-                key = *reinterpret_cast<const char4 *>(&packed);
+        };
+        auto finish = [&](int seq, float sum, const float (&val)[4]) {
+            if (head < heads && lane < streamLanes) {
+                const int8_t *key = plan.Base[seq] >= slot0 ? g.K8 + (seq - seq0) * p.PerGroup * D + head * D + z : nullptr;
+                FinishColumns<D>(p, plan.Pos[seq], seq, head0 + head, z, key, sum, make_float4(val[0], val[1], val[2], val[3]));
             }
-            StoreKvProduct(p.Kv8 + ((size_t)seq * hs + (head0 + head) * D) * 4, D, z, key, val);
+        };
+        auto chunksHere = [&](int seq, int &c0, int &c1) { // the unit's chunks of a sequence
+            c0 = max(plan.Base[seq] - slot0, 0);
+            c1 = min(plan.Base[seq] + plan.Count[seq] - slot0, slots);
+            return c1 - c0;
+        };
+        bool shared = false; // a row that other units have chunks of: its partials go to L2
+        for (int seq = seq0; seq <= seq1; ++seq) {
+            int c0, c1;
+            const bool whole = chunksHere(seq, c0, c1) == plan.Count[seq];
+            shared |= !whole;
+            float mAll = 0; // the sink has logit 0 (softMax.Add(0), cpu_infer.cpp:444)
+            if (whole) {
+                for (int k = c0 * plan.Parts; k < c1 * plan.Parts; ++k) {
+                    mAll = fmaxf(mAll, shareOf(k)[0]);
+                }
+            }
+            float sumAll = exp2f(-mAll), valAll[4] = {0, 0, 0, 0};
+            for (int c = c0; c < c1; ++c) {
+                float m, sum, val[4];
+                mergeChunk(c, m, sum, val);
+                if (whole) {
+                    const float f = exp2f(m - mAll);
+                    sumAll = fmaf(f, sum, sumAll);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        valAll[i] = fmaf(f, val[i], valAll[i]);
+                    }
+                } else if (head < heads && lane < streamLanes) {
+                    float *dst = p.Partial + ((size_t)(slot0 + c) * p.Heads + head0 + head) * PITCH;
+                    __stcg(reinterpret_cast<float4 *>(dst + z), make_float4(val[0], val[1], val[2], val[3]));
+                    if (z == 0) {
+                        __stcg(reinterpret_cast<float2 *>(dst + D), make_float2(m, sum));
+                    }
+                }
+            }
+            if (whole) {
+                finish(seq, sumAll, valAll);
+            }
         }
-        at = vg.Next;
-        if (at < 0) {
-            unit += PS_GROUPS * gridDim.x;
-            at = unit / p.HeadGroups * plan.Quantum;
+        if (shared) {
+            // at most the first and the last sequence; the unit that arrives last merges all chunks of the row
+            GroupSync(group);
+            if (tid % 128 < 2) {
+                const int seq = tid % 128 == 0 ? seq0 : seq1;
+                int c0, c1, last = 0;
+                const int here = chunksHere(seq, c0, c1);
+                if (here != plan.Count[seq] && (tid % 128 == 0 || seq1 != seq0)) {
+                    int *arrived = p.Arrived + seq * p.HeadGroups + hg;
+                    int before;
+                    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(before) : "l"(arrived), "r"(here) : "memory");
+                    last = before + here == plan.Count[seq];
+                    if (last) {
+                        *arrived = 0; // for the next layer
+                    }
+                }
+                g.Last[tid % 128] = last;
+            }
+            GroupSync(group);
+            for (int k = 0; k < 2; ++k) {
+                if (!g.Last[k]) {
+                    continue;
+                }
+                const int seq = k == 0 ? seq0 : seq1, chunks = plan.Count[seq];
+                float sumAll, valAll[4];
+                MergePartials<D>(p, p.Partial + ((size_t)plan.Base[seq] * p.Heads + head0 + min(head, heads - 1)) * PITCH, chunks, z, sumAll, valAll);
+                finish(seq, sumAll, valAll);
+            }
         }
-        GroupSync(group); // the group's shared memory is used again by its next chunk
+        GroupSync(group); // the group's shared memory is used again by its next unit
     }
 }
 
@@ -931,6 +1033,9 @@ __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
             ProductPhase(p, sm, l, phase, cursor);
         }
         GridArrive(p);
+        if (!attention && phase == PH_PROJ) {
+            PrepareAttention(p, sm, l);
+        }
         RefillRing(p, sm, &cursor);
         if (!attention && phase == PH_PROJ) {
             attention = true;
@@ -959,7 +1064,7 @@ __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
     }
 }
 
-// PS_THREADS x 168 registers and 195 KB of shared memory: one CTA per SM.
+// PS_THREADS x 168 registers and nearly all of the shared memory: one CTA per SM.
 template <int D>
 __global__ void __launch_bounds__(PS_THREADS, 1) InferLayersKernel(const __grid_constant__ TStepParams p)
 {
@@ -973,6 +1078,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) InferLayersKernel(const __grid_
         sm.Failed = 0;
         sm.Passed = 0;
         sm.Plan[0].Window = sm.Plan[1].Window = -1;
+        sm.PlanOf = 0;
     }
     if (tid < 32) {
         TmemAlloc(&sm.TmemBase, 64);
@@ -1012,7 +1118,6 @@ int InferLayersPersistent(const tsa_infer_model *model, const tsa_kv_seq *const 
     if (rc != TSA_OK) {
         return rc;
     }
-    sms = sms < PS_MAX_SLOTS / PS_GROUPS ? sms : PS_MAX_SLOTS / PS_GROUPS;
     TStepParams p;
     auto shape = [&](int tiles, int columns) {
         // as many items as SMs, each with the same number of column chunks
@@ -1035,7 +1140,11 @@ int InferLayersPersistent(const tsa_infer_model *model, const tsa_kv_seq *const 
     p.HeadSize = D;
     p.PerGroup = AttGroupHeads(d.head_count, D);
     p.HeadGroups = (d.head_count + p.PerGroup - 1) / p.PerGroup;
-    p.PerLoad = 512 / D / p.PerGroup;
+    const int perLoad = 512 / D / p.PerGroup; // a power of two for every size of a group
+    p.PerLoadLog = perLoad >= 8 ? 3 : perLoad >= 4 ? 2 : perLoad >= 2 ? 1 : 0;
+    // as the decode kernel's four warps share the heads of a chunk, 512 columns each
+    const int wide = (hs + 511) / 512;
+    p.Split = wide == 1 ? 4 : wide == 2 ? 2 : 1;
     p.ReluDim = d.relu_dim;
     p.Capacity = capacity;
     p.MaxCtx = maxCtx + 1;
