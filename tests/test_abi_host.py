@@ -74,6 +74,29 @@ def test_bad_arguments_return_status_not_abort():
     assert ctypes.sizeof(abi.InferLayer) == 80 and ctypes.sizeof(abi.InferDims) == 28
 
 
+@pytest.mark.parametrize("matrix", ["qk", "qv", "k", "v", "combiner", "expand", "contract"])
+@pytest.mark.parametrize("address", [None, 4096 + 8])
+def test_infer_layer_matrices_are_checked_before_any_launch(matrix, address):
+    """A matrix off the 16-byte grid (or none) is an error status, whatever layer it belongs to; the addresses are never dereferenced."""
+    lib = abi.lib()
+    layers = (abi.InferLayer * 2)()
+    for layer in layers:
+        for nm in ("qk", "qv", "k", "v", "combiner", "expand", "contract"):
+            setattr(layer, nm, 4096)
+        layer.attention_width = 64
+    setattr(layers[1], matrix, address)
+    im = abi.InferModel()
+    im.dims = abi.InferDims(256, 64, 4, 512, 1000, 1000, 2)
+    im.layers = ctypes.cast(layers, ctypes.POINTER(abi.InferLayer))
+    for nm in ("label_embed", "final_layer", "bias", "rope"):
+        setattr(im, nm, 4096)
+    im.rope_len = 32
+    seqs = (ctypes.c_void_p * 2)(4096, 4096)
+    need = lib.tsa_infer_workspace_bytes(ctypes.byref(im), 1, 8)
+    assert lib.tsa_infer_step(ctypes.byref(im), seqs, 4096, 16, 4096, 1, 1, 8, 4096, None, 4096, need, None, None) == abi.TSA_BAD_ARG
+    assert b"layer 1" in lib.tsa_last_error()
+
+
 @pytest.mark.parametrize("name", ["att_w64_slope05", "att_full_slope0", "att_w1_d32", "att_handmade"])
 def test_span_helpers_match_reference_fixtures(golden_dir, name):
     z = np.load(os.path.join(golden_dir, name + ".npz"))

@@ -330,6 +330,15 @@ extern "C" __attribute__((visibility("default"))) int tsa_infer_step(const tsa_i
     TSA_REQUIRE(d.layer_count == 0 || (model->layers && layerSeqs), "tsa_infer_step: null layers");
     TSA_REQUIRE(model->label_embed && model->final_layer && model->bias && model->rope && model->rope_len > maxCtx,
         "tsa_infer_step: model tables (the rope table must cover position maxCtx = %d, it has %d rows)", maxCtx, model->rope_len);
+    for (int l = 0; l < d.layer_count; ++l) {
+        const tsa_infer_layer &layer = model->layers[l];
+        const void *matrices[7] = {layer.qk, layer.qv, layer.k, layer.v, layer.combiner, layer.expand, layer.contract};
+        for (const void *m : matrices) {
+            TSA_REQUIRE(m && layerSeqs[l], "tsa_infer_step: layer %d has a null matrix or cache", l);
+            TSA_REQUIRE((uintptr_t)m % 16 == 0, "tsa_infer_step: a matrix of layer %d is not 16-byte aligned", l); // copied 16 bytes at a time
+        }
+        TSA_REQUIRE(layer.attention_width >= 0, "tsa_infer_step: layer %d has a negative attention width", l);
+    }
     const TInferBuffers need = CarveInferBuffers(model, nSeq, nullptr);
     TSA_REQUIRE(workspace && workspaceBytes >= need.Total && (uintptr_t)workspace % 256 == 0, "tsa_infer_step: workspace of %zu bytes, 256-byte aligned, needed",
         need.Total);

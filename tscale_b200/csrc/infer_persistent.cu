@@ -1169,12 +1169,6 @@ int InferLayersPersistent(const tsa_infer_model *model, const tsa_kv_seq *const 
     p.NormState = b.NormState;
     p.Partial = b.Partial;
     p.Status = statusWord;
-    for (int l = 0; l < d.layer_count; ++l) {
-        const tsa_infer_layer &layer = model->layers[l];
-        TSA_REQUIRE(layer.qk && layer.qv && layer.k && layer.v && layer.combiner && layer.expand && layer.contract && layerSeqs[l],
-            "tsa_infer_step: layer %d has a null matrix or cache", l);
-        TSA_REQUIRE(layer.attention_width >= 0, "tsa_infer_step: layer %d has a negative attention width", l);
-    }
     int done = 0;
     do {
         p.LayerCount = d.layer_count - done < PS_LAYERS ? d.layer_count - done : PS_LAYERS;
