@@ -136,3 +136,17 @@ def test_batch_of_twenty_sequences():
         assert np.array_equal(logits[s, 0], want_logits), s
     for s in range(2, 20):
         assert np.array_equal(logits[s], logits[s % 2]) and np.array_equal(pred[s], pred[s % 2]), s
+
+
+@pytest.mark.parametrize("offset", [1, 2])
+def test_embedding_table_at_any_address(offset):
+    from tscale_b200 import infer
+    model = O.make_infer_model(97, 256, 64, 2, 1, 96, 16, [(8, 0.0)])
+    gm = infer.InferModel(model, O.fill_rope(64, 4), DEV)
+    labels = torch.tensor([[3, 15], [0, 7]], dtype=torch.int32, device=DEV)
+    want = infer.InferContext(gm, 2, 4).compute_prediction(labels)
+    table = torch.from_numpy(model["label_embed"]).flatten().to(DEV)
+    shifted = torch.zeros(table.numel() + offset, dtype=torch.int8, device=DEV)
+    shifted[offset:] = table
+    gm.c.label_embed = shifted.data_ptr() + offset
+    assert torch.equal(infer.InferContext(gm, 2, 4).compute_prediction(labels), want)

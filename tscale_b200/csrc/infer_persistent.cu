@@ -285,7 +285,8 @@ __device__ __noinline__ float4 EmbedColumns(const TStepParams &p, int s, int col
             }
             continue;
         }
-        const char4 e = *reinterpret_cast<const char4 *>(p.Embed + (size_t)label * p.Dim + col);
+        const int8_t *row = p.Embed + (size_t)label * p.Dim + col;
+        const char4 e = ((uintptr_t)row & 3) == 0 ? *reinterpret_cast<const char4 *>(row) : make_char4(row[0], row[1], row[2], row[3]);
         v.x = __fadd_rn(v.x, __fmul_rn((float)e.x, p.EmbedScale));
         v.y = __fadd_rn(v.y, __fmul_rn((float)e.y, p.EmbedScale));
         v.z = __fadd_rn(v.z, __fmul_rn((float)e.z, p.EmbedScale));
