@@ -130,6 +130,23 @@ def test_decode_window_alibi_and_self():
     _decode_case(6, [40, 0], 2, 128, 64, 0.5)         # an empty sequence gets its first token
 
 
+def test_decode_replaces_a_workspace_that_is_too_small():
+    from tscale_b200 import ops
+    cache = ops.KVCache(2, 40, 4, 64, DEV)
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(8)
+    cache.k.random_(-127, 128, generator=gen)
+    cache.v.random_(-127, 128, generator=gen)
+    cache.k_scale.fill_(1e-3)
+    cache.v_scale.fill_(1e-2)
+    cache.ctx_lens.fill_(30)
+    cache.max_ctx = 30
+    q = torch.ones((2, 256), dtype=torch.int8, device=DEV)
+    want = cache.decode(q, None, 100, 0.0)
+    cache.workspace = torch.empty(64, dtype=torch.uint8, device=DEV)
+    assert torch.equal(cache.decode(q, None, 100, 0.0), want)
+
+
 def test_decode_matches_reference_fixture(golden_dir):
     from tscale_b200 import ops
     z = np.load(os.path.join(golden_dir, "decode_w64.npz"))

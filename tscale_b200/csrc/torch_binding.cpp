@@ -421,6 +421,12 @@ PyObject *KvAppend(PyObject *, PyObject *const *a, Py_ssize_t n)
     });
 }
 
+// cfg, nSeq, heads, maxCtx
+PyObject *AttDecodeWorkspaceBytes(PyObject *, PyObject *const *a, Py_ssize_t n)
+{
+    return Guard<4>(n, [&] { return PyLong_FromSize_t(g.AttDecodeWs(Struct<tsa_decode_cfg>(a[0]), (int)Int(a[1]), (int)Int(a[2]), (int)Int(a[3]))); });
+}
+
 // cfg, seqs, ctxLens, nSeq, maxCtx, q, qScale, window, slope, out, heads, workspace (None: the library's static scratch), status
 PyObject *AttDecode(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
@@ -467,6 +473,7 @@ PyObject *InferStep(PyObject *, PyObject *const *a, Py_ssize_t n)
 PyMethodDef g_methods[] = {FAST("bind", Bind), FAST("att_fwd", AttFwd), FAST("att_bwd", AttBwd), FAST("quant_rows", QuantRows),
     FAST("norm_rope_quant", NormRopeQuant), FAST("matmul_norm_rope_quant", MatmulNormRopeQuant), FAST("rope_norm_bwd", RopeNormBwd),
     FAST("kv_product", KvProduct), FAST("kv_product_bwd", KvProductBwd), FAST("calc_dscale", CalcDScale), FAST("kv_append", KvAppend),
+    FAST("att_decode_workspace_bytes", AttDecodeWorkspaceBytes),
     FAST("att_decode", AttDecode), FAST("infer_step", InferStep), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", "torch-tensor binding of libtsa_b200.so", -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 

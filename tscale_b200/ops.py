@@ -336,8 +336,8 @@ class KVCache:
         self.max_ctx = min(self.capacity, self.max_ctx + 1)
 
     def decode(self, q, q_scale, window, slope, out=None, status=None):
-        if self.workspace is None:
-            need = abi.lib().tsa_att_decode_workspace_bytes(ctypes.byref(self.cfg), self.n_seq, self.heads, self.capacity)
+        need = _native.att_decode_workspace_bytes(self.cfg, self.n_seq, self.heads, self.capacity)
+        if self.workspace is None or self.workspace.numel() < need:
             self.workspace = torch.empty(max(1, need), dtype=torch.uint8, device=q.device)
         rc, out = _native.att_decode(self.cfg, self.seqs, self.ctx_lens, self.n_seq, self.max_ctx, q, q_scale, window, slope, out, self.heads,
                                      self.workspace, status)
