@@ -166,3 +166,13 @@ def test_header_is_plain_c_and_links(tmp_path):
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
     assert int(out[0]) == len(names) == len(abi.EXPORTS)
     assert int(out[1]) == 4 + 2      # one span per row that has keys: rows 1..4 of the first fragment, rows 1..2 of the second
+
+
+def test_masks_saved_without_the_last_device_load():
+    """A mask whose saved state has only the arrays and the table of device copies."""
+    import torch
+    saved = ops.Mask.window([70, 3], 0)
+    mask = ops.Mask.__new__(ops.Mask)
+    mask.__dict__.update({k: v for k, v in vars(saved).items() if k != "_last"})
+    for _ in range(2):
+        assert all(torch.equal(a, b) for a, b in zip(mask.dev(torch.device("cpu")), saved.dev(torch.device("cpu"))))

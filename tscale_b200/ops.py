@@ -43,13 +43,14 @@ class Mask:
     """Attention mask in the grouped form the kernels take (TAttentionSpanGroup<64> records), for the
     mask itself and for its transpose.  Built on the host by the library's span helpers."""
 
+    _last = (None, None)  # device of the last call of dev and its arrays; of the class, as saved masks may not have it
+
     def __init__(self, length, groups, group_ptr, rev_groups, rev_group_ptr):
         self.len = length
         self.len_att_tiles = (length + abi.ATT_GROUP - 1) // abi.ATT_GROUP
         self.groups, self.group_ptr = groups, group_ptr          # numpy int32 [n][130], [tiles+1]
         self.rev_groups, self.rev_group_ptr = rev_groups, rev_group_ptr
         self._dev = {}
-        self._last = (None, None)  # device of the last call and its arrays
 
     @staticmethod
     def _run_grouper(fn, cap):
