@@ -4,6 +4,7 @@ host span helpers agree with the reference's preprocessing (golden files) and wi
 import ctypes
 import os
 import re
+import subprocess
 
 import numpy as np
 import pytest
@@ -176,3 +177,11 @@ def test_masks_saved_without_the_last_device_load():
     mask.__dict__.update({k: v for k, v in vars(saved).items() if k != "_last"})
     for _ in range(2):
         assert all(torch.equal(a, b) for a, b in zip(mask.dev(torch.device("cpu")), saved.dev(torch.device("cpu"))))
+
+
+def test_library_builds_without_python():
+    """The default target is the C ABI library alone; the torch binding, which needs Python and torch's headers, has its own."""
+    csrc = os.path.join(ROOT, "tscale_b200", "csrc")
+    plan = lambda *t: subprocess.run(["make", "-n", "-B", "-C", csrc, *t], check=True, capture_output=True, text=True).stdout
+    assert "libtsa_b200.so" in plan() and "torch" not in plan()
+    assert "torch_binding.cpp" in plan("binding")

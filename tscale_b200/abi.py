@@ -176,7 +176,7 @@ def native():
         try:
             from . import _native
         except ImportError as e:
-            raise ImportError("tscale_b200: _native.so cannot be loaded (%s); build it with `make -C tscale_b200/csrc` "
+            raise ImportError("tscale_b200: _native.so cannot be loaded (%s); build it with `make -C tscale_b200/csrc binding` "
                               "(or __graft_entry__.build())." % e) from e
         _native.bind(lib()._handle)
         _binding = _native
