@@ -6,8 +6,8 @@
 // logit 0, softmax in base 2, out = sum softmax * vScale[to][h] * v[to].
 //
 // Layout: per sequence K and V are [capacity][H*D] int8 with the heads of one token contiguous, so a
-// token range of a sequence is one contiguous byte range.  A CTA owns (sequence, chunk of DEC_CHUNK
-// tokens) and all heads: a 128-bit load per lane covers 512 contiguous bytes per warp = 32/LPH heads
+// token range of a sequence is one contiguous byte range.  A CTA owns a chunk of a
+// sequence's tokens and all heads: a 128-bit load per lane covers 512 contiguous bytes per warp = 32/LPH heads
 // of one token (LPH = D/16 lanes per head).  The int8 dot uses dp4a (exact int32), partial sums are
 // reduced over the LPH lanes of a head with shuffles.  Each CTA keeps an online (max, sum, acc[D])
 // per head and writes it to the scratch buffer; a second kernel merges the chunks of a sequence and
@@ -25,7 +25,6 @@ struct TDecodeParams {
     int NSeq;
     int HeadCount;
     int Window;
-    int ScaleDtype;
     int OutDtype;
     float Slope;
     float DotScale;  // attDotScale
@@ -39,28 +38,13 @@ struct TDecodeParams {
     int *Status;     // device status word (may be null)
     int MaxSlots;    // TargetCtas + nSeq
     int MaxCtx;      // the caller's upper bound of CtxLens: sizes the grid, checked on the device
-    // inference step only (null otherwise): the merge kernel also writes the combiner input
-    // kv[seq][head][blk][z] = int8(KvKey[seq][head][z ^ blk] * out[seq][head][z]), blk = 0..3 (KVProduct, cpu_infer.cpp:318-337)
-    const int8_t *KvKey;
-    int8_t *KvOut;
-    int CtxBias;     // added to every CtxLens entry: 1 when the caller has written the new token but not yet counted it
 };
-
-__device__ __forceinline__ int CtxLenOf(const TDecodeParams &p, int s)
-{
-    return p.CtxLens[s] + p.CtxBias;
-}
-
-__device__ __forceinline__ float LoadScale(const void *base, size_t idx, int dt)
-{
-    return dt == TSA_F16 ? __half2float(((const __half *)base)[idx]) : ((const float *)base)[idx];
-}
 
 constexpr int DEC_MIN_CHUNK = 16; // keys: short windows are spread over several CTAs of two batches rather than one CTA of eight
 
-__device__ __forceinline__ int SeqKeys(const int *ctxLens, int ctxBias, int s, int window)
+__device__ __forceinline__ int SeqKeys(const int *ctxLens, int s, int window)
 {
-    int ctxLen = ctxLens[s] + ctxBias;
+    int ctxLen = ctxLens[s];
     if (ctxLen <= 0) {
         return 0;
     }
@@ -69,16 +53,16 @@ __device__ __forceinline__ int SeqKeys(const int *ctxLens, int ctxBias, int s, i
     return j1 - j0;
 }
 
-// Balanced plan: all keys of all sequences are cut into chunks of (nearly) the same size C = total / TargetCtas, so
-// that every CTA streams the same number of bytes whatever the mix of context lengths.  Chunk slots are numbered
-// sequence by sequence.  Every CTA derives the plan from ctxLens itself (a block-wide sum and scan); CTA 0 also
-// writes it to the workspace header for the merge kernel.  Returns false if this CTA has no chunk.
-// barrier of the DEC_WARPS * 32 planning threads (the producer warp does not take part)
+// barrier of the CTA's DEC_WARPS * 32 threads
 __device__ __forceinline__ void PlanSync()
 {
     asm volatile("bar.sync 1, %0;" ::"n"(DEC_WARPS * 32) : "memory");
 }
 
+// Balanced plan: all keys of all sequences are cut into chunks of (nearly) the same size C = total / TargetCtas, so
+// that every CTA streams the same number of bytes whatever the mix of context lengths.  Chunk slots are numbered
+// sequence by sequence.  Every CTA derives the plan from ctxLens itself (a block-wide sum and scan); CTA 0 also
+// writes it to the workspace header for the merge kernel.  Returns false if this CTA has no chunk.
 __device__ bool DecodePlan(const TDecodeParams &p, int slot, int *pSeq, int *pBeg, int *pEnd)
 {
     __shared__ int red[DEC_WARPS];
@@ -88,8 +72,8 @@ __device__ bool DecodePlan(const TDecodeParams &p, int slot, int *pSeq, int *pBe
     // total number of keys
     int sum = 0;
     for (int s = tid; s < p.NSeq; s += nThreads) {
-        sum += SeqKeys(p.CtxLens, p.CtxBias, s, p.Window);
-        if (CtxLenOf(p, s) > p.MaxCtx && blockIdx.x == 0 && p.Status) {
+        sum += SeqKeys(p.CtxLens, s, p.Window);
+        if (p.CtxLens[s] > p.MaxCtx && blockIdx.x == 0 && p.Status) {
             atomicOr(p.Status, kDevBadSpan); // the grid was sized for shorter sequences
         }
     }
@@ -118,7 +102,7 @@ __device__ bool DecodePlan(const TDecodeParams &p, int slot, int *pSeq, int *pBe
             const int mid = (lo + hi) >> 1;
             int cnt = 0;
             for (int s = tid; s < p.NSeq; s += nThreads) {
-                cnt += (SeqKeys(p.CtxLens, p.CtxBias, s, p.Window) + mid * 8 - 1) / (mid * 8);
+                cnt += (SeqKeys(p.CtxLens, s, p.Window) + mid * 8 - 1) / (mid * 8);
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
@@ -146,7 +130,7 @@ __device__ bool DecodePlan(const TDecodeParams &p, int slot, int *pSeq, int *pBe
     const int s0 = tid * per, s1 = min(s0 + per, p.NSeq);
     int mine = 0;
     for (int s = s0; s < s1; ++s) {
-        mine += (SeqKeys(p.CtxLens, p.CtxBias, s, p.Window) + chunk - 1) / chunk;
+        mine += (SeqKeys(p.CtxLens, s, p.Window) + chunk - 1) / chunk;
     }
     // exclusive scan over the threads' counts: shuffles inside a warp, the warps' sums through shared memory (one thread walking
     // 128 sums in shared memory took 2 us of every call)
@@ -174,13 +158,13 @@ __device__ bool DecodePlan(const TDecodeParams &p, int slot, int *pSeq, int *pBe
         p.Plan[0] = chunk;
     }
     for (int s = s0; s < s1; ++s) {
-        int keys = SeqKeys(p.CtxLens, p.CtxBias, s, p.Window);
+        int keys = SeqKeys(p.CtxLens, s, p.Window);
         int n = (keys + chunk - 1) / chunk;
         if (writePlan) {
             p.Plan[1 + s] = base;
         }
         if (slot >= base && slot < base + n) {
-            int ctxLen = CtxLenOf(p, s);
+            int ctxLen = p.CtxLens[s];
             int j0, j1;
             KeyRange(ctxLen, p.Window, &j0, &j1);
             found[0] = s;
@@ -203,7 +187,7 @@ __device__ bool DecodePlan(const TDecodeParams &p, int slot, int *pSeq, int *pBe
 // V (16 bytes each) in flight; four such CTAs are resident per SM.
 // FINAL: every sequence attends so few keys (a short window or short contexts, decided on the host from its bound) that
 // one CTA takes a whole sequence: no plan, no partials and no merge kernel -- the CTA adds the sink and writes the
-// result (and the inference step's combiner input) itself.
+// result itself.
 template <int D, int DEC_UNROLL, bool SCALE_F16, bool FINAL>
 __global__ void __launch_bounds__(DEC_WARPS * 32, 4) DecodePartialKernel(TDecodeParams p)
 {
@@ -215,7 +199,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 4) DecodePartialKernel(TDecode
     PdlWait();
     if (FINAL) {
         seq = blockIdx.x;
-        const int len = CtxLenOf(p, seq);
+        const int len = p.CtxLens[seq];
         if (len > p.MaxCtx && threadIdx.x == 0 && p.Status) {
             atomicOr(p.Status, kDevBadSpan); // the launch was sized for shorter sequences
         }
@@ -227,7 +211,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 4) DecodePartialKernel(TDecode
     } else if (!DecodePlan(p, chunk, &seq, &cBeg, &cEnd)) {
         return;
     }
-    const int ctxLen = CtxLenOf(p, seq);
+    const int ctxLen = p.CtxLens[seq];
     const int cur = ctxLen - 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane % LPH;             // 16-byte slice inside the head
@@ -293,25 +277,11 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, 4) DecodePartialKernel(TDecode
                 const float mAll = fmaxf(m, 0.0f);
                 const float f = exp2f(m - mAll);
                 const float lAll = exp2f(-mAll) + f * l;
-                const size_t rowSize = (size_t)H * D;
-                int4 keyWords = make_int4(0, 0, 0, 0);
-                if (p.KvOut) {
-                    keyWords = *reinterpret_cast<const int4 *>(p.KvKey + seq * rowSize + head * D + sub * 16);
-                }
-                const int8_t *key = reinterpret_cast<const int8_t *>(&keyWords);
-                int8_t *kv = p.KvOut ? p.KvOut + (seq * rowSize + head * D) * 4 : nullptr;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const float res = ctxLen > 0 ? (f * acc[i]) / lAll : 0.0f;
                     const int x = sub * 16 + i;
                     StoreFromFloat(p.Out.Row(seq), head * D + x, p.OutDtype, res);
-                    if (kv) {
-#pragma unroll
-                        for (int blk = 0; blk < 4; ++blk) {
-                            // ConvertToInt8 (cpu_infer.cpp:88-92): round to nearest even, clamp to +-127
-                            kv[blk * D + x] = (int8_t)max(-127, min(127, __float2int_rn(__fmul_rn((float)key[i ^ blk], res))));
-                        }
-                    }
                 }
             }
         } else if (headOk && tokenPart == 0) {
@@ -346,7 +316,7 @@ __global__ void __launch_bounds__(DEC_MERGE_THREADS) DecodeCombineKernel(TDecode
     const int group = tid / LPC, sub = tid % LPC;
     PdlTrigger();
     PdlWait();
-    const int ctxLen = CtxLenOf(p, seq);
+    const int ctxLen = p.CtxLens[seq];
     float m = 0; // the sink has logit 0 (softMax.Add(0), cpu_infer.cpp:444)
     if (ctxLen > 0) {
         const int first = p.Plan[1 + seq];
@@ -400,16 +370,6 @@ __global__ void __launch_bounds__(DEC_MERGE_THREADS) DecodeCombineKernel(TDecode
         res = acc / l;
     }
     StoreFromFloat(p.Out.Row(seq), head * D + x, p.OutDtype, res);
-    if (p.KvOut) {
-        const size_t rowSize = (size_t)p.HeadCount * D;
-        const int8_t *key = p.KvKey + seq * rowSize + head * D;
-        int8_t *kv = p.KvOut + (seq * rowSize + head * D) * 4;
-#pragma unroll
-        for (int blk = 0; blk < 4; ++blk) {
-            // ConvertToInt8 (cpu_infer.cpp:88-92): round to nearest even, clamp to +-127
-            kv[blk * D + x] = (int8_t)max(-127, min(127, __float2int_rn(__fmul_rn((float)key[x ^ blk], res))));
-        }
-    }
 }
 
 __global__ void KvAppendKernel(const tsa_kv_seq *seqs, int *ctxLens, int nSeq, int capacity, int rowBytes, int headCount, int scaleBytes,
@@ -448,7 +408,10 @@ __global__ void KvAppendKernel(const tsa_kv_seq *seqs, int *ctxLens, int nSeq, i
     }
 }
 
-constexpr int DEC_SINGLE_KEYS = 16;       // up to this many keys per sequence (one batch per warp) one CTA takes the whole sequence; with 64 keys four CTAs and the merge kernel are faster (0.80 against 0.81 ms per inference step)
+// Up to this many keys per sequence (one batch per warp) one CTA takes the whole sequence.  With a bound of 64 a call whose window is 64 takes
+// 7.7 instead of 6.5 us for one sequence and 10.8 instead of 7.7 for eight (16 heads x 128), 11.1 instead of 12.0 for 64; with a
+// window of 32 batches of 64 gain (10.8 -> 7.9 us) and of eight lose (7.4 -> 7.7).
+constexpr int DEC_SINGLE_KEYS = 16;
 constexpr int DEC_MAX_TARGET_CTAS = 1024; // workspace is sized for this many chunk slots plus one per sequence
 
 static size_t DecodeHeaderBytes(int nSeq)
@@ -462,12 +425,8 @@ size_t DecodeWorkspaceBytes(int headDim, int nSeq, int headCount, int maxCtx)
     return DecodeHeaderBytes(nSeq) + (size_t)(DEC_MAX_TARGET_CTAS + nSeq) * headCount * (headDim + 4) * sizeof(float);
 }
 
-int LaunchDecode(const tsa_decode_cfg *cfg, TDecodeParams p, int maxCtx, cudaStream_t stream, const int8_t *kvKey = nullptr, int8_t *kvOut = nullptr,
-    int ctxBias = 0)
+int LaunchDecode(const tsa_decode_cfg *cfg, TDecodeParams p, int maxCtx, cudaStream_t stream)
 {
-    p.KvKey = kvKey;
-    p.KvOut = kvOut;
-    p.CtxBias = ctxBias;
     int dev = 0, sms = 0;
     int rc = CheckCuda(cudaGetDevice(&dev), "cudaGetDevice");
     if (rc == TSA_OK) {
@@ -535,12 +494,9 @@ extern "C" __attribute__((visibility("default"))) size_t tsa_att_decode_workspac
     return DecodeWorkspaceBytes(cfg->head_dim, nSeq, headCount, maxCtx);
 }
 
-namespace tsa {
-// tsa_att_decode plus the inference step's combiner input written by the merge kernel (kvKey int8 [nSeq][H*D] packed,
-// kvOut int8 [nSeq][4*H*D] packed; both null for the plain entry point); ctxBias is added to every ctxLens entry
-int DecodeWithKvProduct(const tsa_decode_cfg *cfg, const tsa_kv_seq *seqs, const int *ctxLens, int nSeq, int maxCtx,
+extern "C" __attribute__((visibility("default"))) int tsa_att_decode(const tsa_decode_cfg *cfg, const tsa_kv_seq *seqs, const int *ctxLens, int nSeq, int maxCtx,
     tsa_ptr2d q, tsa_ptr2d qScale, int window, float alibiSlope, tsa_ptr2d out, int headCount,
-    void *workspace, size_t workspaceBytes, int *statusWord, tsa_stream_t stream, const int8_t *kvKey, int8_t *kvOut, int ctxBias)
+    void *workspace, size_t workspaceBytes, int *statusWord, tsa_stream_t stream)
 {
     int rc = CheckDecodeCfg(cfg, "tsa_att_decode");
     if (rc != TSA_OK) {
@@ -568,7 +524,6 @@ int DecodeWithKvProduct(const tsa_decode_cfg *cfg, const tsa_kv_seq *seqs, const
     p.NSeq = nSeq;
     p.HeadCount = headCount;
     p.Window = window;
-    p.ScaleDtype = cfg->scale_dtype;
     p.OutDtype = cfg->out_dtype;
     p.Slope = alibiSlope;
     p.DotScale = HostAttDotScale(cfg->head_dim);
@@ -577,16 +532,7 @@ int DecodeWithKvProduct(const tsa_decode_cfg *cfg, const tsa_kv_seq *seqs, const
     p.QScale = P2D<float>(qScale);
     p.Out = P2D<char>(out);
     p.Partial = (float *)workspace;
-    return LaunchDecode(cfg, p, maxCtx, (cudaStream_t)stream, kvKey, kvOut, ctxBias);
-}
-} // namespace tsa
-
-extern "C" __attribute__((visibility("default"))) int tsa_att_decode(const tsa_decode_cfg *cfg, const tsa_kv_seq *seqs, const int *ctxLens, int nSeq, int maxCtx,
-    tsa_ptr2d q, tsa_ptr2d qScale, int window, float alibiSlope, tsa_ptr2d out, int headCount,
-    void *workspace, size_t workspaceBytes, int *statusWord, tsa_stream_t stream)
-{
-    return DecodeWithKvProduct(cfg, seqs, ctxLens, nSeq, maxCtx, q, qScale, window, alibiSlope, out, headCount, workspace, workspaceBytes, statusWord, stream,
-        nullptr, nullptr, 0);
+    return LaunchDecode(cfg, p, maxCtx, (cudaStream_t)stream);
 }
 
 extern "C" __attribute__((visibility("default"))) int tsa_kv_append(const tsa_decode_cfg *cfg, const tsa_kv_seq *seqs, int *ctxLens, int nSeq, int capacity,
@@ -686,6 +632,6 @@ extern "C" __attribute__((visibility("default"))) int tsa_att_decode_static(cons
     if (rc != TSA_OK) {
         return rc;
     }
-    return DecodeWithKvProduct(cfg, seqs, ctxLens, nSeq, maxCtx, q, qScale, window, alibiSlope, out, headCount, scratch, kStaticScratchBytes,
-        statusWord, stream, nullptr, nullptr, 0);
+    return tsa_att_decode(cfg, seqs, ctxLens, nSeq, maxCtx, q, qScale, window, alibiSlope, out, headCount, scratch, kStaticScratchBytes,
+        statusWord, stream);
 }

@@ -41,14 +41,6 @@ __device__ __forceinline__ int4 LoadRow(const int4 *p)
 {
     return COHERENT ? __ldcg(p) : __ldg(p);
 }
-// sum of four (unsigned byte of a) x (signed byte of b) products, plus c
-__device__ __forceinline__ int Dp4aUS(uint32_t a, uint32_t b, int c)
-{
-    int d;
-    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-
 // two 16-bit x 8-bit products added to c: a = (w0 | w1 << 16) unsigned, b bytes signed; lo takes bytes 0 and 1 of b, hi bytes 2 and 3
 __device__ __forceinline__ int Dp2aLoUS(uint32_t a, uint32_t b, int c)
 {
