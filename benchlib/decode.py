@@ -216,10 +216,10 @@ def run(args, rank, world, local_rank, emit=True, quick=False):
                 "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
                 "peak_source": "MEASURED_PEAKS.json copy bandwidth (%s)" % peaks["_source"], "frac_of_8tbs_nominal": achieved / 8000.0,
                 "ms_per_launch": k_ms, "algorithmic_bytes_per_launch": k_bytes,
-                # not measured in this run: the ratio comes from the ncu capture of this workload at this size
-                # (profiles/decode_partial_i8_d128_64seq.md: 1.1588 GB of DRAM traffic for 1.166 GB algorithmic)
-                "traffic": 0.994 * k_bytes, "traffic_source": "algorithmic bytes x 0.994, the dram/algorithmic ratio of the committed ncu capture "
-                                                                "profiles/decode_partial_i8_d128_64seq.md (same workload and size); not re-measured per run"}
+                # not measured in this run: the ratio comes from an ncu capture of this workload at this size (1.1588 GB of DRAM
+                # traffic for 1.166 GB algorithmic)
+                "traffic": 0.994 * k_bytes, "traffic_source": "algorithmic bytes x 0.994, the dram/algorithmic ratio of an ncu capture of the same "
+                                                                "workload and size; not re-measured per run"}
     cpu_baseline = None
     if world == 1 and not args.no_cpu_baseline and not quick:
         threads = os.cpu_count() or 1

@@ -145,7 +145,7 @@ def run(args, rank, world, local_rank):
     ctx.set_lengths(ctx0)
     labels = torch.randint(0, VOCAB, (N_SEQ, 1), generator=gen, device=dev, dtype=torch.int32)
     pred = torch.empty((N_SEQ, VOCAB), dtype=torch.float32, device=dev)
-    launches_per_step = 2 + LAYERS * 7 + 4   # embedding, first normalise; per layer 4 matrix products, rope, 2 attention kernels; count, final layer, 2 softmax kernels
+    launches_per_step = 4   # all layers, final layer, 2 softmax kernels
 
     # one eager step (also sets the kernels' attributes), then the step as a CUDA graph
     ctx.compute_prediction(labels, prediction=pred)
@@ -224,7 +224,7 @@ def run(args, rank, world, local_rank):
     peaks = load_peaks()
     step_bytes = nbytes / steps
     achieved = step_bytes / (ms_step * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "whole step: DecodePartialKernel<64> on the wide layers + int8 matrix products", "achieved": achieved,
+    roofline = {"bound": "hbm", "kernel": "whole step: InferLayersKernel<64> (all layers), final layer and softmax", "achieved": achieved,
                 "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
                 "peak_source": "MEASURED_PEAKS.json copy bandwidth (%s)" % peaks["_source"], "ms_per_launch": ms_step,
                 "algorithmic_bytes_per_launch": step_bytes, "kv_bytes_per_step": step_bytes - weight_bytes(), "weight_bytes_per_step": weight_bytes(),

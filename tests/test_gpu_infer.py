@@ -90,7 +90,7 @@ def test_first_step_bit_exact_and_batch_independence():
 
 
 def test_wide_matrices_chunked_through_shared_memory():
-    """64 sequences with a combiner input of 4 * 1536 columns: the batch's vectors do not fit shared memory at once."""
+    """64 sequences with a combiner input of 4 * 1536 columns, which many CTAs share."""
     model = O.make_infer_model(92, 256, 128, 12, 1, 64, 16, [(8, 0.0)])
     rng = np.random.default_rng(93)
     steps = 3
@@ -123,7 +123,7 @@ def test_bad_arguments():
 
 
 def test_batch_of_twenty_sequences():
-    """17 to 32 sequences take the matrix products' two-way sequence split: exact first-step logits, identical slots."""
+    """Accumulator columns past the batch: exact first-step logits, identical slots."""
     model = O.make_infer_model(95, 256, 64, 2, 1, 96, 16, [(8, 0.0), (32, 0.5)])
     rng = np.random.default_rng(96)
     steps = 4

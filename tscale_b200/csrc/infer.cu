@@ -1,21 +1,20 @@
-// One-token inference step of the int8 model over a batch of sequences with per-layer int8 KV caches: the caller of
-// the decode attention kernel.  Replaces NCPUInfer::ComputePrediction / AddLookupProduct of the reference
+// One-token inference step of the int8 model over a batch of sequences with per-layer int8 KV caches.  Replaces NCPUInfer::ComputePrediction / AddLookupProduct of the reference
 // (code/gpt/train/cpu_infer.cpp:466-560), which runs one sequence on the CPU, by a batch of sequences on the GPU:
 //
 //   state = sum of label embeddings * scale                                    (cpu_infer.cpp:536-543)
 //   per layer (cpu_infer.cpp:466-527):
 //     norm   = NormalizeState(state, tiles of 128)            -> int8
 //     qk, qv, k, v = int8 matrix * norm (exact int32), rope on qk and qv, NormalizeState per head -> int8
-//     cache.append(qv, qvScale * QVScale * VEC_SCALE * dotScale(dim), v)  (written by the rope kernel);  val = decode attention(qk, cache)
-//     kv     = int8(k[z ^ blk] * val[z]), 4 blocks per head (written by the decode merge kernel); state += Combiner * kv * scale
+//     cache.append(qv, qvScale * QVScale * VEC_SCALE * dotScale(dim), v);  val = decode attention(qk, cache)
+//     kv     = int8(k[z ^ blk] * val[z]), 4 blocks per head; state += Combiner * kv * scale
 //     norm   = NormalizeState(state);  relu = max(0, NormalizeState(Expand * norm, per head));  state += Contract * relu * scale
 //   prediction = softmax2(FinalLayer * NormalizeState(state) * scale + bias)    (cpu_infer.cpp:549-558)
 //
-// Everything but the attention weights and the last softmax is integer or single-rounded float arithmetic in the
-// reference's order (sums of squares are accumulated sequentially like the scalar loops there), so those stages are
-// bit-identical to the CPU code; the attention (tsa_att_decode) and the softmax use exp2 instead of the CPU's
-// polynomial.  The matrix products read every int8 weight once per step for the whole batch (tcgen05 kind::i8, exact
-// int32 accumulators); at realistic context lengths the step is dominated by the KV-cache stream of the decode kernel.
+// The layers are one persistent kernel (infer_persistent.cu); here are the final layer, the softmax and the entry points.  Everything but
+// the attention weights and the last softmax is integer or single-rounded float arithmetic in the reference's order (sums of squares
+// are accumulated sequentially like the scalar loops there), so those stages are bit-identical to the CPU code; the attention and the
+// softmax use exp2 instead of the CPU's polynomial.  The matrix products read every int8 weight once per step for the whole batch (tcgen05
+// kind::i8, exact int32 accumulators).
 #include "att_sm100_common.cuh"
 #include "infer_internal.cuh"
 
@@ -269,8 +268,7 @@ TInferBuffers CarveInferBuffers(const tsa_infer_model *m, int nSeq, void *base)
         off += Align256(bytes);
         return p;
     };
-    b.SyncInts = 64 + Align256((size_t)nSeq * headGroups * sizeof(int)) / sizeof(int);
-    b.Sync = (int *)take(sizeof(int) * b.SyncInts);
+    b.Sync = (int *)take(sizeof(int) * (64 + (size_t)nSeq * headGroups));
     b.Proj = (int *)take(sizeof(int) * nSeq * 4 * hs);
     b.Comb = (int *)take(sizeof(int) * nSeq * d.dim);
     b.Expand = (int *)take(sizeof(int) * nSeq * d.relu_dim);

@@ -55,8 +55,8 @@ inline int AttGroupHeads(int heads, int headDim)
 
 struct TInferBuffers {
     float *StateA, *StateB, *Logits, *SoftmaxPart, *Partial;
-    int *Sync;      // grid barrier and the attention chunks' counters, then the int32 sums: zeroed before every step
-    size_t SyncInts, ZeroBytes;
+    int *Sync;      // grid barrier (64 words), counters of chunks done, then the int32 sums: zeroed before every step
+    size_t ZeroBytes;
     int *Proj, *Comb, *Expand, *Contract;
     int8_t *NormState, *K8, *Kv8;
     size_t Total;

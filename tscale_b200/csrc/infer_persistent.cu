@@ -47,7 +47,7 @@ constexpr int PS_CHUNKS_PER_SM = 4;            // the keys of a layer are cut in
 constexpr int PS_MIN_CHUNK = 16;               // keys
 constexpr long long PS_WAIT_CYCLES = 1ll << 31;
 
-enum { PH_PROJ = 0, PH_COMB = 1, PH_EXPAND = 2, PH_CONTRACT = 3, PH_FINAL = 4 };
+enum { PH_PROJ = 0, PH_COMB = 1, PH_EXPAND = 2, PH_CONTRACT = 3 };
 enum { SRC_EMBED = 0, SRC_SUM = 1, SRC_STATE = 2 }; // where the first product of a launch gets the state from
 
 struct TStepLayer {
@@ -466,51 +466,49 @@ __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm
     for (int index = sm.PhaseBegin[phase]; index < end; ++index) {
         const TWeightTile t = TileAt(p, sm, index);
         const int chunk = t.Chunk, tile = t.Matrix == 0 || t.Matrix > 3 ? t.Tile : -1; // tile 0 of the phase also keeps the new state
-        {
-            if (phase == PH_PROJ || phase == PH_EXPAND) {
-                // StateA and StateB take turns: the first holds the state in front of the attention block, the second behind it
-                const bool proj = phase == PH_PROJ;
-                const int source = proj && l == 0 ? p.FirstSource : SRC_SUM;
-                StageState(p, sm, chunk, source, proj == (source == SRC_SUM) ? p.StateB : p.StateA, proj ? p.Contract : p.Comb,
-                    proj ? (l > 0 ? p.Layers[l - 1].ContractScale : 0.0f) : layer.CombScale, tile != 0 || source == SRC_STATE ? nullptr : proj ? p.StateA : p.StateB);
-                NormaliseStaged(p, sm);
-            } else if (phase == PH_COMB) {
-                for (int i = tid; i < p.NSeq * 8; i += PS_THREADS) {
-                    StoreCodes(sm.B, i >> 3, i & 7, __ldcg(reinterpret_cast<const int4 *>(p.Kv8 + (size_t)(i >> 3) * 4 * hs + chunk * 128 + (i & 7) * 16)));
-                }
-            } else {
-                NormaliseRelu(p, sm, chunk);
+        if (phase == PH_PROJ || phase == PH_EXPAND) {
+            // StateA and StateB take turns: the first holds the state in front of the attention block, the second behind it
+            const bool proj = phase == PH_PROJ;
+            const int source = proj && l == 0 ? p.FirstSource : SRC_SUM;
+            StageState(p, sm, chunk, source, proj == (source == SRC_SUM) ? p.StateB : p.StateA, proj ? p.Contract : p.Comb,
+                proj ? (l > 0 ? p.Layers[l - 1].ContractScale : 0.0f) : layer.CombScale, tile != 0 || source == SRC_STATE ? nullptr : proj ? p.StateA : p.StateB);
+            NormaliseStaged(p, sm);
+        } else if (phase == PH_COMB) {
+            for (int i = tid; i < p.NSeq * 8; i += PS_THREADS) {
+                StoreCodes(sm.B, i >> 3, i & 7, __ldcg(reinterpret_cast<const int4 *>(p.Kv8 + (size_t)(i >> 3) * 4 * hs + chunk * 128 + (i & 7) * 16)));
             }
-            // this thread's part of the tile has landed: the groups requested behind it (one per tile, at most PS_RING - 1 tiles are
-            // requested and not used up) may still be on their way
-            if (cursor.Requested - cursor.Used == PS_RING - 1) {
-                CpAsyncWait<PS_RING - 2>();
-            } else {
-                CpAsyncWait<0>();
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            TcFenceBefore();
-            __syncthreads();
-            TcFenceAfter();
-            if (warp == 0 && ElectOne()) {
-                const uint32_t sA = SmemAddr(sm.Ring[cursor.Used % PS_RING]), sB = SmemAddr(sm.B);
+        } else {
+            NormaliseRelu(p, sm, chunk);
+        }
+        // this thread's part of the tile has landed: the groups requested behind it (one per tile, at most PS_RING - 1 tiles are
+        // requested and not used up) may still be on their way
+        if (cursor.Requested - cursor.Used == PS_RING - 1) {
+            CpAsyncWait<PS_RING - 2>();
+        } else {
+            CpAsyncWait<0>();
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        TcFenceBefore();
+        __syncthreads();
+        TcFenceAfter();
+        if (warp == 0 && ElectOne()) {
+            const uint32_t sA = SmemAddr(sm.Ring[cursor.Used % PS_RING]), sB = SmemAddr(sm.B);
 #pragma unroll
-                for (int ks = 0; ks < 4; ++ks) {
-                    MmaI8SS(sm.TmemBase, MakeSmemDesc(sA + ks * 32, 16, 1024, 128), MakeSmemDesc(sB + ks * 32, 16, 1024, 128), idesc,
-                        (!(t.Flags & TILE_FIRST) || ks > 0) ? 1u : 0u);
-                }
-                MmaCommit(&sm.MmaDone);
+            for (int ks = 0; ks < 4; ++ks) {
+                MmaI8SS(sm.TmemBase, MakeSmemDesc(sA + ks * 32, 16, 1024, 128), MakeSmemDesc(sB + ks * 32, 16, 1024, 128), idesc,
+                    (!(t.Flags & TILE_FIRST) || ks > 0) ? 1u : 0u);
             }
-            if (!WaitBar(&sm.MmaDone, cursor.Used & 1)) {
-                sm.Failed = 1;
-                if (p.Status) {
-                    atomicOr(p.Status, kDevTimeoutMma);
-                }
+            MmaCommit(&sm.MmaDone);
+        }
+        if (!WaitBar(&sm.MmaDone, cursor.Used & 1)) {
+            sm.Failed = 1;
+            if (p.Status) {
+                atomicOr(p.Status, kDevTimeoutMma);
             }
-            ++cursor.Used;
-            if (cursor.Requested - cursor.Used < PS_RING / 2) {
-                RefillRing(p, sm, &cursor); // a phase with many tiles for one CTA: do not wait for its end
-            }
+        }
+        ++cursor.Used;
+        if (cursor.Requested - cursor.Used < PS_RING / 2) {
+            RefillRing(p, sm, &cursor); // a phase with many tiles for one CTA: do not wait for its end
         }
         if (!(t.Flags & TILE_LAST)) {
             continue;
