@@ -37,16 +37,16 @@ __device__ __forceinline__ float AddSquares(float sum2, float4 v)
     return __fadd_rn(sum2, __fmul_rn(v.w, v.w));
 }
 
-// Heads the attention of the step takes together.  A warp-wide 16-byte load covers 512 columns: some heads of one token, or, with
-// fewer heads, those of several tokens.  Taken: the size that needs the fewest loads for a token's row (12 heads of 64: three groups of
-// four heads, two tokens per load, instead of eight and four heads or twice six with idle lanes), the largest of those.
+// Heads the attention of the step takes together.  A warp-wide 16-byte load covers 512 columns: some heads of one stream of keys, or,
+// with fewer heads, those of several streams.  Taken: the size that needs the fewest loads for a token's row (12 heads of 64: three groups
+// of four heads, two streams per load, instead of eight and four heads or twice six with idle lanes), the largest of those.
 inline int AttGroupHeads(int heads, int headDim)
 {
     const int most = 512 / headDim;
     int best = 1;
     for (int g = 1; g <= most && g <= heads; ++g) {
         const int groups = (heads + g - 1) / g, bestGroups = (heads + best - 1) / best;
-        if (groups * (most / best) <= bestGroups * (most / g)) { // groups / tokens per load, cross-multiplied
+        if (groups * (most / best) <= bestGroups * (most / g)) { // groups / streams per load, cross-multiplied
             best = g;
         }
     }
