@@ -335,6 +335,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                 }
                 const long long t0 = clock64();
                 for (;;) {
+#pragma unroll 1
                     for (int i = 0; i < 64; ++i) {
                         __nanosleep(20);
                         if (*turn == index) {

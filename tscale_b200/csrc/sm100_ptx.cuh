@@ -80,6 +80,7 @@ __device__ __forceinline__ bool MbarTryWait(uint64_t *bar, uint32_t parity)
 // Every wait in this library is bounded so that a lost signal ends in an error code, not a hang.
 __device__ __forceinline__ bool MbarWaitBounded(uint64_t *bar, uint32_t parity, uint32_t maxSpins)
 {
+#pragma unroll 1
     for (uint32_t i = 0; i < maxSpins; ++i) {
         if (MbarTryWait(bar, parity)) {
             return true;
