@@ -105,6 +105,16 @@ def test_projection_tiles(dst, rows, length, dim, heads, d, with_rope):
     assert not bool(got[length:].view(want.dtype).float().any())
 
 
+@pytest.mark.parametrize("dst", ["i8", torch.bfloat16])
+@pytest.mark.parametrize("rows,dim,heads,d", [
+    (1, 64, 1, 64), (128, 192, 1, 128), (129, 64, 3, 64), (256, 320, 5, 64), (257, 2048, 3, 128), (20000, 192, 5, 128),
+])
+def test_projection_pairs(dst, rows, dim, heads, d):
+    """Tiles of 256 rows x 256 columns shared by two CTAs, 128 columns of x at a time: a second CTA without rows, half or all of
+    its columns' weights past the matrix, an inner size that ends in half a chunk, rings that wrap."""
+    test_projection_tiles(dst, rows, rows, dim, heads, d, True)
+
+
 @pytest.mark.parametrize("ctx,heads,d,window,slope", [
     ([9001], 5, 128, 100000, 0.0), ([4097, 3, 0, 2000], 2, 64, 3000, 0.25), ([1], 7, 64, 100000, 0.0),
 ])

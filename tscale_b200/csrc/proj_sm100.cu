@@ -8,34 +8,117 @@
 //   per head: discr = sqrt(sum y^2 / D) * vecScale;  z = y / discr;  rope (elements k and k + 32 of a 64-block);
 //             dst = quantise(z) (int8 or e4m3);  scale[head][t] = discr
 //
-// Persistent: one CTA per SM takes tiles of 128 rows of x times 256 output columns (4 heads of 64 or 2 of 128), tcgen05.mma kind::i8,
-// M = 128, N = 256, exact int32 accumulators in 256 tensor-memory columns, two such sets in turn.  One warp streams both operands
-// through a TMA ring of 64-column chunks that runs on across tiles, one issues the MMAs, and eight work on the epilogue of the tile
-// before: a row belongs to two threads, each with half of the tile's heads, so a head's sum of squares, the rotation partners and the
-// 64 output bytes of a block are all in one thread: no exchange between threads, sums in the scalar loop's order (bit-identical to
-// the stand-alone normalise + rope + quantise of the CPU code on the same projection).  A CTA's tiles are neighbours along the
+// Persistent, in pairs of CTAs (clusters of two, one CTA per SM): a pair takes tiles of 256 rows of x times 256 output columns (4 heads of
+// 64 or 2 of 128), tcgen05.mma cta_group::2, M = 256, N = 256: each CTA copies 128 rows of x and the weights of 128 columns, the first
+// one issues the products, which read the operands of both, and each has the accumulators of its own rows: 256 tensor-memory columns,
+// two such sets in turn.  One warp of each CTA streams its operands through a TMA ring of 128-column chunks that runs on across tiles
+// (both CTAs' copies count on the first one's barriers; a commit frees a stage in both), and eight warps work on the epilogue of
+// the tile before: a row belongs to two threads, each with half of the tile's heads, so a head's sum of squares, the rotation partners
+// and the 64 output bytes of a block are all in one thread: no exchange between threads, sums in the scalar loop's order (bit-identical
+// to the stand-alone normalise + rope + quantise of the CPU code on the same projection).  A pair's tiles are neighbours along the
 // columns, so its rows of x stay in L2 and its rows of the rope table in shared memory.
-// Bound by the operand stream out of L2 (24 KB per 256 clocks of MMA, more than the 64 bytes per clock an SM gets) and the epilogue's
-// issue slots.  Before, two CTAs per SM each ran load, multiply and epilogue in sequence with two chunks in flight: the tensor cores
-// waited for the latency of every chunk.  12345 rows x 2048 -> 16 heads of 128: 82 us (66 to 96 with the variant) before, 67 to 74 now,
-// where 67 us is the 24-KB stages through L2 at 9 TB/s; the four projections and the attention of a block 752 -> 606 us.
+// Bound by the operand stream out of L2: with a tile of 128 x 256 per CTA, 24 KB for every 64 columns, 12345 rows x 2048 -> 16 heads of 128
+// took 58 to 64 us; pairs copy two thirds of that: 43 to 51 us.  Chunks of 64 columns in pairs: 58 us, every stage pays its round trip
+// of commit, copy and barrier across the two SMs.
 #include "att_sm100_common.cuh"
 
 namespace tsa {
 
-constexpr int PROJ_MAX_STAGES = 9;
-constexpr int PROJ_M = 128, PROJ_N = 256, PROJ_KB = 64;
-constexpr int PROJ_STAGE_BYTES = (PROJ_M + PROJ_N) * PROJ_KB;
+constexpr int PROJ_MAX_STAGES = 8;
+// a pair's tile: PROJ_M rows and the weights of PROJ_N / 2 columns come from each CTA
+constexpr int PROJ_M = 128, PROJ_N = 256, PROJ_KB = 128;
+constexpr int PROJ_STAGE_BYTES = (PROJ_M + PROJ_N / 2) * PROJ_KB;
 constexpr int PROJ_LOAD_WARP = 0, PROJ_MMA_WARP = 1, PROJ_EPI_WARPS = 8;
 constexpr int PROJ_EPI_THREADS = PROJ_EPI_WARPS * 32, PROJ_THREADS = PROJ_EPI_THREADS + 64;
 constexpr int PROJ_SMEM_MAX = 227 * 1024;
 
 struct TProjMisc {
-    uint64_t Full[PROJ_MAX_STAGES], Empty[PROJ_MAX_STAGES]; // ring: copies landed / MMAs that read them retired
-    uint64_t AccFull[2], AccEmpty[2];                        // accumulator set complete / read out (one arrival per epilogue warp)
+    uint64_t Full[PROJ_MAX_STAGES], Empty[PROJ_MAX_STAGES]; // ring: in the first CTA: the copies of both landed / MMAs that read them retired (both CTAs)
+    uint64_t AccFull[2], AccEmpty[2];                       // accumulator set complete (both CTAs) / in the first CTA: read out, an arrival per epilogue warp of both
     uint32_t TmemBase;
     int Abort; // a bounded wait ran out somewhere in the CTA
 };
+
+// arrival, with release at cluster scope, on the barrier that lies in the first CTA of the pair where `bar` lies in this one
+__device__ __forceinline__ void ArriveInFirst(uint64_t *bar)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .b32 remote;\n\t"
+        "mapa.shared::cluster.u32 remote, %0, 0;\n\t"
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remote];\n\t"
+        "}" ::"r"(SmemAddr(bar))
+        : "memory");
+}
+// WaitBarA for a barrier the other CTA of the pair arrives on
+__device__ __forceinline__ bool WaitBarPair(uint64_t *bar, uint32_t parity, const int *abortFlag)
+{
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 32; ++i) {
+            uint32_t ok;
+            asm volatile(
+                "{\n\t"
+                ".reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.b32 %0, 1, 0, p;\n\t"
+                "}"
+                : "=r"(ok)
+                : "r"(SmemAddr(bar)), "r"(parity)
+                : "memory");
+            if (ok) {
+                return true;
+            }
+        }
+        if (*(const volatile int *)abortFlag || clock64() - t0 > WAIT_CYCLES) {
+            return false;
+        }
+    }
+}
+// 2-D tile load into this CTA's shared memory, counted on the barrier that lies in the first CTA of the pair where `bar` lies in this one
+__device__ __forceinline__ void TmaLoadPair(void *smemDst, const void *tensorMap, int x, int y, uint64_t *bar)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .b32 first;\n\t"
+        "mapa.shared::cluster.u32 first, %4, 0;\n\t"
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [first];\n\t"
+        "}" ::"r"(SmemAddr(smemDst)), "l"(tensorMap), "r"(x), "r"(y), "r"(SmemAddr(bar))
+        : "memory");
+}
+__device__ __forceinline__ void PairSync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// D (M = 256: each CTA's 128 rows in its own tensor memory) (+)= A B^T, A's rows and B's rows split between the two CTAs' shared memory
+template <bool E4M3>
+__device__ __forceinline__ void MmaPairSS(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate)
+{
+    if (E4M3) {
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
+            "}" ::"r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    } else {
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t"
+            "}" ::"r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    }
+}
+// arrive on the barrier of both CTAs when all MMAs issued so far by this thread have completed
+__device__ __forceinline__ void MmaCommitPair(uint64_t *bar)
+{
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(SmemAddr(bar)), "h"((uint16_t)3)
+                 : "memory");
+}
 
 __device__ __forceinline__ uint32_t PackBf16(float lo, float hi)
 {
@@ -57,11 +140,11 @@ struct TProjArgs {
 // cores (kind::f8f6f4); otherwise int8 x int8 with exact int32 accumulators (kind::i8).
 // DST: TSA_I8, TSA_E4M3 (quantised) or TSA_F16 / TSA_BF16 (the normalised, rotated values themselves: the reference's K16).
 template <int D, int DST, bool X_E4M3>
-__global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, TProjArgs a,
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, TProjArgs a,
     int *status)
 {
     // s32 accumulators, s8 x s8 -- or f32 accumulators, e4m3 x e4m3; both operands K-major
-    constexpr uint32_t IDESC = X_E4M3 ? MakeInstrDesc(1, 0, 0, 0, 0, PROJ_M, PROJ_N) : MakeInstrDesc(2, 1, 1, 0, 0, PROJ_M, PROJ_N);
+    constexpr uint32_t IDESC = X_E4M3 ? MakeInstrDesc(1, 0, 0, 0, 0, 2 * PROJ_M, PROJ_N) : MakeInstrDesc(2, 1, 1, 0, 0, 2 * PROJ_M, PROJ_N);
     auto accValue = [](uint32_t bits) { return X_E4M3 ? __uint_as_float(bits) : (float)(int32_t)bits; };
     constexpr int HPC = PROJ_N / D;                                          // heads per tile
     extern __shared__ uint8_t projSmemRaw[];
@@ -69,6 +152,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
     TProjMisc &misc = *reinterpret_cast<TProjMisc *>(smem + a.Stages * PROJ_STAGE_BYTES);
     float *ropeTile = reinterpret_cast<float *>(smem + a.Stages * PROJ_STAGE_BYTES + 1024);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = blockIdx.x & 1; // in the pair
     if (tid == 0) {
         for (int s = 0; s < a.Stages; ++s) {
             MbarInit(&misc.Full[s], 1);
@@ -76,17 +160,18 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
         }
         for (int b = 0; b < 2; ++b) {
             MbarInit(&misc.AccFull[b], 1);
-            MbarInit(&misc.AccEmpty[b], PROJ_EPI_WARPS);
+            MbarInit(&misc.AccEmpty[b], 2 * PROJ_EPI_WARPS);
         }
         misc.Abort = 0;
         FenceBarrierInit();
     }
     if (warp == PROJ_MMA_WARP) {
-        TmemAlloc(&misc.TmemBase, 2 * PROJ_N);
-        TmemRelinquish();
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(&misc.TmemBase)), "r"(2 * PROJ_N) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     TcFenceBefore();
     __syncthreads();
+    PairSync(); // the other CTA's barriers and tensor memory are set up too
     TcFenceAfter();
     const uint32_t tmem = misc.TmemBase;
     PdlTrigger(); // behind the allocation: a CTA of the next kernel may hold tensor memory of this SM from here on
@@ -98,7 +183,9 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
             atomicOr(status, code);
         }
     };
-    const int itemBegin = (int)((long long)a.Items * blockIdx.x / gridDim.x), itemEnd = (int)((long long)a.Items * (blockIdx.x + 1) / gridDim.x);
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int itemBegin = (int)((long long)a.Items * pair / pairs), itemEnd = (int)((long long)a.Items * (pair + 1) / pairs);
+    auto rowOf = [&](int item) { return (item / a.ColTiles * 2 + rank) * PROJ_M; };
     if (warp == PROJ_LOAD_WARP) {
         if (lane == 0) {
             PrefetchTensorMap(&tmX);
@@ -106,7 +193,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
             int s = 0, phase = 0, requested = 0; // ring slot, its parity, chunks requested
             bool failed = false;
             for (int item = itemBegin; item < itemEnd && !failed; ++item) {
-                const int rowBase = item / a.ColTiles * PROJ_M, colBase = item % a.ColTiles * PROJ_N;
+                const int rowBase = rowOf(item), colBase = item % a.ColTiles * PROJ_N + rank * (PROJ_N / 2);
                 for (int c = 0; c < a.Chunks; ++c) {
                     if (requested >= a.Stages && !WaitBarA(&misc.Empty[s], phase ^ 1, abortFlag)) {
                         failed = true;
@@ -114,9 +201,11 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
                         break;
                     }
                     uint8_t *sA = smem + s * PROJ_STAGE_BYTES;
-                    MbarExpectTx(&misc.Full[s], PROJ_STAGE_BYTES);
-                    TmaLoad2D(sA, &tmX, c * PROJ_KB, rowBase, &misc.Full[s]);
-                    TmaLoad2D(sA + PROJ_M * PROJ_KB, &tmW, c * PROJ_KB, colBase, &misc.Full[s]);
+                    if (rank == 0) {
+                        MbarExpectTx(&misc.Full[s], 2 * PROJ_STAGE_BYTES);
+                    }
+                    TmaLoadPair(sA, &tmX, c * PROJ_KB, rowBase, &misc.Full[s]);
+                    TmaLoadPair(sA + PROJ_M * PROJ_KB, &tmW, c * PROJ_KB, colBase, &misc.Full[s]);
                     ++requested;
                     if (++s == a.Stages) {
                         s = 0;
@@ -124,8 +213,9 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
                     }
                 }
             }
-            if (failed || *(volatile int *)&misc.Abort) {
-                // copies that were requested but never consumed must not land after the CTA is gone: wait (bounded) for them
+            if (rank == 0 && (failed || *(volatile int *)&misc.Abort)) {
+                // copies that were requested but never consumed must not land after the CTA is gone: wait (bounded) for both CTAs' (the
+                // second one leaves behind the first)
                 for (int k = max(0, requested - a.Stages); k < requested; ++k) {
                     WaitBar(&misc.Full[k % a.Stages], (k / a.Stages) & 1);
                 }
@@ -133,11 +223,12 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
         }
         __syncwarp();
     } else if (warp == PROJ_MMA_WARP) {
+        if (rank == 0) {
         // the whole warp runs the loop and the waits, one elected lane issues (descriptors stay in uniform registers that way)
         int s = 0, phase = 0, n = 0;
         bool failed = false;
         auto wait = [&](uint64_t *bar, uint32_t parity, int code) {
-            if (!__all_sync(0xffffffffu, WaitBarA(bar, parity, abortFlag))) {
+            if (!__all_sync(0xffffffffu, WaitBarPair(bar, parity, abortFlag))) {
                 failed = true;
                 if (lane == 0) {
                     fail(code);
@@ -161,15 +252,11 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
                     for (int ks = 0; ks < PROJ_KB / 32; ++ks) {
                         const uint64_t aDesc = MakeSmemDesc(sA + ks * 32, 16, 8 * PROJ_KB, PROJ_KB);
                         const uint64_t bDesc = MakeSmemDesc(sB + ks * 32, 16, 8 * PROJ_KB, PROJ_KB);
-                        if (X_E4M3) {
-                            MmaF8SS(acc, aDesc, bDesc, IDESC, (c > 0 || ks > 0) ? 1u : 0u);
-                        } else {
-                            MmaI8SS(acc, aDesc, bDesc, IDESC, (c > 0 || ks > 0) ? 1u : 0u);
-                        }
+                        MmaPairSS<X_E4M3>(acc, aDesc, bDesc, IDESC, (c > 0 || ks > 0) ? 1u : 0u);
                     }
-                    MmaCommit(&misc.Empty[s]);
+                    MmaCommitPair(&misc.Empty[s]);
                     if (c == a.Chunks - 1) {
-                        MmaCommit(&misc.AccFull[n & 1]);
+                        MmaCommitPair(&misc.AccFull[n & 1]);
                     }
                 }
                 __syncwarp();
@@ -178,6 +265,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
                     phase ^= 1;
                 }
             }
+        }
         }
         __syncwarp();
     } else {
@@ -198,7 +286,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
         int ropeRow = -1, n = 0; // first row of the rope table's rows in shared memory
         bool failed = false;
         for (int item = itemBegin; item < itemEnd; ++item, ++n) {
-            const int rowBase = item / a.ColTiles * PROJ_M, headBase = item % a.ColTiles * HPC;
+            const int rowBase = rowOf(item), headBase = item % a.ColTiles * HPC;
             if (!WaitBarA(&misc.AccFull[n & 1], (n >> 1) & 1, abortFlag)) {
                 failed = true;
                 fail(kDevTimeoutMma);
@@ -325,14 +413,15 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
             TcFenceBefore();
             __syncwarp();
             if (lane == 0) {
-                MbarArrive(&misc.AccEmpty[n & 1]);
+                ArriveInFirst(&misc.AccEmpty[n & 1]);
             }
         }
     }
     TcFenceBefore();
     __syncthreads();
+    PairSync(); // neither CTA leaves while the other's MMAs may still read its operands or arrive on its barriers
     if (warp == PROJ_MMA_WARP) {
-        TmemDealloc(tmem, 2 * PROJ_N);
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * PROJ_N) : "memory");
     }
 }
 
@@ -349,8 +438,8 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     TSA_REQUIRE(x.data && w.data && dst.data, "tsa_matmul_norm_rope_quant: null x / w / dst");
     TSA_REQUIRE(headCount > 0 && (headDim == 64 || headDim == 128), "tsa_matmul_norm_rope_quant: head size %d must be 64 or 128", headDim);
     const int dim = x.xsize, outCols = headCount * headDim;
-    TSA_REQUIRE(dim > 0 && dim % PROJ_KB == 0 && w.xsize == dim, "tsa_matmul_norm_rope_quant: inner size %d (x) / %d (w) must be equal multiples of %d", dim,
-        w.xsize, PROJ_KB);
+    TSA_REQUIRE(dim > 0 && dim % 64 == 0 && w.xsize == dim, "tsa_matmul_norm_rope_quant: inner size %d (x) / %d (w) must be equal multiples of 64", dim,
+        w.xsize);
     TSA_REQUIRE(w.ysize >= outCols && dst.xsize >= outCols, "tsa_matmul_norm_rope_quant: w has %d rows, dst %d columns, H*D = %d", w.ysize, dst.xsize, outCols);
     TSA_REQUIRE(len >= 0 && len <= x.ysize && len <= dst.ysize, "tsa_matmul_norm_rope_quant: len %d exceeds buffers (%d, %d rows)", len, x.ysize, dst.ysize);
     TSA_REQUIRE((uintptr_t)x.data % 16 == 0 && x.stride_bytes % 16 == 0 && (uintptr_t)w.data % 16 == 0 && w.stride_bytes % 16 == 0 &&
@@ -373,7 +462,7 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     if (rc == TSA_OK) {
         tsa_ptr2d wv = w;
         wv.ysize = outCols;
-        rc = MakeTileMapEx(&mw, wv, 1, PROJ_KB, PROJ_N, "w");
+        rc = MakeTileMapEx(&mw, wv, 1, PROJ_KB, PROJ_N / 2, "w");
     }
     if (rc != TSA_OK) {
         return rc;
@@ -388,9 +477,9 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     a.Len = len;
     a.Rows = dst.ysize;
     a.HeadCount = headCount;
-    a.Chunks = dim / PROJ_KB;
+    a.Chunks = (dim + PROJ_KB - 1) / PROJ_KB; // columns past the end read as zeros
     a.ColTiles = (outCols + PROJ_N - 1) / PROJ_N;
-    a.Items = (dst.ysize + PROJ_M - 1) / PROJ_M * a.ColTiles;
+    a.Items = (dst.ysize + 2 * PROJ_M - 1) / (2 * PROJ_M) * a.ColTiles;
     // as many ring stages as fit beside the rope rows
     const int ropeBytes = rope.data ? PROJ_M * (headDim + 1) * (int)sizeof(float) : 0;
     a.Stages = (PROJ_SMEM_MAX - 2048 - ropeBytes) / PROJ_STAGE_BYTES;
@@ -422,5 +511,5 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
         return rc;
     }
     void *args[] = {&mx, &mw, &a, &statusWord};
-    return CheckCuda(LaunchPdl(kern, dim3(a.Items < sms ? a.Items : sms), dim3(PROJ_THREADS), smemBytes, (cudaStream_t)stream, args), "tsa_matmul_norm_rope_quant launch");
+    return CheckCuda(LaunchPdl(kern, dim3(2 * (a.Items < sms / 2 ? a.Items : sms / 2)), dim3(PROJ_THREADS), smemBytes, (cudaStream_t)stream, args), "tsa_matmul_norm_rope_quant launch");
 }
