@@ -179,45 +179,40 @@ __device__ __forceinline__ void TmemStore8(uint32_t taddr, const uint32_t *r)
 }
 
 // Slow path of the softmax: the row's reference moves up by d whole units, so what has been accumulated shrinks by
-// alpha = 2^-d: the O accumulator (D columns) and this tile's e4m3 weights that are already in tensor memory.  The
-// weights of the 32-key block b sit in columns [32b, 32b + 8) and their residuals in [32b + 8, 32b + 16);
-// quads [firstQuad, firstQuad + nQuads) are the 4-column (16-key) groups written and not yet handed to the MMA.  All lanes of the warp execute the
-// tensor-memory accesses; a lane whose row needs no change passes alpha = 1.  Kept out of line and in small pieces:
-// it is rare, and inlined it costs the common path registers.
+// alpha = 2^-d: the O accumulator (D columns) and this tile's e4m3 weights that are in tensor memory and not yet handed to the MMA:
+// none, or those of one 32-key block (storedBlock >= 0), weights in columns [32b, 32b + 8), residuals in [32b + 8, 32b + 16).  All lanes
+// of the warp execute the tensor-memory accesses; a lane whose row needs no change passes alpha = 1.  Kept out of line: inlined it
+// costs the common path registers.  32 columns at a time: with 8 the round trips to tensor memory took four times as long, and rows
+// whose scores spread (queries and keys of unit variance) come here in most of their first tiles.
 template <int D>
-__device__ __noinline__ void ShrinkAccumulated(uint32_t tLane, float alpha, int hasO, int firstQuad, int nQuads, int withResidual)
+__device__ __noinline__ void ShrinkAccumulated(uint32_t tLane, float alpha, int hasO, int storedBlock)
 {
     TmemWaitSt(); // the weights stored so far have landed
     if (hasO) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < D; c0 += 8) {
-            uint32_t o[8];
-            TmemLd8(tLane + TMEM_O_COL + c0, o);
-            TmemWaitLd();
+        for (int c0 = 0; c0 < D; c0 += 32) {
+            uint32_t o[32];
+            TmemLoad32(tLane + TMEM_O_COL + c0, o);
+            TmemWait32(o);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < 32; ++c) {
                 o[c] = __float_as_uint(__uint_as_float(o[c]) * alpha);
             }
-            TmemStN<8>(tLane + TMEM_O_COL + c0, o);
+            TmemSt32(tLane + TMEM_O_COL + c0, o);
         }
     }
-    const __half2 ah = __float2half2_rn(alpha);
-    const uint32_t ah2 = *reinterpret_cast<const uint32_t *>(&ah);
-#pragma unroll 1
-    for (int q = firstQuad; q < firstQuad + nQuads; ++q) {
-#pragma unroll 1
-        for (int part = 0; part < (withResidual ? 2 : 1); ++part) {
-            const uint32_t col = 32 * (q >> 1) + 4 * (q & 1) + 8 * part;
-#pragma unroll 1
-            for (int k = 0; k < 4; k += 2) {
-                uint32_t w0, w1;
-                TmemLd2(tLane + col + k, w0, w1);
-                TmemWaitLd();
-                w0 = ScaleE4M3x4(w0, ah2);
-                w1 = ScaleE4M3x4(w1, ah2);
-                TmemSt2(tLane + col + k, w0, w1);
-            }
+    if (storedBlock >= 0) {
+        const __half2 ah = __float2half2_rn(alpha);
+        const uint32_t ah2 = *reinterpret_cast<const uint32_t *>(&ah);
+        uint32_t w[16];
+        TmemLd16(tLane + 32 * storedBlock, w);
+        TmemWaitLd();
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            w[c] = ScaleE4M3x4(w[c], ah2);
         }
+        TmemStore8(tLane + 32 * storedBlock, w);
+        TmemStore8(tLane + 32 * storedBlock + 8, w + 8);
     }
     TmemWaitSt();
 }
@@ -940,7 +935,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
 
                 // the reference moves up by d whole units: everything accumulated so far shrinks by 2^-d, and the W logits in s
                 // drop by d.  storedQuads: 16-key groups of this tile whose weights are in tensor memory.
-                auto raise = [&](float mxc, int storedQuads, uint32_t *s, auto widthTag, int withResidual) {
+                auto raise = [&](float mxc, int storedQuads, uint32_t *s, auto widthTag) {
                     constexpr int W = decltype(widthTag)::value;
                     const float d = (mxc > headroom) ? floorf(mxc - 7.0f) : 0.0f;
                     const float alpha = exp2f(-d);
@@ -960,7 +955,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                         }
                         TcFenceAfter();
                     }
-                    ShrinkAccumulated<D>(tLane, alpha, oLive ? 1 : 0, firstQuad, storedQuads - firstQuad, withResidual);
+                    ShrinkAccumulated<D>(tLane, alpha, oLive ? 1 : 0, storedQuads > firstQuad ? firstQuad >> 1 : -1);
                     lacc2.x *= alpha;
                     lacc2.y *= alpha;
                     m += d;
@@ -1009,7 +1004,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                     TmemWait32(s + 32);
                     mx = scaleGroup(s + 32, h * 64 + 32, mx, TW32());
                     if (__any_sync(0xffffffffu, mx > headroom)) {
-                        raise(mx, h * 4, s, TW64(), 0);
+                        raise(mx, h * 4, s, TW64());
                     }
 #pragma unroll
                     for (int c = 0; c < 64; c += 4) {
@@ -1049,7 +1044,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                                 s[c + 1] = __float_as_uint(tt.y);
                             }
                             if (__any_sync(0xffffffffu, mx > headroom)) {
-                                raise(mx, blk * 2, s, TW32(), 1);
+                                raise(mx, blk * 2, s, TW32());
                             }
 #pragma unroll
                             for (int c = 0; c < 32; c += 4) {
