@@ -98,6 +98,7 @@ struct TBwdMisc {
     uint64_t BarEmpty[8];     // MMA warp -> loader: the half stage's output products have retired
     uint64_t BarS[2];         // control -> half h: S and dP columns of the half ready
     uint64_t BarP[2];         // half h -> control: A1 / A2 of the half written (8 warp arrivals)
+    uint64_t ColFull[2];      // first four arithmetic warps -> all of them: the column factors of a tile are staged
     uint64_t BarOut;          // MMA warps -> arithmetic: every output product of the item has retired
     uint32_t TmemBase;
 };
@@ -161,6 +162,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
             MbarInit(&misc.BarS[h], 1);
             MbarInit(&misc.BarP[h], BWD_ARITH_THREADS / 32);
         }
+        MbarInit(&misc.ColFull[0], TILE_ROWS / 32);
+        MbarInit(&misc.ColFull[1], TILE_ROWS / 32);
         MbarInit(&misc.BarOut, 2);
         misc.Abort = 0;
         misc.Turn = 0;
@@ -540,13 +543,19 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                     misc.ColA[buf][tid] = pfA;
                     misc.ColT[buf][tid] = MODE_DKV ? -pfT - p.Slope * (float)tid : p.Slope * (float)tid;
                     misc.ColB[buf][tid] = MODE_DKV ? -pfB * dsMult : pfB * dsMult;
+                    __syncwarp();
+                    if (lane == 0) {
+                        MbarArrive(&misc.ColFull[buf]);
+                    }
                 }
                 const int c0 = cur.J0;
                 const int ls = spanS - c0, lf = min(spanF, p.Rows - 1) - c0; // span in tile-local columns
                 const bool rowFull = ls <= 0 && lf >= TILE_ROWS - 1;
                 const bool warpMasked = !__all_sync(0xffffffffu, rowFull);
-                // publishes the staged columns; a failed wait is carried here so the arithmetic threads leave together
-                if (BarRedOr(BAR_ARITH, BWD_ARITH_THREADS, failed || (*(volatile int *)&misc.Abort != 0))) {
+                // The staged columns, double buffered: a warp that stages tile t + 2 has seen the scores of tile t + 1's second half, and
+                // those were asked for when all 16 warps had handed over tile t.  (A barrier of the 512 threads per tile kept the warps in
+                // step.)  A thread whose wait fails goes to the threads' next common barrier, where they leave together.
+                if (!__all_sync(0xffffffffu, !failed && WaitBarA<true>(&misc.ColFull[buf], (it >> 1) & 1, abortFlag))) {
                     failed = true;
                     break;
                 }
