@@ -1138,13 +1138,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                         loadKeys(0, kcur);
                     }
                 }
-                if (tilesInItem > 0) {
-                    if (!wait(&misc.BarOFull, oCount & 1, kDevTimeoutMma)) {
-                        break;
-                    }
-                    ++oCount;
-                    TcFenceAfter();
-                }
+                // all that does not need O comes in front of the wait for the last output products
                 const float lTot = (lacc2.x + lacc2.y) * (1.0f / 128.0f) + exp2f(-m);
                 const float outMult = (HAS_VSCALE ? invK : p.VVecScale) * (1.0f / 128.0f) / lTot;
                 if (rowOk && p.Lse.Valid()) {
@@ -1172,6 +1166,13 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                         put(p.OutCopy[0].Row(row) + rowOff);
                     }
                 };
+                if (tilesInItem > 0) {
+                    if (!wait(&misc.BarOFull, oCount & 1, kDevTimeoutMma)) {
+                        break;
+                    }
+                    ++oCount;
+                    TcFenceAfter();
+                }
 #pragma unroll 1
                 for (int c0 = 0; c0 < D; c0 += 32) {
                     uint32_t o[32];
