@@ -18,11 +18,11 @@
 // phases and layers, in flight in a ring of shared memory (cp.async), so that their DRAM latency is never on the path.
 //
 // Measured, twelve layers, dim 768, 12 heads x 64, vocabulary 50304, a whole token with the final layer and softmax, launches / graph:
-//     1 sequence, 500 tokens of context       744 / 568 -> 334 / 328 us, of which 312 are there with windows of 64 tokens in all
-//                                             layers: sixty phases at some 5 us, the barrier, the sums through L2 and the norm, in a
-//                                             chain; the bytes take 20 us
-//     64 sequences, 1024 to 8192 tokens       968 / 801 -> 735 / 727 us (three of four layers see 64 tokens): 473 us with the short
-//                                             windows in all layers, and 85 us for every wide layer, whose keys and values then
+//     1 sequence, 500 tokens of context       744 / 568 -> 325 us, of which 303 are there with windows of 64 tokens in all layers: sixty
+//                                             phases at some 5 us, the barrier, the sums through L2 and the norm, in a chain; the
+//                                             bytes take 20 us
+//     64 sequences, 1024 to 8192 tokens       968 / 801 -> 714 / 714 us (three of four layers see 64 tokens): 462 us with the short
+//                                             windows in all layers, and 84 us for every wide layer, whose keys and values then
 //                                             stream at 5.8 TB/s
 // Head counts whose chunks need a whole group of four warps leave a quarter of the groups a second unit: with 16 heads x 64 such a
 // batch takes 975 / 968 us, where separate launches, 16 warps per SM in the attention, took 1085 / 897.
@@ -42,6 +42,7 @@ constexpr int PS_TILE = 128 * 128;             // bytes of a weight tile: 128 ro
 constexpr int PS_B_BYTES = INF_MAX_SEQ * 128;  // the chunk's vectors, one row of 128 int8 per sequence
 constexpr int PS_F_PITCH = 132;                // floats per row of the fp32 chunk: 16-byte rows that fall into different banks
 constexpr int PS_MERGE_PITCH = 19;
+constexpr int PS_STAGE_AHEAD = 3;              // quads of columns whose loads a thread has in flight (6: spills, +4 %)
 constexpr int PS_LAYERS = 32;                  // layers per launch
 constexpr int PS_CHUNKS_PER_SM = 4;            // the keys of a layer are cut into no more chunks than this times the SMs
 constexpr int PS_MIN_CHUNK = 16;               // keys
@@ -116,6 +117,12 @@ struct TWeightTile {
 };
 constexpr int PS_TABLE = 512; // tiles per CTA and layer kept in shared memory (1.2 GB of weights in one layer); beyond it they are computed
 
+// what the critical path reads of a layer
+struct TLayerNow {
+    float QvMult, CombScale, PrevContractScale, Slope;
+    int Window;
+};
+
 struct TStepSmem {
     uint8_t Ring[PS_RING][PS_TILE];
     uint8_t B[PS_B_BYTES];
@@ -129,6 +136,7 @@ struct TStepSmem {
     TWeightTile Table[PS_TABLE];
     int PhaseBegin[5];            // first tile of each phase, and their number
     TAttPlan Plan[2];             // of the last two windows: the layers of a model alternate between two or so
+    TLayerNow Now;                // of the present layer: a first read of a kernel parameter waits for the constant cache
     int PlanOf;                   // which of them is the present layer's
     tsa_kv_seq Seqs[INF_MAX_SEQ]; // the present layer's caches
     uint64_t MmaDone;
@@ -311,13 +319,15 @@ __device__ __forceinline__ void StageState(const TStepParams &p, TStepSmem &sm, 
         __syncthreads();
         return;
     }
-    // two quads of columns per thread and step, their loads before the first use (all of a thread's quads at once took the registers
+    // a few quads of columns per thread and step, their loads before the first use (all of a thread's quads at once took the registers
     // the attention loop needs)
-    for (int base = threadIdx.x; base < p.NSeq * 32; base += 2 * PS_THREADS) {
-        float4 v[2];
-        int4 add[2];
+    constexpr int AHEAD = PS_STAGE_AHEAD;
+#pragma unroll 1
+    for (int base = threadIdx.x; base < p.NSeq * 32; base += AHEAD * PS_THREADS) {
+        float4 v[AHEAD];
+        int4 add[AHEAD];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < AHEAD; ++k) {
             const int i = base + k * PS_THREADS, s = i >> 5, col = chunk * 128 + (i & 31) * 4;
             if (i < p.NSeq * 32) {
                 v[k] = __ldcg(reinterpret_cast<const float4 *>(state + (size_t)s * p.Dim + col));
@@ -327,7 +337,7 @@ __device__ __forceinline__ void StageState(const TStepParams &p, TStepSmem &sm, 
             }
         }
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < AHEAD; ++k) {
             const int i = base + k * PS_THREADS, s = i >> 5, x = (i & 31) * 4;
             if (i < p.NSeq * 32) {
                 if (source == SRC_SUM) { // AddScaled, cpu_infer.cpp:296-303
@@ -346,25 +356,23 @@ __device__ __forceinline__ void StageState(const TStepParams &p, TStepSmem &sm, 
     __syncthreads();
 }
 
-// int8 codes of the staged columns [x0, x0 + 16 pieces * 16) under sm.Mult, into the operand tile
-__device__ __forceinline__ void QuantiseStaged(const TStepParams &p, TStepSmem &sm, int piece0, int pieces, bool relu)
+// int8 codes of the staged columns [4 quad0, 4 (quad0 + quads)) under sm.Mult, into the operand tile; four columns per thread and step
+// (sixteen left all but eight threads without work for one sequence and were four times the code)
+__device__ __forceinline__ void QuantiseStaged(const TStepParams &p, TStepSmem &sm, int quad0, int quads, bool relu)
 {
-    for (int i = threadIdx.x; i < p.NSeq * pieces; i += PS_THREADS) {
-        const int s = i / pieces, c16 = piece0 + i - s * pieces;
+#pragma unroll 2
+    for (int i = threadIdx.x; i < p.NSeq * quads; i += PS_THREADS) {
+        const int s = i / quads, x = (quad0 + i - s * quads) * 4;
         const float mult = sm.Mult[s];
-        uint32_t w[4];
+        const float4 v = *reinterpret_cast<const float4 *>(&sm.F[s][x]);
+        int q[4] = {ToInt8Clamp127(__fmul_rn(v.x, mult)), ToInt8Clamp127(__fmul_rn(v.y, mult)), ToInt8Clamp127(__fmul_rn(v.z, mult)),
+            ToInt8Clamp127(__fmul_rn(v.w, mult))};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float4 v = *reinterpret_cast<const float4 *>(&sm.F[s][c16 * 16 + k * 4]);
-            int q[4] = {ToInt8Clamp127(__fmul_rn(v.x, mult)), ToInt8Clamp127(__fmul_rn(v.y, mult)), ToInt8Clamp127(__fmul_rn(v.z, mult)),
-                ToInt8Clamp127(__fmul_rn(v.w, mult))};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                q[j] = relu ? max(q[j], 0) : q[j];
-            }
-            w[k] = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
+        for (int j = 0; j < 4; ++j) {
+            q[j] = relu ? max(q[j], 0) : q[j];
         }
-        StoreCodes(sm.B, s, c16, make_int4((int)w[0], (int)w[1], (int)w[2], (int)w[3]));
+        const uint32_t w = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
+        *reinterpret_cast<uint32_t *>(sm.B + s * 128 + (((x >> 4) ^ (s & 7)) << 4) + (x & 15)) = w;
     }
 }
 
@@ -383,7 +391,7 @@ __device__ __forceinline__ void NormaliseStaged(const TStepParams &p, TStepSmem 
         sm.Mult[s] = mult;
     }
     __syncthreads();
-    QuantiseStaged(p, sm, 0, 8, false);
+    QuantiseStaged(p, sm, 0, 32, false);
 }
 
 // The contract product's input: relu of the expand sums normalised per head (groups of ReluDim / Heads columns).  A group that lies
@@ -447,7 +455,7 @@ __device__ __forceinline__ void NormaliseRelu(const TStepParams &p, TStepSmem &s
         }
         __syncthreads();
         const int lo = max(g0, c0) - c0, hi = min(g1, c0 + 128) - c0;
-        QuantiseStaged(p, sm, lo / 16, (hi - lo) / 16, true);
+        QuantiseStaged(p, sm, lo / 4, (hi - lo) / 4, true);
         if (g1 < c0 + 128) {
             __syncthreads(); // the next group overwrites sm.Mult
         }
@@ -457,7 +465,6 @@ __device__ __forceinline__ void NormaliseRelu(const TStepParams &p, TStepSmem &s
 // All of this CTA's items of one matrix product.
 __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm, int l, int phase, TTileCursor &cursor)
 {
-    const TStepLayer &layer = p.Layers[l];
     const int tid = threadIdx.x, warp = tid >> 5;
     const int hs = p.Heads * p.HeadSize;
     const int nCols = (p.NSeq + 15) & ~15; // accumulator columns
@@ -471,9 +478,10 @@ __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm
             const bool proj = phase == PH_PROJ;
             const int source = proj && l == 0 ? p.FirstSource : SRC_SUM;
             StageState(p, sm, chunk, source, proj == (source == SRC_SUM) ? p.StateB : p.StateA, proj ? p.Contract : p.Comb,
-                proj ? (l > 0 ? p.Layers[l - 1].ContractScale : 0.0f) : layer.CombScale, tile != 0 || source == SRC_STATE ? nullptr : proj ? p.StateA : p.StateB);
+                proj ? sm.Now.PrevContractScale : sm.Now.CombScale, tile != 0 || source == SRC_STATE ? nullptr : proj ? p.StateA : p.StateB);
             NormaliseStaged(p, sm);
         } else if (phase == PH_COMB) {
+#pragma unroll 2
             for (int i = tid; i < p.NSeq * 8; i += PS_THREADS) {
                 StoreCodes(sm.B, i >> 3, i & 7, __ldcg(reinterpret_cast<const int4 *>(p.Kv8 + (size_t)(i >> 3) * 4 * hs + chunk * 128 + (i & 7) * 16)));
             }
@@ -514,7 +522,8 @@ __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm
             continue;
         }
         TcFenceAfter();
-        // 128 rows x 16 sequences per warp: the item's sums join the others' in L2
+        // 128 rows x 16 sequences per warp: the item's sums join the others' in L2.  Written as sixteen predicated additions they were
+        // a kilobyte of instructions that every phase fetched anew, for one sequence too (1 K of the 7 K clocks of a phase)
         int *out = phase == PH_PROJ ? p.Proj + t.Matrix * hs : phase == PH_COMB ? p.Comb : phase == PH_EXPAND ? p.Expand : p.Contract;
         const int rows = phase == PH_PROJ ? hs : phase == PH_EXPAND ? p.ReluDim : p.Dim, pitch = phase == PH_PROJ ? 4 * hs : rows;
         const int quad = warp & 3, row = t.Tile * 128 + quad * 32 + (tid & 31);
@@ -523,10 +532,18 @@ __device__ __forceinline__ void ProductPhase(const TStepParams &p, TStepSmem &sm
             TmemLd16(sm.TmemBase + ((uint32_t)(quad * 32) << 16) + s0, acc);
             TmemWaitLd();
             if (row < rows) {
+                int *dst = out + (size_t)s0 * pitch + row;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    if (s0 + j < p.NSeq) {
-                        atomicAdd(out + (size_t)(s0 + j) * pitch + row, (int)acc[j]);
+                for (int j = 0; j < 16; j += 4) {
+                    if (s0 + j >= p.NSeq) { // the rest has no sequences: nor its instructions to be fetched
+                        break;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (s0 + j + k < p.NSeq) {
+                            atomicAdd(dst, (int)acc[j + k]);
+                        }
+                        dst += pitch;
                     }
                 }
             }
@@ -682,7 +699,7 @@ __device__ __forceinline__ void StoreKvProduct(int8_t *kv, int headSize, int z, 
 // One matrix (m: qk, qv, k, v) of a head group of one sequence, by one warp: rope on qk and qv (ReferenceApplyRope,
 // code/gpt/att/rope.cpp:28-46), NormalizeState per head, codes into shared memory (qk, k: at `codes`) or the sequence's cache (qv, v).
 template <int D>
-__device__ __noinline__ void ProjectHeads(const TStepParams &p, const TStepLayer &layer, TAttGroupSmem &g, const tsa_kv_seq &sq, int m, int seq, int codes,
+__device__ __noinline__ void ProjectHeads(const TStepParams &p, float qvMult, TAttGroupSmem &g, const tsa_kv_seq &sq, int m, int seq, int codes,
     int head0, int heads, int pos)
 {
     const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 3, hs = p.Heads * D;
@@ -734,7 +751,7 @@ __device__ __noinline__ void ProjectHeads(const TStepParams &p, const TStepLayer
         NormScales(sum2, D, &discr, &mult);
         g.Mult[warp][lane] = mult;
         if (m == 1) {
-            ((float *)sq.kScale)[(size_t)pos * p.Heads + head0 + lane] = __fmul_rn(discr, layer.QvMult);
+            ((float *)sq.kScale)[(size_t)pos * p.Heads + head0 + lane] = __fmul_rn(discr, qvMult);
         } else if (m == 3) {
             ((float *)sq.vScale)[(size_t)pos * p.Heads + head0 + lane] = INF_VEC_SCALE;
         }
@@ -831,11 +848,10 @@ __device__ __forceinline__ void AttendRange(const int4 qv, float logitMult, floa
 }
 
 template <int D>
-__device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
+__device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm)
 {
     constexpr int LPH = D / 16;  // lanes per head
     constexpr int PITCH = D + 4; // of a partial: columns, maximum, sum
-    const TStepLayer &layer = p.Layers[l];
     const TAttPlan &plan = sm.Plan[sm.PlanOf];
     const int tid = threadIdx.x, lane = tid & 31, group = tid >> 7, w = (tid >> 5) & 3;
     const int hs = p.Heads * D;
@@ -852,7 +868,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
         for (int seq = seq0; seq <= seq1; ++seq) {
             const int m = (w + seq - seq0) & 3, pos = plan.Pos[seq];
             if (PosOk(p, pos) && (m == 0 || plan.Base[seq] >= slot0)) {
-                ProjectHeads<D>(p, layer, g, sm.Seqs[seq], m, seq, (seq - seq0) * p.PerGroup * D, head0, heads, pos);
+                ProjectHeads<D>(p, sm.Now.QvMult, g, sm.Seqs[seq], m, seq, (seq - seq0) * p.PerGroup * D, head0, heads, pos);
             }
         }
         GroupSync(group);
@@ -864,7 +880,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
             if (chunk < slots) {
                 seq = plan.SeqOf[slot0 + chunk];
                 int j0, j1;
-                KeyRange(plan.Pos[seq] + 1, layer.Window, &j0, &j1);
+                KeyRange(plan.Pos[seq] + 1, sm.Now.Window, &j0, &j1);
                 const int cBeg = j0 + (slot0 + chunk - plan.Base[seq]) * plan.Chunk, cEnd = min(cBeg + plan.Chunk, j1);
                 const int perPart = (((cEnd - cBeg + p.Split - 1) >> (p.Split >> 1)) + 7) & ~7, beg = cBeg + part * perPart, end = min(beg + perPart, cEnd);
                 if (beg < end && PosOk(p, plan.Pos[seq])) {
@@ -877,7 +893,7 @@ __device__ void AttentionPhase(const TStepParams &p, TStepSmem &sm, int l)
             const tsa_kv_seq &sq = sm.Seqs[seq];
             const int4 qv = *reinterpret_cast<const int4 *>(g.Q8 + (seq - seq0) * p.PerGroup * D + (headC - head0) * D + sub * 16);
             const size_t off = (size_t)tBeg * hs + headC * D + sub * 16, soff = (size_t)tBeg * p.Heads + headC;
-            AttendRange<D>(qv, p.DotScale * INF_VEC_SCALE, layer.Slope, plan.Pos[seq], (const int8_t *)sq.k + off, (const int8_t *)sq.v + off,
+            AttendRange<D>(qv, p.DotScale * INF_VEC_SCALE, sm.Now.Slope, plan.Pos[seq], (const int8_t *)sq.k + off, (const int8_t *)sq.v + off,
                 (const float *)sq.kScale + soff, (const float *)sq.vScale + soff, p.Heads, tBeg, tEnd, batches, g.Merge[w][lane]);
         }
         GroupSync(group);
@@ -989,6 +1005,17 @@ __device__ __forceinline__ void ZeroSums(int *sums, int n)
     }
 }
 
+__device__ __forceinline__ TLayerNow LayerNow(const TStepParams &p, int l)
+{
+    TLayerNow n;
+    n.QvMult = p.Layers[l].QvMult;
+    n.CombScale = p.Layers[l].CombScale;
+    n.PrevContractScale = l > 0 ? p.Layers[l - 1].ContractScale : 0.0f;
+    n.Slope = p.Layers[l].Slope;
+    n.Window = p.Layers[l].Window;
+    return n;
+}
+
 template <int D>
 __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
 {
@@ -1002,6 +1029,9 @@ __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
             }
         }
         sm.PhaseBegin[tid] = n;
+    }
+    if (tid == PS_THREADS - 1 && p.LayerCount > 0) {
+        sm.Now = LayerNow(p, 0);
     }
     __syncthreads();
     for (int i = tid; i < sm.PhaseBegin[4] && i < PS_TABLE; i += PS_THREADS) {
@@ -1019,7 +1049,7 @@ __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
     while (l < p.LayerCount) {
         if (attention) {
             ZeroSums(l > 0 ? p.Contract : p.Comb, p.NSeq * p.Dim);
-            AttentionPhase<D>(p, sm, l);
+            AttentionPhase<D>(p, sm);
         } else {
             int *done = phase == PH_PROJ ? p.Expand : phase == PH_COMB ? p.Proj : p.Comb;
             const int doneInts = p.NSeq * (phase == PH_PROJ ? p.ReluDim : phase == PH_COMB ? 4 * hs : p.Dim);
@@ -1034,6 +1064,9 @@ __device__ void RunLayers(const TStepParams &p, TStepSmem &sm)
         GridArrive(p);
         if (!attention && phase == PH_PROJ) {
             PrepareAttention(p, sm, l);
+        }
+        if (!attention && phase == PH_CONTRACT && tid == PS_THREADS - 1 && l + 1 < p.LayerCount) {
+            sm.Now = LayerNow(p, l + 1);
         }
         RefillRing(p, sm, &cursor);
         if (!attention && phase == PH_PROJ) {
