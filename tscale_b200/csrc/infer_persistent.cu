@@ -361,8 +361,11 @@ __device__ __forceinline__ void StageState(const TStepParams &p, TStepSmem &sm, 
 __device__ __forceinline__ void QuantiseStaged(const TStepParams &p, TStepSmem &sm, int quad0, int quads, bool relu)
 {
 #pragma unroll 2
-    for (int i = threadIdx.x; i < p.NSeq * quads; i += PS_THREADS) {
-        const int s = i / quads, x = (quad0 + i - s * quads) * 4;
+    for (int i = threadIdx.x; i < p.NSeq * 32; i += PS_THREADS) {
+        const int s = i >> 5, x = (i & 31) * 4;
+        if ((unsigned)((i & 31) - quad0) >= (unsigned)quads) {
+            continue;
+        }
         const float mult = sm.Mult[s];
         const float4 v = *reinterpret_cast<const float4 *>(&sm.F[s][x]);
         int q[4] = {ToInt8Clamp127(__fmul_rn(v.x, mult)), ToInt8Clamp127(__fmul_rn(v.y, mult)), ToInt8Clamp127(__fmul_rn(v.z, mult)),
@@ -398,11 +401,25 @@ __device__ __forceinline__ void NormaliseStaged(const TStepParams &p, TStepSmem 
 // inside the chunk is summed from shared memory, one that reaches beyond it from L2.
 __device__ __forceinline__ void NormaliseRelu(const TStepParams &p, TStepSmem &sm, int chunk)
 {
-#pragma unroll 8
-    for (int i = threadIdx.x; i < p.NSeq * 32; i += PS_THREADS) {
-        const int s = i >> 5, x = (i & 31) * 4;
-        const int4 a = __ldcg(reinterpret_cast<const int4 *>(p.Expand + (size_t)s * p.ReluDim + chunk * 128 + x));
-        *reinterpret_cast<float4 *>(&sm.F[s][x]) = make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w);
+    // three loads of a thread before the first use (an unrolled loop ran its five or six iterations in the remainder, one load after the
+    // other)
+#pragma unroll 1
+    for (int base = threadIdx.x; base < p.NSeq * 32; base += PS_STAGE_AHEAD * PS_THREADS) {
+        int4 a[PS_STAGE_AHEAD];
+#pragma unroll
+        for (int k = 0; k < PS_STAGE_AHEAD; ++k) {
+            const int i = base + k * PS_THREADS;
+            if (i < p.NSeq * 32) {
+                a[k] = __ldcg(reinterpret_cast<const int4 *>(p.Expand + (size_t)(i >> 5) * p.ReluDim + chunk * 128 + (i & 31) * 4));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < PS_STAGE_AHEAD; ++k) {
+            const int i = base + k * PS_THREADS;
+            if (i < p.NSeq * 32) {
+                *reinterpret_cast<float4 *>(&sm.F[i >> 5][(i & 31) * 4]) = make_float4((float)a[k].x, (float)a[k].y, (float)a[k].z, (float)a[k].w);
+            }
+        }
     }
     __syncthreads();
     const int group = p.ReluDim / p.Heads, c0 = chunk * 128;
