@@ -20,8 +20,9 @@
 //              key tile in two halves of 64, finds the largest of a half, and exponentiates the half in one straight run
 //              against the reference m it already holds.  Only when a score exceeds m by more than the e4m3 headroom
 //              (weights up to 2^8.75 < 448) does the warp first raise m and shrink O and the sum.  The run has no branch
-//              or vote inside, so loads, exponentials, conversions and stores of a half overlap: 16 columns at a time
-//              with a vote each took 836 us where this takes 720 (16 documents of 4096 rows, 12 heads x 64, no window).
+//              or vote inside, so loads, exponentials, conversions and stores of a half overlap, and its first weights are
+//              formed in front of the vote (FW_EARLY).  16 documents of 4096 rows, 12 heads x 64, no window: 836 us with 16
+//              columns and a vote at a time, 712 with halves, 659 with early weights.
 //              Tiles the span mask cuts through add a second e4m3 residual term (P split into
 //              e4m3(P) + e4m3(P - e4m3(P)), two MMAs), which removes the 3-bit-mantissa rounding where it is not
 //              averaged out over many keys (rows with few keys see only such tiles).

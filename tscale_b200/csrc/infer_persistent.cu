@@ -18,12 +18,12 @@
 // phases and layers, in flight in a ring of shared memory (cp.async), so that their DRAM latency is never on the path.
 //
 // Measured, twelve layers, dim 768, 12 heads x 64, vocabulary 50304, a whole token with the final layer and softmax, launches / graph:
-//     1 sequence, 500 tokens of context       744 / 568 -> 325 us, of which 303 are there with windows of 64 tokens in all layers: sixty
+//     1 sequence, 500 tokens of context       744 / 568 -> 323 us, of which 305 are there with windows of 64 tokens in all layers: sixty
 //                                             phases at some 5 us, the barrier, the sums through L2 and the norm, in a chain; the
 //                                             bytes take 20 us
-//     64 sequences, 1024 to 8192 tokens       968 / 801 -> 714 / 714 us (three of four layers see 64 tokens): 462 us with the short
-//                                             windows in all layers, and 84 us for every wide layer, whose keys and values then
-//                                             stream at 5.8 TB/s
+//     64 sequences, 1024 to 8192 tokens       968 / 801 -> 707 / 701 us (three of four layers see 64 tokens): 439 us with the short
+//                                             windows in all layers, and 89 us for every wide layer, whose keys and values then
+//                                             stream at 5.5 TB/s
 // Head counts whose chunks need a whole group of four warps leave a quarter of the groups a second unit: with 16 heads x 64 such a
 // batch takes 975 / 968 us, where separate launches, 16 warps per SM in the attention, took 1085 / 897.
 #include "att_sm100_common.cuh"
