@@ -46,6 +46,42 @@ def test_fwd_half_tiles(length, d, qk_dtype, v_dtype, slope):
     assert util.err_stats(lse, ref["lse"])[0] < 2e-3, util.describe(lse, ref["lse"])
 
 
+@pytest.mark.parametrize("step", [-0.05, 0.02, 0.11, 3.0])   # log2 units from key to key: no raise, one now and then, one per group, one per key
+@pytest.mark.parametrize("d,qk_dtype,window", [(64, "e4m3", 0), (128, "e4m3", 0), (128, "i8", 0), (64, "i8", 200)])
+def test_fwd_rising_logits(step, d, qk_dtype, window):
+    """Logits that rise along the keys: the reference moves in full halves and in masked blocks, first groups and later ones, and the
+    weights formed in front of the vote have to be formed again.  A weight is rounded to three mantissa bits at worst, a relative
+    error of 2^-4, and so is the output at most; the sum of the weights is not rounded."""
+    from tscale_b200 import abi, ops
+    rows, heads = 420, 2
+    c = 0.5 / np.sqrt(d) / 0.693147
+    one = 0x38 if qk_dtype == "e4m3" else 1   # the vectors are all ones, their product is d
+    q8 = torch.full((rows, heads * d), one, dtype=torch.uint8, device=DEV)
+    sk = (torch.arange(rows, dtype=torch.float64) * step / (d * c)).to(torch.float32).expand(heads, rows).contiguous()
+    sq = torch.ones(heads, rows)
+    gen = torch.Generator().manual_seed(60)
+    v8 = torch.randn(rows, heads * d, generator=gen).to(torch.float8_e4m3fn)
+    sv = torch.rand(heads, rows, generator=gen) + 0.5
+    cfg = ops.make_cfg(qk_dtype, "e4m3", d, d, out_dtype=torch.float32)
+    ws = torch.empty(max(1, abi.lib().tsa_att_fwd_workspace_bytes(cfg, heads, rows)), dtype=torch.uint8, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    out, lse = ops.att_fwd(cfg, q8, q8, v8.view(torch.uint8).to(DEV), sk.to(DEV), ops.Mask.window([rows], window), 0.0, heads, qk_scale=sq.to(DEV),
+                           v_scale=sv.to(DEV), workspace=ws, status=status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    i = torch.arange(rows)
+    seen = (i[None, :] < i[:, None]) & ((i[None, :] >= i[:, None] - window) if window else True)
+    z = (sk[0].double() * d * c).expand(rows, rows).masked_fill(~seen, -np.inf)
+    m = z.amax(1, keepdim=True).clamp_min(0)
+    w = torch.exp2(z - m)
+    total = w.sum(1, keepdim=True) + torch.exp2(-m)
+    v = v8.double().view(rows, heads, d) * sv.t().double()[:, :, None]
+    want = torch.einsum("ij,jhd->ihd", w / total, v).reshape(rows, heads * d)
+    want_lse = (m + torch.log2(total))[:, 0]
+    assert (out.cpu().double() - want).abs().max() <= 2.0 ** -4 * v.abs().max()
+    assert ((lse.cpu().double() - want_lse).abs() <= 2e-5 + 1e-6 * want_lse.abs()).all()
+
+
 @pytest.mark.parametrize("length,heads", [(1, 1), (129, 3), (391, 2), (2200, 10)])   # the last: more items than CTAs
 @pytest.mark.parametrize("d,grad,pad", [(64, torch.bfloat16, 0), (128, torch.float32, 4), (64, torch.float16, 8), (128, torch.bfloat16, 8)])
 def test_bwd_work_items(length, heads, d, grad, pad):
