@@ -589,9 +589,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                     const bool rowEmpty = lsC > lfC;
                     const int lsQ = lsC - cb;
                     const unsigned spanW = rowEmpty ? 0u : (unsigned)(lfC - lsC);
-                    const bool anyCh = !warpMasked || __any_sync(0xffffffffu, !rowEmpty);
                     uint32_t a1[8], a2[8];
-                    if (anyCh) {
+                    // The arithmetic of a half's 16 columns, with and without the mask: as one piece of code every pair of columns carried
+                    // six instructions that only tiles at the mask's edge need.
+                    auto weigh = [&](auto maskedTag) {
+                        constexpr bool MASKED = decltype(maskedTag)::value;
                         float2 s[8], d[8];
                         TmemLd16x2Pairs(tLane + BWD_S_COL + cb, tLane + BWD_DP_COL + cb, s, d);
                         const float4 *A4 = reinterpret_cast<const float4 *>(misc.ColA[buf] + cb);
@@ -609,7 +611,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                                 const float2 u = __fmul2_rn(s[i], ca);
                                 const float2 e = __ffma2_rn(u, rowMult2, __fadd2_rn(ct, rowConst2));
                                 float2 pij = FastExp2Pair(e);
-                                if (warpMasked) {
+                                if (MASKED) {
                                     pij.x = (!rowEmpty && (unsigned)(c + 2 * k - lsQ) <= spanW) ? pij.x : 0.0f;
                                     pij.y = (!rowEmpty && (unsigned)(c + 2 * k + 1 - lsQ) <= spanW) ? pij.y : 0.0f;
                                 }
@@ -619,6 +621,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                                 a2[i] = PackBf16x2(pij.x, pij.y);
                             }
                         }
+                    };
+                    if (!warpMasked) {
+                        weigh(std::false_type());
+                    } else if (__any_sync(0xffffffffu, !rowEmpty)) {
+                        weigh(std::true_type());
                     } else {
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {
