@@ -213,6 +213,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
                     }
                 }
             }
+            // the commits that free the last stages arrive in both CTAs: none may be on its way to one that has left
+            for (int k = max(0, requested - a.Stages); k < requested && !failed; ++k) {
+                if (!WaitBarA(&misc.Empty[k % a.Stages], (k / a.Stages) & 1, abortFlag)) {
+                    failed = true;
+                    fail(kDevTimeoutMma);
+                }
+            }
             if (rank == 0 && (failed || *(volatile int *)&misc.Abort)) {
                 // copies that were requested but never consumed must not land after the CTA is gone: wait (bounded) for both CTAs' (the
                 // second one leaves behind the first)
@@ -419,7 +426,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
     }
     TcFenceBefore();
     __syncthreads();
-    PairSync(); // neither CTA leaves while the other's MMAs may still read its operands or arrive on its barriers
+    PairSync(); // neither CTA leaves while the other may still arrive on its barriers
     if (warp == PROJ_MMA_WARP) {
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * PROJ_N) : "memory");
     }
