@@ -73,6 +73,47 @@ def test_forward_with_a_withheld_copy_times_out_cleanly_and_recovers():
     assert mx < util.OUT_MAX_ABS and mean < util.OUT_MEAN_ABS
 
 
+@pytest.mark.parametrize("chunk", [0, 5, 16, 47])   # of 48: the first, inside the first tile, the first of the third tile, the last
+@pytest.mark.parametrize("with_rope", [False, True])
+def test_projection_pair_with_a_withheld_copy_times_out_cleanly_and_recovers(chunk, with_rope):
+    """The second CTA of every pair requests a chunk of x that never arrives: both CTAs give up within the bound, wait for the copies
+    and products that are under way, some of them on the other one's barriers, and leave together; the next call is right."""
+    from tscale_b200 import abi, ops
+    lib = abi.lib()
+    heads, d, dim, rows = 4, 64, 1024, 6 * 74 * 256   # six tiles of 256 rows x 256 columns per pair, eight chunks each
+    gen = torch.Generator(device=DEV).manual_seed(70)
+    x = torch.randint(-127, 128, (rows, dim), dtype=torch.int8, device=DEV, generator=gen)
+    w = torch.randint(-127, 128, (heads * d, dim), dtype=torch.int8, device=DEV, generator=gen)
+    rope = torch.randn(rows, d, device=DEV, generator=gen) if with_rope else None
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def project():
+        return ops.matmul_norm_rope_quant(x, w, rope, "i8", heads, d, vec_scale=1 / 24.0, src_scale=1 / 4096.0, status=status)
+
+    want = project()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    abi.check(lib.tsa_selftest_fwd_withhold_copy(2000000, chunk))
+    try:
+        begin.record()
+        project()
+        end.record()
+        torch.cuda.synchronize()
+    finally:
+        abi.check(lib.tsa_selftest_fwd_withhold_copy(0, -1))
+    word = int(status.item())
+    assert word & 0x30 and lib.tsa_status_from_word(word) == abi.TSA_TIMEOUT, hex(word)
+    # two waits of about a millisecond, each looked at after at most 32 suspended polls of 0.2 ms; one CTA that had to find out by
+    # itself would add the production bound of about a second
+    assert begin.elapsed_time(end) < 500
+    status.zero_()
+    got = project()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
 def _banded(rows, cols, dtype, pad_rows=3, pad_cols=16):
     """A [rows][cols] view inside a larger buffer filled with the guard pattern; returns (view, whole buffer)."""
     whole = torch.empty((rows + 2 * pad_rows, cols + pad_cols), dtype=dtype, device=DEV)

@@ -1531,6 +1531,10 @@ void SetFwdScoreDump(const TFwdDump &d)
 {
     g_dump = d;
 }
+const TFwdDump &TestHooks()
+{
+    return g_dump;
+}
 
 template <int D, bool QK_I8, bool HAS_VSCALE, bool HAS_ALIBI, bool V_I8, bool FORWARD, bool KV = false>
 static int LaunchFwdT2(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const CUtensorMap &mv2, const TFwdParams &fp, cudaStream_t stream)

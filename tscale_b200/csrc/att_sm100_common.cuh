@@ -32,7 +32,7 @@ __device__ __forceinline__ bool WaitBar(uint64_t *bar, uint32_t parity, long lon
 // the same with an abort flag of the CTA: returns false as soon as another thread has given up.
 // FAST polls without a suspend hint (the waiting thread's wake-up latency is on the critical path).
 template <bool FAST = false>
-__device__ __forceinline__ bool WaitBarA(uint64_t *bar, uint32_t parity, const int *abortFlag)
+__device__ __forceinline__ bool WaitBarA(uint64_t *bar, uint32_t parity, const int *abortFlag, long long limit = WAIT_CYCLES)
 {
     if (FAST ? MbarTryWaitFast(bar, parity) : MbarTryWait(bar, parity)) {
         return true;
@@ -48,7 +48,7 @@ __device__ __forceinline__ bool WaitBarA(uint64_t *bar, uint32_t parity, const i
         if (*(const volatile int *)abortFlag) {
             return false;
         }
-        if (clock64() - t0 > WAIT_CYCLES) {
+        if (clock64() - t0 > limit) {
             return false;
         }
     }

@@ -36,7 +36,9 @@ struct TProjMisc {
     uint64_t Full[PROJ_MAX_STAGES], Empty[PROJ_MAX_STAGES]; // ring: in the first CTA: the copies of both landed / MMAs that read them retired (both CTAs)
     uint64_t AccFull[2], AccEmpty[2];                       // accumulator set complete (both CTAs) / in the first CTA: read out, an arrival per epilogue warp of both
     uint32_t TmemBase;
-    int Abort; // a bounded wait ran out somewhere in the CTA
+    int Abort;        // a bounded wait ran out somewhere in the pair (both CTAs)
+    int Requested[2]; // in the first CTA: chunks whose copies either one's loader has requested
+    int Issued;       // chunks whose products were issued (both CTAs)
 };
 
 // arrival, with release at cluster scope, on the barrier that lies in the first CTA of the pair where `bar` lies in this one
@@ -50,8 +52,25 @@ __device__ __forceinline__ void ArriveInFirst(uint64_t *bar)
         "}" ::"r"(SmemAddr(bar))
         : "memory");
 }
+// `value` into the word that lies in the given CTA of the pair where `word` lies in this one
+__device__ __forceinline__ void StoreInPair(int *word, int value, int rank)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .b32 remote;\n\t"
+        "mapa.shared::cluster.u32 remote, %0, %2;\n\t"
+        "st.relaxed.cluster.shared::cluster.u32 [remote], %1;\n\t"
+        "}" ::"r"(SmemAddr(word)),
+        "r"(value), "r"(rank)
+        : "memory");
+}
+// counts bytes as landed that nobody copies
+__device__ __forceinline__ void MbarCompleteTx(uint64_t *bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(SmemAddr(bar)), "r"(bytes) : "memory");
+}
 // WaitBarA for a barrier the other CTA of the pair arrives on
-__device__ __forceinline__ bool WaitBarPair(uint64_t *bar, uint32_t parity, const int *abortFlag)
+__device__ __forceinline__ bool WaitBarPair(uint64_t *bar, uint32_t parity, const int *abortFlag, long long limit)
 {
     const long long t0 = clock64();
     for (;;) {
@@ -71,7 +90,7 @@ __device__ __forceinline__ bool WaitBarPair(uint64_t *bar, uint32_t parity, cons
                 return true;
             }
         }
-        if (*(const volatile int *)abortFlag || clock64() - t0 > WAIT_CYCLES) {
+        if (*(const volatile int *)abortFlag || clock64() - t0 > limit) {
             return false;
         }
     }
@@ -134,6 +153,10 @@ struct TProjArgs {
     int Len, Rows, HeadCount, Chunks;
     int ColTiles, Items; // tiles along the output columns, and all of them
     int Stages;          // of the ring
+    // self-test of the failure path: bound of every barrier wait in clock cycles (about a second in production) and the index, in a pair's
+    // own sequence, of a chunk of x that the second CTA requests but never copies (-1: none)
+    long long WaitCycles;
+    int WithholdChunk;
 };
 
 // X_E4M3: both operands are e4m3 bytes (MulForwardFp8, gpt_cuda.cu:488-491), products accumulate in f32 on the tensor
@@ -179,6 +202,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
     const int *abortFlag = &misc.Abort;
     auto fail = [&](int code) {
         *(volatile int *)&misc.Abort = 1;
+        StoreInPair(&misc.Abort, 1, rank ^ 1);
         if (status) {
             atomicOr(status, code);
         }
@@ -195,7 +219,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
             for (int item = itemBegin; item < itemEnd && !failed; ++item) {
                 const int rowBase = rowOf(item), colBase = item % a.ColTiles * PROJ_N + rank * (PROJ_N / 2);
                 for (int c = 0; c < a.Chunks; ++c) {
-                    if (requested >= a.Stages && !WaitBarA(&misc.Empty[s], phase ^ 1, abortFlag)) {
+                    if (requested >= a.Stages && !WaitBarA(&misc.Empty[s], phase ^ 1, abortFlag, a.WaitCycles)) {
                         failed = true;
                         fail(kDevTimeoutMma);
                         break;
@@ -204,7 +228,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
                     if (rank == 0) {
                         MbarExpectTx(&misc.Full[s], 2 * PROJ_STAGE_BYTES);
                     }
-                    TmaLoadPair(sA, &tmX, c * PROJ_KB, rowBase, &misc.Full[s]);
+                    if (rank == 0 || requested != a.WithholdChunk) { // self-test: the bytes of a withheld copy never arrive
+                        TmaLoadPair(sA, &tmX, c * PROJ_KB, rowBase, &misc.Full[s]);
+                    }
                     TmaLoadPair(sA + PROJ_M * PROJ_KB, &tmW, c * PROJ_KB, colBase, &misc.Full[s]);
                     ++requested;
                     if (++s == a.Stages) {
@@ -215,27 +241,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
             }
             // the commits that free the last stages arrive in both CTAs: none may be on its way to one that has left
             for (int k = max(0, requested - a.Stages); k < requested && !failed; ++k) {
-                if (!WaitBarA(&misc.Empty[k % a.Stages], (k / a.Stages) & 1, abortFlag)) {
+                if (!WaitBarA(&misc.Empty[k % a.Stages], (k / a.Stages) & 1, abortFlag, a.WaitCycles)) {
                     failed = true;
                     fail(kDevTimeoutMma);
                 }
             }
-            if (rank == 0 && (failed || *(volatile int *)&misc.Abort)) {
-                // copies that were requested but never consumed must not land after the CTA is gone: wait (bounded) for both CTAs' (the
-                // second one leaves behind the first)
-                for (int k = max(0, requested - a.Stages); k < requested; ++k) {
-                    WaitBar(&misc.Full[k % a.Stages], (k / a.Stages) & 1);
-                }
-            }
+            StoreInPair(&misc.Requested[rank], requested, 0);
         }
         __syncwarp();
     } else if (warp == PROJ_MMA_WARP) {
         if (rank == 0) {
         // the whole warp runs the loop and the waits, one elected lane issues (descriptors stay in uniform registers that way)
-        int s = 0, phase = 0, n = 0;
+        int s = 0, phase = 0, n = 0, issued = 0;
         bool failed = false;
         auto wait = [&](uint64_t *bar, uint32_t parity, int code) {
-            if (!__all_sync(0xffffffffu, WaitBarPair(bar, parity, abortFlag))) {
+            if (!__all_sync(0xffffffffu, WaitBarPair(bar, parity, abortFlag, a.WaitCycles))) {
                 failed = true;
                 if (lane == 0) {
                     fail(code);
@@ -267,11 +287,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
                     }
                 }
                 __syncwarp();
+                ++issued;
                 if (++s == a.Stages) {
                     s = 0;
                     phase ^= 1;
                 }
             }
+        }
+        if (lane < 2) {
+            StoreInPair(&misc.Issued, issued, lane);
         }
         }
         __syncwarp();
@@ -294,7 +318,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
         bool failed = false;
         for (int item = itemBegin; item < itemEnd; ++item, ++n) {
             const int rowBase = rowOf(item), headBase = item % a.ColTiles * HPC;
-            if (!WaitBarA(&misc.AccFull[n & 1], (n >> 1) & 1, abortFlag)) {
+            if (!WaitBarA(&misc.AccFull[n & 1], (n >> 1) & 1, abortFlag, a.WaitCycles)) {
                 failed = true;
                 fail(kDevTimeoutMma);
             }
@@ -427,6 +451,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
     TcFenceBefore();
     __syncthreads();
     PairSync(); // neither CTA leaves while the other may still arrive on its barriers
+    if (*(volatile int *)&misc.Abort) {
+        // A wait ran out, which both CTAs see here.  What was started and nobody has waited for must not reach a CTA that has left: the
+        // products issued, and copies of either CTA, all counted in the first one, that no product has waited for.
+        if (tid == PROJ_LOAD_WARP * 32) {
+            const int issued = misc.Issued, tiles = issued / a.Chunks;
+            for (int k = max(0, issued - a.Stages); k < issued; ++k) {
+                WaitBar(&misc.Empty[k % a.Stages], (k / a.Stages) & 1, a.WaitCycles);
+            }
+            for (int n = max(0, tiles - 2); n < tiles; ++n) {
+                WaitBar(&misc.AccFull[n & 1], (n >> 1) & 1, a.WaitCycles);
+            }
+            if (rank == 0) {
+                const int mine = misc.Requested[0], others = misc.Requested[1];
+                for (int k = issued; k < max(mine, others); ++k) {
+                    uint64_t *bar = &misc.Full[k % a.Stages];
+                    if (k >= mine) {
+                        MbarExpectTx(bar, PROJ_STAGE_BYTES); // the second CTA alone requested it
+                    } else if (k >= others) {
+                        MbarCompleteTx(bar, PROJ_STAGE_BYTES); // the first CTA alone
+                    }
+                    WaitBar(bar, (k / a.Stages) & 1, a.WaitCycles);
+                }
+            }
+        }
+        __syncthreads();
+        PairSync();
+    }
     if (warp == PROJ_MMA_WARP) {
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * PROJ_N) : "memory");
     }
@@ -491,6 +542,8 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     const int ropeBytes = rope.data ? PROJ_M * (headDim + 1) * (int)sizeof(float) : 0;
     a.Stages = (PROJ_SMEM_MAX - 2048 - ropeBytes) / PROJ_STAGE_BYTES;
     a.Stages = a.Stages < PROJ_MAX_STAGES ? a.Stages : PROJ_MAX_STAGES;
+    a.WaitCycles = TestHooks().WaitCycles > 0 ? TestHooks().WaitCycles : WAIT_CYCLES;
+    a.WithholdChunk = TestHooks().WithholdTile;
     const int smemBytes = a.Stages * PROJ_STAGE_BYTES + 1024 /* barriers */ + 1024 /* alignment */ + ropeBytes;
     int dev = 0, sms = 0;
     rc = CheckCuda(cudaGetDevice(&dev), "cudaGetDevice");
