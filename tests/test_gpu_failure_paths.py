@@ -114,6 +114,49 @@ def test_projection_pair_with_a_withheld_copy_times_out_cleanly_and_recovers(chu
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
+@pytest.mark.parametrize("tile", [0, 3])
+def test_backward_with_withheld_column_factors_times_out_cleanly_and_recovers(tile):
+    """The factors of a tile's columns are never announced: the warp whose wait runs out first reports it and stops the others.  Left
+    to themselves the other warps and the MMA warps would each run out their own production bound of about a second."""
+    from tscale_b200 import abi, ops
+    lib = abi.lib()
+    heads, d, seq = 2, 64, 1024
+    q, k, v = util.make_qkv(71, seq, heads, d, d, 0.5)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
+    (q8, sq, _), (k8, sk, _), (v8, sv, _) = util.quantize(q, "i8", d), util.quantize(k, "i8", d), util.quantize(v, "e4m3", d)
+    g = dict(q=t(q8.view(np.uint8)), k=t(k8.view(np.uint8)), v=t(v8.view(np.uint8)), sq=t(sq), sk=t(sk), sv=t(sv))
+    mask = ops.Mask.window([seq], 0)
+    cfg = ops.make_cfg("i8", "e4m3", d, d, out_dtype=torch.float32, grad_dtype=torch.float32)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    out, lse = ops.att_fwd(cfg, g["q"], g["k"], g["v"], g["sk"], mask, 0.0, heads, qk_scale=g["sq"], v_scale=g["sv"], status=status)
+    d_out = t((np.random.default_rng(72).standard_normal((seq, heads * d)) * 1e-2).astype(np.float32))
+
+    def bwd():
+        return ops.att_bwd(cfg, g["q"], g["k"], g["v"], g["sk"], d_out, out, lse, mask, 0.0, heads, qk_scale=g["sq"], v_scale=g["sv"], status=status)
+
+    want = bwd()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    abi.check(lib.tsa_selftest_fwd_withhold_copy(2000000, tile))
+    try:
+        begin.record()
+        bwd()
+        end.record()
+        torch.cuda.synchronize()
+    finally:
+        abi.check(lib.tsa_selftest_fwd_withhold_copy(0, -1))
+    word = int(status.item())
+    assert word & 0x30 and lib.tsa_status_from_word(word) == abi.TSA_TIMEOUT, hex(word)
+    assert begin.elapsed_time(end) < 500, begin.elapsed_time(end)
+    status.zero_()
+    got = bwd()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
 def _banded(rows, cols, dtype, pad_rows=3, pad_cols=16):
     """A [rows][cols] view inside a larger buffer filled with the guard pattern; returns (view, whole buffer)."""
     whole = torch.empty((rows + 2 * pad_rows, cols + pad_cols), dtype=dtype, device=DEV)

@@ -63,6 +63,10 @@ struct TBwdParams {
     int Ascending;    // order of the row tiles: the long ones come first
     int *Counter;     // work-item counter, zero at launch
     int *Status;
+    // self-test of the failure path: bound, in clock cycles, of the wait for a tile's column factors (about a second in production) and
+    // the index, in a CTA's own sequence, of a tile whose factors are staged but never announced (-1: none)
+    long long WaitCycles;
+    int WithholdTile;
 };
 
 template <int D>
@@ -97,7 +101,7 @@ struct TBwdMisc {
     uint64_t BarFull[8];      // TMA: half stage (64 rows of C1 and C2) landed
     uint64_t BarEmpty[8];     // MMA warp -> loader: the half stage's output products have retired
     uint64_t BarS[2];         // control -> half h: S and dP columns of the half ready
-    uint64_t BarP[2];         // half h -> control: A1 / A2 of the half written (8 warp arrivals)
+    uint64_t BarP[2];         // half h -> control: A1 / A2 of the half written (an arrival per arithmetic warp)
     uint64_t ColFull[2];      // first four arithmetic warps -> all of them: the column factors of a tile are staged
     uint64_t BarOut;          // MMA warps -> arithmetic: every output product of the item has retired
     uint32_t TmemBase;
@@ -544,7 +548,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                     misc.ColT[buf][tid] = MODE_DKV ? -pfT - p.Slope * (float)tid : p.Slope * (float)tid;
                     misc.ColB[buf][tid] = MODE_DKV ? -pfB * dsMult : pfB * dsMult;
                     __syncwarp();
-                    if (lane == 0) {
+                    if (lane == 0 && it != p.WithholdTile) {
                         MbarArrive(&misc.ColFull[buf]);
                     }
                 }
@@ -555,8 +559,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                 // The staged columns, double buffered: a warp that stages tile t + 2 has seen the scores of tile t + 1's second half, and
                 // those were asked for when all 16 warps had handed over tile t.  (A barrier of the 512 threads per tile kept the warps in
                 // step.)  A thread whose wait fails goes to the threads' next common barrier, where they leave together.
-                if (!__all_sync(0xffffffffu, !failed && WaitBarA<true>(&misc.ColFull[buf], (it >> 1) & 1, abortFlag))) {
+                if (!__all_sync(0xffffffffu, !failed && WaitBarA<true>(&misc.ColFull[buf], (it >> 1) & 1, abortFlag, p.WaitCycles))) {
                     failed = true;
+                    *(volatile int *)&misc.Abort = 1;
+                    if (p.Status) {
+                        atomicOr(p.Status, kDevTimeoutMma);
+                    }
                     break;
                 }
                 {
@@ -961,6 +969,8 @@ int LaunchSm100Bwd(const tsa_att_cfg *cfg, const TGenParams &p, tsa_ptr2d qk, ts
     bp.GradMult = p.GradMult;
     bp.GradDtype = p.GradDtype;
     bp.Status = statusWord;
+    bp.WaitCycles = TestHooks().WaitCycles > 0 ? TestHooks().WaitCycles : WAIT_CYCLES;
+    bp.WithholdTile = TestHooks().WithholdTile;
     const int rowTiles = (lenAttTiles + 1) / 2;
     // dQ pass: rows = queries
     bp.Spans = p.Spans;

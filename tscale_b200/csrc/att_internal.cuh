@@ -47,8 +47,8 @@ int LaunchDScale(int outDtype, int gradDtype, tsa_ptr2d out, tsa_ptr2d dOut, tsa
 struct TFwdDump {
     int32_t *Dst = nullptr; // [128][128] int32 in device memory, null = off
     int Head = 0, QTile = 0, Tile = 0;
-    long long WaitCycles = 0; // self-test: bound of the barrier waits of the forward and the projection (0: the production bound)
-    int WithholdTile = -1;    // self-test: a key tile (projection: a chunk of x) whose copy is requested but never issued (-1: none)
+    long long WaitCycles = 0; // self-test: bound of barrier waits (0: the production bound)
+    int WithholdTile = -1;    // self-test: a key tile (projection: chunk of x; backward: factors of a tile) that is asked for but never comes (-1: none)
 };
 int LaunchBoundedWaitSelfTest(long long limitCycles, int *statusWord, cudaStream_t stream);
 void SetFwdScoreDump(const TFwdDump &d);
