@@ -75,12 +75,14 @@ def test_forward_with_a_withheld_copy_times_out_cleanly_and_recovers():
 
 @pytest.mark.parametrize("chunk", [0, 5, 16, 47])   # of 48: the first, inside the first tile, the first of the third tile, the last
 @pytest.mark.parametrize("with_rope", [False, True])
-def test_projection_pair_with_a_withheld_copy_times_out_cleanly_and_recovers(chunk, with_rope):
-    """The second CTA of every pair requests a chunk of x that never arrives: both CTAs give up within the bound, wait for the copies
-    and products that are under way, some of them on the other one's barriers, and leave together; the next call is right."""
+@pytest.mark.parametrize("dim,rows", [(1024, 6 * 74 * 256), (512, 6 * 148 * 128)])   # pairs, single CTAs: six tiles each, eight chunks per tile
+def test_projection_with_a_withheld_copy_times_out_cleanly_and_recovers(dim, rows, chunk, with_rope):
+    """The second CTA of every pair, or every single CTA, requests a chunk of x that never arrives: both CTAs give up within the bound,
+    wait for the copies and products that are under way, some of them on the other one's barriers, and leave together; the next call is
+    right."""
     from tscale_b200 import abi, ops
     lib = abi.lib()
-    heads, d, dim, rows = 4, 64, 1024, 6 * 74 * 256   # six tiles of 256 rows x 256 columns per pair, eight chunks each
+    heads, d = 4, 64
     gen = torch.Generator(device=DEV).manual_seed(70)
     x = torch.randint(-127, 128, (rows, dim), dtype=torch.int8, device=DEV, generator=gen)
     w = torch.randint(-127, 128, (heads * d, dim), dtype=torch.int8, device=DEV, generator=gen)

@@ -119,7 +119,7 @@ def test_bwd_work_items(length, heads, d, grad, pad):
 ])
 @pytest.mark.parametrize("dst", ["i8", torch.float16])
 def test_projection_tiles(dst, rows, length, dim, heads, d, with_rope):
-    """Remainders of the 128 x 256 tiles; the last shape hands every CTA several tiles, so ring and accumulator sets wrap."""
+    """Remainders of the 128 x 256 tiles of single CTAs."""
     from tscale_b200 import ops
     rng = np.random.default_rng(rows + dim)
     x = rng.integers(-127, 128, (rows, dim)).astype(np.int8)
@@ -146,9 +146,58 @@ def test_projection_tiles(dst, rows, length, dim, heads, d, with_rope):
     (1, 64, 1, 64), (128, 192, 1, 128), (129, 64, 3, 64), (256, 320, 5, 64), (257, 2048, 3, 128), (20000, 192, 5, 128),
 ])
 def test_projection_pairs(dst, rows, dim, heads, d):
-    """Tiles of 256 rows x 256 columns shared by two CTAs, 128 columns of x at a time: a second CTA without rows, half or all of
-    its columns' weights past the matrix, an inner size that ends in half a chunk, rings that wrap."""
+    """One to three row tiles, heads that leave part of the columns' weights past the matrix, one chunk to many."""
     test_projection_tiles(dst, rows, rows, dim, heads, d, True)
+
+
+@pytest.mark.parametrize("dst", ["i8", torch.bfloat16])
+@pytest.mark.parametrize("rows,length,dim,heads,d", [
+    (1, 1, 1344, 1, 64), (128, 128, 1344, 1, 128), (129, 128, 1280, 3, 64), (256, 200, 1344, 5, 64), (385, 385, 1408, 2, 128),
+    (300, 300, 1024, 4, 64), (300, 300, 1088, 4, 64), (300, 300, 1216, 4, 64),   # on both sides of the lines between single CTAs and pairs
+])
+def test_projection_pair_tiles(dst, rows, length, dim, heads, d):
+    """Tiles of 256 rows x 256 columns shared by two CTAs, 128 columns of x at a time: a second CTA without rows, half or all of
+    its columns' weights past the matrix, an inner size that ends in half a chunk."""
+    test_projection_tiles(dst, rows, length, dim, heads, d, True)
+
+
+@pytest.mark.parametrize("src,dst", [("i8", "i8"), ("i8", torch.float16), ("e4m3", "i8")])
+@pytest.mark.parametrize("rows,dim,heads,d,with_rope", [
+    (69, 64, 2100, 128, True), (4000, 192, 132, 64, False),      # single CTAs: 1050 and 32 x 33 tiles on 148, at least seven each
+    (257, 1344, 520, 128, True), (2048, 1280, 268, 64, False),   # pairs: 2 x 260 and 8 x 67 tiles on 74, at least seven each
+])
+def test_projection_many_tiles(src, dst, rows, dim, heads, d, with_rope):
+    """Several tiles for every CTA or pair: the ring goes round many times, both accumulator sets are waited for in both parities, the
+    rope rows change under way.  e4m3 operands: the sums are formed in f32, in steps of 32 products; with a rounding of 2^-22 of a sum
+    per step (nothing is known of the order inside) a value is off by dim / 32 * 2^-22 of the largest partial sum, and so is a scale at most.
+    A code changes where the value lies that close to a rounding boundary: 2 * 127 * that bound of them."""
+    from tscale_b200 import ops
+    gen = torch.Generator(device=DEV).manual_seed(rows + dim)
+    if src == "i8":
+        x, w = (torch.randint(-127, 128, (n, dim), dtype=torch.int8, device=DEV, generator=gen) for n in (rows, heads * d))
+        src_scale = float(np.float32(1.0 / 4096))
+    else:
+        x, w = ((torch.randn(n, dim, device=DEV, generator=gen) * 0.7).to(torch.float8_e4m3fn) for n in (rows, heads * d))
+        src_scale = 1.0
+    # float64 holds every sum of these products exactly
+    y = (x.double() @ w.double().t()).float().cpu().numpy() * np.float32(src_scale)
+    table = O.fill_rope(d, rows) if with_rope else None
+    vec = 1 / 24.0 if src == "e4m3" else 0.5
+    want_b, want_s, roped = O.norm_rope_quant("i8", vec, y, table, d)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got, got_s = ops.matmul_norm_rope_quant(x.view(torch.int8), w.view(torch.int8), None if table is None else torch.from_numpy(table).to(DEV), dst,
+                                            heads, d, vec_scale=vec, src_scale=src_scale, status=status, src=src)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    got, got_s = got.cpu(), got_s.cpu().numpy()
+    if src == "e4m3":
+        bound = dim / 32 * 2.0 ** -22
+        codes, want = got.view(torch.int8).numpy().astype(np.int32), want_b.view(np.int8).astype(np.int32)
+        assert np.abs(got_s - want_s).max() <= bound * want_s.max()
+        assert np.abs(codes - want).max() <= 1 and np.mean(codes != want) <= 2 * 127 * bound
+    else:
+        want = torch.from_numpy(want_b.view(np.int8)) if dst == "i8" else torch.from_numpy(roped).to(dst)
+        assert np.array_equal(got_s, want_s) and torch.equal(got.view(want.dtype), want)
 
 
 @pytest.mark.parametrize("ctx,heads,d,window,slope", [

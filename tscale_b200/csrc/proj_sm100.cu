@@ -8,30 +8,50 @@
 //   per head: discr = sqrt(sum y^2 / D) * vecScale;  z = y / discr;  rope (elements k and k + 32 of a 64-block);
 //             dst = quantise(z) (int8 or e4m3);  scale[head][t] = discr
 //
-// Persistent, in pairs of CTAs (clusters of two, one CTA per SM): a pair takes tiles of 256 rows of x times 256 output columns (4 heads of
-// 64 or 2 of 128), tcgen05.mma cta_group::2, M = 256, N = 256: each CTA copies 128 rows of x and the weights of 128 columns, the first
-// one issues the products, which read the operands of both, and each has the accumulators of its own rows: 256 tensor-memory columns,
-// two such sets in turn.  One warp of each CTA streams its operands through a TMA ring of 128-column chunks that runs on across tiles
-// (both CTAs' copies count on the first one's barriers; a commit frees a stage in both), and eight warps work on the epilogue of
-// the tile before: a row belongs to two threads, each with half of the tile's heads, so a head's sum of squares, the rotation partners
-// and the 64 output bytes of a block are all in one thread: no exchange between threads, sums in the scalar loop's order (bit-identical
-// to the stand-alone normalise + rope + quantise of the CPU code on the same projection).  A pair's tiles are neighbours along the
-// columns, so its rows of x stay in L2 and its rows of the rope table in shared memory.
-// Bound by the operand stream out of L2: with a tile of 128 x 256 per CTA, 24 KB for every 64 columns, 12345 rows x 2048 -> 16 heads of 128
-// took 58 to 64 us; pairs copy two thirds of that: 43 to 51 us.  Chunks of 64 columns in pairs: 58 us, every stage pays its round trip
-// of commit, copy and barrier across the two SMs.
+// Persistent, one CTA per SM, single or in pairs (clusters of two).
+// Single: a CTA takes tiles of 128 rows of x times 256 output columns (4 heads of 64 or 2 of 128), tcgen05.mma M = 128, N = 256, with a ring
+// of 64-column chunks.
+// Pair: a tile has 256 rows; tcgen05.mma cta_group::2, M = 256, N = 256: each CTA copies 128 rows of x and the weights of 128 columns, the
+// first one issues the products, which read the operands of both, and each has the accumulators of its own rows; both CTAs' copies
+// count on the first one's barriers, a commit frees a stage in both.  Chunks of 128 columns: with 64 every stage pays its round trip
+// of commit, copy and barrier across the two SMs (58 us where 128 take 43 to 51).
+// Either way the accumulators are 256 tensor-memory columns per CTA, two such sets in turn.  One warp of each CTA streams its operands
+// through a TMA ring that runs on across tiles, one issues the MMAs, and eight warps work on the epilogue of the tile before: a row
+// belongs to two threads, each with half of the tile's heads, so a head's sum of squares, the rotation partners and the 64 output
+// bytes of a block are all in one thread: no exchange between threads, sums in the scalar loop's order (bit-identical to the
+// stand-alone normalise + rope + quantise of the CPU code on the same projection).  Tiles in a row are neighbours along the
+// columns, so the rows of x stay in L2 and the rows of the rope table in shared memory.
+// What bounds it: at large inner sizes the operand stream out of L2, 24 KB for every 64 columns in a single CTA, of which pairs copy two
+// thirds; at small ones the epilogue, and a pair's epilogues wait for each other.
 #include "att_sm100_common.cuh"
 
 namespace tsa {
 
-constexpr int PROJ_MAX_STAGES = 8;
-// a pair's tile: PROJ_M rows and the weights of PROJ_N / 2 columns come from each CTA
-constexpr int PROJ_M = 128, PROJ_N = 256, PROJ_KB = 128;
-constexpr int PROJ_STAGE_BYTES = (PROJ_M + PROJ_N / 2) * PROJ_KB;
+constexpr int PROJ_M = 128, PROJ_N = 256; // rows of a CTA, columns of a tile
 constexpr int PROJ_LOAD_WARP = 0, PROJ_MMA_WARP = 1, PROJ_EPI_WARPS = 8;
 constexpr int PROJ_EPI_THREADS = PROJ_EPI_WARPS * 32, PROJ_THREADS = PROJ_EPI_THREADS + 64;
 constexpr int PROJ_SMEM_MAX = 227 * 1024;
 
+// The inner size from which on pairs are taken: below, tiles of single CTAs were faster at some number of rows (1 to 131072), from there on
+// pairs were as fast or faster at all of them.  The longer a tile's epilogue (16-bit results are twice the bytes), the later.  Single ->
+// pair, 32768 rows without rope: int8 to e4m3 30.2 -> 32.1 us (768 -> 12 x 64), 40.6 -> 39.2 (1024 -> 16 x 64), 133 -> 105 (2048 -> 16 x 128);
+// int8 to bf16 35.6 -> 37.8, 44.0 -> 47.0, 61.5 -> 59.1 (1280 -> 20 x 64), 147 -> 120; e4m3 to int8 with rope 37.2 -> 39.4, 49.8 -> 51.2,
+// 62.0 -> 60.8 (1152 -> 18 x 64), 167 -> 149.
+inline int ProjPairFrom(bool srcE4M3, bool dst16)
+{
+    return dst16 ? 1280 : srcE4M3 ? 1152 : 1024;
+}
+// what a CTA copies of a chunk: PROJ_M rows of x, W_ROWS of w, KB columns of both
+template <bool PAIR>
+struct TProjShape {
+    static constexpr int CTAS = PAIR ? 2 : 1;
+    static constexpr int KB = PAIR ? 128 : 64;
+    static constexpr int W_ROWS = PROJ_N / CTAS;
+    static constexpr int STAGE_BYTES = (PROJ_M + W_ROWS) * KB;
+};
+constexpr int PROJ_MAX_STAGES = (PROJ_SMEM_MAX - 2048) / TProjShape<false>::STAGE_BYTES;
+
+// (without a pair the CTA itself is the first one, and the only one)
 struct TProjMisc {
     uint64_t Full[PROJ_MAX_STAGES], Empty[PROJ_MAX_STAGES]; // ring: in the first CTA: the copies of both landed / MMAs that read them retired (both CTAs)
     uint64_t AccFull[2], AccEmpty[2];                       // accumulator set complete (both CTAs) / in the first CTA: read out, an arrival per epilogue warp of both
@@ -153,8 +173,8 @@ struct TProjArgs {
     int Len, Rows, HeadCount, Chunks;
     int ColTiles, Items; // tiles along the output columns, and all of them
     int Stages;          // of the ring
-    // self-test of the failure path: bound of every barrier wait in clock cycles (about a second in production) and the index, in a pair's
-    // own sequence, of a chunk of x that the second CTA requests but never copies (-1: none)
+    // self-test of the failure path: bound of every barrier wait in clock cycles (about a second in production) and the index, in a CTA's
+    // own sequence, of a chunk of x that it (of a pair the second one) requests but never copies (-1: none)
     long long WaitCycles;
     int WithholdChunk;
 };
@@ -162,20 +182,22 @@ struct TProjArgs {
 // X_E4M3: both operands are e4m3 bytes (MulForwardFp8, gpt_cuda.cu:488-491), products accumulate in f32 on the tensor
 // cores (kind::f8f6f4); otherwise int8 x int8 with exact int32 accumulators (kind::i8).
 // DST: TSA_I8, TSA_E4M3 (quantised) or TSA_F16 / TSA_BF16 (the normalised, rotated values themselves: the reference's K16).
-template <int D, int DST, bool X_E4M3>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, TProjArgs a,
+template <int D, int DST, bool X_E4M3, bool PAIR>
+__global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, TProjArgs a,
     int *status)
 {
+    using SH = TProjShape<PAIR>;
+    constexpr int CTAS = SH::CTAS, KB = SH::KB, STAGE_BYTES = SH::STAGE_BYTES;
     // s32 accumulators, s8 x s8 -- or f32 accumulators, e4m3 x e4m3; both operands K-major
-    constexpr uint32_t IDESC = X_E4M3 ? MakeInstrDesc(1, 0, 0, 0, 0, 2 * PROJ_M, PROJ_N) : MakeInstrDesc(2, 1, 1, 0, 0, 2 * PROJ_M, PROJ_N);
+    constexpr uint32_t IDESC = X_E4M3 ? MakeInstrDesc(1, 0, 0, 0, 0, CTAS * PROJ_M, PROJ_N) : MakeInstrDesc(2, 1, 1, 0, 0, CTAS * PROJ_M, PROJ_N);
     auto accValue = [](uint32_t bits) { return X_E4M3 ? __uint_as_float(bits) : (float)(int32_t)bits; };
     constexpr int HPC = PROJ_N / D;                                          // heads per tile
     extern __shared__ uint8_t projSmemRaw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)projSmemRaw + 1023) & ~(uintptr_t)1023);
-    TProjMisc &misc = *reinterpret_cast<TProjMisc *>(smem + a.Stages * PROJ_STAGE_BYTES);
-    float *ropeTile = reinterpret_cast<float *>(smem + a.Stages * PROJ_STAGE_BYTES + 1024);
+    TProjMisc &misc = *reinterpret_cast<TProjMisc *>(smem + a.Stages * STAGE_BYTES);
+    float *ropeTile = reinterpret_cast<float *>(smem + a.Stages * STAGE_BYTES + 1024);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int rank = blockIdx.x & 1; // in the pair
+    const int rank = blockIdx.x % CTAS; // in the pair
     if (tid == 0) {
         for (int s = 0; s < a.Stages; ++s) {
             MbarInit(&misc.Full[s], 1);
@@ -183,33 +205,48 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
         }
         for (int b = 0; b < 2; ++b) {
             MbarInit(&misc.AccFull[b], 1);
-            MbarInit(&misc.AccEmpty[b], 2 * PROJ_EPI_WARPS);
+            MbarInit(&misc.AccEmpty[b], CTAS * PROJ_EPI_WARPS);
         }
         misc.Abort = 0;
         FenceBarrierInit();
     }
     if (warp == PROJ_MMA_WARP) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(&misc.TmemBase)), "r"(2 * PROJ_N) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(&misc.TmemBase)), "r"(2 * PROJ_N) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            TmemAlloc(&misc.TmemBase, 2 * PROJ_N);
+            TmemRelinquish();
+        }
     }
     TcFenceBefore();
     __syncthreads();
-    PairSync(); // the other CTA's barriers and tensor memory are set up too
+    if constexpr (PAIR) {
+        PairSync(); // the other CTA's barriers and tensor memory are set up too
+    }
     TcFenceAfter();
     const uint32_t tmem = misc.TmemBase;
     PdlTrigger(); // behind the allocation: a CTA of the next kernel may hold tensor memory of this SM from here on
     PdlWait();
     const int *abortFlag = &misc.Abort;
+    auto store = [&](int *word, int value, int toRank) {
+        if constexpr (PAIR) {
+            StoreInPair(word, value, toRank);
+        } else {
+            *(volatile int *)word = value;
+        }
+    };
     auto fail = [&](int code) {
-        *(volatile int *)&misc.Abort = 1;
-        StoreInPair(&misc.Abort, 1, rank ^ 1);
+        for (int r = 0; r < CTAS; ++r) {
+            store(&misc.Abort, 1, r);
+        }
         if (status) {
             atomicOr(status, code);
         }
     };
-    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int pair = blockIdx.x / CTAS, pairs = gridDim.x / CTAS;
     const int itemBegin = (int)((long long)a.Items * pair / pairs), itemEnd = (int)((long long)a.Items * (pair + 1) / pairs);
-    auto rowOf = [&](int item) { return (item / a.ColTiles * 2 + rank) * PROJ_M; };
+    auto rowOf = [&](int item) { return (item / a.ColTiles * CTAS + rank) * PROJ_M; };
     if (warp == PROJ_LOAD_WARP) {
         if (lane == 0) {
             PrefetchTensorMap(&tmX);
@@ -217,21 +254,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
             int s = 0, phase = 0, requested = 0; // ring slot, its parity, chunks requested
             bool failed = false;
             for (int item = itemBegin; item < itemEnd && !failed; ++item) {
-                const int rowBase = rowOf(item), colBase = item % a.ColTiles * PROJ_N + rank * (PROJ_N / 2);
+                const int rowBase = rowOf(item), colBase = item % a.ColTiles * PROJ_N + rank * SH::W_ROWS;
                 for (int c = 0; c < a.Chunks; ++c) {
                     if (requested >= a.Stages && !WaitBarA(&misc.Empty[s], phase ^ 1, abortFlag, a.WaitCycles)) {
                         failed = true;
                         fail(kDevTimeoutMma);
                         break;
                     }
-                    uint8_t *sA = smem + s * PROJ_STAGE_BYTES;
+                    uint8_t *sA = smem + s * STAGE_BYTES, *sB = sA + PROJ_M * KB;
                     if (rank == 0) {
-                        MbarExpectTx(&misc.Full[s], 2 * PROJ_STAGE_BYTES);
+                        MbarExpectTx(&misc.Full[s], CTAS * STAGE_BYTES);
                     }
-                    if (rank == 0 || requested != a.WithholdChunk) { // self-test: the bytes of a withheld copy never arrive
-                        TmaLoadPair(sA, &tmX, c * PROJ_KB, rowBase, &misc.Full[s]);
+                    const bool withheld = rank == CTAS - 1 && requested == a.WithholdChunk; // self-test: the bytes of a withheld copy never arrive
+                    if constexpr (PAIR) {
+                        if (!withheld) {
+                            TmaLoadPair(sA, &tmX, c * KB, rowBase, &misc.Full[s]);
+                        }
+                        TmaLoadPair(sB, &tmW, c * KB, colBase, &misc.Full[s]);
+                    } else {
+                        if (!withheld) {
+                            TmaLoad2D(sA, &tmX, c * KB, rowBase, &misc.Full[s]);
+                        }
+                        TmaLoad2D(sB, &tmW, c * KB, colBase, &misc.Full[s]);
                     }
-                    TmaLoadPair(sA + PROJ_M * PROJ_KB, &tmW, c * PROJ_KB, colBase, &misc.Full[s]);
                     ++requested;
                     if (++s == a.Stages) {
                         s = 0;
@@ -239,64 +284,84 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
                     }
                 }
             }
-            // the commits that free the last stages arrive in both CTAs: none may be on its way to one that has left
-            for (int k = max(0, requested - a.Stages); k < requested && !failed; ++k) {
-                if (!WaitBarA(&misc.Empty[k % a.Stages], (k / a.Stages) & 1, abortFlag, a.WaitCycles)) {
+            // the commits that free the last stages: none may be on its way to a CTA that has left
+            for (int k = 0; k < min(requested, a.Stages) && !failed; ++k) {
+                if (!WaitBarA(&misc.Empty[k], k < s ? phase : phase ^ 1, abortFlag, a.WaitCycles)) {
                     failed = true;
                     fail(kDevTimeoutMma);
                 }
             }
-            StoreInPair(&misc.Requested[rank], requested, 0);
+            store(&misc.Requested[rank], requested, 0);
         }
         __syncwarp();
     } else if (warp == PROJ_MMA_WARP) {
         if (rank == 0) {
-        // the whole warp runs the loop and the waits, one elected lane issues (descriptors stay in uniform registers that way)
-        int s = 0, phase = 0, n = 0, issued = 0;
-        bool failed = false;
-        auto wait = [&](uint64_t *bar, uint32_t parity, int code) {
-            if (!__all_sync(0xffffffffu, WaitBarPair(bar, parity, abortFlag, a.WaitCycles))) {
-                failed = true;
-                if (lane == 0) {
-                    fail(code);
+            // the whole warp runs the loop and the waits, one elected lane issues (descriptors stay in uniform registers that way)
+            int s = 0, phase = 0, n = 0, issued = 0;
+            bool failed = false;
+            auto wait = [&](uint64_t *bar, uint32_t parity, int code) {
+                bool ok;
+                if constexpr (PAIR) {
+                    ok = WaitBarPair(bar, parity, abortFlag, a.WaitCycles);
+                } else {
+                    ok = WaitBarA(bar, parity, abortFlag, a.WaitCycles);
                 }
-            }
-            return !failed;
-        };
-        for (int item = itemBegin; item < itemEnd && !failed; ++item, ++n) {
-            const uint32_t acc = tmem + (n & 1) * PROJ_N;
-            if (n >= 2 && !wait(&misc.AccEmpty[n & 1], ((n >> 1) - 1) & 1, kDevTimeoutMma)) {
-                break;
-            }
-            for (int c = 0; c < a.Chunks; ++c) {
-                if (!wait(&misc.Full[s], phase, kDevTimeoutTma)) {
+                if (!__all_sync(0xffffffffu, ok)) {
+                    failed = true;
+                    if (lane == 0) {
+                        fail(code);
+                    }
+                }
+                return !failed;
+            };
+            for (int item = itemBegin; item < itemEnd && !failed; ++item, ++n) {
+                const uint32_t acc = tmem + (n & 1) * PROJ_N;
+                if (n >= 2 && !wait(&misc.AccEmpty[n & 1], ((n >> 1) - 1) & 1, kDevTimeoutMma)) {
                     break;
                 }
-                TcFenceAfter();
-                if (ElectOne()) {
-                    const uint32_t sA = SmemAddr(smem + s * PROJ_STAGE_BYTES), sB = sA + PROJ_M * PROJ_KB;
+                for (int c = 0; c < a.Chunks; ++c) {
+                    if (!wait(&misc.Full[s], phase, kDevTimeoutTma)) {
+                        break;
+                    }
+                    TcFenceAfter();
+                    if (ElectOne()) {
+                        const uint32_t sA = SmemAddr(smem + s * STAGE_BYTES), sB = sA + PROJ_M * KB;
 #pragma unroll
-                    for (int ks = 0; ks < PROJ_KB / 32; ++ks) {
-                        const uint64_t aDesc = MakeSmemDesc(sA + ks * 32, 16, 8 * PROJ_KB, PROJ_KB);
-                        const uint64_t bDesc = MakeSmemDesc(sB + ks * 32, 16, 8 * PROJ_KB, PROJ_KB);
-                        MmaPairSS<X_E4M3>(acc, aDesc, bDesc, IDESC, (c > 0 || ks > 0) ? 1u : 0u);
+                        for (int ks = 0; ks < KB / 32; ++ks) {
+                            const uint64_t aDesc = MakeSmemDesc(sA + ks * 32, 16, 8 * KB, KB);
+                            const uint64_t bDesc = MakeSmemDesc(sB + ks * 32, 16, 8 * KB, KB);
+                            const uint32_t accumulate = (c > 0 || ks > 0) ? 1u : 0u;
+                            if constexpr (PAIR) {
+                                MmaPairSS<X_E4M3>(acc, aDesc, bDesc, IDESC, accumulate);
+                            } else if constexpr (X_E4M3) {
+                                MmaF8SS(acc, aDesc, bDesc, IDESC, accumulate);
+                            } else {
+                                MmaI8SS(acc, aDesc, bDesc, IDESC, accumulate);
+                            }
+                        }
+                        auto commit = [&](uint64_t *bar) {
+                            if constexpr (PAIR) {
+                                MmaCommitPair(bar);
+                            } else {
+                                MmaCommit(bar);
+                            }
+                        };
+                        commit(&misc.Empty[s]);
+                        if (c == a.Chunks - 1) {
+                            commit(&misc.AccFull[n & 1]);
+                        }
                     }
-                    MmaCommitPair(&misc.Empty[s]);
-                    if (c == a.Chunks - 1) {
-                        MmaCommitPair(&misc.AccFull[n & 1]);
+                    __syncwarp();
+                    ++issued;
+                    if (++s == a.Stages) {
+                        s = 0;
+                        phase ^= 1;
                     }
-                }
-                __syncwarp();
-                ++issued;
-                if (++s == a.Stages) {
-                    s = 0;
-                    phase ^= 1;
                 }
             }
-        }
-        if (lane < 2) {
-            StoreInPair(&misc.Issued, issued, lane);
-        }
+            if (lane < CTAS) {
+                store(&misc.Issued, issued, lane);
+            }
         }
         __syncwarp();
     } else {
@@ -444,13 +509,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
             TcFenceBefore();
             __syncwarp();
             if (lane == 0) {
-                ArriveInFirst(&misc.AccEmpty[n & 1]);
+                if constexpr (PAIR) {
+                    ArriveInFirst(&misc.AccEmpty[n & 1]);
+                } else {
+                    MbarArrive(&misc.AccEmpty[n & 1]);
+                }
             }
         }
     }
     TcFenceBefore();
     __syncthreads();
-    PairSync(); // neither CTA leaves while the other may still arrive on its barriers
+    if constexpr (PAIR) {
+        PairSync(); // neither CTA leaves while the other may still arrive on its barriers
+    }
     if (*(volatile int *)&misc.Abort) {
         // A wait ran out, which both CTAs see here.  What was started and nobody has waited for must not reach a CTA that has left: the
         // products issued, and copies of either CTA, all counted in the first one, that no product has waited for.
@@ -463,23 +534,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PROJ_THREADS, 1) Pro
                 WaitBar(&misc.AccFull[n & 1], (n >> 1) & 1, a.WaitCycles);
             }
             if (rank == 0) {
-                const int mine = misc.Requested[0], others = misc.Requested[1];
+                const int mine = misc.Requested[0], others = misc.Requested[CTAS - 1];
                 for (int k = issued; k < max(mine, others); ++k) {
                     uint64_t *bar = &misc.Full[k % a.Stages];
                     if (k >= mine) {
-                        MbarExpectTx(bar, PROJ_STAGE_BYTES); // the second CTA alone requested it
+                        MbarExpectTx(bar, STAGE_BYTES); // the second CTA alone requested it
                     } else if (k >= others) {
-                        MbarCompleteTx(bar, PROJ_STAGE_BYTES); // the first CTA alone
+                        MbarCompleteTx(bar, STAGE_BYTES); // the first CTA alone
                     }
                     WaitBar(bar, (k / a.Stages) & 1, a.WaitCycles);
                 }
             }
         }
         __syncthreads();
-        PairSync();
+        if constexpr (PAIR) {
+            PairSync();
+        }
     }
     if (warp == PROJ_MMA_WARP) {
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * PROJ_N) : "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * PROJ_N) : "memory");
+        } else {
+            TmemDealloc(tmem, 2 * PROJ_N);
+        }
     }
 }
 
@@ -513,14 +590,17 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     if (dst.ysize == 0) {
         return TSA_OK;
     }
+    const bool pair = dim >= ProjPairFrom(srcDtype == TSA_E4M3, dstDtype == TSA_F16 || dstDtype == TSA_BF16);
+    const int ctas = pair ? 2 : 1, kb = pair ? TProjShape<true>::KB : TProjShape<false>::KB;
+    const int stageBytes = pair ? TProjShape<true>::STAGE_BYTES : TProjShape<false>::STAGE_BYTES;
     CUtensorMap mx, mw;
     tsa_ptr2d xv = x;
     xv.ysize = len; // rows past len read as zeros
-    int rc = len > 0 ? MakeTileMapEx(&mx, xv, 1, PROJ_KB, PROJ_M, "x") : MakeTileMapEx(&mx, x, 1, PROJ_KB, PROJ_M, "x");
+    int rc = len > 0 ? MakeTileMapEx(&mx, xv, 1, kb, PROJ_M, "x") : MakeTileMapEx(&mx, x, 1, kb, PROJ_M, "x");
     if (rc == TSA_OK) {
         tsa_ptr2d wv = w;
         wv.ysize = outCols;
-        rc = MakeTileMapEx(&mw, wv, 1, PROJ_KB, PROJ_N / 2, "w");
+        rc = MakeTileMapEx(&mw, wv, 1, kb, PROJ_N / ctas, "w");
     }
     if (rc != TSA_OK) {
         return rc;
@@ -535,16 +615,15 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     a.Len = len;
     a.Rows = dst.ysize;
     a.HeadCount = headCount;
-    a.Chunks = (dim + PROJ_KB - 1) / PROJ_KB; // columns past the end read as zeros
+    a.Chunks = (dim + kb - 1) / kb; // columns past the end read as zeros
     a.ColTiles = (outCols + PROJ_N - 1) / PROJ_N;
-    a.Items = (dst.ysize + 2 * PROJ_M - 1) / (2 * PROJ_M) * a.ColTiles;
+    a.Items = (dst.ysize + ctas * PROJ_M - 1) / (ctas * PROJ_M) * a.ColTiles;
     // as many ring stages as fit beside the rope rows
     const int ropeBytes = rope.data ? PROJ_M * (headDim + 1) * (int)sizeof(float) : 0;
-    a.Stages = (PROJ_SMEM_MAX - 2048 - ropeBytes) / PROJ_STAGE_BYTES;
-    a.Stages = a.Stages < PROJ_MAX_STAGES ? a.Stages : PROJ_MAX_STAGES;
+    a.Stages = (PROJ_SMEM_MAX - 2048 - ropeBytes) / stageBytes; // at most PROJ_MAX_STAGES
     a.WaitCycles = TestHooks().WaitCycles > 0 ? TestHooks().WaitCycles : WAIT_CYCLES;
     a.WithholdChunk = TestHooks().WithholdTile;
-    const int smemBytes = a.Stages * PROJ_STAGE_BYTES + 1024 /* barriers */ + 1024 /* alignment */ + ropeBytes;
+    const int smemBytes = a.Stages * stageBytes + 1024 /* barriers */ + 1024 /* alignment */ + ropeBytes;
     int dev = 0, sms = 0;
     rc = CheckCuda(cudaGetDevice(&dev), "cudaGetDevice");
     if (rc == TSA_OK) {
@@ -555,9 +634,9 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     }
     const bool x8 = srcDtype == TSA_E4M3;
     const void *kern = nullptr;
-#define TSA_PROJ_CASE(DD, DT, X8)                                       \
-    if (headDim == DD && dstDtype == DT && x8 == X8) {                  \
-        kern = (const void *)ProjNormRopeKernel<DD, DT, X8>;            \
+#define TSA_PROJ_CASE(DD, DT, X8)                                                                                             \
+    if (headDim == DD && dstDtype == DT && x8 == X8) {                                                                        \
+        kern = pair ? (const void *)ProjNormRopeKernel<DD, DT, X8, true> : (const void *)ProjNormRopeKernel<DD, DT, X8, false>; \
     }
 #define TSA_PROJ_CASES(DD, X8) TSA_PROJ_CASE(DD, TSA_I8, X8) TSA_PROJ_CASE(DD, TSA_E4M3, X8) TSA_PROJ_CASE(DD, TSA_F16, X8) TSA_PROJ_CASE(DD, TSA_BF16, X8)
     TSA_PROJ_CASES(64, false)
@@ -571,5 +650,5 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
         return rc;
     }
     void *args[] = {&mx, &mw, &a, &statusWord};
-    return CheckCuda(LaunchPdl(kern, dim3(2 * (a.Items < sms / 2 ? a.Items : sms / 2)), dim3(PROJ_THREADS), smemBytes, (cudaStream_t)stream, args), "tsa_matmul_norm_rope_quant launch");
+    return CheckCuda(LaunchPdl(kern, dim3(ctas * (a.Items < sms / ctas ? a.Items : sms / ctas)), dim3(PROJ_THREADS), smemBytes, (cudaStream_t)stream, args, ctas), "tsa_matmul_norm_rope_quant launch");
 }

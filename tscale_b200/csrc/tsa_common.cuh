@@ -221,18 +221,23 @@ __device__ __forceinline__ void PdlTrigger()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-inline cudaError_t LaunchPdl(const void *kern, dim3 grid, dim3 block, size_t smemBytes, cudaStream_t stream, void **args)
+// cluster: CTAs of a thread-block cluster, side by side in x
+inline cudaError_t LaunchPdl(const void *kern, dim3 grid, dim3 block, size_t smemBytes, cudaStream_t stream, void **args, unsigned cluster = 1)
 {
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = grid;
     lc.blockDim = block;
     lc.dynamicSmemBytes = smemBytes;
     lc.stream = stream;
     lc.attrs = attr;
-    lc.numAttrs = 1;
+    lc.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelExC(&lc, kern, args);
 }
 
