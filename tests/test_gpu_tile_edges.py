@@ -47,11 +47,21 @@ def test_fwd_half_tiles(length, d, qk_dtype, v_dtype, slope):
 
 
 @pytest.mark.parametrize("step", [-0.05, 0.02, 0.11, 3.0])   # log2 units from key to key: no raise, one now and then, one per group, one per key
-@pytest.mark.parametrize("d,qk_dtype,window", [(64, "e4m3", 0), (128, "e4m3", 0), (128, "i8", 0), (64, "i8", 200)])
-def test_fwd_rising_logits(step, d, qk_dtype, window):
+@pytest.mark.parametrize("d,qk_dtype,v_dtype,window,slope,form", [
+    (64, "e4m3", "e4m3", 0, 0.0, "plain"), (128, "e4m3", "e4m3", 0, 0.0, "plain"), (128, "i8", "e4m3", 0, 0.0, "plain"),
+    (64, "i8", "e4m3", 200, 0.0, "plain"), (64, "e4m3", "e4m3", 0, 0.01, "plain"), (64, "i8", "i8", 0, 0.0, "plain"),
+    (64, "e4m3", "e4m3", 0, 0.0, "to"), (128, "i8", "e4m3", 0, 0.01, "to"), (64, "i8", "e4m3", 200, 0.0, "to"),
+    (64, "e4m3", "e4m3", 0, 0.01, "kv"), (128, "i8", "e4m3", 0, 0.0, "kv"),
+])
+def test_fwd_rising_logits(step, d, qk_dtype, v_dtype, window, slope, form):
     """Logits that rise along the keys: the reference moves in full halves and in masked blocks, first groups and later ones, and the
-    weights formed in front of the vote have to be formed again.  A weight is rounded to three mantissa bits at worst, a relative
-    error of 2^-4, and so is the output at most; the sum of the weights is not rounded."""
+    weights formed in front of the vote have to be formed again.  Also with int8 values, with two further destinations and with the
+    fused consumer, which are kernels of their own.
+
+    The values are positive, so that an output is bounded by its own size.  P = 128 w sv / svRef is rounded to e4m3: by 2^-4 of itself at
+    most, or by 2^-10 where it is subnormal (svRef, the power of two at or above the scales, is 2); with int8 values the residual takes all
+    but 2^-4 of that away again, or down to 2^-10.  2^-10 stands for 2^-17 svRef in the sum of w v.  A block that is shrunk again is rounded
+    once more, on what the residual left (2^-8).  The sum of the weights is not rounded; a bf16 output by 2^-9."""
     from tscale_b200 import abi, ops
     rows, heads = 420, 2
     c = 0.5 / np.sqrt(d) / 0.693147
@@ -60,26 +70,41 @@ def test_fwd_rising_logits(step, d, qk_dtype, window):
     sk = (torch.arange(rows, dtype=torch.float64) * step / (d * c)).to(torch.float32).expand(heads, rows).contiguous()
     sq = torch.ones(heads, rows)
     gen = torch.Generator().manual_seed(60)
-    v8 = torch.randn(rows, heads * d, generator=gen).to(torch.float8_e4m3fn)
+    if v_dtype == "e4m3":
+        v8 = (torch.randn(rows, heads * d, generator=gen).abs() + 0.25).to(torch.float8_e4m3fn)
+    else:
+        v8 = torch.randint(1, 128, (rows, heads * d), generator=gen, dtype=torch.int8)
     sv = torch.rand(heads, rows, generator=gen) + 0.5
-    cfg = ops.make_cfg(qk_dtype, "e4m3", d, d, out_dtype=torch.float32)
+    out_dtype = torch.bfloat16 if form == "kv" else torch.float32
+    cfg = ops.make_cfg(qk_dtype, v_dtype, d, d, out_dtype=out_dtype)
     ws = torch.empty(max(1, abi.lib().tsa_att_fwd_workspace_bytes(cfg, heads, rows)), dtype=torch.uint8, device=DEV)
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
-    out, lse = ops.att_fwd(cfg, q8, q8, v8.view(torch.uint8).to(DEV), sk.to(DEV), ops.Mask.window([rows], window), 0.0, heads, qk_scale=sq.to(DEV),
-                           v_scale=sv.to(DEV), workspace=ws, status=status)
+    copies = [torch.zeros(rows, heads * d, dtype=out_dtype, device=DEV) for _ in range(2)] if form == "to" else None
+    comb = torch.ones(rows, heads * d, dtype=torch.bfloat16, device=DEV) if form == "kv" else None
+    out, lse, *kv = ops.att_fwd(cfg, q8, q8, v8.view(torch.uint8).to(DEV), sk.to(DEV), ops.Mask.window([rows], window), slope, heads,
+                                qk_scale=sq.to(DEV), v_scale=sv.to(DEV), workspace=ws, status=status, out_copies=copies, combiner_k=comb)
     torch.cuda.synchronize()
     assert int(status.item()) == 0
     i = torch.arange(rows)
     seen = (i[None, :] < i[:, None]) & ((i[None, :] >= i[:, None] - window) if window else True)
-    z = (sk[0].double() * d * c).expand(rows, rows).masked_fill(~seen, -np.inf)
+    z = ((sk[0].double() * d * c).expand(rows, rows) - slope * (i[:, None] - i[None, :])).masked_fill(~seen, -np.inf)
     m = z.amax(1, keepdim=True).clamp_min(0)
     w = torch.exp2(z - m)
     total = w.sum(1, keepdim=True) + torch.exp2(-m)
-    v = v8.double().view(rows, heads, d) * sv.t().double()[:, :, None]
-    want = torch.einsum("ij,jhd->ihd", w / total, v).reshape(rows, heads * d)
+    v = v8.double().view(rows, heads, d)
+    want = torch.einsum("ij,jhd->ihd", w / total, v * sv.t().double()[:, :, None])
+    bound = (2.0 ** -4 + 2.0 ** -8 if v_dtype == "e4m3" else 2.0 ** -8 + 2.0 ** -8) * want
+    bound += 2.0 ** -17 * 2 * torch.einsum("ij,jhd->ihd", seen.double() / total, v)
+    if form == "kv":
+        bound += 2.0 ** -9 * want
+    err = (out.cpu().double().view(rows, heads, d) - want).abs()
+    assert (err <= bound).all(), float((err / bound.clamp_min(1e-30)).max())
     want_lse = (m + torch.log2(total))[:, 0]
-    assert (out.cpu().double() - want).abs().max() <= 2.0 ** -4 * v.abs().max()
     assert ((lse.cpu().double() - want_lse).abs() <= 2e-5 + 1e-6 * want_lse.abs()).all()
+    for copy in copies or []:
+        assert torch.equal(copy, out)
+    if kv:   # keys of one: each of the four blocks is the output
+        assert torch.equal(kv[0].view(rows, heads, 4, d), out.view(rows, heads, 1, d).expand(-1, -1, 4, -1))
 
 
 @pytest.mark.parametrize("length,heads", [(1, 1), (129, 3), (391, 2), (2200, 10)])   # the last: more items than CTAs
