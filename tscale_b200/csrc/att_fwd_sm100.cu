@@ -21,7 +21,7 @@
 //              against the reference m it already holds.  Only when a score exceeds m by more than the e4m3 headroom
 //              (weights up to 2^8.75 < 448) does the warp first raise m and shrink O and the sum.  The run has no branch
 //              or vote inside, so loads, exponentials, conversions and stores of a half overlap, and its first weights are
-//              formed in front of the vote (FW_EARLY).  16 documents of 4096 rows, 12 heads x 64, no window: 836 us with 16
+//              formed in front of the vote (TFwdTune).  16 documents of 4096 rows, 12 heads x 64, no window: 836 us with 16
 //              columns and a vote at a time, 712 with halves, 659 with early weights.
 //              Tiles the span mask cuts through add a second e4m3 residual term (P split into
 //              e4m3(P) + e4m3(P - e4m3(P)), two MMAs), which removes the 3-bit-mantissa rounding where it is not
@@ -58,11 +58,27 @@ constexpr int Q_SLOTS = 2;
 // a weight is 2^t with t = z - m + 7; e4m3 holds up to 448 = 2^8.8, so t may reach 8.75 before m has to move
 constexpr float P_HEADROOM = 8.75f;
 
-// Weights formed before the outcome of the vote on a group's maximum is known, of the 64 of a half and of the 32 of a masked block.
-// Full-causal / window-64 layer (16 documents of 4096 rows, 12 heads x 64) without any: 712 / 113.1 us; 8: 699; 16: 676; 24 or 32 and 16:
-// 662 / 111.6; 48 spills: 688; 40 and 32: 673 / 115.0.  Full-causal 131072 rows x 32 x 128: 27.4 -> 26.2 ms until the power limit holds
-// the clock down, 27.4 behind it.  Rows that raise often form them twice: the short training block loses the 1 % again.
-constexpr int FW_EARLY = 24, FW_EARLY_MASKED = 16;
+// Weights formed before the outcome of the vote on a group's maximum is known, of the 64 of a half and of the 32 of a masked block, and
+// the columns of O that a rescale takes at a time.  Full-causal / window-64 layer (16 documents of 4096 rows, 12 heads x 64) without any
+// early weight: 712 / 113.1 us; 8: 699; 16: 676; 24 or 32 and 16: 662 / 111.6; 48 spills: 688; 40 and 32: 673 / 115.0.  Full-causal 131072
+// rows x 32 x 128: 27.4 -> 26.2 ms until the power limit holds the clock down, 27.4 behind it.  Rows that raise often form them
+// twice: the short training block loses the 1 % again.
+// The instances with a lower register limit were measured by themselves (us): with no early weights and a rescale in steps of 8, then with
+// 24, 16, 32 (FORWARD: 104 to 172 bytes of spills at its 128 registers, KV: 26 to 58 at 168), then FORWARD with 16, 16, 8 (none in
+// twelve of the sixteen instances, 40 bytes at most):
+//     layer                                                        FORWARD, three destinations       KV
+//     4 x 4096 rows, 12 x 64, e4m3, full-causal                    302 / 279 / 271                   307 / 276
+//     16 x 4096, 12 x 64, e4m3, window 64                          273 / 264 / 236                   325 / 304
+//     2 x 8192, 16 x 128, e4m3, window 1024, ALiBi                 210 / 242 / 197                   267 / 258
+//     8192, 16 x 128, e4m3, full-causal                            356 / 335 / 328                   356 / 333
+//     8192, 16 x 128, int8, full-causal, logits of a third         328 / 336 / 316                   344 / 329
+//     8192, 16 x 128, int8, full-causal                            384 / 379 / 383                   409 / 376
+//     443 + 2000 + 999, 12 x 64, int8, window 512, ALiBi, wide     58.4 / 54.4 / 55.1                58.0 / 50.7
+// KV keeps the plain kernel's: without spills (steps of 8) the first, second, fourth, fifth and last take 280, 297, 338, 318, 52.7.
+template <bool FORWARD>
+struct TFwdTune {
+    static constexpr int EARLY = FORWARD ? 16 : 24, EARLY_MASKED = 16, RESCALE = FORWARD ? 8 : 32;
+};
 
 enum { RF_FIRST = 1, RF_LAST = 2, RF_END = 4 };
 
@@ -196,37 +212,57 @@ __device__ __forceinline__ void TmemStore8(uint32_t taddr, const uint32_t *r)
 // alpha = 2^-d: the O accumulator (D columns) and this tile's e4m3 weights that are in tensor memory and not yet handed to the MMA:
 // none, or those of one 32-key block (storedBlock >= 0), weights in columns [32b, 32b + 8), residuals in [32b + 8, 32b + 16).  All lanes
 // of the warp execute the tensor-memory accesses; a lane whose row needs no change passes alpha = 1.  Kept out of line: inlined it
-// costs the common path registers.  32 columns at a time: with 8 the round trips to tensor memory took four times as long, and rows
-// whose scores spread (queries and keys of unit variance) come here in most of their first tiles.
-template <int D>
+// costs the common path registers.  With 8 columns at a time the round trips to tensor memory take four times as long as with 32, and rows
+// whose scores spread (queries and keys of unit variance) come here in most of their first tiles; the registers of 32 are the caller's to save.
+template <int D, int STEP>
 __device__ __noinline__ void ShrinkAccumulated(uint32_t tLane, float alpha, int hasO, int storedBlock)
 {
+    static_assert(STEP == 8 || STEP == 32, "columns at a time");
     TmemWaitSt(); // the weights stored so far have landed
     if (hasO) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < D; c0 += 32) {
-            uint32_t o[32];
-            TmemLoad32(tLane + TMEM_O_COL + c0, o);
-            TmemWait32(o);
+        for (int c0 = 0; c0 < D; c0 += STEP) {
+            uint32_t o[STEP];
+            if constexpr (STEP == 32) {
+                TmemLoad32(tLane + TMEM_O_COL + c0, o);
+                TmemWait32(o);
+            } else {
+                TmemLd8(tLane + TMEM_O_COL + c0, o);
+                TmemWaitLd();
+            }
 #pragma unroll
-            for (int c = 0; c < 32; ++c) {
+            for (int c = 0; c < STEP; ++c) {
                 o[c] = __float_as_uint(__uint_as_float(o[c]) * alpha);
             }
-            TmemSt32(tLane + TMEM_O_COL + c0, o);
+            if constexpr (STEP == 32) {
+                TmemSt32(tLane + TMEM_O_COL + c0, o);
+            } else {
+                TmemStore8(tLane + TMEM_O_COL + c0, o);
+            }
         }
     }
     if (storedBlock >= 0) {
         const __half2 ah = __float2half2_rn(alpha);
         const uint32_t ah2 = *reinterpret_cast<const uint32_t *>(&ah);
-        uint32_t w[16];
-        TmemLd16(tLane + 32 * storedBlock, w);
-        TmemWaitLd();
+        constexpr int W = STEP < 16 ? STEP : 16; // weights and residuals at once, or one after the other
+#pragma unroll 1
+        for (int c0 = 0; c0 < 16; c0 += W) {
+            uint32_t w[W];
+            if constexpr (W == 16) {
+                TmemLd16(tLane + 32 * storedBlock, w);
+            } else {
+                TmemLd8(tLane + 32 * storedBlock + c0, w);
+            }
+            TmemWaitLd();
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-            w[c] = ScaleE4M3x4(w[c], ah2);
+            for (int c = 0; c < W; ++c) {
+                w[c] = ScaleE4M3x4(w[c], ah2);
+            }
+#pragma unroll
+            for (int c = 0; c < W; c += 8) {
+                TmemStore8(tLane + 32 * storedBlock + c0 + c, w + c);
+            }
         }
-        TmemStore8(tLane + 32 * storedBlock, w);
-        TmemStore8(tLane + 32 * storedBlock + 8, w + 8);
     }
     TmemWaitSt();
 }
@@ -267,6 +303,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
     TFwdParams p)
 {
     using SM = TFwdSmem<D, V_I8>;
+    using TUNE = TFwdTune<FORWARD>;
     constexpr int NV = SM::NV;
     constexpr int STAGES = SM::STAGES;
     constexpr int SWZ = (D == 128) ? 128 : 64;
@@ -948,13 +985,14 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                 float eoff = rowOff - m + 7.0f;
 
                 // the reference moves up by d whole units: everything accumulated so far shrinks by 2^-d, and the W logits in s
-                // drop by d.  storedQuads: 16-key groups of this tile whose weights are in tensor memory.
+                // drop by d.  storedQuads: 16-key groups of this tile whose weights are in tensor memory; of those not yet handed over there is
+                // one block of 32 keys (the first of a masked half, when its second one raises) or none.
                 auto raise = [&](float mxc, int storedQuads, uint32_t *s, auto widthTag) {
                     constexpr int W = decltype(widthTag)::value;
                     const float d = (mxc > headroom) ? floorf(mxc - 7.0f) : 0.0f;
                     const float alpha = exp2f(-d);
                     // the group voted on is the next one to be stored: it lies in half storedQuads / 4, whose earlier
-                    // quads are still this thread's; O holds something once a PV group of this item has been enabled,
+                    // block, if there is one, is still this thread's; O holds something once a PV group of this item has been enabled,
                     // and may be touched once the last enabled group has retired
                     const int firstQuad = storedQuads & ~3;
                     const bool oLive = hasO || firstQuad > 0;
@@ -969,7 +1007,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                         }
                         TcFenceAfter();
                     }
-                    ShrinkAccumulated<D>(tLane, alpha, oLive ? 1 : 0, storedQuads > firstQuad ? firstQuad >> 1 : -1);
+                    ShrinkAccumulated<D, TUNE::RESCALE>(tLane, alpha, oLive ? 1 : 0, storedQuads > firstQuad ? firstQuad >> 1 : -1);
                     lacc2.x *= alpha;
                     lacc2.y *= alpha;
                     m += d;
@@ -1026,7 +1064,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                     float mx = scaleGroup(s, h * 64, -INFINITY, TW32());
                     TmemWait32(s + 32);
                     mx = scaleGroup(s + 32, h * 64 + 32, mx, TW32());
-                    float early[FW_EARLY];
+                    float early[TUNE::EARLY];
                     earlyWeights(s, early);
                     if (__any_sync(0xffffffffu, mx > headroom)) {
                         raise(mx, h * 4, s, TW64());
@@ -1035,7 +1073,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
 #pragma unroll
                     for (int c = 0; c < 64; c += 4) {
                         float2 e[2];
-                        weighQuad(s + c, h * 64 + c, e, c < FW_EARLY ? early + c : nullptr);
+                        weighQuad(s + c, h * 64 + c, e, c < TUNE::EARLY ? early + c : nullptr);
                         pk[c >> 2] = PackE4M3x4(e[0].x, e[0].y, e[1].x, e[1].y);
                         if (c == 28) {
                             TmemStore8(cols, pk);
@@ -1069,7 +1107,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
                                 s[c] = __float_as_uint(tt.x);
                                 s[c + 1] = __float_as_uint(tt.y);
                             }
-                            float early[FW_EARLY_MASKED];
+                            float early[TUNE::EARLY_MASKED];
                             earlyWeights(s, early);
                             if (__any_sync(0xffffffffu, mx > headroom)) {
                                 raise(mx, blk * 2, s, TW32());
@@ -1078,7 +1116,7 @@ __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) 
 #pragma unroll
                             for (int c = 0; c < 32; c += 4) {
                                 float2 e[2];
-                                weighQuad(s + c, blk * 32 + c, e, c < FW_EARLY_MASKED ? early + c : nullptr);
+                                weighQuad(s + c, blk * 32 + c, e, c < TUNE::EARLY_MASKED ? early + c : nullptr);
                                 const uint32_t hi4 = PackE4M3x4(e[0].x, e[0].y, e[1].x, e[1].y);
                                 pk[c >> 2] = hi4;
                                 pl[c >> 2] = ResidualE4M3x2(e[0].x, e[0].y, hi4 & 0xffff) | (ResidualE4M3x2(e[1].x, e[1].y, hi4 >> 16) << 16);
