@@ -205,8 +205,9 @@ int tsa_att_fwd_set_score_dump(int32_t *dst, int head, int queryTile, int keyTil
  * arrives on, and must come back with 0x10 in *statusWord; tsa_selftest_fwd_withhold_copy makes the following
  * tsa_att_fwd calls (tensor-core path) wait at most waitCycles cycles per barrier and leave out the copy of every CTA's
  * withholdTile-th key tile, so the forward must notice, drain its other copies, free its tensor memory and return with
- * the time-out bits set, and the following tsa_matmul_norm_rope_quant calls likewise with the withholdTile-th chunk of x of
- * every CTA (of a pair the second one), and the following tsa_att_bwd calls with the announcement of the factors of every CTA's withholdTile-th tile (waitCycles = 0, withholdTile = -1 restores production behaviour).  Process-wide, for tests. */
+ * the time-out bits set.  The following tsa_matmul_norm_rope_quant calls do likewise with the withholdTile-th chunk of x of
+ * every CTA (of a pair the second one), the following tsa_att_bwd calls with the announcement of the factors of every CTA's
+ * first (0) or second (1) tile.  waitCycles = 0, withholdTile = -1 restores production behaviour.  Process-wide, for tests. */
 int tsa_status_from_word(int statusWord);
 int tsa_selftest_bounded_wait(long long limitCycles, int *statusWord, tsa_stream_t stream);
 int tsa_selftest_fwd_withhold_copy(long long waitCycles, int withholdTile);

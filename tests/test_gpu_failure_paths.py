@@ -116,7 +116,7 @@ def test_projection_with_a_withheld_copy_times_out_cleanly_and_recovers(dim, row
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
-@pytest.mark.parametrize("tile", [0, 3])
+@pytest.mark.parametrize("tile", [0, 1])
 def test_backward_with_withheld_column_factors_times_out_cleanly_and_recovers(tile):
     """The factors of a tile's columns are never announced: the warp whose wait runs out first reports it and stops the others.  Left
     to themselves the other warps and the MMA warps would each run out their own production bound of about a second."""
