@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
             for (int o = 0; o < OUTPUTS; ++o) {
 #pragma unroll
                 for (int c = 0; c < QUARTER_D; c += 8) {
-                    TmemStN<8>(tLane + BWD_OUT_COL + o * D + quarter * QUARTER_D + c, zero);
+                    TmemSt8(tLane + BWD_OUT_COL + o * D + quarter * QUARTER_D + c, zero);
                 }
             }
             TmemWaitSt();
@@ -644,9 +644,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) BwdSm100Kernel(const __grid_co
                         }
                     }
                     // 16 bf16 values = 8 columns, written over the first half of the 16 columns this thread has just read
-                    TmemStN<8>(tLane + BWD_S_COL + cb, a1);
+                    TmemSt8(tLane + BWD_S_COL + cb, a1);
                     if (MODE_DKV) {
-                        TmemStN<8>(tLane + BWD_DP_COL + cb, a2);
+                        TmemSt8(tLane + BWD_DP_COL + cb, a2);
                     }
                     TmemWaitSt();
                     TcFenceBefore();

@@ -201,7 +201,7 @@ __device__ __forceinline__ float PinnedExp2(float x)
     asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// eight columns of this thread's lane, without the memory clobber of TmemStN
+// eight columns of this thread's lane, without the memory clobber of TmemSt8
 __device__ __forceinline__ void TmemStore8(uint32_t taddr, const uint32_t *r)
 {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),

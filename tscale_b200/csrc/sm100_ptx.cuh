@@ -29,11 +29,6 @@ __device__ __forceinline__ void MbarExpectTx(uint64_t *bar, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(SmemAddr(bar)), "r"(bytes) : "memory");
 }
-// adds to the transaction count of the current phase without arriving (the arrival follows separately)
-__device__ __forceinline__ void MbarExpectTxOnly(uint64_t *bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(SmemAddr(bar)), "r"(bytes) : "memory");
-}
 // one poll with the default (short) suspend time: for the thread whose wake-up latency is on the critical path
 __device__ __forceinline__ bool MbarTryWaitFast(uint64_t *bar, uint32_t parity)
 {
@@ -48,17 +43,6 @@ __device__ __forceinline__ bool MbarTryWaitFast(uint64_t *bar, uint32_t parity)
         : "r"(SmemAddr(bar)), "r"(parity)
         : "memory");
     return ok != 0;
-}
-// register reallocation between the warpgroups of a CTA (all four warps of the warpgroup execute it)
-template <int N>
-__device__ __forceinline__ void RegDealloc()
-{
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
-}
-template <int N>
-__device__ __forceinline__ void RegAlloc()
-{
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
 }
 // upper bound, in nanoseconds, for which one try_wait may keep the thread suspended before it returns false
 constexpr uint32_t kTryWaitHintNs = 200000;
@@ -253,19 +237,6 @@ __device__ __forceinline__ void MmaI8SS(uint32_t dTmem, uint64_t aDesc, uint64_t
         : "r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void MmaF8TS(uint32_t dTmem, uint32_t aTmem, uint64_t bDesc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t"
-        "}"
-        :
-        : "r"(dTmem), "r"(aTmem), "l"(bDesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 // bf16 operands, f32 accumulation
 __device__ __forceinline__ void MmaF16SS(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate)
 {
@@ -277,18 +248,6 @@ __device__ __forceinline__ void MmaF16SS(uint32_t dTmem, uint64_t aDesc, uint64_
         "}"
         :
         : "r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void MmaF16TS(uint32_t dTmem, uint32_t aTmem, uint64_t bDesc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-        "}"
-        :
-        : "r"(dTmem), "r"(aTmem), "l"(bDesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // ---- grouped issue -----------------------------------------------------------------------------
