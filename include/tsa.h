@@ -275,7 +275,7 @@ int tsa_kv_product_bwd(int inDtype, int gradDtype, tsa_ptr2d k, tsa_ptr2d valLoo
  * bit for bit what tsa_kv_product(bf16, bf16) gives on the stored output.  The thread that rounds a row of the output to
  * bf16 multiplies it with the row of combiner keys (prefetched into L2 while the block is computed) and stores the four
  * products with streaming 32-byte stores, so the stand-alone kernel's launch and its re-read of the output go away.
- * Measured on B200 the two calls it replaces are as fast or faster (the forward is bound by the instruction issue of
+ * Measured on B200 the two calls it replaces are faster (the forward is bound by the instruction issue of
  * the threads that would do this work, the stand-alone product by memory bandwidth, which it reaches): prefer them
  * where speed decides.  combinerK bf16 [>= len][>= H*D], kv bf16 [>= len][>= 4*H*D],
  * both 16-byte aligned; out dtype bf16, e4m3 values, head size 64 or 128 (otherwise TSA_UNSUPPORTED: call tsa_att_fwd
