@@ -293,10 +293,10 @@ __device__ __forceinline__ int ValueScaleExponent(float x)
 // KV: the epilogue also forms the consumer's input (the reference's KVProduct) from the row it has just rounded to bf16.
 // Measured against the two launches it replaces (attention, then the stand-alone product, which streams at 0.94 of the copy
 // bandwidth): slower on a full-causal layer of 16 x 4096 x 12 x 64 (0.783 against 0.752 ms), on the window-64 layer (0.232 against
-// 0.200 ms) and on 32768 x 16 x 128 (3.80 against 3.69 ms).  A kernel that carries this code runs its hot
-// loop 6-7 % slower even when none of the consumer's memory accesses execute, and the same held for the two other forms
-// that were built (0.231 / 0.941 / 3.95 ms the one that stayed, then): the products as a pass of their own that reads the stored row back from L2 (same register count as the
-// plain kernel; 0.290 / 0.949 / 3.99 ms) and a seventh warp that takes finished blocks from L2 (0.271 / 1.075 / 4.00 ms).
+// 0.200 ms) and on 32768 x 16 x 128 (3.80 against 3.69 ms).  A kernel that carries this code runs its hot loop 6-7 % slower even
+// when none of the consumer's memory accesses execute, and the same held for the two other forms that were built beside this one
+// (0.231 / 0.941 / 3.95 ms then): the products as a pass of their own that reads the stored row back from L2 (same register
+// count as the plain kernel; 0.290 / 0.949 / 3.99 ms) and a seventh warp that takes finished blocks from L2 (0.271 / 1.075 / 4.00 ms).
 template <int D, bool QK_I8, bool HAS_VSCALE, bool HAS_ALIBI, bool V_I8, bool FORWARD = false, bool KV = false>
 __global__ void __launch_bounds__(FORWARD ? FW_THREADS_FORWARD : FW_THREADS, 2) FwdSm100Kernel(const __grid_constant__ CUtensorMap tmQ,
     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmV2,
