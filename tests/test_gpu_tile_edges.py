@@ -178,7 +178,8 @@ def test_projection_pairs(dst, rows, dim, heads, d):
 @pytest.mark.parametrize("dst", ["i8", torch.bfloat16])
 @pytest.mark.parametrize("rows,length,dim,heads,d", [
     (1, 1, 1344, 1, 64), (128, 128, 1344, 1, 128), (129, 128, 1280, 3, 64), (256, 200, 1344, 5, 64), (385, 385, 1408, 2, 128),
-    (300, 300, 1024, 4, 64), (300, 300, 1088, 4, 64), (300, 300, 1216, 4, 64),   # on both sides of the lines between single CTAs and pairs
+    # on both sides of the lines between single CTAs and pairs: the inner size, and one tile of 128 x 256 for each of 148 SMs or one more
+    (300, 300, 960, 4, 64), (300, 300, 1024, 4, 64), (18944, 18900, 1024, 4, 64), (18945, 18945, 1024, 4, 64), (18945, 18945, 1088, 4, 64),
 ])
 def test_projection_pair_tiles(dst, rows, length, dim, heads, d):
     """Tiles of 256 rows x 256 columns shared by two CTAs, 128 columns of x at a time: a second CTA without rows, half or all of

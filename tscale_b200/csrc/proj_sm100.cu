@@ -32,14 +32,15 @@ constexpr int PROJ_LOAD_WARP = 0, PROJ_MMA_WARP = 1, PROJ_EPI_WARPS = 8;
 constexpr int PROJ_EPI_THREADS = PROJ_EPI_WARPS * 32, PROJ_THREADS = PROJ_EPI_THREADS + 64;
 constexpr int PROJ_SMEM_MAX = 227 * 1024;
 
-// The inner size from which on pairs are taken: below, tiles of single CTAs were faster at some number of rows (1 to 131072), from there on
+// Whether pairs are taken.  Below these inner sizes tiles of single CTAs were faster at some number of rows (1 to 131072), from there on
 // pairs were as fast or faster at all of them.  The longer a tile's epilogue (16-bit results are twice the bytes), the later.  Single ->
 // pair, 32768 rows without rope: int8 to e4m3 30.2 -> 32.1 us (768 -> 12 x 64), 40.6 -> 39.2 (1024 -> 16 x 64), 133 -> 105 (2048 -> 16 x 128);
 // int8 to bf16 35.6 -> 37.8, 44.0 -> 47.0, 61.5 -> 59.1 (1280 -> 20 x 64), 147 -> 120; e4m3 to int8 with rope 37.2 -> 39.4, 49.8 -> 51.2,
-// 62.0 -> 60.8 (1152 -> 18 x 64), 167 -> 149.
-inline int ProjPairFrom(bool srcE4M3, bool dst16)
+// 62.0 -> 60.8 (1152 -> 18 x 64), 167 -> 149.  With no more tiles than SMs no epilogue waits for another one, and pairs win from 1024 on
+// (128 rows, 1024 -> 16 x 64: 10.5 -> 10.1 us to bf16, 11.6 -> 11.3 from e4m3).
+inline bool ProjInPairs(int dim, bool srcE4M3, bool dst16, long long singleTiles, int sms)
 {
-    return dst16 ? 1280 : srcE4M3 ? 1152 : 1024;
+    return dim >= (dst16 ? 1280 : srcE4M3 ? 1152 : 1024) || (dim >= 1024 && singleTiles <= sms);
 }
 // what a CTA copies of a chunk: PROJ_M rows of x, W_ROWS of w, KB columns of both
 template <bool PAIR>
@@ -55,6 +56,7 @@ constexpr int PROJ_MAX_STAGES = (PROJ_SMEM_MAX - 2048) / TProjShape<false>::STAG
 struct TProjMisc {
     uint64_t Full[PROJ_MAX_STAGES], Empty[PROJ_MAX_STAGES]; // ring: in the first CTA: the copies of both landed / MMAs that read them retired (both CTAs)
     uint64_t AccFull[2], AccEmpty[2];                       // accumulator set complete (both CTAs) / in the first CTA: read out, an arrival per epilogue warp of both
+    uint64_t Drained;                                       // a wait ran out: the products issued have retired (both CTAs)
     uint32_t TmemBase;
     int Abort;        // a bounded wait ran out somewhere in the pair (both CTAs)
     int Requested[2]; // in the first CTA: chunks whose copies either one's loader has requested
@@ -179,6 +181,69 @@ struct TProjArgs {
     int WithholdChunk;
 };
 
+// `value` into the word of one of the pair's CTAs
+template <bool PAIR>
+__device__ __forceinline__ void ProjStore(int *word, int value, int toRank)
+{
+    if constexpr (PAIR) {
+        StoreInPair(word, value, toRank);
+    } else {
+        *(volatile int *)word = value;
+    }
+}
+// What happens when a wait runs out is out of line: a CTA runs most of its code once, and every instruction of it has to be fetched.  Written
+// out, these two functions cost 0.3 to 0.5 us of a launch that takes 8 to 12.
+template <bool PAIR>
+__device__ __noinline__ void ProjFail(TProjMisc &misc, int *status, int code)
+{
+    for (int r = 0; r < TProjShape<PAIR>::CTAS; ++r) {
+        ProjStore<PAIR>(&misc.Abort, 1, r);
+    }
+    if (status) {
+        atomicOr(status, code);
+    }
+}
+// All threads of the pair.  What was started and nobody has waited for must not reach a CTA that has left: the products issued, the commits
+// behind them, and copies of either CTA, all counted in the first one, that no product has waited for.
+template <bool PAIR>
+__device__ __noinline__ void ProjDrain(TProjMisc &misc, int stages, int chunks, long long waitCycles, int rank, int refilled)
+{
+    using SH = TProjShape<PAIR>;
+    if (rank == 0 && (threadIdx.x >> 5) == PROJ_MMA_WARP && ElectOne()) { // the lane that issued the products
+        if constexpr (PAIR) {
+            MmaCommitPair(&misc.Drained);
+        } else {
+            MmaCommit(&misc.Drained);
+        }
+    }
+    if (threadIdx.x == PROJ_LOAD_WARP * 32) {
+        const int issued = misc.Issued, freed = min(issued, max(refilled, 0)), tiles = issued / chunks;
+        WaitBar(&misc.Drained, 0, waitCycles);
+        for (int k = max(0, freed - stages); k < freed; ++k) {
+            WaitBar(&misc.Empty[k % stages], (k / stages) & 1, waitCycles);
+        }
+        for (int n = max(0, tiles - 2); n < tiles; ++n) {
+            WaitBar(&misc.AccFull[n & 1], (n >> 1) & 1, waitCycles);
+        }
+        if (rank == 0) {
+            const int mine = misc.Requested[0], others = misc.Requested[SH::CTAS - 1];
+            for (int k = issued; k < max(mine, others); ++k) {
+                uint64_t *bar = &misc.Full[k % stages];
+                if (k >= mine) {
+                    MbarExpectTx(bar, SH::STAGE_BYTES); // the second CTA alone requested it
+                } else if (k >= others) {
+                    MbarCompleteTx(bar, SH::STAGE_BYTES); // the first CTA alone
+                }
+                WaitBar(bar, (k / stages) & 1, waitCycles);
+            }
+        }
+    }
+    __syncthreads();
+    if constexpr (PAIR) {
+        PairSync();
+    }
+}
+
 // X_E4M3: both operands are e4m3 bytes (MulForwardFp8, gpt_cuda.cu:488-491), products accumulate in f32 on the tensor
 // cores (kind::f8f6f4); otherwise int8 x int8 with exact int32 accumulators (kind::i8).
 // DST: TSA_I8, TSA_E4M3 (quantised) or TSA_F16 / TSA_BF16 (the normalised, rotated values themselves: the reference's K16).
@@ -207,6 +272,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
             MbarInit(&misc.AccFull[b], 1);
             MbarInit(&misc.AccEmpty[b], CTAS * PROJ_EPI_WARPS);
         }
+        MbarInit(&misc.Drained, 1);
         misc.Abort = 0;
         FenceBarrierInit();
     }
@@ -229,23 +295,10 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
     PdlTrigger(); // behind the allocation: a CTA of the next kernel may hold tensor memory of this SM from here on
     PdlWait();
     const int *abortFlag = &misc.Abort;
-    auto store = [&](int *word, int value, int toRank) {
-        if constexpr (PAIR) {
-            StoreInPair(word, value, toRank);
-        } else {
-            *(volatile int *)word = value;
-        }
-    };
-    auto fail = [&](int code) {
-        for (int r = 0; r < CTAS; ++r) {
-            store(&misc.Abort, 1, r);
-        }
-        if (status) {
-            atomicOr(status, code);
-        }
-    };
+    auto fail = [&](int code) { ProjFail<PAIR>(misc, status, code); };
     const int pair = blockIdx.x / CTAS, pairs = gridDim.x / CTAS;
     const int itemBegin = (int)((long long)a.Items * pair / pairs), itemEnd = (int)((long long)a.Items * (pair + 1) / pairs);
+    const int refilled = (itemEnd - itemBegin) * a.Chunks - a.Stages; // chunks whose stage is used again: only those are reported free
     auto rowOf = [&](int item) { return (item / a.ColTiles * CTAS + rank) * PROJ_M; };
     if (warp == PROJ_LOAD_WARP) {
         if (lane == 0) {
@@ -284,14 +337,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
                     }
                 }
             }
-            // the commits that free the last stages: none may be on its way to a CTA that has left
-            for (int k = 0; k < min(requested, a.Stages) && !failed; ++k) {
-                if (!WaitBarA(&misc.Empty[k], k < s ? phase : phase ^ 1, abortFlag, a.WaitCycles)) {
-                    failed = true;
-                    fail(kDevTimeoutMma);
-                }
-            }
-            store(&misc.Requested[rank], requested, 0);
+            ProjStore<PAIR>(&misc.Requested[rank], requested, 0);
         }
         __syncwarp();
     } else if (warp == PROJ_MMA_WARP) {
@@ -346,7 +392,9 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
                                 MmaCommit(bar);
                             }
                         };
-                        commit(&misc.Empty[s]);
+                        if (issued < refilled) { // nobody waits for a later arrival, and it could reach a CTA that has left
+                            commit(&misc.Empty[s]);
+                        }
                         if (c == a.Chunks - 1) {
                             commit(&misc.AccFull[n & 1]);
                         }
@@ -360,7 +408,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
                 }
             }
             if (lane < CTAS) {
-                store(&misc.Issued, issued, lane);
+                ProjStore<PAIR>(&misc.Issued, issued, lane);
             }
         }
         __syncwarp();
@@ -522,34 +570,8 @@ __global__ void __launch_bounds__(PROJ_THREADS, 1) ProjNormRopeKernel(const __gr
     if constexpr (PAIR) {
         PairSync(); // neither CTA leaves while the other may still arrive on its barriers
     }
-    if (*(volatile int *)&misc.Abort) {
-        // A wait ran out, which both CTAs see here.  What was started and nobody has waited for must not reach a CTA that has left: the
-        // products issued, and copies of either CTA, all counted in the first one, that no product has waited for.
-        if (tid == PROJ_LOAD_WARP * 32) {
-            const int issued = misc.Issued, tiles = issued / a.Chunks;
-            for (int k = max(0, issued - a.Stages); k < issued; ++k) {
-                WaitBar(&misc.Empty[k % a.Stages], (k / a.Stages) & 1, a.WaitCycles);
-            }
-            for (int n = max(0, tiles - 2); n < tiles; ++n) {
-                WaitBar(&misc.AccFull[n & 1], (n >> 1) & 1, a.WaitCycles);
-            }
-            if (rank == 0) {
-                const int mine = misc.Requested[0], others = misc.Requested[CTAS - 1];
-                for (int k = issued; k < max(mine, others); ++k) {
-                    uint64_t *bar = &misc.Full[k % a.Stages];
-                    if (k >= mine) {
-                        MbarExpectTx(bar, STAGE_BYTES); // the second CTA alone requested it
-                    } else if (k >= others) {
-                        MbarCompleteTx(bar, STAGE_BYTES); // the first CTA alone
-                    }
-                    WaitBar(bar, (k / a.Stages) & 1, a.WaitCycles);
-                }
-            }
-        }
-        __syncthreads();
-        if constexpr (PAIR) {
-            PairSync();
-        }
+    if (*(volatile int *)&misc.Abort) { // which both CTAs see alike here
+        ProjDrain<PAIR>(misc, a.Stages, a.Chunks, a.WaitCycles, rank, refilled);
     }
     if (warp == PROJ_MMA_WARP) {
         if constexpr (PAIR) {
@@ -590,13 +612,22 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     if (dst.ysize == 0) {
         return TSA_OK;
     }
-    const bool pair = dim >= ProjPairFrom(srcDtype == TSA_E4M3, dstDtype == TSA_F16 || dstDtype == TSA_BF16);
+    int dev = 0, sms = 0;
+    int rc = CheckCuda(cudaGetDevice(&dev), "cudaGetDevice");
+    if (rc == TSA_OK) {
+        rc = CheckCuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+    }
+    if (rc != TSA_OK) {
+        return rc;
+    }
+    const int colTiles = (outCols + PROJ_N - 1) / PROJ_N;
+    const bool pair = ProjInPairs(dim, srcDtype == TSA_E4M3, dstDtype == TSA_F16 || dstDtype == TSA_BF16, (long long)((dst.ysize + PROJ_M - 1) / PROJ_M) * colTiles, sms);
     const int ctas = pair ? 2 : 1, kb = pair ? TProjShape<true>::KB : TProjShape<false>::KB;
     const int stageBytes = pair ? TProjShape<true>::STAGE_BYTES : TProjShape<false>::STAGE_BYTES;
     CUtensorMap mx, mw;
     tsa_ptr2d xv = x;
     xv.ysize = len; // rows past len read as zeros
-    int rc = len > 0 ? MakeTileMapEx(&mx, xv, 1, kb, PROJ_M, "x") : MakeTileMapEx(&mx, x, 1, kb, PROJ_M, "x");
+    rc = len > 0 ? MakeTileMapEx(&mx, xv, 1, kb, PROJ_M, "x") : MakeTileMapEx(&mx, x, 1, kb, PROJ_M, "x");
     if (rc == TSA_OK) {
         tsa_ptr2d wv = w;
         wv.ysize = outCols;
@@ -616,22 +647,14 @@ extern "C" __attribute__((visibility("default"))) int tsa_matmul_norm_rope_quant
     a.Rows = dst.ysize;
     a.HeadCount = headCount;
     a.Chunks = (dim + kb - 1) / kb; // columns past the end read as zeros
-    a.ColTiles = (outCols + PROJ_N - 1) / PROJ_N;
-    a.Items = (dst.ysize + ctas * PROJ_M - 1) / (ctas * PROJ_M) * a.ColTiles;
+    a.ColTiles = colTiles;
+    a.Items = (dst.ysize + ctas * PROJ_M - 1) / (ctas * PROJ_M) * colTiles;
     // as many ring stages as fit beside the rope rows
     const int ropeBytes = rope.data ? PROJ_M * (headDim + 1) * (int)sizeof(float) : 0;
     a.Stages = (PROJ_SMEM_MAX - 2048 - ropeBytes) / stageBytes; // at most PROJ_MAX_STAGES
     a.WaitCycles = TestHooks().WaitCycles > 0 ? TestHooks().WaitCycles : WAIT_CYCLES;
     a.WithholdChunk = TestHooks().WithholdTile;
     const int smemBytes = a.Stages * stageBytes + 1024 /* barriers */ + 1024 /* alignment */ + ropeBytes;
-    int dev = 0, sms = 0;
-    rc = CheckCuda(cudaGetDevice(&dev), "cudaGetDevice");
-    if (rc == TSA_OK) {
-        rc = CheckCuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
-    }
-    if (rc != TSA_OK) {
-        return rc;
-    }
     const bool x8 = srcDtype == TSA_E4M3;
     const void *kern = nullptr;
 #define TSA_PROJ_CASE(DD, DT, X8)                                                                                             \
